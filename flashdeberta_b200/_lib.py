@@ -14,7 +14,7 @@ FDB_OK = 0
 FDB_BF16, FDB_FP32, FDB_E4M3 = 0, 1, 2
 FDB_DEV_TIMEOUT, FDB_DEV_BAD_SEQLEN, FDB_DEV_BAD_INDEX, FDB_DEV_BAD_MASK = 1, 2, 4, 8
 STATIC_SCRATCH_BYTES = 8 << 20
-ABI_VERSION = 4
+ABI_VERSION = 5
 PREPARED_SCHEDULE, PREPARED_TABLES = 1, 2  # fdb_attn_params.prepared
 TUNE_ONE_LAUNCH, TUNE_TWO_LAUNCHES = 1, 2  # fdb_attn_params.tune
 
@@ -49,7 +49,8 @@ EXPORTS = (
     "fdb_abi_version", "fdb_last_error", "fdb_status_string", "fdb_build_bucket_lut", "fdb_relative_index",
     "fdb_attn_workspace_bytes", "fdb_attn_fwd", "fdb_attn_fwd_static", "fdb_attn_fwd_check", "fdb_relative_index_matrix",
     "fdb_quantize_e4m3", "fdb_add_layernorm", "fdb_linear_gelu", "fdb_embed_layernorm",
-    "fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums",
+    "fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums", "fdb_expanded_rows", "fdb_expand_tables", "fdb_encoder_create",
+    "fdb_encoder_destroy", "fdb_encoder_workspace_bytes", "fdb_encoder_forward",
 )
 
 _lib = None
@@ -106,6 +107,20 @@ def load() -> C.CDLL:
     for name in ("fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums"):  # (const fdb_bwd_block*, stream); struct in backward.py
         getattr(lib, name).restype = C.c_int
         getattr(lib, name).argtypes = [C.c_void_p, C.c_void_p]
+    lib.fdb_expanded_rows.restype = C.c_int32
+    lib.fdb_expanded_rows.argtypes = [C.c_int32, C.c_int32]
+    lib.fdb_expand_tables.restype = C.c_int
+    lib.fdb_expand_tables.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int32, C.c_int32, C.c_void_p, C.c_int32,
+                                      C.c_int32, C.c_void_p]
+    # the encoder's structs are in engine.py
+    lib.fdb_encoder_create.restype = C.c_int
+    lib.fdb_encoder_create.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_void_p]
+    lib.fdb_encoder_destroy.restype = None
+    lib.fdb_encoder_destroy.argtypes = [C.c_void_p]
+    lib.fdb_encoder_workspace_bytes.restype = C.c_uint64
+    lib.fdb_encoder_workspace_bytes.argtypes = [C.c_void_p]
+    lib.fdb_encoder_forward.restype = C.c_int
+    lib.fdb_encoder_forward.argtypes = [C.c_void_p, C.c_void_p]
     if lib.fdb_abi_version() != ABI_VERSION:
         raise RuntimeError(f"libfdb_b200.so has ABI {lib.fdb_abi_version()}, this package expects {ABI_VERSION}: rebuild")
     _lib = lib

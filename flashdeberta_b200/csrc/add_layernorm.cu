@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 
 #include "internal.h"
+#include "launch.h"
+#include "sm100_ptx.cuh"
 
 namespace fdb {
 namespace {
@@ -31,29 +33,47 @@ __device__ __forceinline__ float warp_sum(float v) {
   return v;
 }
 
+// The attention mask of a token as the eager expression multiplies by it: cast to the activation type first.
+__device__ __forceinline__ float mask_value(const void* mask, int type, int64_t i) {
+  switch (type) {
+    case kMaskF32Exact: return static_cast<const float*>(mask)[i];
+    case kMaskF32: return round_bf16(static_cast<const float*>(mask)[i]);
+    case kMaskI64: return round_bf16((float)static_cast<const int64_t*>(mask)[i]);
+    case kMaskI32: return round_bf16((float)static_cast<const int32_t*>(mask)[i]);
+    case kMaskU8: return (float)static_cast<const uint8_t*>(mask)[i];
+    default: return __bfloat162float(static_cast<const __nv_bfloat16*>(mask)[i]);
+  }
+}
+
 template <int VEC>
-__global__ void __launch_bounds__(32 * kRowsPerBlock) add_layernorm_kernel(const uint4* __restrict__ x,
-                                                                          const uint4* __restrict__ residual,
-                                                                          const uint4* __restrict__ gamma,
-                                                                          const uint4* __restrict__ beta,
-                                                                          uint4* __restrict__ out, int64_t rows, float eps,
-                                                                          const int64_t* __restrict__ ids, int64_t table_rows,
-                                                                          const float* __restrict__ row_scale,
-                                                                          int32_t* __restrict__ status) {
+__global__ void __launch_bounds__(32 * kRowsPerBlock) add_layernorm_kernel(const LayerNormCall c) {
   const int lane = threadIdx.x & 31;
   const int64_t row = (int64_t)blockIdx.x * kRowsPerBlock + (threadIdx.x >> 5);
-  if (row >= rows) return;
+  ptx::grid_launch();
+  ptx::grid_wait();
   constexpr int kVecPerRow = VEC * 32;
+  const int64_t rows = c.rows_dev != nullptr ? (int64_t)*c.rows_dev : c.rows;
+  if (row >= rows) {
+    if (c.zero_tail != nullptr && row < c.rows && row < rows + kTileN) {
+      uint4* z = static_cast<uint4*>(c.zero_tail) + row * kVecPerRow;
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) z[i * 32 + lane] = make_uint4(0, 0, 0, 0);
+    }
+    return;
+  }
   int64_t src = row;
-  if (ids != nullptr) {  // embedding form: x is a table, this row is table[ids[row]]
-    src = ids[row];
-    if (src < 0 || src >= table_rows) {
-      if (lane == 0 && status != nullptr) atomicOr(reinterpret_cast<unsigned int*>(status), FDB_DEV_BAD_INDEX);
-      src = src < 0 ? 0 : table_rows - 1;
+  float scale = 1.f;
+  if (c.ids != nullptr) {  // embedding form: x is a table, this row is table[ids[token]]
+    const int64_t token = c.token_index != nullptr ? c.token_index[row] : row;
+    if (c.mask != nullptr) scale = mask_value(c.mask, c.mask_type, token);
+    src = c.ids[token];
+    if (src < 0 || src >= c.table_rows) {
+      if (lane == 0 && c.status != nullptr) atomicOr(reinterpret_cast<unsigned int*>(c.status), FDB_DEV_BAD_INDEX);
+      src = src < 0 ? 0 : c.table_rows - 1;
     }
   }
-  const uint4* xr = x + src * kVecPerRow;
-  const uint4* rr = residual != nullptr ? residual + row * kVecPerRow : nullptr;
+  const uint4* xr = static_cast<const uint4*>(c.x) + src * kVecPerRow;
+  const uint4* rr = c.residual != nullptr ? static_cast<const uint4*>(c.residual) + row * kVecPerRow : nullptr;
   float v[VEC * 8];
   float sum = 0.f;
 #pragma unroll
@@ -86,9 +106,10 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) add_layernorm_kernel(const
     const float d = v[k] - mean;
     sq = fmaf(d, d, sq);
   }
-  const float rstd = rsqrtf(warp_sum(sq) * kInv + eps);
-  uint4* orow = out + row * kVecPerRow;
-  const float scale = row_scale != nullptr ? row_scale[row] : 1.f;
+  const float rstd = rsqrtf(warp_sum(sq) * kInv + c.eps);
+  uint4* orow = static_cast<uint4*>(c.out) + (c.out_index != nullptr ? (int64_t)c.out_index[row] : row) * kVecPerRow;
+  const uint4* gamma = static_cast<const uint4*>(c.gamma);
+  const uint4* beta = static_cast<const uint4*>(c.beta);
 #pragma unroll
   for (int i = 0; i < VEC; ++i) {
     const uint4 g = __ldg(gamma + i * 32 + lane), b = __ldg(beta + i * 32 + lane);
@@ -98,7 +119,7 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) add_layernorm_kernel(const
     for (int k = 0; k < 4; ++k) {
       float lo = fmaf((v[i * 8 + 2 * k] - mean) * rstd, bf16_lo(gw[k]), bf16_lo(bw[k]));
       float hi = fmaf((v[i * 8 + 2 * k + 1] - mean) * rstd, bf16_hi(gw[k]), bf16_hi(bw[k]));
-      if (row_scale != nullptr) {  // the normalised row is rounded before it is scaled, as two separate kernels would
+      if (c.mask != nullptr) {  // the normalised row is rounded before it is scaled, as two separate kernels would
         lo = round_bf16(lo) * scale;
         hi = round_bf16(hi) * scale;
       }
@@ -109,19 +130,36 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) add_layernorm_kernel(const
 }
 
 template <int VEC>
-int launch(const void* x, const void* residual, const void* gamma, const void* beta, void* out, int64_t rows, float eps,
-           cudaStream_t s, const int64_t* ids = nullptr, int64_t table_rows = 0, const float* row_scale = nullptr,
-           int32_t* status = nullptr) {
-  const int64_t blocks = (rows + kRowsPerBlock - 1) / kRowsPerBlock;
-  add_layernorm_kernel<VEC><<<(unsigned)blocks, 32 * kRowsPerBlock, 0, s>>>(
-      static_cast<const uint4*>(x), static_cast<const uint4*>(residual), static_cast<const uint4*>(gamma),
-      static_cast<const uint4*>(beta), static_cast<uint4*>(out), rows, eps, ids, table_rows, row_scale, status);
-  const cudaError_t e = cudaGetLastError();
+int launch(const LayerNormCall& c, cudaStream_t s) {
+  const dim3 grid((unsigned)((c.rows + kRowsPerBlock - 1) / kRowsPerBlock));
+  const cudaError_t e = launch_kernel<LayerNormCall>(add_layernorm_kernel<VEC>, c, grid, 32 * kRowsPerBlock, 0, c.chained, s);
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "add_layernorm launch: %s", cudaGetErrorString(e));
   return FDB_OK;
 }
 
 }  // namespace
+
+int launch_layernorm(const LayerNormCall& c, void* stream) {
+  if (c.rows < 0 || c.rows > (int64_t(1) << 31) * kRowsPerBlock - 1) return fail(FDB_ERR_LIMIT, "rows = %lld", (long long)c.rows);
+  if (c.hidden <= 0 || c.hidden % 256 != 0 || c.hidden > 2048)
+    return fail(FDB_ERR_UNSUPPORTED, "hidden = %d: the kernel handles multiples of 256 up to 2048", c.hidden);
+  const uintptr_t all = reinterpret_cast<uintptr_t>(c.x) | reinterpret_cast<uintptr_t>(c.residual) |
+                        reinterpret_cast<uintptr_t>(c.gamma) | reinterpret_cast<uintptr_t>(c.beta) | reinterpret_cast<uintptr_t>(c.out);
+  if ((all & 15u) != 0) return fail(FDB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
+  if (c.rows == 0) return FDB_OK;
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  switch (c.hidden / 256) {
+    case 1: return launch<1>(c, s);
+    case 2: return launch<2>(c, s);
+    case 3: return launch<3>(c, s);
+    case 4: return launch<4>(c, s);
+    case 5: return launch<5>(c, s);
+    case 6: return launch<6>(c, s);
+    case 7: return launch<7>(c, s);
+    default: return launch<8>(c, s);
+  }
+}
+
 }  // namespace fdb
 
 using namespace fdb;
@@ -131,24 +169,10 @@ extern "C" FDB_API int fdb_add_layernorm(const void* x, const void* residual, co
   clear_error();
   if (x == nullptr || gamma == nullptr || beta == nullptr || out == nullptr)
     return fail(FDB_ERR_INVALID_ARGUMENT, "x, gamma, beta and out must not be NULL");
-  if (rows < 0 || rows > (int64_t(1) << 31) * kRowsPerBlock - 1) return fail(FDB_ERR_LIMIT, "rows = %lld", (long long)rows);
-  if (hidden <= 0 || hidden % 256 != 0 || hidden > 2048)
-    return fail(FDB_ERR_UNSUPPORTED, "hidden = %d: the kernel handles multiples of 256 up to 2048", hidden);
-  const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(residual) |
-                        reinterpret_cast<uintptr_t>(gamma) | reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(out);
-  if ((all & 15u) != 0) return fail(FDB_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
-  if (rows == 0) return FDB_OK;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  switch (hidden / 256) {
-    case 1: return launch<1>(x, residual, gamma, beta, out, rows, eps, s);
-    case 2: return launch<2>(x, residual, gamma, beta, out, rows, eps, s);
-    case 3: return launch<3>(x, residual, gamma, beta, out, rows, eps, s);
-    case 4: return launch<4>(x, residual, gamma, beta, out, rows, eps, s);
-    case 5: return launch<5>(x, residual, gamma, beta, out, rows, eps, s);
-    case 6: return launch<6>(x, residual, gamma, beta, out, rows, eps, s);
-    case 7: return launch<7>(x, residual, gamma, beta, out, rows, eps, s);
-    default: return launch<8>(x, residual, gamma, beta, out, rows, eps, s);
-  }
+  LayerNormCall c = {};
+  c.x = x; c.residual = residual; c.gamma = gamma; c.beta = beta; c.out = out;
+  c.rows = rows; c.hidden = hidden; c.eps = eps;
+  return launch_layernorm(c, stream);
 }
 
 extern "C" FDB_API int fdb_embed_layernorm(const int64_t* ids, const void* table, int64_t table_rows, const void* gamma,
@@ -158,22 +182,9 @@ extern "C" FDB_API int fdb_embed_layernorm(const int64_t* ids, const void* table
   if (ids == nullptr || table == nullptr || gamma == nullptr || beta == nullptr || out == nullptr)
     return fail(FDB_ERR_INVALID_ARGUMENT, "ids, table, gamma, beta and out must not be NULL");
   if (table_rows <= 0) return fail(FDB_ERR_INVALID_ARGUMENT, "table_rows = %lld", (long long)table_rows);
-  if (rows < 0 || rows > (int64_t(1) << 31) * kRowsPerBlock - 1) return fail(FDB_ERR_LIMIT, "rows = %lld", (long long)rows);
-  if (hidden <= 0 || hidden % 256 != 0 || hidden > 2048)
-    return fail(FDB_ERR_UNSUPPORTED, "hidden = %d: the kernel handles multiples of 256 up to 2048", hidden);
-  const uintptr_t all = reinterpret_cast<uintptr_t>(table) | reinterpret_cast<uintptr_t>(gamma) |
-                        reinterpret_cast<uintptr_t>(beta) | reinterpret_cast<uintptr_t>(out);
-  if ((all & 15u) != 0) return fail(FDB_ERR_ALIGNMENT, "table, gamma, beta and out must be 16-byte aligned");
-  if (rows == 0) return FDB_OK;
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  switch (hidden / 256) {
-    case 1: return launch<1>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    case 2: return launch<2>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    case 3: return launch<3>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    case 4: return launch<4>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    case 5: return launch<5>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    case 6: return launch<6>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    case 7: return launch<7>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-    default: return launch<8>(table, nullptr, gamma, beta, out, rows, eps, s, ids, table_rows, row_scale, status);
-  }
+  LayerNormCall c = {};
+  c.x = table; c.gamma = gamma; c.beta = beta; c.out = out;
+  c.rows = rows; c.hidden = hidden; c.eps = eps;
+  c.ids = ids; c.table_rows = table_rows; c.mask = row_scale; c.mask_type = kMaskF32Exact; c.status = status;
+  return launch_layernorm(c, stream);
 }

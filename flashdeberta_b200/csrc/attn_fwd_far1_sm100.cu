@@ -24,6 +24,7 @@
 
 #include "attn_fwd_common.cuh"
 #include "internal.h"
+#include "launch.h"
 #include "sm100_ptx.cuh"
 #include "tensor_map.cuh"
 
@@ -407,7 +408,8 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
 
 int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream) {
   const FwdArgs& a = *static_cast<const FwdArgs*>(fwd_args);
-  cudaError_t e = cudaFuncSetAttribute(attn_fwd_far1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  static std::atomic<uint64_t> smem_done{0};
+  cudaError_t e = allow_smem(smem_done, reinterpret_cast<const void*>(attn_fwd_far1_kernel), (int)kSmemBytes);
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   attn_fwd_far1_kernel<<<dim3((unsigned)slots, heads), kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(a);
   e = cudaGetLastError();

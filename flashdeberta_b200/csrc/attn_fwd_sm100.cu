@@ -41,6 +41,7 @@
 #include <cuda_runtime.h>
 
 #include "internal.h"
+#include "launch.h"
 #include "sm100_ptx.cuh"
 #include "tensor_map.cuh"
 #include "attn_fwd_common.cuh"
@@ -736,16 +737,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 
 }  // namespace
 
-int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const WorkspaceLayout& w, void* stream) {
+int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream) {
   const bool f8 = p.dtype == FDB_E4M3;
   FwdArgs a;
-  char* ws = static_cast<char*>(p.workspace);
   int rc;
   if ((rc = make_map_rows(&a.tm_q, p.q, p.total_rows, p.heads, p.q_row_stride, p.q_head_stride, kTileM, f8, "q"))) return rc;
   if ((rc = make_map_rows(&a.tm_k, p.k, p.total_rows, p.heads, p.k_row_stride, p.k_head_stride, kTileN, f8, "k"))) return rc;
   if ((rc = make_map_rows(&a.tm_v, p.v, p.total_rows, p.heads, p.v_row_stride, p.v_head_stride, kTileN, f8, "v"))) return rc;
-  a.xk = p.pos_key ? ws + w.exp_key : nullptr;
-  a.xq = p.pos_query ? ws + w.exp_query : nullptr;
+  a.xk = b.exp_key;
+  a.xq = b.exp_query;
   a.q_scale = p.q_scale; a.k_scale = p.k_scale; a.v_scale = p.v_scale;
   a.xk_scale = p.pos_key_scale; a.xq_scale = p.pos_query_scale;
   // a map is always encoded so the kernel argument is well formed; an unused one points at q
@@ -754,16 +754,16 @@ int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, con
   if (a.xq) { if ((rc = make_map_table(&a.tm_xq_sat, a.xq, g.rows, p.heads, f8, "saturated pos_query rows", 8))) return rc; } else a.tm_xq_sat = a.tm_q;
   a.out = static_cast<__nv_bfloat16*>(p.out);
   a.o_rs = p.out_row_stride; a.o_hs = p.out_head_stride;
-  a.seq_info = reinterpret_cast<const int32_t*>(ws + w.seq_info);
-  a.tile_first = reinterpret_cast<const int32_t*>(ws + w.tile_first);
-  a.slot_info = reinterpret_cast<const int4*>(ws + w.slot_info);
+  a.seq_info = b.seq_info;
+  a.tile_first = b.tile_first;
+  a.slot_info = reinterpret_cast<const int4*>(b.slot_info);
   a.lse = p.lse; a.status = p.status;
   a.batch = p.batch; a.heads = p.heads; a.packed = p.cu_seqlens != nullptr; a.max_seqlen = p.max_seqlen;
   a.sat_lo = g.sat_lo; a.sat_hi = g.sat_hi; a.d_first = g.d_first; a.xrows = g.rows;
   a.scale_log2 = p.sm_scale * 1.4426950408889634f;
-  a.part_o = w.split ? reinterpret_cast<float*>(ws + w.part_o) : nullptr;
-  a.part_ml = w.split ? reinterpret_cast<float*>(ws + w.part_ml) : nullptr;
-  a.band_only = w.split ? 1 : 0;
+  a.part_o = b.part_o;
+  a.part_ml = b.part_ml;
+  a.band_only = b.split ? 1 : 0;
   a.split_len = (p.tune & FDB_TUNE_TWO_LAUNCHES) ? 0 : kSplitSeqlen;  // forced two launches: every sequence is split
 #ifdef FDB_TRACE
   a.trace = trace_buffer_from_env();
@@ -777,14 +777,15 @@ int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, con
   // bf16: key tiles with saturated (or no) position terms go to the far kernel (half an SM per CTA, two CTAs per SM); with
   // position terms the band tiles follow in attn_fwd_kernel, which picks up the partial result on the same stream.
   const bool no_pos = a.xk == nullptr && a.xq == nullptr;
-  if (!f8 && (w.split || (no_pos && !(p.tune & FDB_TUNE_ONE_LAUNCH)))) {
+  if (!f8 && (b.split || (no_pos && !(p.tune & FDB_TUNE_ONE_LAUNCH)))) {
     rc = launch_attn_fwd_far1(&a, slots, p.heads, stream);
     if (rc != FDB_OK) return rc;
     if (no_pos) return FDB_OK;
   }
 
   auto kernel = f8 ? attn_fwd_kernel<true> : attn_fwd_kernel<false>;
-  cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes);
+  static std::atomic<uint64_t> smem_done[2];
+  cudaError_t e = allow_smem(smem_done[f8 ? 1 : 0], reinterpret_cast<const void*>(kernel), (int)kSmemBytes);
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
   kernel<<<dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(a);
   e = cudaGetLastError();

@@ -28,7 +28,7 @@ ExpandGeometry expand_geometry(int32_t lut_d_min, int32_t lut_len) {
 static inline uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 
 // Two launches pay off once a query tile has key tiles with saturated position terms on both sides of the band.
-static bool want_split(const fdb_attn_params& p) {
+bool want_split(const fdb_attn_params& p) {
   if (p.dtype == FDB_E4M3 || (p.pos_key == nullptr && p.pos_query == nullptr)) return false;
   if (p.tune & FDB_TUNE_ONE_LAUNCH) return false;
   if (p.tune & FDB_TUNE_TWO_LAUNCHES) return true;
@@ -191,29 +191,49 @@ __global__ void expand_tables_kernel(const uint4* __restrict__ pos_key, const ui
 
 }  // namespace
 
-int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const WorkspaceLayout& w, void* stream) {
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
+AttnBuffers attn_buffers(const fdb_attn_params& p, const WorkspaceLayout& w) {
   char* ws = static_cast<char*>(p.workspace);
-  if ((p.prepared & FDB_PREPARED_SCHEDULE) == 0)
-    seq_info_kernel<<<1, kScanThreads, 0, s>>>(p.cu_seqlens, p.seq_lens, p.batch, p.max_seqlen, p.total_rows,
-                                               reinterpret_cast<int32_t*>(ws + w.seq_info),
-                                               reinterpret_cast<int32_t*>(ws + w.tile_first),
-                                               reinterpret_cast<int4*>(ws + w.slot_info), (int)tile_slots(p), p.status);
-  cudaError_t e = cudaGetLastError();
+  AttnBuffers b;
+  b.seq_info = reinterpret_cast<int32_t*>(ws + w.seq_info);
+  b.tile_first = reinterpret_cast<int32_t*>(ws + w.tile_first);
+  b.slot_info = reinterpret_cast<int32_t*>(ws + w.slot_info);
+  b.exp_key = p.pos_key != nullptr ? ws + w.exp_key : nullptr;
+  b.exp_query = p.pos_query != nullptr ? ws + w.exp_query : nullptr;
+  b.part_o = w.split ? reinterpret_cast<float*>(ws + w.part_o) : nullptr;
+  b.part_ml = w.split ? reinterpret_cast<float*>(ws + w.part_ml) : nullptr;
+  b.split = w.split;
+  return b;
+}
+
+int launch_seq_info(const fdb_attn_params& p, const AttnBuffers& b, void* stream) {
+  seq_info_kernel<<<1, kScanThreads, 0, static_cast<cudaStream_t>(stream)>>>(
+      p.cu_seqlens, p.seq_lens, p.batch, p.max_seqlen, p.total_rows, b.seq_info, b.tile_first,
+      reinterpret_cast<int4*>(b.slot_info), (int)tile_slots(p), p.status);
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "seq_info launch: %s", cudaGetErrorString(e));
-  if ((p.pos_key != nullptr || p.pos_query != nullptr) && (p.prepared & FDB_PREPARED_TABLES) == 0) {
-    const int esz = p.dtype == FDB_E4M3 ? 1 : 2;
-    const int vec_per_row = kHeadDim * esz / 16;
-    const int table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
-    const int64_t total = (int64_t)p.heads * g.rows * vec_per_row;
-    expand_tables_kernel<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(
-        static_cast<const uint4*>(p.pos_key), static_cast<const uint4*>(p.pos_query),
-        reinterpret_cast<uint4*>(ws + w.exp_key), reinterpret_cast<uint4*>(ws + w.exp_query), p.bucket_lut,
-        p.lut_d_min, p.lut_len, g.d_first, g.rows, table_rows, p.heads, vec_per_row);
-    e = cudaGetLastError();
-    if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "expand_tables launch: %s", cudaGetErrorString(e));
-  }
   return FDB_OK;
+}
+
+int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream) {
+  const int esz = p.dtype == FDB_E4M3 ? 1 : 2;
+  const int vec_per_row = kHeadDim * esz / 16;
+  const int table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
+  const int64_t total = (int64_t)p.heads * g.rows * vec_per_row;
+  expand_tables_kernel<<<(unsigned)((total + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+      static_cast<const uint4*>(p.pos_key), static_cast<const uint4*>(p.pos_query), static_cast<uint4*>(b.exp_key),
+      static_cast<uint4*>(b.exp_query), p.bucket_lut, p.lut_d_min, p.lut_len, g.d_first, g.rows, table_rows, p.heads,
+      vec_per_row);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "expand_tables launch: %s", cudaGetErrorString(e));
+  return FDB_OK;
+}
+
+int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream) {
+  int rc = FDB_OK;
+  if ((p.prepared & FDB_PREPARED_SCHEDULE) == 0) rc = launch_seq_info(p, b, stream);
+  if (rc == FDB_OK && (p.pos_key != nullptr || p.pos_query != nullptr) && (p.prepared & FDB_PREPARED_TABLES) == 0)
+    rc = launch_expand_tables(p, g, b, stream);
+  return rc;
 }
 
 }  // namespace fdb

@@ -53,16 +53,53 @@ struct WorkspaceLayout {
   bool split;          // far key tiles and band key tiles run as two launches
   uint64_t total;
 };
+// Whether a call's longest sequences run as two launches.
+bool want_split(const fdb_attn_params& p);
 // `allow_split` false keeps every key tile in one launch (no partial-result buffers in the workspace).
 WorkspaceLayout workspace_layout(const fdb_attn_params& p, const ExpandGeometry& g, bool allow_split = true);
 // Query-tile slots of a call: dense -> every tile of the padded row range; packed -> an upper bound on the tiles of the
 // sequences (the exact number is only known on the device).
 int64_t tile_slots(const fdb_attn_params& p);
 
+// What the attention kernels read and write beside q, k, v and the output, as pointers: the sequence tables of
+// seq_info_kernel, the expanded position tables and, when the call is split, the partial results.
+struct AttnBuffers {
+  int32_t *seq_info, *tile_first, *slot_info;
+  void *exp_key, *exp_query;  // NULL without the term
+  float *part_o, *part_ml;
+  bool split;
+};
+AttnBuffers attn_buffers(const fdb_attn_params& p, const WorkspaceLayout& w);
+
+// ---- LayerNorm (add_layernorm.cu): out = LayerNorm(x + residual), or LayerNorm(x[ids[token]]) * mask[token] -----------
+// Element type of a mask: FDB_MASK_* of the public header, and fp32 taken as it is.
+enum MaskType : int { kMaskF32 = FDB_MASK_F32, kMaskI64 = FDB_MASK_I64, kMaskI32 = FDB_MASK_I32, kMaskU8 = FDB_MASK_U8,
+                      kMaskBf16 = FDB_MASK_BF16, kMaskF32Exact = 100 };
+struct LayerNormCall {
+  const void *x, *residual, *gamma, *beta;
+  void* out;
+  int64_t rows;
+  const int32_t* rows_dev;     // device: the actual number of rows (at most `rows`), or NULL
+  int hidden;
+  float eps;
+  const int64_t* ids;          // embedding form when set
+  int64_t table_rows;
+  const int32_t* token_index;  // row -> token of ids and mask; NULL: the row itself
+  const void* mask;
+  int mask_type;
+  const int32_t* out_index;    // row -> row of `out`; NULL: the row itself
+  void* zero_tail;             // rows of this (rows, hidden) buffer behind the actual number are zeroed, one key tile of them
+  int32_t* status;
+  bool chained;                // launch with programmatic stream serialisation
+};
+int launch_layernorm(const LayerNormCall& c, void* stream);
+
 // ---- launchers (defined in the .cu files) --------------------------------------------------------------------------
 int launch_attn_check(const fdb_attn_params& p, void* stream);
-int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const WorkspaceLayout& w, void* stream);
-int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const WorkspaceLayout& w, void* stream);
+int launch_seq_info(const fdb_attn_params& p, const AttnBuffers& b, void* stream);
+int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream);
+int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream);
+int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream);
 int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream);  // fwd_args: fwd::FwdArgs
 int launch_relative_index_matrix(const int16_t* lut, int32_t d_min, int32_t len, int32_t lq, int32_t lk, int32_t* out,
                                  void* stream);

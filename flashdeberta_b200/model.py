@@ -42,6 +42,7 @@ from transformers.models.deberta_v2.modeling_deberta_v2 import (
 
 from . import ops
 from .attention import FlashDisentangledSelfAttention, PackedSequences, lengths_from_mask
+from .engine import EncoderEngine
 
 __all__ = [
     "DEBERTA_SELF_ATTENTION_CLASSES", "FlashDebertaV2Attention", "FlashDebertaV2Layer", "FlashDebertaV2Encoder",
@@ -263,7 +264,25 @@ class FlashDebertaV2Model(DebertaV2Model):
         self.encoder = FlashDebertaV2Encoder(config)
         if self.encoder._fused:
             self.embeddings = FlashDebertaV2Embeddings(config)
+        self._engine = EncoderEngine()
         self.post_init()
+
+    def _engine_forward(self, input_ids, attention_mask, cu_seqlens, max_seqlen):
+        """The last hidden state through ``fdb_encoder_forward`` when the call is one it covers (inference, CUDA, no hidden
+        states of the layers asked for), else None."""
+        if (self.training or torch.is_grad_enabled() or not input_ids.is_cuda or input_ids.numel() == 0 or self.z_steps > 1
+                or torch.compiler.is_compiling() or torch.is_autocast_enabled()):
+            return None
+        if cu_seqlens is not None:
+            if max_seqlen is None or input_ids.dim() > 2 or (input_ids.dim() == 2 and input_ids.shape[0] != 1):
+                return None  # the module path says what is wrong
+            cu = cu_seqlens.to(device=input_ids.device, dtype=torch.int32).contiguous()
+            return self._engine.forward(self, input_ids.view(1, -1) if input_ids.dim() == 1 else input_ids, None, cu, int(max_seqlen))
+        if input_ids.dim() != 2 or not getattr(self.config, "pack_sequences", True):
+            return None
+        if attention_mask is not None and attention_mask.shape != input_ids.shape:
+            return None
+        return self._engine.forward(self, input_ids, attention_mask, None, input_ids.shape[1])
 
     def forward(self, input_ids: Optional[torch.Tensor] = None, attention_mask: Optional[torch.Tensor] = None,
                 token_type_ids: Optional[torch.Tensor] = None, position_ids: Optional[torch.Tensor] = None,
@@ -299,6 +318,10 @@ class FlashDebertaV2Model(DebertaV2Model):
             input_shape, device = inputs_embeds.size()[:-1], inputs_embeds.device
         else:
             raise ValueError("You have to specify either input_ids or inputs_embeds")
+        if input_ids is not None and not output_hidden_states:
+            last = self._engine_forward(input_ids, attention_mask, cu_seqlens, max_seqlen)
+            if last is not None:
+                return BaseModelOutput(last_hidden_state=last) if return_dict else (last,)
         if cu_seqlens is not None:
             return self._forward_packed_ids(input_ids, inputs_embeds, cu_seqlens, max_seqlen, output_hidden_states,
                                             return_dict)

@@ -21,7 +21,7 @@
 extern "C" {
 #endif
 
-#define FDB_ABI_VERSION 4
+#define FDB_ABI_VERSION 5
 
 #if defined(__GNUC__)
 #define FDB_API __attribute__((visibility("default")))
@@ -314,6 +314,74 @@ FDB_API int fdb_embed_layernorm(const int64_t* ids, const void* table, int64_t t
  */
 FDB_API int fdb_linear_gelu(const void* x, const void* weight, const void* bias, void* out, int64_t rows,
                             int32_t in_features, int32_t out_features, int32_t* status, void* stream);
+
+/*
+ * Rows of the position tables gathered through the bucket index, as fdb_attn_fwd does on every call that is not prepared:
+ * exp_*[h][u] = pos_*[h][idx(d_first + u)], (heads, fdb_expanded_rows(lut_d_min, lut_len), 64) bf16 each.  Either pair may be
+ * NULL.  pos_* as in fdb_attn_params.
+ */
+FDB_API int32_t fdb_expanded_rows(int32_t lut_d_min, int32_t lut_len);
+FDB_API int fdb_expand_tables(const void* pos_key, const void* pos_query, void* exp_key, void* exp_query, int32_t heads,
+                              int32_t table_rows, const int16_t* lut, int32_t lut_d_min, int32_t lut_len, void* stream);
+
+/*
+ * The whole encoder (inference, bf16) as one launch sequence: the embedding stage, then per layer the three projections of
+ * one input as one kernel, the attention, the output projection, add + LayerNorm, linear + erf GELU, the second
+ * feed-forward linear, add + LayerNorm.  The reference runs the same steps module by module (FlashDebertaV2Model.forward
+ * over FlashDebertaV2Layer, src/flashdeberta/model.py:259-310, :394-496).  Kernels are chained by programmatic dependent
+ * launch; nothing synchronises with the host, the number of valid tokens of a masked batch stays on the device.
+ *
+ * fdb_encoder_create copies the layer descriptions and encodes the weights' tensor maps; the weights themselves stay the
+ * caller's and must outlive the plan at these addresses (their contents may change).  hidden = heads * 64, hidden a
+ * multiple of 256 up to 2048, ffn a multiple of 64; every pointer 16-byte aligned; biases may be NULL.
+ */
+typedef struct fdb_encoder_layer {
+  const void *wq, *bq, *wk, *bk, *wv, *bv; /* (hidden, hidden) and (hidden) */
+  const void *wo, *bo;                     /* attention output block */
+  const void *ln1_gamma, *ln1_beta;
+  const void *wi, *bi;                     /* (ffn, hidden) */
+  const void *wd, *bd;                     /* (hidden, ffn) */
+  const void *ln2_gamma, *ln2_beta;
+  const void *exp_key, *exp_query;         /* fdb_expand_tables of the layer's projected tables, or NULL */
+  float ln1_eps, ln2_eps;
+} fdb_encoder_layer;
+
+FDB_API int fdb_encoder_create(const fdb_encoder_layer* layers, int32_t n_layers, int32_t hidden, int32_t heads, int32_t ffn,
+                               void** plan);
+FDB_API void fdb_encoder_destroy(void* plan);
+
+/* Element type of a mask: token i is valid where mask[i] != 0, and its embedding is multiplied by mask[i]. */
+#define FDB_MASK_F32 0
+#define FDB_MASK_I64 1
+#define FDB_MASK_I32 2
+#define FDB_MASK_U8 3
+#define FDB_MASK_BF16 4
+
+typedef struct fdb_encoder_call {
+  uint32_t struct_bytes; /* sizeof(fdb_encoder_call), checked */
+  int32_t mask_type;     /* FDB_MASK_* */
+  const void* plan;
+  const int64_t* ids;    /* dense: batch * max_seqlen ids; packed: total_rows ids */
+  const void* mask;      /* dense: batch * max_seqlen values, any layout of valid tokens; NULL = every token valid */
+  const int32_t* cu_seqlens; /* packed ids: device, batch+1 entries (mask must be NULL); or NULL */
+  int32_t batch, max_seqlen, total_rows;
+  int32_t position_buckets, max_relative_positions;
+  int32_t lut_d_min, lut_len;
+  const int16_t* lut;    /* bucket table as in fdb_attn_params; NULL without position terms */
+  float sm_scale;
+  float emb_eps;
+  const void *emb_table, *emb_gamma, *emb_beta; /* (emb_rows, hidden), (hidden), (hidden) bf16 */
+  int64_t emb_rows;
+  void* out;             /* total_rows rows of hidden, bf16; rows of invalid tokens are written as zeros */
+  void* workspace;       /* device, >= fdb_encoder_workspace_bytes(), 256-byte aligned */
+  uint64_t workspace_bytes;
+  int32_t* status;       /* device word, OR-ed with FDB_DEV_* bits */
+  void* const* attn_events; /* NULL, or 2 * n_layers cudaEvent_t recorded around every layer's attention */
+  int32_t launches;      /* out: kernels launched */
+} fdb_encoder_call;
+
+FDB_API uint64_t fdb_encoder_workspace_bytes(const fdb_encoder_call* c);
+FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream);
 
 #ifdef __cplusplus
 }

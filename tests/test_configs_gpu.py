@@ -510,3 +510,54 @@ def test_model_packed_ids_entry():
         assert torch.equal(got[0, at:at + n], want[b, :n]), b
         at += n
     _ops().check_status()
+
+
+# ---------------------------------------------------------------------------------------------------------------------
+# the encoder in one call (fdb_encoder_forward) against the module walk
+# ---------------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("B,L,lens,mask_dtype", [
+    (1, 1, (1,), torch.int64), (1, 29, (29,), torch.int64), (2, 129, (129, 1), torch.bool), (3, 255, (0, 255, 7), torch.float32),
+    (2, 700, (700, 513), torch.int32), (5, 2048, (2048, 1025, 64, 0, 1777), torch.bfloat16)])  # the last counts per chunk
+def test_encoder_call_matches_the_module_walk(B, L, lens, mask_dtype):
+    """Same weights, same batch through ``fdb_encoder_forward`` and (asked for the layers' hidden states, which only the
+    modules give) layer by layer: linear layers and attention are rounded alike, so only the GEMM's own order of summation
+    is left.  Rows of padding are zero; a mask with holes packs the same tokens."""
+    from flashdeberta_b200 import FlashDebertaV2Model, ops
+    torch.manual_seed(0)
+    model = FlashDebertaV2Model(_small_config("b200")).eval().to(DEV).bfloat16()
+    ids, mask = _ragged(B, L, lens)
+    holes = mask.clone()
+    holes[:, 3::5] = 0
+    for m in (mask, holes):
+        with torch.no_grad():
+            n0 = ops.launch_count()
+            got = model(input_ids=ids, attention_mask=m.to(mask_dtype)).last_hidden_state
+            assert model._engine.plan is not None and model._engine.plan.ok and ops.launch_count() - n0 >= 2 + 7 * 3
+            want = model(input_ids=ids, attention_mask=m, output_hidden_states=True).last_hidden_state
+        valid = m.bool().unsqueeze(-1)
+        assert torch.count_nonzero(got * ~valid) == 0
+        _close(got, want, 0.1, 5e-3, "one call")
+    ops.check_status()
+
+
+def test_encoder_call_notices_changes_of_the_model():
+    """A weight replaced, a module swapped, a hook, training mode: each is seen on the next call."""
+    from flashdeberta_b200 import FlashDebertaV2Model
+    torch.manual_seed(0)
+    model = FlashDebertaV2Model(_small_config("b200")).eval().to(DEV).bfloat16()
+    ids, mask = _ragged()
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    with torch.no_grad():
+        first = run()
+        dense = model.encoder.layer[1].output.dense
+        dense.weight = torch.nn.Parameter(dense.weight * 2)
+        second = run()
+        assert not torch.equal(first, second)
+        dense.weight.data = dense.weight.data / 2     # same parameter, other storage
+        assert torch.equal(run(), first)
+        seen = []
+        hook = model.encoder.layer[0].register_forward_hook(lambda *a: seen.append(1))
+        _close(run(), first, 0.1, 5e-3, "with a hook")
+        assert seen == [1]
+        hook.remove()
+        assert torch.equal(run(), first)
