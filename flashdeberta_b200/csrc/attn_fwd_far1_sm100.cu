@@ -56,8 +56,8 @@ enum Bar : uint32_t {
   kBarKFree = 5,    // 2: the score MMAs that read the stage finished
   kBarVFree = 7,    // 2: the P.V that read the stage finished
   kBarS = 9,        // S is in tensor memory
-  kBarSFree = 10,   // (count 128) the softmax threads hold the scores in registers
-  kBarP = 11,       // (count 128) P is in tensor memory
+  kBarSFree = 10,   // (count 4, a warp each) the softmax threads hold the scores in registers
+  kBarP = 11,       // (count 4, a warp each) P is in tensor memory
   kBarO = 12,       // P.V finished
   kNumBars = 13
 };
@@ -66,12 +66,14 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem - smem_u32(smem_raw));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)uniform(uint32_t(tid) >> 5), lane = tid & 31;
   const int head = blockIdx.y;
 
+  grid_launch();
+  grid_wait();
   const int4 slot = __ldg(args.slot_info + blockIdx.x);  // (sequence, first row of the tile in it, its first row, its length)
   if (slot.x < 0) return;                                  // slot past the last sequence
-  const int m0 = slot.y, seq_row0 = slot.z, len = slot.w;
+  const int m0 = (int)uniform(slot.y), seq_row0 = (int)uniform(slot.z), len = (int)uniform(slot.w);
   const int row_limit = args.packed ? len : args.max_seqlen;
   const bool has_c2p = args.xk != nullptr, has_p2c = args.xq != nullptr;
   const bool has_pos = has_c2p || has_p2c;
@@ -105,7 +107,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
 
   if (tid == 0) {
     *abort_flag = 0u;
-    for (uint32_t i = 0; i < kNumBars; ++i) mbar_init(bar(i), (i == kBarSFree || i == kBarP) ? 128u : 1u);
+    for (uint32_t i = 0; i < kNumBars; ++i) mbar_init(bar(i), (i == kBarSFree || i == kBarP) ? 4u : 1u);
     fence_barrier_init();
   }
   if (warp == kScoreWarp) {
@@ -115,17 +117,21 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBars + 8u * kNumBars);
+  const uint32_t tmem_base = uniform(*reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBars + 8u * kNumBars));
 
   bool ok = true;
+  auto wait = [&](uint32_t b, uint32_t parity) {  // whole warps wait, the result is warp-uniform
+    if (ok) ok = mbar_wait_warp(b, parity, abort_flag);
+  };
+  auto arrive = [&](uint32_t b) {  // one arrival per warp
+    __syncwarp();
+    if (elect_one()) mbar_arrive(b);
+  };
 
   if (warp >= kScoreWarp) {
     reg_dealloc<kProducerRegs>();
-    auto wait = [&](uint32_t b, uint32_t parity) {
-      if (ok && !mbar_wait_abortable(b, parity, abort_flag)) { ok = false; *abort_flag = 1u; }
-    };
     if (warp == kTmaWarp) {
-      if (lane == 0) {
+      if (elect_one()) {
         tma_prefetch_desc(&args.tm_q); tma_prefetch_desc(&args.tm_k); tma_prefetch_desc(&args.tm_v);
         mbar_expect_tx(bar(kBarQ), 16384u + (has_p2c ? 2048u : 0u));
         tma_load_3d(smem + kSmemQ, &args.tm_q, bar(kBarQ), 0, head, seq_row0 + m0);
@@ -135,37 +141,40 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
           tma_load_3d(smem + kSmemSat, &args.tm_xq_sat, bar(kBarQ), 0, args.xrows - 8, head);
           tma_load_3d(smem + kSmemSat + 1024, &args.tm_xq_sat, bar(kBarQ), 0, 0, head);
         }
+      }
 #pragma unroll 1
-        for (int i = 0; i < n_far; ++i) {
-          const int st = i & 1;
-          const uint32_t use = uint32_t(i >> 1);
-          const int row = seq_row0 + tile_of(i) * kTileN;
-          if (use > 0) wait(bar(kBarKFree + st), (use - 1u) & 1u);
-          if (!ok) break;
+      for (int i = 0; i < n_far; ++i) {
+        const int st = i & 1;
+        const uint32_t use = uint32_t(i >> 1);
+        const int row = seq_row0 + tile_of(i) * kTileN;
+        if (use > 0) wait(bar(kBarKFree + st), (use - 1u) & 1u);
+        if (!ok) break;
+        if (elect_one()) {
           mbar_expect_tx(bar(kBarK + st), 16384);
           tma_load_3d(smem + kSmemK + st * 16384, &args.tm_k, bar(kBarK + st), 0, head, row);
-          if (use > 0) wait(bar(kBarVFree + st), (use - 1u) & 1u);
-          if (!ok) break;
+        }
+        if (use > 0) wait(bar(kBarVFree + st), (use - 1u) & 1u);
+        if (!ok) break;
+        if (elect_one()) {
           mbar_expect_tx(bar(kBarV + st), 16384);
           tma_load_3d(smem + kSmemV + st * 16384, &args.tm_v, bar(kBarV + st), 0, head, row);
         }
       }
-      __syncwarp();
     } else if (warp == kScoreWarp) {
-      if (lane == 0) {
-        const uint32_t idesc_s = instr_desc(128, 128, 1, 0, 0);
-        const uint64_t dq = smem_desc_sw128(smem + kSmemQ, 1024, 16);
-        const uint64_t dk0 = smem_desc_sw128(smem + kSmemK, 1024, 16);
-        const uint64_t dsat = smem_desc_sw128(smem + kSmemSat, 0, 16);  // group stride 0: 8 identical rows serve all 128
-        wait(bar(kBarQ), 0);
+      const uint32_t idesc_s = instr_desc(128, 128, 1, 0, 0);
+      const uint64_t dq = smem_desc_sw128(smem + kSmemQ, 1024, 16);
+      const uint64_t dk0 = smem_desc_sw128(smem + kSmemK, 1024, 16);
+      const uint64_t dsat = smem_desc_sw128(smem + kSmemSat, 0, 16);  // group stride 0: 8 identical rows serve all 128
+      wait(bar(kBarQ), 0);
 #pragma unroll 1
-        for (int i = 0; i < n_far; ++i) {
-          const int st = i & 1;
-          const int kind = kind_of(tile_of(i));
-          const uint64_t dk = dk0 + uint64_t(st) * (16384u >> 4);
-          if (i > 0) wait(bar(kBarSFree), uint32_t(i - 1) & 1u);  // the softmax threads have pulled the previous scores
-          wait(bar(kBarK + st), uint32_t(i >> 1) & 1u);
-          tc_fence_after();
+      for (int i = 0; i < n_far; ++i) {
+        const int st = i & 1;
+        const int kind = kind_of(tile_of(i));
+        const uint64_t dk = dk0 + uint64_t(st) * (16384u >> 4);
+        if (i > 0) wait(bar(kBarSFree), uint32_t(i - 1) & 1u);  // the softmax threads have pulled the previous scores
+        wait(bar(kBarK + st), uint32_t(i >> 1) & 1u);
+        tc_fence_after();
+        if (elect_one()) {
           if (ok) {
 #pragma unroll
             for (int ks = 0; ks < 4; ++ks)
@@ -181,18 +190,17 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
           mma_commit(bar(kBarKFree + st));
         }
       }
-      __syncwarp();
     } else if (warp == kPvWarp) {
-      if (lane == 0) {
-        const uint32_t idesc_pv = instr_desc(128, 64, 1, 0, 1);
-        const uint64_t dv0 = smem_desc_sw128(smem + kSmemV, 1024, 16);
+      const uint32_t idesc_pv = instr_desc(128, 64, 1, 0, 1);
+      const uint64_t dv0 = smem_desc_sw128(smem + kSmemV, 1024, 16);
 #pragma unroll 1
-        for (int i = 0; i < n_far; ++i) {
-          const int st = i & 1;
-          const uint64_t dv = dv0 + uint64_t(st) * (16384u >> 4);
-          wait(bar(kBarV + st), uint32_t(i >> 1) & 1u);
-          wait(bar(kBarP), uint32_t(i) & 1u);
-          tc_fence_after();
+      for (int i = 0; i < n_far; ++i) {
+        const int st = i & 1;
+        const uint64_t dv = dv0 + uint64_t(st) * (16384u >> 4);
+        wait(bar(kBarV + st), uint32_t(i >> 1) & 1u);
+        wait(bar(kBarP), uint32_t(i) & 1u);
+        tc_fence_after();
+        if (elect_one()) {
           if (ok) {
 #pragma unroll
             for (int ks = 0; ks < 8; ++ks)
@@ -203,7 +211,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
           mma_commit(bar(kBarVFree + st));
         }
       }
-      __syncwarp();
     }
   } else {
     // =================================================== softmax ========================================================
@@ -212,12 +219,6 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
     const int r = quad * 32 + lane;
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
     const int my_row = m0 + r;
-    auto wait = [&](uint32_t b, uint32_t parity) {
-      const bool mine = ok && mbar_wait_abortable(b, parity, abort_flag);
-      const bool all = __all_sync(0xffffffffu, mine);
-      if (ok && !all) *abort_flag = 1u;
-      ok = all;
-    };
 
     wait(bar(kBarQ), 0);
     float rc_lo = 0.f, rc_hi = 0.f;
@@ -265,7 +266,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
         tmem_wait_ld();
       }
       tc_fence_before();
-      mbar_arrive(bar(kBarSFree));  // the scores are in registers: the next tile's may be computed
+      arrive(bar(kBarSFree));  // the scores are in registers: the next tile's may be computed
       float mx[4];
 #pragma unroll
       for (int q = 0; q < 4; ++q) mx[q] = max3(__uint_as_float(a0[q]), __uint_as_float(a0[4 + q]), __uint_as_float(a1[q]));
@@ -351,7 +352,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
       if (lane == 0 && quad == 0) FDB_STAMP(0, i, 4);
       tmem_wait_st();
       tc_fence_before();
-      mbar_arrive(bar(kBarP));
+      arrive(bar(kBarP));
       if (lane == 0 && quad == 0) FDB_STAMP(0, i, 5);
     }
 
@@ -406,13 +407,12 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
 
 }  // namespace
 
-int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream) {
+int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream, bool chained) {
   const FwdArgs& a = *static_cast<const FwdArgs*>(fwd_args);
   static std::atomic<uint64_t> smem_done{0};
   cudaError_t e = allow_smem(smem_done, reinterpret_cast<const void*>(attn_fwd_far1_kernel), (int)kSmemBytes);
-  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  attn_fwd_far1_kernel<<<dim3((unsigned)slots, heads), kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(a);
-  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_kernel<FwdArgs>(attn_fwd_far1_kernel, a, dim3((unsigned)slots, heads), kThreads, kSmemBytes, chained, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_fwd_far1 launch: %s", cudaGetErrorString(e));
   return FDB_OK;
 }

@@ -94,12 +94,12 @@ enum Bar : uint32_t {
   kBarWin = 9,       // 1   position windows landed (TMA)
   kBarWinFree = 10,  // 1   the MMAs that read the windows finished
   kBarS = 11,        // 1   S (and the p2c product) of a tile are in tensor memory
-  kBarSFree = 12,    // 256 both softmax groups hold their scores in registers: S and R may be overwritten
-  kBarP = 13,        // 256 P of a tile is in tensor memory
+  kBarSFree = 12,    // 8   both softmax groups hold their scores in registers: S and R may be overwritten
+  kBarP = 13,        // 8   P of a tile is in tensor memory
   kBarO = 14,        // 1   P.V of a tile finished
   kBarC2p = 15,      // 1   the c2p product of a band tile is in R
-  kBarStage = 16,    // 128 the drain group has written the c2p stage (R may be overwritten, the stage may be read)
-  kBarGather = 17,   // 256 both softmax groups are done reading the c2p stage
+  kBarStage = 16,    // 4   the drain group has written the c2p stage (R may be overwritten, the stage may be read)
+  kBarGather = 17,   // 8   both softmax groups are done reading the c2p stage
   kNumBars = 18
 };
 
@@ -109,13 +109,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem - smem_u32(smem_raw));
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, warp = (int)uniform(uint32_t(tid) >> 5), lane = tid & 31;
   const int head = blockIdx.y;
 
+  grid_launch();
+  grid_wait();
   // ---- which tile ------------------------------------------------------------------------------------------------
   const int4 slot = __ldg(args.slot_info + blockIdx.x);  // (sequence, first row of the tile in it, its first row, its length)
   if (slot.x < 0) return;                                  // slot past the last sequence
-  const int seq = slot.x, m0 = slot.y, seq_row0 = slot.z, len = slot.w;
+  const int seq = (int)uniform(slot.x), m0 = (int)uniform(slot.y), seq_row0 = (int)uniform(slot.z), len = (int)uniform(slot.w);
   // rows of this tile that may be written: packed -> the sequence's own rows; dense -> the padded row range
   const int row_limit = args.packed ? len : args.max_seqlen;
 
@@ -155,8 +157,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     *abort_flag = 0u;
     for (uint32_t i = 0; i < kNumBars; ++i) {
       uint32_t count = 1u;
-      if (i == kBarSFree || i == kBarP || i == kBarGather) count = kSoftmaxThreads;
-      if (i == kBarStage) count = kDrainThreads;
+      if (i == kBarSFree || i == kBarP || i == kBarGather) count = kSoftmaxThreads / 32;  // one arrival per warp
+      if (i == kBarStage) count = kDrainThreads / 32;
       mbar_init(bar(i), count);
     }
     fence_barrier_init();
@@ -179,9 +181,16 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBars + 8u * kNumBars);
+  const uint32_t tmem_base = uniform(*reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBars + 8u * kNumBars));
 
   bool ok = true;
+  auto wait = [&](uint32_t b, uint32_t parity) {  // whole warps wait, the result is warp-uniform
+    if (ok) ok = mbar_wait_warp(b, parity, abort_flag);
+  };
+  auto arrive = [&](uint32_t b) {  // one arrival per warp
+    __syncwarp();
+    if (elect_one()) mbar_arrive(b);
+  };
 
   if (warp >= kDrainWarp0) {
     // =================================================== drain group ====================================================
@@ -189,12 +198,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     const int quad = warp & 3;
     const int r = quad * 32 + lane;  // TMEM lane = position row inside a 128-position block
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
-    auto wait = [&](uint32_t b, uint32_t parity) {  // warp-uniform result
-      const bool mine = ok && mbar_wait_abortable(b, parity, abort_flag);
-      const bool all = __all_sync(0xffffffffu, mine);
-      if (ok && !all) *abort_flag = 1u;
-      ok = all;
-    };
     uint32_t band_idx = 0;
     for (int jj = 0; jj < n_proc; ++jj) {
       const int j = j_first + jj;
@@ -246,17 +249,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         }
       }
       tc_fence_before();
-      mbar_arrive(bar(kBarStage));
+      arrive(bar(kBarStage));
       ++band_idx;
     }
   } else if (warp >= kMmaWarp) {
     reg_dealloc<kProducerRegs>();
     if (warp == kTmaWarp) {
       // ================================================= TMA producer ===================================================
-      if (lane == 0) {
-        auto wait = [&](uint32_t b, uint32_t parity) {
-          if (ok && !mbar_wait_abortable(b, parity, abort_flag)) { ok = false; *abort_flag = 1u; }
-        };
+      if (elect_one()) {
         tma_prefetch_desc(&args.tm_q); tma_prefetch_desc(&args.tm_k); tma_prefetch_desc(&args.tm_v);
         mbar_expect_tx(bar(kBarQ), G::kTile + (has_p2c ? 16u * G::kRow : 0u));
         tma_load_3d(smem + kSmemQ, &args.tm_q, bar(kBarQ), 0, head, seq_row0 + m0);
@@ -266,178 +266,176 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           tma_load_3d(smem + kSmemSat, &args.tm_xq_sat, bar(kBarQ), 0, args.xrows - 8, head);
           tma_load_3d(smem + kSmemSat + 1024, &args.tm_xq_sat, bar(kBarQ), 0, 0, head);
         }
-        int band_idx = 0;
-        for (int jj = 0; jj < n_proc && ok; ++jj) {
-          const int j = j_first + jj;
-          const int s = jj & 1;
-          const uint32_t use = uint32_t(jj >> 1);  // how often this stage was used before
-          FDB_STAMP(3, j, 0);
-          if (jj >= 2) wait(bar(kBarKFree + s), (use - 1u) & 1u);
-          if (!ok) break;
-          FDB_STAMP(3, j, 1);
+      }
+      int band_idx = 0;
+#pragma unroll 1
+      for (int jj = 0; jj < n_proc && ok; ++jj) {
+        const int j = j_first + jj;
+        const int s = jj & 1;
+        const uint32_t use = uint32_t(jj >> 1);  // how often this stage was used before
+        FDB_STAMP(3, j, 0);
+        if (jj >= 2) wait(bar(kBarKFree + s), (use - 1u) & 1u);
+        if (!ok) break;
+        FDB_STAMP(3, j, 1);
+        if (elect_one()) {
           mbar_expect_tx(bar(kBarK + s), G::kTile);
           tma_load_3d(smem + kSmemK + s * 16384, &args.tm_k, bar(kBarK + s), 0, head, seq_row0 + j * kTileN);
-          if (tile_kind(j) == kBand) {
-            if (band_idx > 0) wait(bar(kBarWinFree), uint32_t(band_idx - 1) & 1u);
-            if (!ok) break;
-            const int u0 = m0 - j * kTileN - (kTileN - 1) - args.d_first;
+        }
+        if (tile_kind(j) == kBand) {
+          if (band_idx > 0) wait(bar(kBarWinFree), uint32_t(band_idx - 1) & 1u);
+          if (!ok) break;
+          const int u0 = m0 - j * kTileN - (kTileN - 1) - args.d_first;
+          if (elect_one()) {
             mbar_expect_tx(bar(kBarWin), (has_c2p ? G::kWin : 0u) + (has_p2c ? G::kWin : 0u));
             if (has_c2p) tma_load_3d(smem + kSmemWinK, &args.tm_xk, bar(kBarWin), 0, u0, head);
             if (has_p2c) tma_load_3d(smem + kSmemWinQ, &args.tm_xq, bar(kBarWin), 0, u0, head);
-            ++band_idx;
           }
-          if (jj >= 2) wait(bar(kBarVFree + s), (use - 1u) & 1u);
-          if (!ok) break;
-          FDB_STAMP(3, j, 2);
+          ++band_idx;
+        }
+        if (jj >= 2) wait(bar(kBarVFree + s), (use - 1u) & 1u);
+        if (!ok) break;
+        FDB_STAMP(3, j, 2);
+        if (elect_one()) {
           mbar_expect_tx(bar(kBarV + s), G::kTile);
           tma_load_3d(smem + kSmemV + s * 16384, &args.tm_v, bar(kBarV + s), 0, head, seq_row0 + j * kTileN);
         }
       }
-      __syncwarp();  // lanes 1-31 wait here for lane 0: the block-wide barrier below must be reached by whole warps
     } else if (warp == kMmaWarp) {
       // ================================================= score MMA issuer ===============================================
       // S = Q.K^T (+ saturated p2c) and the position products of band tiles.  Descriptors are built once; per MMA only the
       // start-address field moves (a 64-bit add), which keeps the single issuing thread short of instructions.
-      if (lane == 0) {
-        auto wait = [&](uint32_t b, uint32_t parity) {
-          if (ok && !mbar_wait_abortable(b, parity, abort_flag)) { ok = false; *abort_flag = 1u; }
-        };
-        const uint32_t idesc_s = instr_desc(128, 128, G::kFmt, 0, 0);
-        const uint32_t idesc_p2c = instr_desc(128, 32, G::kFmt, 0, 0);
-        const uint32_t idesc_p2c64 = instr_desc(128, 64, G::kFmt, 0, 0);
-        const uint64_t dq = G::desc(smem + kSmemQ, G::kGroup);
-        const uint64_t dk0 = G::desc(smem + kSmemK, G::kGroup);
-        const uint64_t dwk = G::desc(smem + kSmemWinK, G::kGroup);
-        const uint64_t dwq = G::desc(smem + kSmemWinQ, G::kGroup);
-        const uint64_t dsat = G::desc(smem + kSmemSat, 0);  // group stride 0: every 8-row group is the same rows
-        int band_idx = 0;
-        wait(bar(kBarQ), 0);
+      const uint32_t idesc_s = instr_desc(128, 128, G::kFmt, 0, 0);
+      const uint32_t idesc_p2c = instr_desc(128, 32, G::kFmt, 0, 0);
+      const uint32_t idesc_p2c64 = instr_desc(128, 64, G::kFmt, 0, 0);
+      const uint64_t dq = G::desc(smem + kSmemQ, G::kGroup);
+      const uint64_t dk0 = G::desc(smem + kSmemK, G::kGroup);
+      const uint64_t dwk = G::desc(smem + kSmemWinK, G::kGroup);
+      const uint64_t dwq = G::desc(smem + kSmemWinQ, G::kGroup);
+      const uint64_t dsat = G::desc(smem + kSmemSat, 0);  // group stride 0: every 8-row group is the same rows
+      int band_idx = 0;
+      wait(bar(kBarQ), 0);
 #pragma unroll 1
-        for (int jj = 0; jj < n_proc; ++jj) {
-          const int j = j_first + jj;
-          const int kind = tile_kind(j);
-          const int s = jj & 1;
-          const uint64_t dk = dk0 + uint64_t(s) * (16384u >> 4);  // stages are 16 KB apart in either build
-          // both softmax groups hold tile j-1 in registers: S and R are free
-          if (jj > 0) wait(bar(kBarSFree), uint32_t(jj - 1) & 1u);
-          wait(bar(kBarK + s), uint32_t(jj >> 1) & 1u);
-          if (kind == kBand) {
-            wait(bar(kBarWin), uint32_t(band_idx) & 1u);
-            tc_fence_after();
-            // Order of issue.  First band tile of the run: c2p (two 128-position blocks) -> R, scores -> S, and once the
-            // drain group has emptied R, the p2c products -> R.  Later tiles bring one c2p block, and it goes to the S
-            // columns (free until this tile's scores are computed), so the p2c products can be issued into R at once and
-            // run while the drain group works; only the four score MMAs wait for the drain.  The same holds for a first
-            // band tile that is the CTA's first tile at all (c2p_outside_r).
-            const bool first = band_idx == 0;
-            if (ok && has_c2p) {
-              // c2p[m][p] = Q[m].X_k[p] in 128-position blocks (later tiles reuse the lower half of the previous window
-              // from the stage)
-              const int nblk = first ? 2 : 1;
+      for (int jj = 0; jj < n_proc; ++jj) {
+        const int j = j_first + jj;
+        const int kind = tile_kind(j);
+        const int s = jj & 1;
+        const uint64_t dk = dk0 + uint64_t(s) * (16384u >> 4);  // stages are 16 KB apart in either build
+        // both softmax groups hold tile j-1 in registers: S and R are free
+        if (jj > 0) wait(bar(kBarSFree), uint32_t(jj - 1) & 1u);
+        wait(bar(kBarK + s), uint32_t(jj >> 1) & 1u);
+        if (kind == kBand) {
+          wait(bar(kBarWin), uint32_t(band_idx) & 1u);
+          tc_fence_after();
+          // Order of issue.  First band tile of the run: c2p (two 128-position blocks) -> R, scores -> S, and once the
+          // drain group has emptied R, the p2c products -> R.  Later tiles bring one c2p block, and it goes to the S
+          // columns (free until this tile's scores are computed), so the p2c products can be issued into R at once and
+          // run while the drain group works; only the four score MMAs wait for the drain.  The same holds for a first
+          // band tile that is the CTA's first tile at all (c2p_outside_r).
+          const bool first = band_idx == 0;
+          if (ok && has_c2p && elect_one()) {
+            // c2p[m][p] = Q[m].X_k[p] in 128-position blocks (later tiles reuse the lower half of the previous window
+            // from the stage)
+            const int nblk = first ? 2 : 1;
 #pragma unroll 1
-              for (int blk = 0; blk < nblk; ++blk)
+            for (int blk = 0; blk < nblk; ++blk)
 #pragma unroll
-                for (int ks = 0; ks < G::kSteps; ++ks)
-                  G::mma(tmem_base + (!first ? kColS : (c2p_outside_r ? (blk == 0 ? kColS : kColO) : kColR + blk * 128)),
-                         dq + uint64_t((ks * 32) >> 4), dwk + uint64_t((blk * G::kTile + ks * 32) >> 4), idesc_s, ks > 0);
+              for (int ks = 0; ks < G::kSteps; ++ks)
+                G::mma(tmem_base + (!first ? kColS : (c2p_outside_r ? (blk == 0 ? kColS : kColO) : kColR + blk * 128)),
+                       dq + uint64_t((ks * 32) >> 4), dwk + uint64_t((blk * G::kTile + ks * 32) >> 4), idesc_s, ks > 0);
+          }
+          if (elect_one()) mma_commit(bar(kBarC2p));
+          const bool scores_last = !first || c2p_outside_r;  // a c2p block sits in the S columns until it is drained
+          if (ok && !scores_last && elect_one()) {
+#pragma unroll
+            for (int ks = 0; ks < G::kSteps; ++ks)
+              G::mma(tmem_base + kColS, dq + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4), idesc_s, ks > 0);
+          }
+          if (!scores_last) {
+            wait(bar(kBarStage), uint32_t(band_idx) & 1u);  // the drain group has moved the c2p product out of R
+            tc_fence_after();
+          }
+          if (ok && has_p2c && elect_one()) {
+            // p2c products.  Key block b (32 keys) needs X_q rows starting at 32(3-b) (t = 0) and 32(4-b) (t = 1); blocks
+            // b and b+1 share the start row 32(3-b), so three 128x64 products cover six of the eight (b, t) pairs and
+            // two 128x32 products the rest (a narrow MMA costs the tensor pipe about as much as a 64-wide one):
+            //   start row 96: keys   0..63  -> R +   0 (b=0,t=0 | b=1,t=1)     start row 128: keys  0..31  -> R + 192 (b=0,t=1)
+            //   start row 64: keys  32..95  -> R +  64 (b=1,t=0 | b=2,t=1)     start row   0: keys 96..127 -> R + 224 (b=3,t=0)
+            //   start row 32: keys  64..127 -> R + 128 (b=2,t=0 | b=3,t=1)
+            const uint64_t blk32 = (32u * G::kRow) >> 4;  // 32 rows of an operand, in descriptor address units
+#pragma unroll 1
+            for (int q = 0; q < 3; ++q) {
+              const uint64_t da = dwq + uint64_t(3 - q) * blk32, db = dk + uint64_t(q) * blk32;
+#pragma unroll
+              for (int ks = 0; ks < G::kSteps; ++ks)
+                G::mma(tmem_base + kColR + 64 * q, da + uint64_t((ks * 32) >> 4), db + uint64_t((ks * 32) >> 4),
+                       idesc_p2c64, ks > 0);
             }
-            mma_commit(bar(kBarC2p));
-            const bool scores_last = !first || c2p_outside_r;  // a c2p block sits in the S columns until it is drained
-            if (ok && !scores_last) {
+#pragma unroll
+            for (int ks = 0; ks < G::kSteps; ++ks)
+              G::mma(tmem_base + kColR + 192, dwq + 4 * blk32 + uint64_t((ks * 32) >> 4),
+                     dk + uint64_t((ks * 32) >> 4), idesc_p2c, ks > 0);
+#pragma unroll
+            for (int ks = 0; ks < G::kSteps; ++ks)
+              G::mma(tmem_base + kColR + 224, dwq + uint64_t((ks * 32) >> 4),
+                     dk + 3 * blk32 + uint64_t((ks * 32) >> 4), idesc_p2c, ks > 0);
+          }
+          if (scores_last) {
+            wait(bar(kBarStage), uint32_t(band_idx) & 1u);  // the drain group has moved the c2p product out of S
+            tc_fence_after();
+            if (ok && elect_one()) {
 #pragma unroll
               for (int ks = 0; ks < G::kSteps; ++ks)
                 G::mma(tmem_base + kColS, dq + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4), idesc_s, ks > 0);
             }
-            if (!scores_last) {
-              wait(bar(kBarStage), uint32_t(band_idx) & 1u);  // the drain group has moved the c2p product out of R
-              tc_fence_after();
-            }
-            if (ok && has_p2c) {
-              // p2c products.  Key block b (32 keys) needs X_q rows starting at 32(3-b) (t = 0) and 32(4-b) (t = 1); blocks
-              // b and b+1 share the start row 32(3-b), so three 128x64 products cover six of the eight (b, t) pairs and
-              // two 128x32 products the rest (a narrow MMA costs the tensor pipe about as much as a 64-wide one):
-              //   start row 96: keys   0..63  -> R +   0 (b=0,t=0 | b=1,t=1)     start row 128: keys  0..31  -> R + 192 (b=0,t=1)
-              //   start row 64: keys  32..95  -> R +  64 (b=1,t=0 | b=2,t=1)     start row   0: keys 96..127 -> R + 224 (b=3,t=0)
-              //   start row 32: keys  64..127 -> R + 128 (b=2,t=0 | b=3,t=1)
-              const uint64_t blk32 = (32u * G::kRow) >> 4;  // 32 rows of an operand, in descriptor address units
-#pragma unroll 1
-              for (int q = 0; q < 3; ++q) {
-                const uint64_t da = dwq + uint64_t(3 - q) * blk32, db = dk + uint64_t(q) * blk32;
-#pragma unroll
-                for (int ks = 0; ks < G::kSteps; ++ks)
-                  G::mma(tmem_base + kColR + 64 * q, da + uint64_t((ks * 32) >> 4), db + uint64_t((ks * 32) >> 4),
-                         idesc_p2c64, ks > 0);
-              }
-#pragma unroll
-              for (int ks = 0; ks < G::kSteps; ++ks)
-                G::mma(tmem_base + kColR + 192, dwq + 4 * blk32 + uint64_t((ks * 32) >> 4),
-                       dk + uint64_t((ks * 32) >> 4), idesc_p2c, ks > 0);
-#pragma unroll
-              for (int ks = 0; ks < G::kSteps; ++ks)
-                G::mma(tmem_base + kColR + 224, dwq + uint64_t((ks * 32) >> 4),
-                       dk + 3 * blk32 + uint64_t((ks * 32) >> 4), idesc_p2c, ks > 0);
-            }
-            if (scores_last) {
-              wait(bar(kBarStage), uint32_t(band_idx) & 1u);  // the drain group has moved the c2p product out of S
-              tc_fence_after();
-              if (ok) {
-#pragma unroll
-                for (int ks = 0; ks < G::kSteps; ++ks)
-                  G::mma(tmem_base + kColS, dq + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4), idesc_s, ks > 0);
-              }
-            }
-            ++band_idx;
-          } else {
-            tc_fence_after();
           }
-          if (ok && kind != kBand) {
+          ++band_idx;
+        } else {
+          tc_fence_after();
+        }
+        if (ok && kind != kBand && elect_one()) {
+#pragma unroll
+          for (int ks = 0; ks < G::kSteps; ++ks)
+            G::mma(tmem_base + kColS, dq + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4), idesc_s, ks > 0);
+          if (has_p2c && (kind == kSatHi || kind == kSatLo)) {
+            // bf16: accumulated straight into S.  e4m3: the term has its own scale, so it goes to the (idle) product
+            // area and the softmax threads add it with the ratio of the scales.
+            const uint64_t ds = dsat + uint64_t(kind == kSatHi ? 0u : (1024u >> 4));
 #pragma unroll
             for (int ks = 0; ks < G::kSteps; ++ks)
-              G::mma(tmem_base + kColS, dq + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4), idesc_s, ks > 0);
-            if (has_p2c && (kind == kSatHi || kind == kSatLo)) {
-              // bf16: accumulated straight into S.  e4m3: the term has its own scale, so it goes to the (idle) product
-              // area and the softmax threads add it with the ratio of the scales.
-              const uint64_t ds = dsat + uint64_t(kind == kSatHi ? 0u : (1024u >> 4));
-#pragma unroll
-              for (int ks = 0; ks < G::kSteps; ++ks)
-                G::mma(tmem_base + (F8 ? kColR : kColS), ds + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4),
-                       idesc_s, (F8 ? ks > 0 : 1));
-            }
+              G::mma(tmem_base + (F8 ? kColR : kColS), ds + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4),
+                     idesc_s, (F8 ? ks > 0 : 1));
           }
+        }
+        if (elect_one()) {
           mma_commit(bar(kBarS));
           mma_commit(bar(kBarKFree + s));
           if (kind == kBand) mma_commit(bar(kBarWinFree));
-          FDB_STAMP(2, j, 0);
         }
+        FDB_STAMP(2, j, 0);
       }
-      __syncwarp();  // as above
     } else if (warp == kPvWarp) {
       // ================================================= P.V MMA issuer =================================================
-      if (lane == 0) {
-        auto wait = [&](uint32_t b, uint32_t parity) {
-          if (ok && !mbar_wait_abortable(b, parity, abort_flag)) { ok = false; *abort_flag = 1u; }
-        };
-        const uint32_t idesc_pv = instr_desc(128, 64, G::kFmt, 0, 1);
-        const uint64_t dv0 = G::desc(smem + kSmemV, G::kGroup);  // V is the MN-major operand: keys run along K
+      const uint32_t idesc_pv = instr_desc(128, 64, G::kFmt, 0, 1);
+      const uint64_t dv0 = G::desc(smem + kSmemV, G::kGroup);  // V is the MN-major operand: keys run along K
 #pragma unroll 1
-        for (int jj = 0; jj < n_proc; ++jj) {
-          const uint64_t dv = dv0 + uint64_t(jj & 1) * (16384u >> 4);
-          wait(bar(kBarV + (jj & 1)), uint32_t(jj >> 1) & 1u);
-          wait(bar(kBarP), uint32_t(jj) & 1u);  // both groups have written P
-          tc_fence_after();
-          FDB_STAMP(2, j_first + jj, 3);
-          if (ok) {
+      for (int jj = 0; jj < n_proc; ++jj) {
+        const uint64_t dv = dv0 + uint64_t(jj & 1) * (16384u >> 4);
+        wait(bar(kBarV + (jj & 1)), uint32_t(jj >> 1) & 1u);
+        wait(bar(kBarP), uint32_t(jj) & 1u);  // both groups have written P
+        tc_fence_after();
+        FDB_STAMP(2, j_first + jj, 3);
+        if (ok && elect_one()) {
 #pragma unroll
-            for (int ks = 0; ks < G::kPvSteps; ++ks)  // one step = 2048 bytes of V in either build (16 x 128 B, 32 x 64 B)
-              G::mma_ts(tmem_base + kColO, tmem_base + kColP + G::kPColsPerStep * ks, dv + uint64_t((ks * 2048) >> 4),
-                        idesc_pv, (jj > 0 || ks > 0 || resume) ? 1u : 0u);
-          }
+          for (int ks = 0; ks < G::kPvSteps; ++ks)  // one step = 2048 bytes of V in either build (16 x 128 B, 32 x 64 B)
+            G::mma_ts(tmem_base + kColO, tmem_base + kColP + G::kPColsPerStep * ks, dv + uint64_t((ks * 2048) >> 4),
+                      idesc_pv, (jj > 0 || ks > 0 || resume) ? 1u : 0u);
+        }
+        if (elect_one()) {
           mma_commit(bar(kBarO));
           mma_commit(bar(kBarVFree + (jj & 1)));
-          FDB_STAMP(2, j_first + jj, 5);
         }
+        FDB_STAMP(2, j_first + jj, 5);
       }
-      __syncwarp();  // as above
     }
   } else {
     // =================================================== softmax groups =================================================
@@ -447,12 +445,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     const int r = quad * 32 + lane;          // row of the tile
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
     const int my_row = m0 + r;
-    auto wait = [&](uint32_t b, uint32_t parity) {  // warp-uniform result
-      const bool mine = ok && mbar_wait_abortable(b, parity, abort_flag);
-      const bool all = __all_sync(0xffffffffu, mine);
-      if (ok && !all) *abort_flag = 1u;
-      ok = all;
-    };
 
     wait(bar(kBarQ), 0);
     float rc_lo = 0.f, rc_hi = 0.f;  // saturated c2p terms of this row: Q[m].X_k[first row], Q[m].X_k[last row]
@@ -560,7 +552,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         }
       }
       tc_fence_before();
-      mbar_arrive(bar(kBarSFree));
+      arrive(bar(kBarSFree));
       if (lane == 0 && quad == 0) FDB_STAMP(g, j, 2);
 
       float row_const = 0.f;
@@ -583,7 +575,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
             }
           }
         }
-        mbar_arrive(bar(kBarGather));
+        arrive(bar(kBarGather));
         ++band_idx;
       } else if (kind == kSatHi) {
         row_const = rc_hi;
@@ -686,7 +678,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         tmem_wait_st();
       }
       tc_fence_before();
-      mbar_arrive(bar(kBarP));
+      arrive(bar(kBarP));
       if (lane == 0 && quad == 0) FDB_STAMP(g, j, 7);
     }
 
@@ -737,7 +729,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 
 }  // namespace
 
-int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream) {
+int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained) {
   const bool f8 = p.dtype == FDB_E4M3;
   FwdArgs a;
   int rc;
@@ -778,7 +770,7 @@ int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, con
   // position terms the band tiles follow in attn_fwd_kernel, which picks up the partial result on the same stream.
   const bool no_pos = a.xk == nullptr && a.xq == nullptr;
   if (!f8 && (b.split || (no_pos && !(p.tune & FDB_TUNE_ONE_LAUNCH)))) {
-    rc = launch_attn_fwd_far1(&a, slots, p.heads, stream);
+    rc = launch_attn_fwd_far1(&a, slots, p.heads, stream, chained);
     if (rc != FDB_OK) return rc;
     if (no_pos) return FDB_OK;
   }
@@ -786,9 +778,8 @@ int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, con
   auto kernel = f8 ? attn_fwd_kernel<true> : attn_fwd_kernel<false>;
   static std::atomic<uint64_t> smem_done[2];
   cudaError_t e = allow_smem(smem_done[f8 ? 1 : 0], reinterpret_cast<const void*>(kernel), (int)kSmemBytes);
-  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-  kernel<<<dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, static_cast<cudaStream_t>(stream)>>>(a);
-  e = cudaGetLastError();
+  if (e == cudaSuccess)
+    e = launch_kernel<FwdArgs>(kernel, a, dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, chained, static_cast<cudaStream_t>(stream));
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_fwd launch: %s", cudaGetErrorString(e));
   return FDB_OK;
 }

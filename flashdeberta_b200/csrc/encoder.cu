@@ -357,7 +357,7 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
     b.exp_key = const_cast<void*>(lp.d.exp_key);
     b.exp_query = const_cast<void*>(lp.d.exp_query);
     if (c->attn_events != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(c->attn_events[2 * i]), s);
-    if ((rc = launch_attn_fwd_sm100(p, g, b, stream)) != FDB_OK) return rc;
+    if ((rc = launch_attn_fwd_sm100(p, g, b, stream, true)) != FDB_OK) return rc;
     if (c->attn_events != nullptr) cudaEventRecord(static_cast<cudaEvent_t>(c->attn_events[2 * i + 1]), s);
     // output block
     lin.groups = 1;

@@ -99,8 +99,8 @@ int launch_attn_check(const fdb_attn_params& p, void* stream);
 int launch_seq_info(const fdb_attn_params& p, const AttnBuffers& b, void* stream);
 int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream);
 int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream);
-int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream);
-int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream);  // fwd_args: fwd::FwdArgs
+int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained = false);
+int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream, bool chained);  // fwd_args: fwd::FwdArgs
 int launch_relative_index_matrix(const int16_t* lut, int32_t d_min, int32_t len, int32_t lq, int32_t lk, int32_t* out,
                                  void* stream);
 int launch_quantize_e4m3(const void* x, int64_t rows, int64_t row_stride, int64_t head_stride, const int32_t* slab_start,

@@ -83,23 +83,18 @@ __device__ __forceinline__ bool elect_one() {
   return p != 0;
 }
 __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __shfl_sync(0xffffffffu, v, 0); }
-// Bounded wait of a whole warp (warp-uniform result, the vote inside the loop keeps the warp converged); raises the abort flag
-// when it gives up.
-static __device__ __noinline__ bool mbar_wait_warp_slow(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+// Bounded wait of a whole warp (warp-uniform result, the vote inside the loop keeps the warp converged): gives up after about
+// two seconds of SM clock, or once another warp of the CTA has, and raises the abort flag.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
   const long long t0 = clock64();
 #pragma unroll 1
-  for (uint32_t i = 0; i < (1u << 30); ++i) {
+  for (uint32_t i = 1; i < (1u << 30); ++i) {
     if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-    if ((i & 63u) == 63u && __any_sync(0xffffffffu, *abort_flag != 0u || clock64() - t0 > 4000000000LL)) break;
+    if ((i & 63u) == 0u && __any_sync(0xffffffffu, *abort_flag != 0u || clock64() - t0 > 4000000000LL)) break;
   }
   *abort_flag = 1u;
   return false;
-}
-__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag) {
-#pragma unroll 1
-  for (int i = 0; i < 32; ++i)
-    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
-  return mbar_wait_warp_slow(bar, parity, abort_flag);
 }
 // Named barrier among `count` threads (count a multiple of 32); id 0 is __syncthreads.
 __device__ __forceinline__ void bar_sync(uint32_t id, uint32_t count) {
