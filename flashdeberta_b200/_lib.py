@@ -50,7 +50,7 @@ EXPORTS = (
     "fdb_attn_workspace_bytes", "fdb_attn_fwd", "fdb_attn_fwd_static", "fdb_attn_fwd_check", "fdb_relative_index_matrix",
     "fdb_quantize_e4m3", "fdb_add_layernorm", "fdb_linear_gelu", "fdb_embed_layernorm",
     "fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums", "fdb_expanded_rows", "fdb_expand_tables", "fdb_encoder_create",
-    "fdb_encoder_destroy", "fdb_encoder_workspace_bytes", "fdb_encoder_forward",
+    "fdb_encoder_destroy", "fdb_encoder_workspace_bytes", "fdb_encoder_forward", "fdb_attn_bwd_workspace_bytes", "fdb_attn_bwd",
 )
 
 _lib = None
@@ -107,6 +107,10 @@ def load() -> C.CDLL:
     for name in ("fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums"):  # (const fdb_bwd_block*, stream); struct in backward.py
         getattr(lib, name).restype = C.c_int
         getattr(lib, name).argtypes = [C.c_void_p, C.c_void_p]
+    lib.fdb_attn_bwd_workspace_bytes.restype = C.c_uint64
+    lib.fdb_attn_bwd_workspace_bytes.argtypes = [C.c_void_p]
+    lib.fdb_attn_bwd.restype = C.c_int
+    lib.fdb_attn_bwd.argtypes = [C.c_void_p, C.c_void_p]
     lib.fdb_expanded_rows.restype = C.c_int32
     lib.fdb_expanded_rows.argtypes = [C.c_int32, C.c_int32]
     lib.fdb_expand_tables.restype = C.c_int

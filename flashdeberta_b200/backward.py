@@ -17,18 +17,35 @@ With  s[m,n] = scale * (q_m.k_n + q_m.pk[i(m-n)] + k_n.pq[i(m-n)]),  p = exp(s -
   dQ_m = sum_n g[m,n] k_n + sum_b GC[m,b] pk_b           dK_n = sum_m g[m,n] q_m + sum_b GP[n,b] pq_b
   dpk_b = sum_m GC[m,b] q_m                              dpq_b = sum_n GP[n,b] k_n
 
-Memory: four (sequences x heads x block rows x keys) buffers at a time (two fp32, two bf16), the block sized to
+Two forms.  ``fdb_attn_bwd`` (csrc/attn_bwd_sm100.cu) is what training runs on: two tcgen05 kernels rebuild P tile by tile
+and leave dQ and dK without the row's own position term, dV, and the bucket sums GC and GP; four GEMMs finish.  The block form
+below it is kept for what that does not cover — a caller that bounds the memory itself (``block_bytes``), bucket tables
+whose index skips rows, other head sizes.
+
+Memory of the block form: four (sequences x heads x block rows x keys) buffers at a time (two fp32, two bf16), the block sized to
 ``block_bytes`` (2 GiB by default: the per-block costs — the fp32 accumulations of dK and dV, the write-back of the p2c
 sums — shrink with the number of blocks).
 """
 from __future__ import annotations
 
 import ctypes as C
-from typing import Optional, Tuple
+from typing import Dict, Optional, Tuple
 
+import numpy as np
 import torch
 
 from . import _lib, bucket
+
+class BwdParams(C.Structure):
+    """Mirror of ``fdb_attn_bwd_params`` (include/fdb_b200.h)."""
+
+    _fields_ = [
+        ("struct_bytes", C.c_uint32), ("reserved", C.c_int32), ("fwd", C.POINTER(_lib.AttnParams)),
+        ("dout", C.c_void_p), ("dout_row_stride", C.c_int64), ("dout_head_stride", C.c_int64),
+        ("dq_core", C.c_void_p), ("dk_core", C.c_void_p), ("dv", C.c_void_p), ("c2p_sums", C.c_void_p), ("p2c_sums", C.c_void_p),
+        ("workspace", C.c_void_p), ("workspace_bytes", C.c_uint64),
+    ]
+
 
 _launches = 0  # kernels of this package launched by the functions below
 
@@ -175,12 +192,70 @@ def _backward_block(q, k, v, o, do, lse, pos_key, pos_query, n_seq, seqlen, seq_
     return _rows_first(dqh, n_seq, H), _rows_first(dkh, n_seq, H), _rows_first(dvh, n_seq, H), dpk, dpq
 
 
+_steps: Dict[Tuple[int, int], bool] = {}
+
+
+def _fused_covers(q, k, v, dout, pos_key, pos_query, position_buckets, max_relative_positions) -> bool:
+    """Whether ``fdb_attn_bwd`` takes the call: bf16 on the GPU, head size 64, a bucket index that rises by at most one."""
+    if not q.is_cuda or q.shape[-1] != 64 or any(t is not None and t.dtype != torch.bfloat16 for t in (q, k, v, dout, pos_key, pos_query)):
+        return False
+    if pos_key is None and pos_query is None:
+        return True
+    key = (int(position_buckets), int(max_relative_positions))
+    if key not in _steps:
+        table, _ = bucket.host_lut(*key)
+        _steps[key] = (len(table) <= 3588 and int(np.diff(table.astype(np.int32)).max()) <= 1
+                       and bucket.att_span(*key) % 4 == 0)
+    return _steps[key]
+
+
+def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
+           max_relative_positions):
+    global _launches
+    from . import ops
+    dev, shape = q.device, q.shape
+    lib = _lib.load()
+    with torch.cuda.device(dev):
+        p, keep = ops._fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
+                                   max_relative_positions, out.contiguous(), lse.contiguous())
+        d3, d_rs, d_hs = ops._rows_view(dout)
+        T, H = d3.shape[0], d3.shape[1]
+        W = 2 * bucket.att_span(position_buckets, max_relative_positions)
+        # rows of a packed batch that belong to no sequence are not visited
+        new = torch.empty if cu_seqlens is None else torch.zeros
+        core = new(2, T, H, 64, dtype=torch.float32, device=dev)
+        dv = new(T, H, 64, dtype=torch.bfloat16, device=dev)
+        gc = torch.empty(H, T, W, dtype=torch.bfloat16, device=dev) if pos_key is not None else None
+        gp = torch.empty(H, T, W, dtype=torch.bfloat16, device=dev) if pos_query is not None else None
+        b = BwdParams()
+        b.struct_bytes, b.fwd = C.sizeof(BwdParams), C.pointer(p)
+        b.dout, b.dout_row_stride, b.dout_head_stride = d3.data_ptr(), d_rs, d_hs
+        b.dq_core, b.dk_core, b.dv = core[0].data_ptr(), core[1].data_ptr(), dv.data_ptr()
+        b.c2p_sums, b.p2c_sums = _ptr(gc), _ptr(gp)
+        need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
+        ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
+        b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
+        _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
+        _launches += 4 + int(W > 0 and (gc is not None or gp is not None))
+        del keep, ws
+    grads = []
+    for core_i, sums, table, other in ((core[0], gc, pos_key, q), (core[1], gp, pos_query, k)):
+        if sums is None:
+            grads += [core_i.to(torch.bfloat16).view(shape), None]
+            continue
+        rows = other.reshape(T, H, 64).permute(1, 0, 2)
+        d = torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev)
+        torch.add(core_i, _bmm(sums, table.view(H, W, 64)).permute(1, 0, 2), out=d)
+        grads += [d.view(shape), _bmm(sums.transpose(1, 2), rows).to(table.dtype).view(table.shape)]
+    return grads[0], grads[2], dv.view(shape), grads[1], grads[3]
+
+
 @torch.no_grad()
 def attention_backward(
     dout: torch.Tensor, q: torch.Tensor, k: torch.Tensor, v: torch.Tensor,
     pos_key: Optional[torch.Tensor], pos_query: Optional[torch.Tensor], out: torch.Tensor, lse: torch.Tensor,
     *, cu_seqlens: Optional[torch.Tensor] = None, seq_lens: Optional[torch.Tensor] = None, max_seqlen: int,
-    sm_scale: float, position_buckets: int = -1, max_relative_positions: int = -1, block_bytes: int = 1 << 31,
+    sm_scale: float, position_buckets: int = -1, max_relative_positions: int = -1, block_bytes: Optional[int] = None,
     status: Optional[torch.Tensor] = None,
 ) -> Tuple[torch.Tensor, torch.Tensor, torch.Tensor, Optional[torch.Tensor], Optional[torch.Tensor]]:
     """Gradients of ``ops.disentangled_attention`` for the bf16 path.  ``out`` and ``lse`` are what the forward returned
@@ -189,6 +264,10 @@ def attention_backward(
     and dtypes of the inputs; rows outside every sequence get zero gradients."""
     H, D = q.shape[-2], q.shape[-1]
     shape = q.shape
+    if block_bytes is None and q.numel() > 0 and _fused_covers(q, k, v, dout, pos_key, pos_query, position_buckets, max_relative_positions):
+        return _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale,
+                      position_buckets, max_relative_positions)
+    block_bytes = (1 << 31) if block_bytes is None else block_bytes
     flat = lambda t: t.reshape(-1, H, D)
     q3, k3, v3, o3, do3 = flat(q), flat(k), flat(v), flat(out), flat(dout)
     lse2 = lse.reshape(-1, H)
