@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
       wait(bar(kBarS), u & 1u);
       tc_fence_after();
       if (lane == 0 && quad == 0) FDB_STAMP(0, i, 0);
-      if (n0 + kTileN > len && ok) {
+      if (n0 + kTileN > len) {
         // ragged last tile of the sequence: overwrite the scores of keys past its end in tensor memory, 32 columns at a
         // time, so the code below is the same for every tile (a select on the 128 register-resident scores under a
         // data-dependent branch made the compiler keep two copies of them)
@@ -258,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
       }
       // pull the 128 scores of this row in four chunks, all on their way at once
       uint32_t a0[32], a1[32], a2[32], a3[32];
-      if (ok) {
+      {
         tmem_ld32(tmem_lane + kColS, a0);
         tmem_ld32(tmem_lane + kColS + 32, a1);
         tmem_ld32(tmem_lane + kColS + 64, a2);
@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
           const float alpha = ex2(m_used - m_new);
           l_run *= alpha;
           m_used = m_new;
-          if (ok) {
+          {
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
               uint32_t o[32];
@@ -339,7 +339,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
         // P is free once the previous P.V has read it.  That P.V was issued when the previous tile's exponentials ended, so
         // it is waited for here, behind the first 64 exponentials of this tile, and not in front of the tile
         if (first && u > 0) { wait(bar(kBarO), (u - 1u) & 1u); tc_fence_after(); }
-        if (ok) tmem_st32(tmem_lane + col, p);
+        tmem_st32(tmem_lane + col, p);
       };
       half(a0, a1, kColP, true);
       half(a2, a3, kColP + 32, false);

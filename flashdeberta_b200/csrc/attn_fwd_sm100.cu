@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
         uint32_t a[32];
-        if (ok) tmem_ld32(tmem_lane + kColS + 64 * g + 32 * ch, a);
+        tmem_ld32(tmem_lane + kColS + 64 * g + 32 * ch, a);
         if (kind == kBand && has_p2c) {
           // key block b = 2g + ch: columns of its two products (see the score-issuing warp)
           const int b = 2 * g + ch;
@@ -509,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 #pragma unroll
             for (int hf = 0; hf < 2; ++hf) {
               uint32_t t0[16], t1[16];
-              if (ok) {
+              {
                 tmem_ld16(tmem_lane + kColR + c0 + 16 * hf, t0);
                 tmem_ld16(tmem_lane + kColR + c1 + 16 * hf, t1);
                 tmem_wait_ld();  // the first wait also covers the 32 scores
@@ -524,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
             }
           } else {
             uint32_t t0[32], t1[32];
-            if (ok) {
+            {
               tmem_ld32(tmem_lane + kColR + c0, t0);
               tmem_ld32(tmem_lane + kColR + c1, t1);
               tmem_wait_ld();
@@ -539,14 +539,14 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         } else if (F8 && has_p2c && (kind == kSatHi || kind == kSatLo)) {
           // e4m3: the saturated p2c term of these keys sits in the product area (same value in every row)
           uint32_t t0[32];
-          if (ok) {
+          {
             tmem_ld32(tmem_lane + kColR + 64 * g + 32 * ch, t0);
             tmem_wait_ld();
           }
 #pragma unroll
           for (int c = 0; c < 32; ++c) s[32 * ch + c] = fmaf(__uint_as_float(t0[c]), ratio_p, __uint_as_float(a[c]));
         } else {
-          if (ok) tmem_wait_ld();
+          tmem_wait_ld();
 #pragma unroll
           for (int c = 0; c < 32; ++c) s[32 * ch + c] = __uint_as_float(a[c]);
         }
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           const float alpha = ex2(m_used - m_new);
           l_run *= alpha;
           m_used = m_new;
-          if (ok) {
+          {
             uint32_t o[32];
             tmem_ld32(tmem_lane + kColO + 32 * g, o);
             tmem_wait_ld();
@@ -642,7 +642,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         }
         l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
         if (lane == 0 && quad == 0) FDB_STAMP(g, j, 6);
-        if (ok) {  // 16 columns of e4m3 quadruples
+        {  // 16 columns of e4m3 quadruples
           uint32_t p[16];
 #pragma unroll
           for (int i = 0; i < 16; ++i) p[i] = pack_e4m3x4(s[4 * i], s[4 * i + 1], s[4 * i + 2], s[4 * i + 3]);
@@ -668,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
             p[i >> 1] = pack_bf16x2(e0, e1);
             p[(i >> 1) + 1] = pack_bf16x2(e2, e3);
           }
-          if (ok) tmem_st16(tmem_lane + kColP + 32 * g + 16 * h, p);
+          tmem_st16(tmem_lane + kColP + 32 * g + 16 * h, p);
         }
         float s0, s1, s2, s3;
         unpack_f32x2(l2[0], s0, s1);
