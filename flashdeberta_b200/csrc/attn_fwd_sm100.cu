@@ -494,61 +494,55 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 
       // ---- this thread's 64 scores (+ p2c through the quadrant shuffle) into registers, then S and R are released ----
       float s[64];
-#pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {
-        uint32_t a[32];
-        tmem_ld32(tmem_lane + kColS + 64 * g + 32 * ch, a);
-        if (kind == kBand && has_p2c) {
-          // key block b = 2g + ch: columns of its two products (see the score-issuing warp)
-          const int b = 2 * g + ch;
+      if (kind == kBand && has_p2c) {
+        // 16 keys at a time, the loads of the next 16 in flight while these are combined (two sets of three 16-register runs)
+        uint32_t a[2][16], t0[2][16], t1[2][16];
+        auto pull = [&](int q) {
+          // key block b = 2g + (q >> 1): columns of its two products (see the score-issuing warp)
+          const int b = 2 * g + (q >> 1);
           const uint32_t c0 = b == 3 ? 224u : 64u * uint32_t(b);
           const uint32_t c1 = b == 0 ? 192u : 64u * uint32_t(b) - 32u;
-          if constexpr (F8) {
-            // the products 16 columns at a time: the e4m3 build has more live values, and three 32-register runs at once
-            // pushed it into spilling
+          const uint32_t hf = 16u * uint32_t(q & 1);
+          tmem_ld16(tmem_lane + kColS + 64 * g + 16 * q, a[q & 1]);
+          tmem_ld16(tmem_lane + kColR + c0 + hf, t0[q & 1]);
+          tmem_ld16(tmem_lane + kColR + c1 + hf, t1[q & 1]);
+        };
+        pull(0);
 #pragma unroll
-            for (int hf = 0; hf < 2; ++hf) {
-              uint32_t t0[16], t1[16];
-              {
-                tmem_ld16(tmem_lane + kColR + c0 + 16 * hf, t0);
-                tmem_ld16(tmem_lane + kColR + c1 + 16 * hf, t1);
-                tmem_wait_ld();  // the first wait also covers the 32 scores
-              }
-#pragma unroll
-              for (int c = 0; c < 16; ++c) {
-                const int cc = 16 * hf + c;
-                const uint32_t x = (lane + cc <= 30) ? t1[c] : t0[c];
-                const uint32_t y = __shfl_sync(0xffffffffu, x, lane + 31 - cc);  // the source lane is taken modulo 32
-                s[32 * ch + cc] = fmaf(__uint_as_float(y), ratio_p, __uint_as_float(a[cc]));
-              }
-            }
-          } else {
-            uint32_t t0[32], t1[32];
-            {
-              tmem_ld32(tmem_lane + kColR + c0, t0);
-              tmem_ld32(tmem_lane + kColR + c1, t1);
-              tmem_wait_ld();
-            }
-#pragma unroll
-            for (int c = 0; c < 32; ++c) {
-              const uint32_t x = (lane + c <= 30) ? t1[c] : t0[c];
-              const uint32_t y = __shfl_sync(0xffffffffu, x, lane + 31 - c);  // the source lane is taken modulo 32
-              s[32 * ch + c] = fmaf(__uint_as_float(y), ratio_p, __uint_as_float(a[c]));
-            }
-          }
-        } else if (F8 && has_p2c && (kind == kSatHi || kind == kSatLo)) {
-          // e4m3: the saturated p2c term of these keys sits in the product area (same value in every row)
-          uint32_t t0[32];
-          {
-            tmem_ld32(tmem_lane + kColR + 64 * g + 32 * ch, t0);
-            tmem_wait_ld();
-          }
-#pragma unroll
-          for (int c = 0; c < 32; ++c) s[32 * ch + c] = fmaf(__uint_as_float(t0[c]), ratio_p, __uint_as_float(a[c]));
-        } else {
+        for (int q = 0; q < 4; ++q) {
           tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 32; ++c) s[32 * ch + c] = __uint_as_float(a[c]);
+          for (int c = 0; c < 16; ++c)  // nothing below uses them in front of the wait
+            asm volatile("" : "+r"(a[q & 1][c]), "+r"(t0[q & 1][c]), "+r"(t1[q & 1][c]));
+          if (q < 3) pull(q + 1);
+#pragma unroll
+          for (int c = 0; c < 16; ++c) {
+            const int cc = 16 * (q & 1) + c;
+            const uint32_t x = (lane + cc <= 30) ? t1[q & 1][c] : t0[q & 1][c];
+            const uint32_t y = __shfl_sync(0xffffffffu, x, lane + 31 - cc);  // the source lane is taken modulo 32
+            s[16 * q + c] = fmaf(__uint_as_float(y), ratio_p, __uint_as_float(a[q & 1][c]));
+          }
+        }
+      } else {
+        uint32_t a0[32], a1[32];
+        tmem_ld32(tmem_lane + kColS + 64 * g, a0);
+        tmem_ld32(tmem_lane + kColS + 64 * g + 32, a1);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; ++c) {
+          s[c] = __uint_as_float(a0[c]);
+          s[32 + c] = __uint_as_float(a1[c]);
+        }
+        if (F8 && has_p2c && kind != kPlain) {
+          // e4m3: the saturated p2c term of these keys sits in the product area (same value in every row)
+#pragma unroll
+          for (int ch = 0; ch < 2; ++ch) {
+            uint32_t t0[32];
+            tmem_ld32(tmem_lane + kColR + 64 * g + 32 * ch, t0);
+            tmem_wait_ld();
+#pragma unroll
+            for (int c = 0; c < 32; ++c) s[32 * ch + c] = fmaf(__uint_as_float(t0[c]), ratio_p, s[32 * ch + c]);
+          }
         }
       }
       tc_fence_before();

@@ -223,8 +223,8 @@ def disentangled_attention(
         if scales is not None or return_lse:
             raise RuntimeError("no gradient is implemented for the e4m3 path or for the LSE output; "
                                "call under torch.no_grad() or detach the inputs")
-        return attn_fwd_train_op(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, int(max_seqlen), float(sm_scale),
-                                 int(position_buckets), int(max_relative_positions))[0]
+        return attn_train(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, int(max_seqlen), float(sm_scale),
+                          int(position_buckets), int(max_relative_positions))
     out = _out_like(q, torch.bfloat16)
     rows = out.numel() // (out.shape[-1] * out.shape[-2])
     lse = torch.empty(rows, q.shape[-2], dtype=torch.float32, device=q.device) if return_lse else None
@@ -612,6 +612,37 @@ def _train_backward(ctx, grad, grad_lse):
 
 
 attn_fwd_train_op.register_autograd(_train_backward, setup_context=_train_setup)
+
+
+class _Train(torch.autograd.Function):
+    """The training call outside tracing: what ``attn_fwd_train`` does, without the custom op's dispatch (some 150 us of
+    host time per forward and backward, more than the kernels of a short batch take)."""
+
+    @staticmethod
+    def forward(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_rel):
+        return disentangled_attention(q, k, v, pos_key, pos_query, cu_seqlens=cu_seqlens, seq_lens=seq_lens,
+                                      max_seqlen=max_seqlen, sm_scale=sm_scale, position_buckets=position_buckets,
+                                      max_relative_positions=max_rel, return_lse=True)
+
+    setup_context = staticmethod(_train_setup)
+
+    @staticmethod
+    @torch.autograd.function.once_differentiable
+    def backward(ctx, grad, grad_lse):
+        from . import backward
+        q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, out, lse = ctx.saved_tensors
+        max_seqlen, sm_scale, position_buckets, max_rel = ctx.fdb_args
+        grads = backward.attention_backward(
+            grad.contiguous(), q, k, v, pos_key, pos_query, out, lse, cu_seqlens=cu_seqlens, seq_lens=seq_lens,
+            max_seqlen=max_seqlen, sm_scale=sm_scale, position_buckets=position_buckets, max_relative_positions=max_rel,
+            status=_status_word(q.device))
+        return (*grads, None, None, None, None, None, None)
+
+
+def attn_train(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_rel):
+    """Output of the attention with autograd recorded: one opaque node under tracing, a plain autograd function otherwise."""
+    call = attn_fwd_train_op if torch.compiler.is_compiling() else _Train.apply
+    return call(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_rel)[0]
 
 
 def wants_grad(*tensors) -> bool:
