@@ -9,24 +9,29 @@
 // exchanged, so one template serves both: "row term" is the position term of the row's own operand (c2p of a query row, p2c
 // of a key row), "column term" the other one.
 //
-// One CTA = 128 rows of one (sequence, head), columns in tiles of 64, two CTAs per SM (256 tensor-memory columns, 107 KB of
+// One CTA = 128 rows of one (sequence, head), columns in tiles of 64, two CTAs per SM (256 tensor-memory columns, 111 KB of
 // shared memory, 32768 registers each): what is serial inside a tile runs beside the other CTA.
-//   warps 0-3  thread r owns row r         warp 4  issues every tcgen05.mma         warp 5  issues every TMA load
+//   warps 0-7    thread r of a half owns row r and 32 of the 64 columns     warps 8-11  run sums of the rows (position gradients)
+//   warp 12      issues every tcgen05.mma                                   warp 13     issues every TMA load
 // Tensor memory: R0 64 | R1 64 | accumulators 64 + 64.  Everything passes through R0 and R1:
 //   row term     the products row . X[window]^T of the tile's 192 window positions, 64 at a time.  Row r needs the 64 positions
-//                r .. r+63: the thread writes them to a shared-memory row of its own as they come and reads them back in the
-//                order of the columns;
+//                r .. r+63, so a thread needs 32 consecutive ones that start at its lane: it shifts 64 registers down by its lane;
 //   column term  the products X[window] . column^T arranged so that the value a thread needs lies in its own 32-lane quarter:
 //                one select and one warp shuffle per element (as in the forward kernel);
-//   S, dP        then P and G go back to R0 as bf16 pairs, the A operand of the accumulating products.
+//   S, dP        then P and G go back over S as bf16 pairs, the A operand of the accumulating products.
 // Tiles whose distances are all saturated have one value per row (a dot product) and one per column (accumulated into S from
 // eight identical rows of the table).
 //
 // Position gradients: along a row the distance falls by one per column and the table row never rises, so the elements that
-// share a table row are one run.  Each thread carries the running sum of its row's run, writes it to a staging row when the
-// table row changes, and the warp copies the staged sums to global memory: (heads, rows, table rows) in bf16, every entry
-// written once, no atomics.  What is left are GEMMs with the sums: dQ += sums . pos_key, dpos_key = sums^T . Q, and the same
-// for the keys.
+// share a table row are one run.  Warps 8-11 carry the running sum of each row's run, park it in shared memory when the table
+// row changes, and write finished groups of eight to global memory: (heads, rows, table rows) in bf16, every entry written
+// once, no atomics.  What is left are GEMMs with the sums: dQ += sums . pos_key, dpos_key = sums^T . Q, and the same for the keys.
+//
+// What bounds it: the chain row term -> column term -> S -> P -> G inside a tile, about 10.5 thousand clocks of which the
+// row-term shift takes 2.4 and the wait for its products 2.2 or more; the run sums (5) lie beside it.  4 x 2048 rows x 12 heads,
+// both terms, us per kernel (<false> / <true>): one warpgroup for the whole tile, row term through shared memory 1345 / 1494; two
+// column halves and run sums of their own warps 570 / 628; the register shift and a second window buffer 558 / 592; run sums from
+// registers, sixteen columns at a time 451 / 468.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -54,12 +59,11 @@ constexpr int kMaxRows = 4096;  // rows of an expanded table (one bit each in sh
 
 constexpr uint32_t kSmemRow = 0;                        // two operands of 128 x 128 B
 constexpr uint32_t kSmemCol = 32768;                    // two operands of 64 x 128 B
-constexpr uint32_t kSmemWin = 49152;                    // 192 x 128 B
-constexpr uint32_t kSmemSat = kSmemWin + kWin * 128;    // 2 x (8 x 128 B) saturated rows of the column table (hi, lo)
-// one row of 32 fp32 values per thread (row r, column half h): the value of its position 32 B + c lies in word 34 r + (c - r) mod 32
-constexpr uint32_t kStagePitch = 34 * 4, kStageHalf = 128 * kStagePitch;
-constexpr uint32_t kSmemStage = kSmemSat + 2048;
-constexpr uint32_t kSmemCols = kSmemStage + 2 * kStageHalf;  // float [2][2][64]: LSE and delta of the columns (<true>)
+constexpr uint32_t kSmemWin = 49152;                    // 192 x 128 B window of the row table, the same of the column table
+constexpr uint32_t kSmemSat = kSmemWin + 2 * kWin * 128;  // 2 x (8 x 128 B) saturated rows of the column table (hi, lo)
+constexpr uint32_t kEmitPitch = 80;                     // per row: finished run sums (bf16), three groups of eight, and padding
+constexpr uint32_t kSmemEmit = kSmemSat + 2048;
+constexpr uint32_t kSmemCols = kSmemEmit + 128 * kEmitPitch;  // float [2][2][64]: LSE and delta of the columns (<true>)
 constexpr uint32_t kSmemBits = kSmemCols + 1024;        // one bit per expanded row: its table row differs from the row before
 constexpr uint32_t kSmemBars = kSmemBits + kMaxRows / 8;
 constexpr uint32_t kSmemBytes = kSmemBars + 128 + 1024;
@@ -69,13 +73,13 @@ enum Bar : uint32_t {
   kBarRow = 0,    // 1  row operands landed
   kBarCol = 1,    // 1  column operands landed
   kBarAcc = 2,    // 1  the accumulating products of a tile finished (the column operands are free)
-  kBarWin = 3,    // 1  window landed
-  kBarWinFree = 4,// 1  the products that read it finished
-  kBarU = 5,      // 1  R0 / R1 filled
-  kBarUFree = 7,  // 8  R0 / R1 read by both halves
-  kBarG = 9,      // 8  P and G are in R0
-  kBarGRead = 10, // 4  the run sums have read G
-  kNumBars = 11
+  kBarWin = 3,    // 1  window of the row / column table landed
+  kBarWinFree = 5,// 1  the products that read it finished
+  kBarU = 7,      // 1  R0 / R1 filled
+  kBarUFree = 9,  // 8  R0 / R1 read by both halves
+  kBarG = 11,     // 8  P and G are in R0
+  kBarGRead = 12, // 4  the run sums have read G
+  kNumBars = 13
 };
 
 struct alignas(64) BwdArgs {
@@ -191,35 +195,36 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
           tma_load_3d(smem + kSmemSat + 1024, &args.tm_xcol_sat, bar(kBarRow), 0, 0, head);
         }
       }
-      uint32_t win = 0;  // windows loaded so far
-      auto load_window = [&](const CUtensorMap* map, int j) {
-        if (win > 0) wait(bar(kBarWinFree), (win - 1u) & 1u);
+      uint32_t n_band = 0;  // band tiles so far
+      auto load_window = [&](uint32_t w, const CUtensorMap* map, int j) {
+        if (n_band > 0) wait(bar(kBarWinFree + w), (n_band - 1u) & 1u);
         if (ok && elect_one()) {
-          mbar_expect_tx(bar(kBarWin), uint32_t(kWin) * 128u);
-          tma_load_3d(smem + kSmemWin, map, bar(kBarWin), 0, r0 - j * kCols - (kCols - 1) - args.d_first, head);
+          mbar_expect_tx(bar(kBarWin + w), uint32_t(kWin) * 128u);
+          tma_load_3d(smem + kSmemWin + w * uint32_t(kWin * 128), map, bar(kBarWin + w), 0, r0 - j * kCols - (kCols - 1) - args.d_first, head);
         }
-        ++win;
       };
 #pragma unroll 1
       for (int j = 0; j < n_tiles && ok; ++j) {
-        const bool band = kind_of(j) == kBand;
-        if (band && row_term) load_window(&args.tm_xrow, j);
+        if (kind_of(j) == kBand) {
+          if (row_term) load_window(0, &args.tm_xrow, j);
+          if (col_term) load_window(1, &args.tm_xcol, j);
+          ++n_band;
+        }
         if (j > 0) wait(bar(kBarAcc), uint32_t(j - 1) & 1u);
         if (ok && elect_one()) {
           mbar_expect_tx(bar(kBarCol), 16384u);
           tma_load_3d(smem + kSmemCol, &args.tm_col[0], bar(kBarCol), 0, head, seq_row0 + j * kCols);
           tma_load_3d(smem + kSmemCol + 8192, &args.tm_col[1], bar(kBarCol), 0, head, seq_row0 + j * kCols);
         }
-        if (band && col_term) load_window(&args.tm_xcol, j);
       }
     } else if (warp == kMmaWarp) {
       // ================================================= MMA issuer =====================================================
       const uint32_t idesc_64 = instr_desc(128, 64, 1, 0, 0), idesc_32 = instr_desc(128, 32, 1, 0, 0);
       const uint32_t idesc_acc = instr_desc(128, 64, 1, 0, 1);
       const uint64_t drow = smem_desc_sw128(smem + kSmemRow, 1024, 16), dcol = smem_desc_sw128(smem + kSmemCol, 1024, 16);
-      const uint64_t dwin = smem_desc_sw128(smem + kSmemWin, 1024, 16), dsat = smem_desc_sw128(smem + kSmemSat, 0, 16);
+      const uint64_t dwin_r = smem_desc_sw128(smem + kSmemWin, 1024, 16), dwin_c = smem_desc_sw128(smem + kSmemWin + kWin * 128, 1024, 16), dsat = smem_desc_sw128(smem + kSmemSat, 0, 16);
       constexpr uint64_t blk32 = (32u * 128u) >> 4;
-      uint32_t win = 0, used[2] = {0, 0};
+      uint32_t n_band = 0, used[2] = {0, 0};
       auto next_use = [&](uint32_t i) {  // R_i may be written again
         if (used[i] > 0) wait(bar(kBarUFree + i), (used[i] - 1u) & 1u);
         ++used[i];
@@ -238,13 +243,12 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
           if (row_term) wait(bar(kBarGRead), uint32_t(j - 1) & 1u);
         }
         if (kind == kBand && row_term) {
-          wait(bar(kBarWin), win & 1u);
-          ++win;
+          wait(bar(kBarWin), n_band & 1u);
 #pragma unroll
           for (uint32_t k = 0; k < 3; ++k) {
             next_use(k & 1u);
             if (ok && elect_one()) {
-              product(tmem_base + kColR + 64u * (k & 1u), drow, dwin + uint64_t(k) * 2u * blk32, idesc_64, 0);
+              product(tmem_base + kColR + 64u * (k & 1u), drow, dwin_r + uint64_t(k) * 2u * blk32, idesc_64, 0);
               mma_commit(bar(kBarU + (k & 1u)));
               if (k == 2) mma_commit(bar(kBarWinFree));
             }
@@ -254,20 +258,20 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
         if (kind == kBand && col_term) {
           // 32-column block b needs the window rows starting at 32(1-b) (t = 0) and 32(2-b) (t = 1); unit u has start row
           // 64 - 32u: block u-1 (t = 0) in its first 32 columns, block u (t = 1) in the last 32
-          wait(bar(kBarWin), win & 1u);
-          ++win;
+          wait(bar(kBarWin + 1), n_band & 1u);
 #pragma unroll
           for (uint32_t u = 0; u < 3; ++u) {
             const uint32_t i = (u & 1u) ^ 1u;
             next_use(i);
             if (ok && elect_one()) {
-              product(tmem_base + kColR + 64u * i + (u == 0 ? 32u : 0u), dwin + uint64_t(2u - u) * blk32,
+              product(tmem_base + kColR + 64u * i + (u == 0 ? 32u : 0u), dwin_c + uint64_t(2u - u) * blk32,
                       dcol + uint64_t(u == 2 ? 1u : 0u) * blk32, u == 1 ? idesc_64 : idesc_32, 0);
               mma_commit(bar(kBarU + i));
-              if (u == 2) mma_commit(bar(kBarWinFree));
+              if (u == 2) mma_commit(bar(kBarWinFree + 1));
             }
           }
         }
+        n_band += kind == kBand ? 1u : 0u;
         next_use(0);
         if (ok && elect_one()) {
           product(tmem_base + kColR, drow, dcol, idesc_64, 0);
@@ -305,46 +309,29 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
     if (row_term) {
       float run = 0.f;                            // sum of the current run
       int b = table_row<DKV>(args, my_row);       // and its table row: falls by one per run (<true>: rises)
-      uint32_t pack[4] = {0u, 0u, 0u, 0u};        // the finished sums of the current group of eight table rows, moved along by 16 bits each
-      __nv_bfloat16* sums = args.sums + ((int64_t)head * args.total_rows + seq_row0 + (valid_row ? my_row : len - 1)) * args.table_rows;
+      // Finished sums wait in a row of three aligned groups of eight table rows: the current group lies in the last one (<true>:
+      // the first), the next ones go towards the other end.  Sixteen columns complete at most two groups.
+      const uint32_t mine = smem + kSmemEmit + uint32_t(quad * 32 + lane) * kEmitPitch;
+      constexpr uint32_t kHome = DKV ? 0u : 32u;  // byte offset of the current group
+      sts_v4(mine + kHome, 0u, 0u, 0u, 0u);
+      uint4* sums = reinterpret_cast<uint4*>(args.sums + ((int64_t)head * args.total_rows + seq_row0 + (valid_row ? my_row : len - 1)) * args.table_rows);
       const uint32_t* bits = reinterpret_cast<const uint32_t*>(smem_gen + kSmemBits);
-      auto push = [&](float v) {
-        const uint32_t x = uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(v)));
-        if (DKV) {
-          pack[0] = __funnelshift_r(pack[0], pack[1], 16); pack[1] = __funnelshift_r(pack[1], pack[2], 16);
-          pack[2] = __funnelshift_r(pack[2], pack[3], 16); pack[3] = (pack[3] >> 16) | (x << 16);
-        } else {
-          pack[3] = __funnelshift_l(pack[2], pack[3], 16); pack[2] = __funnelshift_l(pack[1], pack[2], 16);
-          pack[1] = __funnelshift_l(pack[0], pack[1], 16); pack[0] = (pack[0] << 16) | x;
-        }
-      };
-      auto finish = [&]() {  // the run of table row b is complete
-        push(run);
-        if ((b & 7) == (DKV ? 7 : 0)) *reinterpret_cast<uint4*>(sums + (b & ~7)) = make_uint4(pack[0], pack[1], pack[2], pack[3]);
-        b += DKV ? 1 : -1;
-        run = 0.f;
-      };
 #pragma unroll 1
       for (int j = 0; j < n_tiles; ++j) {
         wait(bar(kBarG), uint32_t(j) & 1u);
         tc_fence_after();
-        uint32_t lo[16], hi[16];
-        {
-          tmem_ld16(tmem_lane + kColR + 16u, lo);
-          tmem_ld16(tmem_lane + kColR + 48u, hi);
-          tmem_wait_ld();
-        }
-        uint32_t g[32];
-#pragma unroll
-        for (int i = 0; i < 16; ++i) { g[i] = lo[i]; g[16 + i] = hi[i]; }
+        uint32_t g[2][16];
+        tmem_ld16(tmem_lane + kColR + 16u, g[0]);
+        tmem_ld16(tmem_lane + kColR + 48u, g[1]);
+        tmem_wait_ld();
         tc_fence_before();
         arrive(bar(kBarGRead));
         if (kind_of(j) != kBand) {
           float a[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            a[i & 1] += __uint_as_float(g[i] << 16);
-            a[2 + (i & 1)] += __uint_as_float(g[i] & 0xffff0000u);
+            a[i & 1] += __uint_as_float(g[i >> 4][i & 15] << 16);
+            a[2 + (i & 1)] += __uint_as_float(g[i >> 4][i & 15] & 0xffff0000u);
           }
           run += (a[0] + a[1]) + (a[2] + a[3]);
           continue;
@@ -363,18 +350,41 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
         }
         if (!valid_row) ends[0] = ends[1] = 0u;
 #pragma unroll
-        for (int n = 0; n < 64; ++n) {
-          run += __uint_as_float((n & 1) ? (g[n >> 1] & 0xffff0000u) : (g[n >> 1] << 16));
-          if (ends[n >> 5] >> (n & 31) & 1u) finish();
+        for (int q = 0; q < 4; ++q) {
+          const int group = b >> 3;
+          uint32_t at = mine + kHome + 2u * uint32_t(b & 7);
+#pragma unroll
+          for (int n = 0; n < 16; ++n) {
+            const uint32_t w = g[q >> 1][(8 * q + (n >> 1)) & 15];
+            run += __uint_as_float((n & 1) ? (w & 0xffff0000u) : (w << 16));
+            const uint32_t end = ends[q >> 1] & (1u << ((16 * q + n) & 31));
+            // predicated, not branched around: with 32 rows one distance apart some lane ends a run at nearly every column
+            asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %0, 0;\n\t@p st.shared.u16 [%1], %2;\n\t}" ::"r"(end), "r"(at),
+                         "h"(__bfloat16_as_ushort(__float2bfloat16_rn(run))) : "memory");
+            at = end ? (DKV ? at + 2u : at - 2u) : at;
+            b = end ? (DKV ? b + 1 : b - 1) : b;
+            run = end ? 0.f : run;
+          }
+          const int full = DKV ? (b >> 3) - group : group - (b >> 3);  // groups completed: 0, 1 or 2
+          if (__any_sync(0xffffffffu, full > 0)) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+              if (full > i) sums[DKV ? group + i : group - i] = lds_v4(mine + (DKV ? 16u * i : 32u - 16u * i));
+            if (full > 0) {  // what is left of the last group goes home
+              const uint4 v = lds_v4(mine + (DKV ? 16u * uint32_t(full) : 32u - 16u * uint32_t(full)));
+              sts_v4(mine + kHome, v.x, v.y, v.z, v.w);
+            }
+          }
         }
       }
-      if (valid_row) {
-        push(run);  // the last run, then zeros up to the end of its group
-        while ((b & 7) != (DKV ? 7 : 0)) {
-          push(0.f);
-          b += DKV ? 1 : -1;
+      if (valid_row) {  // the last run, then zeros up to the end of its group
+        uint32_t at = mine + kHome + 2u * uint32_t(b & 7);
+        sts_u16(at, uint32_t(__bfloat16_as_ushort(__float2bfloat16_rn(run))));
+        for (int i = b & 7; i != (DKV ? 7 : 0); i += DKV ? 1 : -1) {
+          at = DKV ? at + 2u : at - 2u;
+          sts_u16(at, 0u);
         }
-        *reinterpret_cast<uint4*>(sums + (b & ~7)) = make_uint4(pack[0], pack[1], pack[2], pack[3]);
+        sums[b >> 3] = lds_v4(mine + kHome);
       }
     }
   } else {
@@ -386,7 +396,6 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
     const int my_row = r0 + r;
     const bool valid_row = my_row < len;
-    const uint32_t stage = smem + kSmemStage + uint32_t(h) * kStageHalf + uint32_t(r) * kStagePitch;
     const float c_eff = args.sm_scale * 1.4426950408889634f;
     const int64_t rh = (int64_t)(seq_row0 + (valid_row ? my_row : len - 1)) * args.heads + head;
     float row_lse = 0.f, row_delta = 0.f;  // LSE in log2 units
@@ -440,33 +449,36 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
       asm volatile("" : "+r"(lane_i));
       if (kind == kBand && row_term) {
         // position p = r + 63 - column of the window, 32-position blocks, unit k = blocks 2k and 2k+1 in R0, R1, R0.  With
-        // B = quad + 1 - half the thread's positions are the entries c >= lane of block B and c < lane of block B + 1.
+        // B = quad + 1 - half the thread's 32 positions start at entry `lane` of block B: it takes blocks B and B + 1 and
+        // shifts them down by its lane, one bit of it at a time (186 selects; through a shared-memory row of its own the
+        // same took 64 predicated stores, 32 loads and twice the time).
         const int B = quad + 1 - h;
-        const uint32_t place = stage - 4u * uint32_t(lane_i);
+        wait_u(0);  // unit 0
+        if (B >= 2) free_u(0);
+        wait_u(1);  // unit 1
+        if (B >= 3) wait_u(0);  // unit 2
+        uint32_t x[64];
+        tmem_ld32(tmem_lane + kColR + uint32_t(((B >> 1) & 1) * 64 + (B & 1) * 32), reinterpret_cast<uint32_t(&)[32]>(x[0]));
+        tmem_ld32(tmem_lane + kColR + uint32_t((((B + 1) >> 1) & 1) * 64 + ((B + 1) & 1) * 32), reinterpret_cast<uint32_t(&)[32]>(x[32]));
+        tmem_wait_ld();
+        if (B < 2) free_u(0);
+        free_u(1);
+        if (B < 3) wait_u(0);  // unit 2 holds nothing for this warp
+        free_u(0);
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          wait_u(k & 1u);
+        for (int i = 0; i < 47; ++i) x[i] = (lane_i & 16) ? x[i + 16] : x[i];
 #pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int blk = 2 * k + i;
-            if (blk == B || blk == B + 1) {
-              const bool upper = blk == B;
-              const uint32_t at = place + (upper ? 0u : 128u);
+        for (int i = 0; i < 39; ++i) x[i] = (lane_i & 8) ? x[i + 8] : x[i];
 #pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                uint32_t t[16];
-                {
-                  tmem_ld16(tmem_lane + kColR + 64u * (k & 1) + 32u * i + 16u * q, t);
-                  tmem_wait_ld();
-                }
+        for (int i = 0; i < 35; ++i) x[i] = (lane_i & 4) ? x[i + 4] : x[i];
 #pragma unroll
-                for (int c = 0; c < 16; ++c)
-                  if ((16 * q + c >= lane_i) == upper) sts_f32(at + 4u * uint32_t(16 * q + c), __uint_as_float(t[c]));
-              }
-            }
-          }
-          free_u(k & 1u);
-        }
+        for (int i = 0; i < 33; ++i) x[i] = (lane_i & 2) ? x[i + 2] : x[i];
+#pragma unroll
+        for (int n = 0; n < 32; ++n) s[n] = __uint_as_float((lane_i & 1) ? x[32 - n] : x[31 - n]);
+      } else {
+        const float row_const = kind == kSatHi ? rc_hi : (kind == kSatLo ? rc_lo : 0.f);
+#pragma unroll
+        for (int n = 0; n < 32; ++n) s[n] = row_const;
       }
       if (kind == kBand && col_term) {
         // this half's 32-column block: t = 1 from unit h, t = 0 from unit h + 1 (units 0, 1, 2 in R1, R0, R1)
@@ -489,7 +501,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
           for (int c = 0; c < 16; ++c) {
             const int cc = 16 * q + c;
             const uint32_t x = (lane_i + cc <= 30) ? t1[c] : t0[c];
-            s[cc] = __uint_as_float(__shfl_sync(0xffffffffu, x, lane_i + 31 - cc));  // the source lane is taken modulo 32
+            s[cc] += __uint_as_float(__shfl_sync(0xffffffffu, x, lane_i + 31 - cc));  // the source lane is taken modulo 32
           }
         }
         free_u(1);
@@ -498,14 +510,6 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
           wait_u(1);
           free_u(1);
         }
-      } else {
-        const float row_const = kind == kSatHi ? rc_hi : (kind == kSatLo ? rc_lo : 0.f);
-#pragma unroll
-        for (int n = 0; n < 32; ++n) s[n] = row_const;
-      }
-      if (kind == kBand && row_term) {
-#pragma unroll
-        for (int n = 0; n < 32; ++n) s[n] += lds_f32(stage + 4u * uint32_t(31 - n));
       }
       wait_u(0);
 #pragma unroll
