@@ -17,8 +17,9 @@ With  s[m,n] = scale * (q_m.k_n + q_m.pk[i(m-n)] + k_n.pq[i(m-n)]),  p = exp(s -
   dQ_m = sum_n g[m,n] k_n + sum_b GC[m,b] pk_b           dK_n = sum_m g[m,n] q_m + sum_b GP[n,b] pq_b
   dpk_b = sum_m GC[m,b] q_m                              dpq_b = sum_n GP[n,b] k_n
 
-Two forms.  ``fdb_attn_bwd`` (csrc/attn_bwd_sm100.cu) is what training runs on: two tcgen05 kernels rebuild P tile by tile
-and leave dQ and dK without the row's own position term, dV, and the bucket sums GC and GP; four GEMMs finish.  The block form
+Two forms.  ``fdb_attn_bwd`` is what training runs on: two tcgen05 kernels rebuild P tile by tile and leave dQ and dK without the
+row's own position term, dV, and the bucket sums GC and GP (csrc/attn_bwd_sm100.cu); a third one adds what is made of the sums
+(csrc/attn_bwd_tables_sm100.cu).  The block form
 below it is kept for what that does not cover — a caller that bounds the memory itself (``block_bytes``), bucket tables
 whose index skips rows, other head sizes.
 
@@ -42,7 +43,8 @@ class BwdParams(C.Structure):
     _fields_ = [
         ("struct_bytes", C.c_uint32), ("reserved", C.c_int32), ("fwd", C.POINTER(_lib.AttnParams)),
         ("dout", C.c_void_p), ("dout_row_stride", C.c_int64), ("dout_head_stride", C.c_int64),
-        ("dq_core", C.c_void_p), ("dk_core", C.c_void_p), ("dv", C.c_void_p), ("c2p_sums", C.c_void_p), ("p2c_sums", C.c_void_p),
+        ("dq", C.c_void_p), ("dk", C.c_void_p), ("dv", C.c_void_p), ("grad_row_stride", C.c_int64), ("grad_head_stride", C.c_int64),
+        ("dpos_key", C.c_void_p), ("dpos_query", C.c_void_p),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_uint64),
     ]
 
@@ -220,34 +222,23 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
                                    max_relative_positions, out.contiguous(), lse.contiguous())
         d3, d_rs, d_hs = ops._rows_view(dout)
         T, H = d3.shape[0], d3.shape[1]
-        W = 2 * bucket.att_span(position_buckets, max_relative_positions)
-        # rows of a packed batch that belong to no sequence are not visited
-        new = torch.empty if cu_seqlens is None else torch.zeros
-        core = new(2, T, H, 64, dtype=torch.float32, device=dev)
-        dv = new(T, H, 64, dtype=torch.bfloat16, device=dev)
-        gc = torch.empty(H, T, W, dtype=torch.bfloat16, device=dev) if pos_key is not None else None
-        gp = torch.empty(H, T, W, dtype=torch.bfloat16, device=dev) if pos_query is not None else None
+        grads = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)]
+        d_key = torch.empty(pos_key.shape, dtype=torch.bfloat16, device=dev) if pos_key is not None else None
+        d_query = torch.empty(pos_query.shape, dtype=torch.bfloat16, device=dev) if pos_query is not None else None
         b = BwdParams()
         b.struct_bytes, b.fwd = C.sizeof(BwdParams), C.pointer(p)
         b.dout, b.dout_row_stride, b.dout_head_stride = d3.data_ptr(), d_rs, d_hs
-        b.dq_core, b.dk_core, b.dv = core[0].data_ptr(), core[1].data_ptr(), dv.data_ptr()
-        b.c2p_sums, b.p2c_sums = _ptr(gc), _ptr(gp)
+        b.dq, b.dk, b.dv = (g.data_ptr() for g in grads)
+        b.grad_row_stride, b.grad_head_stride = H * 64, 64
+        b.dpos_key, b.dpos_query = _ptr(d_key), _ptr(d_query)
         need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
         ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
         b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
         _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
-        _launches += 4 + int(W > 0 and (gc is not None or gp is not None))
+        terms = int(pos_key is not None) + int(pos_query is not None)
+        _launches += 4 + int(terms > 0) + 2 * terms
         del keep, ws
-    grads = []
-    for core_i, sums, table, other in ((core[0], gc, pos_key, q), (core[1], gp, pos_query, k)):
-        if sums is None:
-            grads += [core_i.to(torch.bfloat16).view(shape), None]
-            continue
-        rows = other.reshape(T, H, 64).permute(1, 0, 2)
-        d = torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev)
-        torch.add(core_i, _bmm(sums, table.view(H, W, 64)).permute(1, 0, 2), out=d)
-        grads += [d.view(shape), _bmm(sums.transpose(1, 2), rows).to(table.dtype).view(table.shape)]
-    return grads[0], grads[2], dv.view(shape), grads[1], grads[3]
+    return (*(g.view(shape) for g in grads), d_key, d_query)
 
 
 @torch.no_grad()

@@ -25,7 +25,8 @@
 // Position gradients: along a row the distance falls by one per column and the table row never rises, so the elements that
 // share a table row are one run.  Warps 8-11 carry the running sum of each row's run, park it in shared memory when the table
 // row changes, and write finished groups of eight to global memory: (heads, rows, table rows) in bf16, every entry written
-// once, no atomics.  What is left are GEMMs with the sums: dQ += sums . pos_key, dpos_key = sums^T . Q, and the same for the keys.
+// once, no atomics (attn_bwd_tables_sm100.cu does the rest: dQ += sums . pos_key, dpos_key = sums^T . Q, the same for the keys).
+// They clear their rows of the sums themselves while the first tile is on its way: a memset in front cost 18 us a side.
 //
 // What bounds it: the chain row term -> column term -> S -> P -> G inside a tile, about 10.5 thousand clocks of which the
 // row-term shift takes 2.4 and the wait for its products 2.2 or more; the run sums (5) lie beside it.  4 x 2048 rows x 12 heads,
@@ -36,6 +37,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "attn_bwd.h"
 #include "attn_fwd_common.cuh"
 #include "internal.h"
 #include "launch.h"
@@ -89,8 +91,10 @@ struct alignas(64) BwdArgs {
   const __nv_bfloat16* xrow;              // expanded table of the row term (heads, xrows, 64), NULL without the term
   const __nv_bfloat16* xcol;              // of the column term
   const float *lse, *delta;               // (rows, heads)
-  float* core;                            // (rows, heads, 64): dQ or dK without the row term's part
-  __nv_bfloat16* dv;                      // <true>: (rows, heads, 64)
+  float* core;                            // with the row term: (rows, heads, 64), dQ or dK without its part
+  __nv_bfloat16* grad;                    // without it: dQ or dK
+  __nv_bfloat16* dv;                      // <true>
+  int64_t grad_rs, grad_hs;               // strides of dQ, dK, dV
   __nv_bfloat16* sums;                    // (heads, rows, table_rows)
   const int16_t* lut;
   int32_t* status;
@@ -108,6 +112,21 @@ __device__ __forceinline__ int table_row(const BwdArgs& a, int d) {
   return a.lut[i];
 }
 
+// `n` threads, this one the `lane`th, clear what this kernel writes of a row outside every sequence
+template <bool DKV>
+__device__ __forceinline__ void zero_row(const BwdArgs& a, int64_t row, int head, int lane, int n) {
+  const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+  for (int i = lane; i < 16; i += n) {
+    const int64_t at = row * a.grad_rs + head * a.grad_hs + (i & 7) * 8;
+    if (a.xrow != nullptr) *reinterpret_cast<uint4*>(a.core + (row * a.heads + head) * 64 + i * 4) = z;
+    else if (i < 8) *reinterpret_cast<uint4*>(a.grad + at) = z;
+    if (DKV && i < 8) *reinterpret_cast<uint4*>(a.dv + at) = z;
+  }
+  if (a.xrow != nullptr)
+    for (int i = lane; i < a.table_rows / 8; i += n)
+      *reinterpret_cast<uint4*>(a.sums + ((int64_t)head * a.total_rows + row) * a.table_rows + i * 8) = z;
+}
+
 template <bool DKV>
 __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant__ BwdArgs args) {
   extern __shared__ uint8_t smem_raw[];
@@ -121,18 +140,12 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
   const int r0 = (int)uniform(slot.y), seq_row0 = (int)uniform(slot.z), len = (int)uniform(slot.w);
   const int row_limit = args.packed ? len : args.max_seqlen;  // rows of the padded batch that this sequence owns
 
-  if (r0 >= len) {  // dense padding: zero gradients (its sums are zero from the start)
-    for (int i = tid; i < 128 * 16; i += kThreads) {
-      const int row = r0 + (i >> 4);
-      if (row >= row_limit) continue;
-      const int64_t at = ((int64_t)(seq_row0 + row) * args.heads + head) * 64 + (i & 15) * 4;
-      *reinterpret_cast<float4*>(args.core + at) = make_float4(0.f, 0.f, 0.f, 0.f);
-      if (DKV) *reinterpret_cast<uint2*>(args.dv + at) = make_uint2(0u, 0u);
-    }
+  const bool row_term = args.xrow != nullptr, col_term = args.xcol != nullptr;
+  if (r0 >= len) {  // dense padding: zero gradients
+    for (int row = r0 + warp; row < min(r0 + 128, row_limit); row += kThreads / 32) zero_row<DKV>(args, seq_row0 + row, head, lane, 32);
     return;
   }
 
-  const bool row_term = args.xrow != nullptr, col_term = args.xcol != nullptr;
   const int n_tiles = (len + kCols - 1) / kCols;
   // tiles [jb, jb + nb) have distances inside the bucketed range; saturated high in front of them, low behind
   int jb = 0, je = 0;
@@ -307,6 +320,13 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
     const bool valid_row = my_row < len;
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
     if (row_term) {
+      for (int i = 0; i < 32; ++i) {  // a row at a time: whole lines (a packed row behind the sequence is another one's)
+        const int row = r0 + quad * 32 + i;
+        if (row >= len && (args.packed || row >= row_limit)) break;
+        uint4* z = reinterpret_cast<uint4*>(args.sums + ((int64_t)head * args.total_rows + seq_row0 + row) * args.table_rows);
+        for (int c = lane; c < args.table_rows / 8; c += 32) z[c] = make_uint4(0u, 0u, 0u, 0u);
+      }
+      __syncwarp();
       float run = 0.f;                            // sum of the current run
       int b = table_row<DKV>(args, my_row);       // and its table row: falls by one per run (<true>: rises)
       // Finished sums wait in a row of three aligned groups of eight table rows: the current group lies in the last one (<true>:
@@ -583,32 +603,34 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
     wait(bar(kBarAcc), uint32_t(n_tiles - 1) & 1u);
     tc_fence_after();
     const bool store = my_row < row_limit;
-    const int64_t at = ((int64_t)(seq_row0 + my_row) * args.heads + head) * 64 + 32 * h;
-    {
-      uint32_t o[32];
-      tmem_ld32(tmem_lane + kColAcc + 32 * h, o);  // whole warps execute this, whatever their rows
+    const int64_t row = seq_row0 + my_row, at = row * args.grad_rs + (int64_t)head * args.grad_hs + 32 * h;
+    uint32_t o[32];
+    auto store_bf16 = [&](__nv_bfloat16* to) {
+      uint4* d = reinterpret_cast<uint4*>(to);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        d[q] = !valid_row ? make_uint4(0u, 0u, 0u, 0u)
+                          : make_uint4(pack_bf16x2(__uint_as_float(o[8 * q + 0]), __uint_as_float(o[8 * q + 1])),
+                                       pack_bf16x2(__uint_as_float(o[8 * q + 2]), __uint_as_float(o[8 * q + 3])),
+                                       pack_bf16x2(__uint_as_float(o[8 * q + 4]), __uint_as_float(o[8 * q + 5])),
+                                       pack_bf16x2(__uint_as_float(o[8 * q + 6]), __uint_as_float(o[8 * q + 7])));
+    };
+    tmem_ld32(tmem_lane + kColAcc + 32 * h, o);  // whole warps execute this, whatever their rows
+    tmem_wait_ld();
+    if (store && row_term) {
+      float4* d = reinterpret_cast<float4*>(args.core + (row * args.heads + head) * 64 + 32 * h);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        d[q] = valid_row ? make_float4(__uint_as_float(o[4 * q]), __uint_as_float(o[4 * q + 1]), __uint_as_float(o[4 * q + 2]), __uint_as_float(o[4 * q + 3]))
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+    } else if (store) {
+      store_bf16(args.grad + at);
+    }
+    __syncwarp();
+    if (DKV) {
+      tmem_ld32(tmem_lane + kColAcc + 64 + 32 * h, o);
       tmem_wait_ld();
-      if (store) {
-        float4* d = reinterpret_cast<float4*>(args.core + at);
-#pragma unroll
-        for (int q = 0; q < 8; ++q)
-          d[q] = valid_row ? make_float4(__uint_as_float(o[4 * q]), __uint_as_float(o[4 * q + 1]), __uint_as_float(o[4 * q + 2]), __uint_as_float(o[4 * q + 3]))
-                           : make_float4(0.f, 0.f, 0.f, 0.f);
-      }
-      if (DKV) {
-        tmem_ld32(tmem_lane + kColAcc + 64 + 32 * h, o);
-        tmem_wait_ld();
-        if (store) {
-          uint4* d = reinterpret_cast<uint4*>(args.dv + at);
-#pragma unroll
-          for (int q = 0; q < 4; ++q)
-            d[q] = !valid_row ? make_uint4(0u, 0u, 0u, 0u)
-                              : make_uint4(pack_bf16x2(__uint_as_float(o[8 * q + 0]), __uint_as_float(o[8 * q + 1])),
-                                           pack_bf16x2(__uint_as_float(o[8 * q + 2]), __uint_as_float(o[8 * q + 3])),
-                                           pack_bf16x2(__uint_as_float(o[8 * q + 4]), __uint_as_float(o[8 * q + 5])),
-                                           pack_bf16x2(__uint_as_float(o[8 * q + 6]), __uint_as_float(o[8 * q + 7])));
-        }
-      }
+      if (store) store_bf16(args.dv + at);
     }
   }
 
@@ -623,10 +645,13 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
   if (warp == kMmaWarp) tmem_dealloc(tmem_base, kTmemCols);
 }
 
-// delta = sum over the head dimension of dO * O, fp32, (rows, heads); eight lanes per (row, head)
+// delta = sum over the head dimension of dO * O, fp32, (rows, heads); eight lanes per (row, head).  Packed rows in front of the
+// first and behind the last sequence, which the tile kernels do not visit, are cleared here (`dq` and `dkv` name the outputs).
 __global__ void __launch_bounds__(256) bwd_delta_kernel(const __nv_bfloat16* __restrict__ dout, int64_t d_rs, int64_t d_hs,
                                                         const __nv_bfloat16* __restrict__ out, int64_t o_rs, int64_t o_hs,
-                                                        int64_t cells, int heads, float* __restrict__ delta) {
+                                                        int64_t cells, int heads, float* __restrict__ delta,
+                                                        const int32_t* __restrict__ cu_seqlens, int batch,
+                                                        const __grid_constant__ BwdArgs dq, const __grid_constant__ BwdArgs dkv) {
   const int64_t cell = ((int64_t)blockIdx.x * 256 + threadIdx.x) >> 3;
   const int sub = threadIdx.x & 7;
   float sum = 0.f;
@@ -644,6 +669,13 @@ __global__ void __launch_bounds__(256) bwd_delta_kernel(const __nv_bfloat16* __r
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   if (sub == 0 && cell < cells) delta[cell] = sum;
+  if (cu_seqlens != nullptr && cell < cells) {
+    const int64_t row = cell / heads;
+    if (row < cu_seqlens[0] || row >= cu_seqlens[batch]) {
+      zero_row<false>(dq, row, (int)(cell % heads), sub, 8);
+      zero_row<true>(dkv, row, (int)(cell % heads), sub, 8);
+    }
+  }
 }
 
 // The four expanded tables: by distance query - key (as in the forward) and by distance key - query (the same rows backwards).
@@ -663,9 +695,11 @@ __global__ void __launch_bounds__(256) bwd_expand_kernel(const uint4* __restrict
   if (pos_query != nullptr) { const uint4 v = pos_query[src]; query[i] = v; query_rev[rev] = v; }
 }
 
+int table_rows_of(const fdb_attn_params& p) { return 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions); }
+
 uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 
-struct Layout { uint64_t seq_info, tile_first, slot_info, delta, table[4], total; };
+struct Layout { uint64_t seq_info, tile_first, slot_info, delta, table[4], core, sums, partial, total; };
 
 Layout layout_of(const fdb_attn_params& p, const ExpandGeometry& g) {
   Layout l;
@@ -676,14 +710,19 @@ Layout layout_of(const fdb_attn_params& p, const ExpandGeometry& g) {
   l.delta = off;      off = align256(off + uint64_t(p.total_rows) * p.heads * 4);
   const uint64_t table = uint64_t(p.heads) * g.rows * kHeadDim * 2;
   for (int i = 0; i < 4; ++i) { l.table[i] = off; off = align256(off + ((i & 1) ? (p.pos_query ? table : 0) : (p.pos_key ? table : 0))); }
+  // the two sides run one after the other and share these
+  const bool terms = p.pos_key != nullptr || p.pos_query != nullptr;
+  const int table_rows = table_rows_of(p);
+  l.core = off;    off = align256(off + (terms ? uint64_t(p.total_rows) * p.heads * kHeadDim * 4 : 0));
+  l.sums = off;    off = align256(off + (terms ? uint64_t(p.total_rows) * p.heads * table_rows * 2 : 0));
+  l.partial = off; off = align256(off + (terms ? bwd_tables_partial_bytes(p.total_rows, p.heads, table_rows) : 0));
   l.total = off;
   return l;
 }
 
 template <bool DKV>
-int launch_bwd(const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layout& l, char* ws, int64_t slots, cudaStream_t stream) {
+int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layout& l, char* ws) {
   const fdb_attn_params& p = *b.fwd;
-  BwdArgs a;
   auto operand = [&](CUtensorMap* m, const void* base, int64_t rs, int64_t hs, int box) {
     return make_map_rows(m, base, p.total_rows, p.heads, rs, hs, box, false, "backward operand");
   };
@@ -704,11 +743,13 @@ int launch_bwd(const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layo
   a.slot_info = reinterpret_cast<const int4*>(ws + l.slot_info);
   a.lse = p.lse;
   a.delta = reinterpret_cast<const float*>(ws + l.delta);
-  a.core = DKV ? b.dk_core : b.dq_core;
+  a.core = reinterpret_cast<float*>(ws + l.core);
+  a.grad = static_cast<__nv_bfloat16*>(DKV ? b.dk : b.dq);
   a.dv = DKV ? static_cast<__nv_bfloat16*>(b.dv) : nullptr;
-  a.sums = static_cast<__nv_bfloat16*>(DKV ? b.p2c_sums : b.c2p_sums);
+  a.grad_rs = b.grad_row_stride; a.grad_hs = b.grad_head_stride;
+  a.sums = reinterpret_cast<__nv_bfloat16*>(ws + l.sums);
   a.lut = p.bucket_lut; a.lut_d_min = p.lut_d_min; a.lut_len = p.lut_len;
-  a.table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
+  a.table_rows = table_rows_of(p);
   a.status = p.status;
   a.heads = p.heads; a.packed = p.cu_seqlens != nullptr; a.max_seqlen = p.max_seqlen; a.total_rows = p.total_rows;
   a.sat_lo = DKV ? -g.sat_hi : g.sat_lo;
@@ -716,12 +757,32 @@ int launch_bwd(const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layo
   a.d_first = a.sat_lo - 254;
   a.xrows = g.rows;
   a.sm_scale = p.sm_scale;
+  return FDB_OK;
+}
+
+template <bool DKV>
+int launch_bwd(const BwdArgs& a, const fdb_attn_bwd_params& b, char* partial, int64_t slots, cudaStream_t stream) {
+  const fdb_attn_params& p = *b.fwd;
   static std::atomic<uint64_t> smem_done{0};
   auto kernel = bwd_kernel<DKV>;
   cudaError_t e = allow_smem(smem_done, reinterpret_cast<const void*>(kernel), (int)kSmemBytes);
   if (e == cudaSuccess) e = launch_kernel<BwdArgs>(kernel, a, dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, false, stream);
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd launch: %s", cudaGetErrorString(e));
-  return FDB_OK;
+  if (a.xrow == nullptr) return FDB_OK;
+  BwdTablesCall c;
+  c.sums = a.sums;
+  c.table = DKV ? p.pos_query : p.pos_key;
+  c.operand = DKV ? p.k : p.q;
+  c.operand_row_stride = DKV ? p.k_row_stride : p.q_row_stride;
+  c.operand_head_stride = DKV ? p.k_head_stride : p.q_head_stride;
+  c.core = a.core;
+  c.out = a.grad;
+  c.out_row_stride = a.grad_rs; c.out_head_stride = a.grad_hs;
+  c.dtable = DKV ? b.dpos_query : b.dpos_key;
+  c.partial = reinterpret_cast<float*>(partial);
+  c.rows = p.total_rows; c.heads = p.heads; c.table_rows = a.table_rows;
+  c.status = p.status;
+  return launch_bwd_tables(c, stream);
 }
 
 int check_bwd(const fdb_attn_bwd_params* b, ExpandGeometry* g) {
@@ -760,12 +821,14 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   if (rc != FDB_OK) return rc;
   const fdb_attn_params& p = *b->fwd;
   if (p.batch == 0 || p.total_rows == 0) return FDB_OK;
-  if (b->dout == nullptr || p.lse == nullptr || b->dq_core == nullptr || b->dk_core == nullptr || b->dv == nullptr ||
-      (p.pos_key != nullptr) != (b->c2p_sums != nullptr) || (p.pos_query != nullptr) != (b->p2c_sums != nullptr))
-    return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_attn_bwd: dout, lse, dq_core, dk_core, dv and the sums of every position term are required");
-  const uintptr_t all = (uintptr_t)b->dout | (uintptr_t)b->dq_core | (uintptr_t)b->dk_core | (uintptr_t)b->dv | (uintptr_t)b->c2p_sums | (uintptr_t)b->p2c_sums;
-  if ((all & 15u) != 0 || b->dout_row_stride <= 0 || b->dout_head_stride <= 0 || b->dout_row_stride % 8 != 0 || b->dout_head_stride % 8 != 0)
-    return fail(FDB_ERR_ALIGNMENT, "fdb_attn_bwd: pointers must be 16-byte aligned, dout strides multiples of 8 elements");
+  if (b->dout == nullptr || p.lse == nullptr || b->dq == nullptr || b->dk == nullptr || b->dv == nullptr ||
+      (p.pos_key != nullptr) != (b->dpos_key != nullptr) || (p.pos_query != nullptr) != (b->dpos_query != nullptr))
+    return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_attn_bwd: dout, lse, dq, dk, dv and the gradient of every position table are required");
+  const uintptr_t all = (uintptr_t)b->dout | (uintptr_t)b->dq | (uintptr_t)b->dk | (uintptr_t)b->dv | (uintptr_t)b->dpos_key | (uintptr_t)b->dpos_query;
+  const int64_t strides[4] = {b->dout_row_stride, b->dout_head_stride, b->grad_row_stride, b->grad_head_stride};
+  bool aligned = (all & 15u) == 0;
+  for (int64_t s : strides) aligned = aligned && s > 0 && s % 8 == 0;
+  if (!aligned) return fail(FDB_ERR_ALIGNMENT, "fdb_attn_bwd: pointers must be 16-byte aligned, strides positive multiples of 8 elements");
   const Layout l = layout_of(p, g);
   if (b->workspace == nullptr || b->workspace_bytes < l.total)
     return fail(FDB_ERR_WORKSPACE, "workspace of %llu bytes needed, %llu given", (unsigned long long)l.total, (unsigned long long)b->workspace_bytes);
@@ -779,25 +842,21 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   buf.tile_first = reinterpret_cast<int32_t*>(ws + l.tile_first);
   buf.slot_info = reinterpret_cast<int32_t*>(ws + l.slot_info);
   if ((rc = launch_seq_info(p, buf, stream)) != FDB_OK) return rc;
-  const int table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
-  const uint64_t sum_bytes = uint64_t(p.heads) * p.total_rows * table_rows * 2;
-  cudaError_t e = cudaSuccess;
-  if (b->c2p_sums != nullptr) e = cudaMemsetAsync(b->c2p_sums, 0, sum_bytes, s);
-  if (e == cudaSuccess && b->p2c_sums != nullptr) e = cudaMemsetAsync(b->p2c_sums, 0, sum_bytes, s);
-  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd memset: %s", cudaGetErrorString(e));
+  BwdArgs dq, dkv;
+  if ((rc = make_args<false>(dq, *b, g, l, ws)) != FDB_OK || (rc = make_args<true>(dkv, *b, g, l, ws)) != FDB_OK) return rc;
   if (p.pos_key != nullptr || p.pos_query != nullptr) {
     const int64_t n = (int64_t)p.heads * g.rows * 8;
     auto table = [&](int i) { return reinterpret_cast<uint4*>(ws + l.table[i]); };
     bwd_expand_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(static_cast<const uint4*>(p.pos_key), static_cast<const uint4*>(p.pos_query),
                                                                  table(0), table(1), table(2), table(3), p.bucket_lut, p.lut_len, g.rows,
-                                                                 table_rows, p.heads);
+                                                                 table_rows_of(p), p.heads);
   }
   const int64_t cells = (int64_t)p.total_rows * p.heads;
   bwd_delta_kernel<<<(unsigned)((cells * 8 + 255) / 256), 256, 0, s>>>(
       static_cast<const __nv_bfloat16*>(b->dout), b->dout_row_stride, b->dout_head_stride, static_cast<const __nv_bfloat16*>(p.out),
-      p.out_row_stride, p.out_head_stride, cells, p.heads, reinterpret_cast<float*>(ws + l.delta));
-  e = cudaGetLastError();
+      p.out_row_stride, p.out_head_stride, cells, p.heads, reinterpret_cast<float*>(ws + l.delta), p.cu_seqlens, p.batch, dq, dkv);
+  const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd set-up: %s", cudaGetErrorString(e));
-  if ((rc = launch_bwd<false>(*b, g, l, ws, slots, s)) != FDB_OK) return rc;
-  return launch_bwd<true>(*b, g, l, ws, slots, s);
+  if ((rc = launch_bwd<false>(dq, *b, ws + l.partial, slots, s)) != FDB_OK) return rc;
+  return launch_bwd<true>(dkv, *b, ws + l.partial, slots, s);
 }

@@ -211,9 +211,7 @@ FDB_API int fdb_attn_fwd_static(const fdb_attn_params* p, void* stream);
 /*
  * Backward pass, fused (bf16, head_dim 64): probabilities rebuilt tile by tile on the tensor cores, nothing quadratic in the
  * sequence length in memory.  Replaces the reference's _bwd_preprocess, _bwd_kv_dise_kernel and _bwd_q_dise_kernel
- * (src/flashdeberta/ops/flash_attention.py:581-940).  What it leaves to the caller are GEMMs with the two sum tensors:
- *   dQ = dq_core + c2p_sums . pos_key        dpos_key   = sum over rows of c2p_sums^T . Q
- *   dK = dk_core + p2c_sums . pos_query      dpos_query = sum over rows of p2c_sums^T . K       (per head)
+ * (src/flashdeberta/ops/flash_attention.py:581-940).
  * The bucket index must rise by at most one from one distance to the next (true of every log-bucket table whose far range
  * is wider than its buckets), 2*att_span must be a multiple of 8, and the bucket table may have at most 3588 entries.
  */
@@ -224,18 +222,15 @@ typedef struct fdb_attn_bwd_params {
                                    and prepared fields are not looked at */
   const void* dout;             /* bf16, gradient of out */
   int64_t dout_row_stride, dout_head_stride;
-  float* dq_core;               /* out (total_rows, heads, 64) */
-  float* dk_core;               /* out (total_rows, heads, 64) */
-  void* dv;                     /* out bf16 (total_rows, heads, 64) */
-  void* c2p_sums;               /* out bf16 (heads, total_rows, 2*att_span), with pos_key: dS of a query row summed over the keys
-                                   that address each table row */
-  void* p2c_sums;               /* out bf16, with pos_query: dS of a key row summed over its queries */
+  void *dq, *dk, *dv;           /* out bf16, (total_rows, heads, 64) with the strides below */
+  int64_t grad_row_stride, grad_head_stride;
+  void *dpos_key, *dpos_query;  /* out bf16 (heads, 2*att_span, 64), each with its table */
   void* workspace;              /* device, >= fdb_attn_bwd_workspace_bytes(), 256-byte aligned */
   uint64_t workspace_bytes;
 } fdb_attn_bwd_params;
 
 FDB_API uint64_t fdb_attn_bwd_workspace_bytes(const fdb_attn_bwd_params* p);
-/* Rows that belong to no sequence: zero in the dense layout, untouched in the packed one (zero the outputs first). */
+/* Rows that belong to no sequence get zero gradients. */
 FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* p, void* stream);
 
 /*

@@ -110,6 +110,45 @@ def test_gradients_at_2048_keys_with_far_tiles():
         _close(a, b, name)
 
 
+@pytest.mark.parametrize("buckets,max_rel,c2p,p2c", [(256, 512, True, True), (512, 1024, True, True), (32, 64, True, False),
+                                                     (-1, 100, False, True), (-1, -1, False, False)])
+@pytest.mark.parametrize("layout", ["packed", "padded"])
+def test_fused_gradients_at_tile_edges_match_the_block_form(buckets, max_rel, c2p, p2c, layout):
+    """Lengths around the edges of the fused kernels' tiles (128 rows, 64 columns), rows outside every sequence, strided inputs,
+    and tables of one, several and more than 512 rows, against the block form of the same gradients."""
+    from flashdeberta_b200 import backward, ops
+    g = torch.Generator().manual_seed(buckets + max_rel)
+    H, D, lens = 2, 64, [1, 63, 64, 65, 0, 127, 128, 129, 191, 600]
+    span = (buckets if buckets > 0 else max_rel) if (c2p or p2c) else 0
+    if layout == "packed":
+        cu = torch.tensor([5 + sum(lens[:i]) for i in range(len(lens) + 1)], dtype=torch.int32, device=DEV)
+        rows, kw = (int(cu[-1]) + 37,), dict(cu_seqlens=cu, max_seqlen=max(lens))
+        inside = torch.arange(rows[0], device=DEV)
+        inside = (inside >= 5) & (inside < int(cu[-1]))
+    else:
+        rows, n = (len(lens), 601), torch.tensor(lens, dtype=torch.int32, device=DEV)
+        kw, inside = dict(seq_lens=n, max_seqlen=601), torch.arange(601, device=DEV)[None, :] < n[:, None]
+    q, k, v = torch.randn(*rows, 3, H, D, generator=g).bfloat16().to(DEV).unbind(-3)
+    dout = torch.randn(*rows, H, D, generator=g).bfloat16().to(DEV)
+    pk = torch.randn(H, 2 * span, D, generator=g).bfloat16().to(DEV) if c2p else None
+    pq = torch.randn(H, 2 * span, D, generator=g).bfloat16().to(DEV) if p2c else None
+    kw.update(sm_scale=oracle.sm_scale_for(D, c2p, p2c), position_buckets=buckets, max_relative_positions=max_rel)
+    with torch.no_grad():
+        out, lse = ops.disentangled_attention(q, k, v, pk, pq, return_lse=True, **kw)
+    out = torch.where(inside[..., None, None], out, 0)
+    lse = torch.where(inside.reshape(-1, 1), lse, 0)
+    got = backward.attention_backward(dout, q, k, v, pk, pq, out, lse, **kw)
+    want = backward.attention_backward(dout * inside[..., None, None], q, k, v, pk, pq, out, lse, block_bytes=1 << 28, **kw)
+    torch.cuda.synchronize()
+    ops.check_status()
+    for name, a, b in zip(("dq", "dk", "dv", "dpos_key", "dpos_query"), got, want):
+        assert (a is None) == (b is None), name
+        if a is not None:
+            _close(a, b.float().cpu(), name)
+    for t in got[:3]:
+        assert t[~inside].abs().max().item() == 0
+
+
 def _small_config(backend, **kw):
     from transformers.models.deberta_v2.configuration_deberta_v2 import DebertaV2Config
     cfg = DebertaV2Config(vocab_size=2000, hidden_size=256, num_hidden_layers=2, num_attention_heads=4,
