@@ -51,6 +51,7 @@ EXPORTS = (
     "fdb_quantize_e4m3", "fdb_add_layernorm", "fdb_linear_gelu", "fdb_embed_layernorm",
     "fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums", "fdb_expanded_rows", "fdb_expand_tables", "fdb_encoder_create",
     "fdb_encoder_destroy", "fdb_encoder_workspace_bytes", "fdb_encoder_forward", "fdb_attn_bwd_workspace_bytes", "fdb_attn_bwd",
+    "fdb_lengths_from_mask", "fdb_column_sums_workspace_bytes", "fdb_column_sums",
 )
 
 _lib = None
@@ -111,6 +112,13 @@ def load() -> C.CDLL:
     lib.fdb_attn_bwd_workspace_bytes.argtypes = [C.c_void_p]
     lib.fdb_attn_bwd.restype = C.c_int
     lib.fdb_attn_bwd.argtypes = [C.c_void_p, C.c_void_p]
+    lib.fdb_lengths_from_mask.restype = C.c_int
+    lib.fdb_lengths_from_mask.argtypes = [C.c_void_p, C.c_int32, C.c_int32, C.c_int32, C.c_int64, C.c_int64, C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.fdb_column_sums_workspace_bytes.restype = C.c_uint64
+    lib.fdb_column_sums_workspace_bytes.argtypes = [C.c_int64, C.c_int64, C.c_int32]
+    lib.fdb_column_sums.restype = C.c_int
+    lib.fdb_column_sums.argtypes = [C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_int64, C.c_int32, C.c_void_p, C.c_void_p, C.c_uint64,
+                                    C.c_void_p]
     lib.fdb_expanded_rows.restype = C.c_int32
     lib.fdb_expanded_rows.argtypes = [C.c_int32, C.c_int32]
     lib.fdb_expand_tables.restype = C.c_int

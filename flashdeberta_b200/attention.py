@@ -20,7 +20,7 @@ from typing import Optional
 import torch
 from transformers.models.deberta_v2.modeling_deberta_v2 import DisentangledSelfAttention
 
-from . import _lib, ops
+from . import _lib, ops, projected
 
 _warned_general = False
 
@@ -86,6 +86,8 @@ def lengths_from_mask(attention_mask: Optional[torch.Tensor], check: bool = True
         m = torch.diagonal(m, dim1=-2, dim2=-1)
     elif m.dim() != 2:
         raise ValueError(f"attention_mask with {attention_mask.dim()} dims is not supported")
+    if check and m.is_cuda and m.dtype in ops.MASK_TYPES and m.dim() == 2 and not torch.compiler.is_compiling():
+        return ops.lengths_from_mask(m)
     valid = m != 0
     lens = valid.sum(dim=-1, dtype=torch.int32)
     if check and not torch.compiler.is_compiling():
@@ -179,6 +181,8 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
         B, L, _ = hidden_states.shape
         H, D = self.num_attention_heads, self.attention_head_size
         in_dtype = hidden_states.dtype
+        if projected.covers(self, hidden_states, query_states, attention_mask, rel_embeddings):
+            return (projected.attention(self, hidden_states, lengths_from_mask(attention_mask), rel_embeddings), None)
 
         q = self.query_proj(query_states).view(B, L, H, D)
         k = self.key_proj(hidden_states).view(B, L, H, D)

@@ -203,6 +203,11 @@ def _fused_covers(q, k, v, dout, pos_key, pos_query, position_buckets, max_relat
         return False
     if pos_key is None and pos_query is None:
         return True
+    return index_covered(position_buckets, max_relative_positions)
+
+
+def index_covered(position_buckets, max_relative_positions) -> bool:
+    """Whether ``fdb_attn_bwd`` takes this bucket table."""
     key = (int(position_buckets), int(max_relative_positions))
     if key not in _steps:
         table, _ = bucket.host_lut(*key)
@@ -212,7 +217,8 @@ def _fused_covers(q, k, v, dout, pos_key, pos_query, position_buckets, max_relat
 
 
 def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
-           max_relative_positions):
+           max_relative_positions, grads=None, table_grads=(None, None)):
+    """``grads`` (rows, 3, H, 64) and ``table_grads`` (each table's shape), when given, take the results."""
     global _launches
     from . import ops
     dev, shape = q.device, q.shape
@@ -222,14 +228,20 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
                                    max_relative_positions, out.contiguous(), lse.contiguous())
         d3, d_rs, d_hs = ops._rows_view(dout)
         T, H = d3.shape[0], d3.shape[1]
-        grads = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)]
-        d_key = torch.empty(pos_key.shape, dtype=torch.bfloat16, device=dev) if pos_key is not None else None
-        d_query = torch.empty(pos_query.shape, dtype=torch.bfloat16, device=dev) if pos_query is not None else None
+        if grads is None:
+            grads, row_stride = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)], H * 64
+        else:
+            grads, row_stride = grads.unbind(1), 3 * H * 64
+        d_key, d_query = table_grads
+        if d_key is None and pos_key is not None:
+            d_key = torch.empty(pos_key.shape, dtype=torch.bfloat16, device=dev)
+        if d_query is None and pos_query is not None:
+            d_query = torch.empty(pos_query.shape, dtype=torch.bfloat16, device=dev)
         b = BwdParams()
         b.struct_bytes, b.fwd = C.sizeof(BwdParams), C.pointer(p)
         b.dout, b.dout_row_stride, b.dout_head_stride = d3.data_ptr(), d_rs, d_hs
         b.dq, b.dk, b.dv = (g.data_ptr() for g in grads)
-        b.grad_row_stride, b.grad_head_stride = H * 64, 64
+        b.grad_row_stride, b.grad_head_stride = row_stride, 64
         b.dpos_key, b.dpos_query = _ptr(d_key), _ptr(d_query)
         need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
         ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)

@@ -17,8 +17,6 @@ from torch import nn
 
 from . import _lib, bucket, ops
 
-_MASK_TYPES = {torch.float32: 0, torch.int64: 1, torch.int32: 2, torch.uint8: 3, torch.bool: 3, torch.bfloat16: 4}
-
 
 class EncoderLayer(C.Structure):
     """Mirror of ``fdb_encoder_layer`` (include/fdb_b200.h)."""
@@ -203,10 +201,10 @@ class EncoderEngine:
         if mask is not None:
             if mask.device != device:
                 mask = mask.to(device, non_blocking=True)
-            if mask.dtype not in _MASK_TYPES:
+            if mask.dtype not in ops.MASK_TYPES:
                 mask = mask.to(torch.float32)
             mask = mask.contiguous()
-            p.mask, p.mask_type = mask.data_ptr(), _MASK_TYPES[mask.dtype]
+            p.mask, p.mask_type = mask.data_ptr(), ops.MASK_TYPES[mask.dtype]
         if cu_seqlens is not None:
             p.cu_seqlens, p.batch = cu_seqlens.data_ptr(), cu_seqlens.numel() - 1
         else:

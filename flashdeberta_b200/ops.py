@@ -5,7 +5,8 @@ src/flashdeberta/ops/flash_attention_varlen.py:485-511).  The signature differs 
 two pre-multiplied bias tensors ``q @ pos_key^T`` and ``k @ pos_query^T`` (model.py:189-192); these take the projected
 position tables themselves and the products never exist in global memory.
 
-Forward only, like the reference's packed op (flash_attention_varlen.py:481-483 raises in backward).
+Where autograd records, the bf16 calls have a backward (backward.py); the reference's packed op raises in its own
+(flash_attention_varlen.py:481-483).
 """
 from __future__ import annotations
 
@@ -21,6 +22,9 @@ __all__ = [
     "disentangled_attention", "disentangled_attention_fp8", "disentangled_attention_static", "disentangled_attention_check", "relative_index_matrix", "quantize_e4m3", "add_layernorm", "can_fuse_add_layernorm", "linear_gelu", "can_fuse_linear_gelu", "embed_layernorm",
     "check_status", "launch_count", "PreparedWorkspace",
 ]
+
+#: element types of a mask (FDB_MASK_*)
+MASK_TYPES = {torch.float32: 0, torch.int64: 1, torch.int32: 2, torch.uint8: 3, torch.bool: 3, torch.bfloat16: 4}
 
 _status: Dict[str, torch.Tensor] = {}
 _launches = 0  # kernels this module asked the library to launch (the benchmark reports it)
@@ -75,6 +79,34 @@ def flag_status(device: torch.device, condition: torch.Tensor, bit: int) -> None
     """OR ``bit`` into the device status word where the 0-d boolean ``condition`` (on that device) is true.  No host
     synchronisation: the word is read by ``check_status``."""
     _status_word(device).bitwise_or_(condition.to(torch.int32) * bit)
+
+
+def lengths_from_mask(mask: torch.Tensor) -> torch.Tensor:
+    """int32 lengths of the rows of a (batch, tokens) mask on the GPU, any strides; flags a mask that is not right-padded in
+    the device status word."""
+    global _launches
+    lens = torch.empty(mask.shape[0], dtype=torch.int32, device=mask.device)
+    with torch.cuda.device(mask.device):
+        _lib.check(_lib.load().fdb_lengths_from_mask(
+            mask.data_ptr(), MASK_TYPES[mask.dtype], mask.shape[0], mask.shape[1], mask.stride(0), mask.stride(1), lens.data_ptr(),
+            _status_word(mask.device).data_ptr(), torch.cuda.current_stream(mask.device).cuda_stream))
+    _launches += 1
+    return lens
+
+
+def column_sums(x: torch.Tensor, more: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """Sums over the rows of a contiguous bf16 matrix, plus those of ``more`` in its first columns: bias gradients."""
+    global _launches
+    lib = _lib.load()
+    out = torch.empty(x.shape[1], dtype=x.dtype, device=x.device)
+    rows, cols = (0, 0) if more is None else more.shape
+    with torch.cuda.device(x.device):
+        need = lib.fdb_column_sums_workspace_bytes(x.shape[0], rows, x.shape[1])
+        ws = torch.empty(need, dtype=torch.uint8, device=x.device)
+        _lib.check(lib.fdb_column_sums(x.data_ptr(), x.shape[0], x.shape[1], None if more is None else more.data_ptr(), rows, cols,
+                                       out.data_ptr(), ws.data_ptr(), need, torch.cuda.current_stream(x.device).cuda_stream))
+    _launches += 2
+    return out
 
 
 def _dtype_code(t: torch.Tensor) -> int:

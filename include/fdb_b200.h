@@ -375,12 +375,23 @@ FDB_API int fdb_encoder_create(const fdb_encoder_layer* layers, int32_t n_layers
                                void** plan);
 FDB_API void fdb_encoder_destroy(void* plan);
 
-/* Element type of a mask: token i is valid where mask[i] != 0, and its embedding is multiplied by mask[i]. */
+/* Element type of a mask: token i is valid where mask[i] != 0 (the encoder multiplies its embedding by mask[i]). */
 #define FDB_MASK_F32 0
 #define FDB_MASK_I64 1
 #define FDB_MASK_I32 2
 #define FDB_MASK_U8 3
 #define FDB_MASK_BF16 4
+
+/* Valid lengths (int32, one per sequence) of a right-padded batch from its mask, element (b, t) at b * batch_stride + t *
+ * token_stride; FDB_DEV_BAD_MASK in `status` (or NULL) when the valid tokens of a sequence are not its first ones. */
+FDB_API int fdb_lengths_from_mask(const void* mask, int32_t mask_type, int32_t batch, int32_t seqlen, int64_t batch_stride,
+                                  int64_t token_stride, int32_t* lens, int32_t* status, void* stream);
+
+/* out[c] = sum over the rows of x (rows, cols) and of more (more_rows, more_cols <= cols), bf16, contiguous, summed in fp32:
+ * the bias gradients of projections of two inputs through the same weights. */
+FDB_API uint64_t fdb_column_sums_workspace_bytes(int64_t rows, int64_t more_rows, int32_t cols);
+FDB_API int fdb_column_sums(const void* x, int64_t rows, int32_t cols, const void* more, int64_t more_rows, int32_t more_cols,
+                            void* out, void* workspace, uint64_t workspace_bytes, void* stream);
 
 typedef struct fdb_encoder_call {
   uint32_t struct_bytes; /* sizeof(fdb_encoder_call), checked */

@@ -161,6 +161,43 @@ def _small_config(backend, **kw):
     return cfg
 
 
+@pytest.mark.parametrize("mask_type,rel_rows,frozen", [(None, 512, ()), (torch.int64, 512, ("rel",)), (torch.bool, 515, ("x", "key_proj")),
+                                                       (torch.bfloat16, 512, ("value_proj", "query_proj", "key_proj"))])
+def test_module_as_one_node_matches_the_operators(monkeypatch, mask_type, rel_rows, frozen):
+    """Training through the module (projections, tables and attention in one autograd node) against the same module operator by
+    operator: output and every gradient, with and without a mask, with inputs and projections that need no gradient."""
+    from flashdeberta_b200 import ops, projected
+    from flashdeberta_b200.attention import FlashDisentangledSelfAttention
+    torch.manual_seed(5)
+    module = FlashDisentangledSelfAttention(_small_config("b200")).to(DEV).bfloat16().train()
+    B, L = 3, 321
+    x, rel = torch.randn(B, L, 256, device=DEV).bfloat16(), torch.randn(rel_rows, 256, device=DEV).bfloat16()
+    dout = torch.randn(B, L, 256, device=DEV).bfloat16()
+    mask = None
+    if mask_type is not None:
+        mask = (torch.arange(L, device=DEV)[None, :] < torch.tensor([321, 128, 1], device=DEV)[:, None]).to(mask_type)
+        dout = dout * mask[..., None].to(dout.dtype)
+    x.requires_grad_("x" not in frozen)
+    rel.requires_grad_("rel" not in frozen)
+    for name in frozen:
+        if hasattr(module, name):
+            getattr(module, name).requires_grad_(False)
+    leaves = {n: p for n, p in [("x", x), ("rel", rel), *module.named_parameters()] if p.requires_grad}
+
+    def run():
+        out, _ = module(x, mask, rel_embeddings=rel)
+        return [out.detach(), *torch.autograd.grad(out, list(leaves.values()), dout)]
+
+    assert projected.covers(module, x, None, mask, rel)
+    got = run()
+    monkeypatch.setattr(projected, "covers", lambda *a: False)
+    want = run()
+    ops.check_status()
+    for name, a, b in zip(["out", *leaves], got, want):
+        assert a.dtype == b.dtype and a.shape == b.shape, name
+        _close(a, b.float().cpu(), name)
+
+
 @pytest.mark.parametrize("pack", [True, False])
 def test_training_step_of_the_model_matches_the_eager_backend(pack):
     """loss.backward() through FlashDebertaV2ForSequenceClassification in train mode on a ragged batch: every parameter's
