@@ -35,7 +35,7 @@ from typing import Dict, Optional, Tuple
 import numpy as np
 import torch
 
-from . import _lib, bucket
+from . import _lib, bucket, ops
 
 class BwdParams(C.Structure):
     """Mirror of ``fdb_attn_bwd_params`` (include/fdb_b200.h)."""
@@ -89,8 +89,8 @@ def _stage_probs(blk: dict) -> Tuple[torch.Tensor, torch.Tensor]:
     p = _block_struct(blk)
     p.scores, p.dprobs, p.c2p, p.p2c = _ptr(s), _ptr(blk["dprobs"]), _ptr(blk["c2p"]), _ptr(blk["p2c"])
     p.lse, p.delta, p.probs, p.dscores = _ptr(blk["lse"]), _ptr(blk["delta"]), _ptr(probs), _ptr(dscores)
-    with torch.cuda.device(s.device):
-        _lib.check(_lib.load().fdb_attn_bwd_probs(C.byref(p), C.c_void_p(torch.cuda.current_stream(s.device).cuda_stream)))
+    with ops.on_device(s.device):
+        _lib.check(_lib.load().fdb_attn_bwd_probs(C.byref(p), C.c_void_p(ops.raw_stream(s.device))))
     _launches += 1
     return probs, dscores
 
@@ -106,8 +106,8 @@ def _stage_sums(blk: dict, dscores: torch.Tensor, want_c2p: bool, p2c_sums: Opti
         c2p_sums = torch.empty(dscores.shape[0], dscores.shape[1], blk["table_rows"], dtype=torch.float32, device=dscores.device)
     p = _block_struct(blk)
     p.dscores, p.c2p_sums, p.p2c_sums = _ptr(dscores), _ptr(c2p_sums), _ptr(p2c_sums)
-    with torch.cuda.device(dscores.device):
-        _lib.check(_lib.load().fdb_attn_bwd_bucket_sums(C.byref(p), C.c_void_p(torch.cuda.current_stream(dscores.device).cuda_stream)))
+    with ops.on_device(dscores.device):
+        _lib.check(_lib.load().fdb_attn_bwd_bucket_sums(C.byref(p), C.c_void_p(ops.raw_stream(dscores.device))))
     _launches += int(want_c2p) + int(p2c_sums is not None)
     return c2p_sums
 
@@ -220,14 +220,13 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
            max_relative_positions, grads=None, table_grads=(None, None)):
     """``grads`` (rows, 3, H, 64) and ``table_grads`` (each table's shape), when given, take the results."""
     global _launches
-    from . import ops
     dev, shape = q.device, q.shape
     lib = _lib.load()
-    with torch.cuda.device(dev):
+    with ops.on_device(dev):
         p, keep = ops._fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
                                    max_relative_positions, out.contiguous(), lse.contiguous())
-        d3, d_rs, d_hs = ops._rows_view(dout)
-        T, H = d3.shape[0], d3.shape[1]
+        d3, d_rs, d_hs, T = ops._rows_view(dout)
+        H = shape[-2]
         if grads is None:
             grads, row_stride = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)], H * 64
         else:
@@ -246,7 +245,7 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
         need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
         ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
         b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
-        _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(torch.cuda.current_stream(dev).cuda_stream)))
+        _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(ops.raw_stream(dev))))
         terms = int(pos_key is not None) + int(pos_query is not None)
         _launches += 4 + int(terms > 0) + 2 * terms
         del keep, ws

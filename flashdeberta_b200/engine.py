@@ -130,7 +130,7 @@ class _Plan:
             d.exp_key = ptr(self.tables[i, 0]) if self.c2p else None
             d.exp_query = ptr(self.tables[i, 1]) if self.p2c else None
         ffn = enc.layer[0].intermediate.dense.out_features
-        with torch.cuda.device(self.device):
+        with ops.on_device(self.device):
             rc = _lib.load().fdb_encoder_create(C.byref(descs), n, self.hidden, self.heads, ffn, C.byref(self.handle))
         self.ok = rc == _lib.FDB_OK
 
@@ -221,8 +221,8 @@ class EncoderEngine:
         out = torch.empty(*ids.shape, plan.hidden, dtype=torch.bfloat16, device=device)
         p.out = out.data_ptr()
         p.status = ops._status_word(device).data_ptr()
-        with torch.cuda.device(device):
-            stream = torch.cuda.current_stream(device).cuda_stream
+        with ops.on_device(device):
+            stream = ops.raw_stream(device)
             ops._launches += plan.refresh_tables(model.encoder, stream)
             if plan.tables is not None and stream != plan.table_stream:
                 torch.cuda.current_stream(device).wait_event(plan.table_event)

@@ -10,6 +10,7 @@ Where autograd records, the bf16 calls have a backward (backward.py); the refere
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes as C
 import math
 from typing import Dict, Optional, Tuple
@@ -81,15 +82,28 @@ def flag_status(device: torch.device, condition: torch.Tensor, bit: int) -> None
     _status_word(device).bitwise_or_(condition.to(torch.int32) * bit)
 
 
+_HERE = contextlib.nullcontext()
+
+
+def on_device(device: torch.device):
+    """``torch.cuda.device(device)``, for next to nothing where it is the current one."""
+    return _HERE if device.index in (None, torch.cuda.current_device()) else torch.cuda.device(device)
+
+
+def raw_stream(device: torch.device) -> int:
+    """Handle of the current stream of a device."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
 def lengths_from_mask(mask: torch.Tensor) -> torch.Tensor:
     """int32 lengths of the rows of a (batch, tokens) mask on the GPU, any strides; flags a mask that is not right-padded in
     the device status word."""
     global _launches
     lens = torch.empty(mask.shape[0], dtype=torch.int32, device=mask.device)
-    with torch.cuda.device(mask.device):
+    with on_device(mask.device):
         _lib.check(_lib.load().fdb_lengths_from_mask(
             mask.data_ptr(), MASK_TYPES[mask.dtype], mask.shape[0], mask.shape[1], mask.stride(0), mask.stride(1), lens.data_ptr(),
-            _status_word(mask.device).data_ptr(), torch.cuda.current_stream(mask.device).cuda_stream))
+            _status_word(mask.device).data_ptr(), raw_stream(mask.device)))
     _launches += 1
     return lens
 
@@ -100,11 +114,11 @@ def column_sums(x: torch.Tensor, more: Optional[torch.Tensor] = None) -> torch.T
     lib = _lib.load()
     out = torch.empty(x.shape[1], dtype=x.dtype, device=x.device)
     rows, cols = (0, 0) if more is None else more.shape
-    with torch.cuda.device(x.device):
+    with on_device(x.device):
         need = lib.fdb_column_sums_workspace_bytes(x.shape[0], rows, x.shape[1])
         ws = torch.empty(need, dtype=torch.uint8, device=x.device)
         _lib.check(lib.fdb_column_sums(x.data_ptr(), x.shape[0], x.shape[1], None if more is None else more.data_ptr(), rows, cols,
-                                       out.data_ptr(), ws.data_ptr(), need, torch.cuda.current_stream(x.device).cuda_stream))
+                                       out.data_ptr(), ws.data_ptr(), need, raw_stream(x.device)))
     _launches += 2
     return out
 
@@ -119,75 +133,75 @@ def _dtype_code(t: torch.Tensor) -> int:
     raise TypeError(f"unsupported dtype {t.dtype}")
 
 
-def _rows_view(x: torch.Tensor) -> Tuple[torch.Tensor, int, int]:
-    """(rows, H, D) view of a (rows, H, D) or (B, L, H, D) tensor without copying when the layout allows it.
-    Returns the view, its row stride and head stride in elements."""
-    if x.dim() == 4:
-        B, L, H, D = x.shape
-        if x.stride(0) != L * x.stride(1):
+def _rows_view(x: torch.Tensor) -> Tuple[torch.Tensor, int, int, int]:
+    """A (rows, H, D) or (B, L, H, D) tensor as rows, without copying when the layout allows it.  Returns the tensor (to be
+    kept alive), its row and head strides in elements and the number of rows."""
+    shape, stride = x.shape, x.stride()
+    if len(shape) == 4:
+        if stride[0] != shape[1] * stride[1] or stride[3] != 1:
             x = x.contiguous()
-        x = x.as_strided((B * L, H, D), (x.stride(1), x.stride(2), x.stride(3)), x.storage_offset())
-    if x.dim() != 3:
+            stride = x.stride()
+        return x, stride[1], stride[2], shape[0] * shape[1]
+    if len(shape) != 3:
         raise ValueError("expected (rows, heads, head_dim) or (batch, seq, heads, head_dim)")
-    if x.stride(2) != 1:
+    if stride[2] != 1:
         x = x.contiguous()
-    return x, x.stride(0), x.stride(1)
+        stride = x.stride()
+    return x, stride[0], stride[1], shape[0]
+
+
+def _int32(t: torch.Tensor) -> torch.Tensor:
+    return t if t.dtype == torch.int32 and t.is_contiguous() else t.to(torch.int32).contiguous()
 
 
 def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
                  max_relative_positions, out, lse, scales=None):
-    dev = q.device
-    q3, q_rs, q_hs = _rows_view(q)
-    k3, k_rs, k_hs = _rows_view(k)
-    v3, v_rs, v_hs = _rows_view(v)
-    rows, H, D = q3.shape
-    if k3.shape != q3.shape or v3.shape != q3.shape:
+    q3, q_rs, q_hs, rows = _rows_view(q)
+    k3, k_rs, k_hs, _ = _rows_view(k)
+    v3, v_rs, v_hs, _ = _rows_view(v)
+    shape = q.shape
+    H, D = shape[-2], shape[-1]
+    if k.shape != shape or v.shape != shape:
         raise ValueError("q, k and v must have the same shape")
-    p = _lib.AttnParams()
-    p.struct_bytes = C.sizeof(_lib.AttnParams)
-    p.dtype = _dtype_code(q3)
     keep = [q3, k3, v3]
-    p.q, p.k, p.v, p.out = q3.data_ptr(), k3.data_ptr(), v3.data_ptr(), out.data_ptr()
-    p.q_row_stride, p.q_head_stride = q_rs, q_hs
-    p.k_row_stride, p.k_head_stride = k_rs, k_hs
-    p.v_row_stride, p.v_head_stride = v_rs, v_hs
-    p.out_row_stride, p.out_head_stride = H * D, D
-    span = bucket.att_span(position_buckets, max_relative_positions)
-    for name, t in (("pos_key", pos_key), ("pos_query", pos_query)):
-        if t is None:
-            continue
-        if t.dim() == 4 and t.shape[0] == 1:
-            t = t[0]
-        if t.shape != (H, 2 * span, D):
-            raise ValueError(f"{name} must be (heads, 2*att_span, head_dim) = {(H, 2 * span, D)}, got {tuple(t.shape)}")
-        if t.dtype != q3.dtype:
-            raise TypeError(f"{name} dtype {t.dtype} differs from q dtype {q3.dtype}")
-        t = t.contiguous()
-        keep.append(t)
-        setattr(p, name, t.data_ptr())
+    tables = [None, None]
+    lut_ptr, d_min, lut_len = None, 0, 0
     if pos_key is not None or pos_query is not None:
-        lut, d_min = bucket.device_lut(position_buckets, max_relative_positions, dev)
-        p.bucket_lut, p.lut_d_min, p.lut_len = lut.data_ptr(), d_min, lut.numel()
+        want = (H, 2 * bucket.att_span(position_buckets, max_relative_positions), D)
+        for i, (name, t) in enumerate((("pos_key", pos_key), ("pos_query", pos_query))):
+            if t is None:
+                continue
+            if t.dim() == 4 and t.shape[0] == 1:
+                t = t[0]
+            if t.shape != want:
+                raise ValueError(f"{name} must be (heads, 2*att_span, head_dim) = {want}, got {tuple(t.shape)}")
+            if t.dtype != q.dtype:
+                raise TypeError(f"{name} dtype {t.dtype} differs from q dtype {q.dtype}")
+            if not t.is_contiguous():
+                t = t.contiguous()
+            keep.append(t)
+            tables[i] = t.data_ptr()
+        lut, d_min = bucket.device_lut(position_buckets, max_relative_positions, q.device)
+        lut_ptr, lut_len = lut.data_ptr(), lut.shape[0]
+    cu_ptr = lens_ptr = None
     if cu_seqlens is not None:
-        if cu_seqlens.dtype != torch.int32 or not cu_seqlens.is_contiguous():
-            cu_seqlens = cu_seqlens.to(torch.int32).contiguous()
+        cu_seqlens = _int32(cu_seqlens)
         keep.append(cu_seqlens)
-        p.cu_seqlens = cu_seqlens.data_ptr()
-        p.batch = cu_seqlens.numel() - 1
+        cu_ptr, batch = cu_seqlens.data_ptr(), cu_seqlens.numel() - 1
     else:
-        if q.dim() != 4:
+        if len(shape) != 4:
             raise ValueError("dense layout needs (batch, seq, heads, head_dim) inputs")
-        p.batch = q.shape[0]
-        if max_seqlen != q.shape[1]:
+        batch = shape[0]
+        if max_seqlen != shape[1]:
             raise ValueError("dense layout: max_seqlen must equal the padded length")
         if seq_lens is not None:
-            if seq_lens.dtype != torch.int32 or not seq_lens.is_contiguous():
-                seq_lens = seq_lens.to(torch.int32).contiguous()
+            seq_lens = _int32(seq_lens)
             keep.append(seq_lens)
-            p.seq_lens = seq_lens.data_ptr()
-    p.max_seqlen, p.total_rows, p.heads, p.head_dim = int(max_seqlen), rows, H, D
-    p.position_buckets, p.max_relative_positions = int(position_buckets), int(max_relative_positions)
-    p.sm_scale = float(sm_scale)
+            lens_ptr = seq_lens.data_ptr()
+    p = _lib.AttnParams(  # in the order of the fields
+        _PARAMS_BYTES, _dtype_code(q), q3.data_ptr(), k3.data_ptr(), v3.data_ptr(), out.data_ptr(), q_rs, q_hs, k_rs, k_hs, v_rs, v_hs,
+        H * D, D, tables[0], tables[1], cu_ptr, lens_ptr, batch, int(max_seqlen), rows, H, D, int(position_buckets),
+        int(max_relative_positions), lut_ptr, d_min, lut_len, float(sm_scale))
     if scales is not None:
         for name, t in scales.items():
             if t is not None:
@@ -196,8 +210,11 @@ def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, 
                 setattr(p, name, t.data_ptr())
     if lse is not None:
         p.lse = lse.data_ptr()
-    p.status = _status_word(dev).data_ptr()
+    p.status = _status_word(q.device).data_ptr()
     return p, keep
+
+
+_PARAMS_BYTES = C.sizeof(_lib.AttnParams)
 
 
 def _out_like(q: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
@@ -260,7 +277,7 @@ def disentangled_attention(
     out = _out_like(q, torch.bfloat16)
     rows = out.numel() // (out.shape[-1] * out.shape[-2])
     lse = torch.empty(rows, q.shape[-2], dtype=torch.float32, device=q.device) if return_lse else None
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         p, keep = _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale,
                                position_buckets, max_relative_positions, out, lse, scales)
         p.tune = int(tune)
@@ -268,7 +285,7 @@ def disentangled_attention(
         if need == 0:  # invalid parameters (raises with the library's message) or an empty batch
             _lib.check(lib.fdb_attn_fwd(C.byref(p), None))
             return (out, lse) if return_lse else out
-        stream = torch.cuda.current_stream(q.device).cuda_stream
+        stream = raw_stream(q.device)
         flags = 0
         if prepared is not None and need <= prepared.max_bytes and prepared.stream in (None, stream):
             prepared.stream = stream  # the buffer stays with the first stream that used it; other streams take scratch
@@ -367,10 +384,10 @@ def disentangled_attention_static(
     lib = _lib.load()
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(q.shape[-1] * (1 + int(pos_key is not None) + int(pos_query is not None)))
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         p, keep = _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale,
                                position_buckets, max_relative_positions, out, None)
-        stream = torch.cuda.current_stream(q.device).cuda_stream
+        stream = raw_stream(q.device)
         _lib.check(lib.fdb_attn_fwd_static(C.byref(p), C.c_void_p(stream)))
         _launches += 2 + int(pos_key is not None or pos_query is not None)
         del keep
@@ -395,10 +412,10 @@ def disentangled_attention_check(
     out = _out_like(q, q.dtype)
     rows = out.numel() // (out.shape[-1] * out.shape[-2])
     lse = torch.empty(rows, q.shape[-2], dtype=torch.float32, device=q.device) if return_lse else None
-    with torch.cuda.device(q.device):
+    with on_device(q.device):
         p, keep = _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale,
                                position_buckets, max_relative_positions, out, lse)
-        stream = torch.cuda.current_stream(q.device).cuda_stream
+        stream = raw_stream(q.device)
         _lib.check(lib.fdb_attn_fwd_check(C.byref(p), C.c_void_p(stream)))
         _launches += 1
     return (out, lse) if return_lse else out
@@ -413,8 +430,8 @@ def relative_index_matrix(len_q: int, len_k: int, position_buckets: int, max_rel
     device = torch.device(device)
     lut, d_min = bucket.device_lut(position_buckets, max_relative_positions, device)
     out = torch.empty(len_q, len_k, dtype=torch.int32, device=device)
-    with torch.cuda.device(device):
-        stream = torch.cuda.current_stream(device).cuda_stream
+    with on_device(device):
+        stream = raw_stream(device)
         _lib.check(lib.fdb_relative_index_matrix(lut.data_ptr(), d_min, lut.numel(), len_q, len_k, out.data_ptr(),
                                                  C.c_void_p(stream)))
         _launches += 1
@@ -426,14 +443,14 @@ def quantize_e4m3(x: torch.Tensor, slab_start: torch.Tensor) -> Tuple[torch.Tens
     (slab, head); slab s = rows [slab_start[s], slab_start[s+1])."""
     global _launches
     lib = _lib.load()
-    x3, rs, hs = _rows_view(x)
-    rows, H, D = x3.shape
+    x3, rs, hs, rows = _rows_view(x)
+    H, D = x.shape[-2:]
     slab_start = slab_start.to(torch.int32).contiguous()
     n = slab_start.numel() - 1
     y = torch.empty(rows, H, D, dtype=torch.float8_e4m3fn, device=x.device)
     scale = torch.empty(n, H, dtype=torch.float32, device=x.device)
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+    with on_device(x.device):
+        stream = raw_stream(x.device)
         _lib.check(lib.fdb_quantize_e4m3(x3.data_ptr(), rows, rs, hs, slab_start.data_ptr(), n, H, D, y.data_ptr(),
                                          scale.data_ptr(), C.c_void_p(stream)))
         _launches += 1
@@ -469,8 +486,8 @@ def add_layernorm(x: torch.Tensor, residual: Optional[torch.Tensor], weight: tor
     out = torch.empty_like(x2)
     if x2.shape[0] == 0:
         return out.view(x.shape)
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+    with on_device(x.device):
+        stream = raw_stream(x.device)
         _lib.check(lib.fdb_add_layernorm(x2.data_ptr(), r2.data_ptr() if r2 is not None else None,
                                          weight.contiguous().data_ptr(), bias.contiguous().data_ptr(), out.data_ptr(),
                                          x2.shape[0], hidden, float(eps), C.c_void_p(stream)))
@@ -499,8 +516,8 @@ def embed_layernorm(ids: torch.Tensor, table: torch.Tensor, weight: torch.Tensor
     out = torch.empty(ids1.numel(), hidden, dtype=torch.bfloat16, device=table.device)
     if ids1.numel() == 0:
         return out.view(*ids.shape, hidden)
-    with torch.cuda.device(table.device):
-        stream = torch.cuda.current_stream(table.device).cuda_stream
+    with on_device(table.device):
+        stream = raw_stream(table.device)
         _lib.check(lib.fdb_embed_layernorm(ids1.data_ptr(), table.data_ptr(), table.shape[0],
                                            weight.contiguous().data_ptr(), bias.contiguous().data_ptr(),
                                            scale1.data_ptr() if scale1 is not None else None, out.data_ptr(),
@@ -533,8 +550,8 @@ def linear_gelu(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tens
     out = torch.empty(x2.shape[0], n, dtype=torch.bfloat16, device=x.device)
     if x2.shape[0] == 0:
         return out.view(*x.shape[:-1], n)
-    with torch.cuda.device(x.device):
-        stream = torch.cuda.current_stream(x.device).cuda_stream
+    with on_device(x.device):
+        stream = raw_stream(x.device)
         _lib.check(lib.fdb_linear_gelu(x2.data_ptr(), weight.data_ptr(), bias.data_ptr() if bias is not None else None,
                                        out.data_ptr(), x2.shape[0], k, n, _status_word(x.device).data_ptr(),
                                        C.c_void_p(stream)))
