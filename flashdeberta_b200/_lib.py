@@ -45,13 +45,21 @@ class AttnParams(C.Structure):
     ]
 
 
+class QuantizeAttnParams(C.Structure):
+    """Mirror of ``fdb_quantize_attn_params``."""
+
+    _fields_ = [("struct_bytes", C.c_uint32), ("reserved", C.c_int32), ("input", C.POINTER(AttnParams))] + [(n, C.c_void_p) for n in (
+        "q", "k", "v", "pos_key", "pos_query", "q_scale", "k_scale", "v_scale", "pos_key_scale", "pos_query_scale", "amax")] + [
+        ("amax_bytes", C.c_uint64)]
+
+
 EXPORTS = (
     "fdb_abi_version", "fdb_last_error", "fdb_status_string", "fdb_build_bucket_lut", "fdb_relative_index",
     "fdb_attn_workspace_bytes", "fdb_attn_fwd", "fdb_attn_fwd_static", "fdb_attn_fwd_check", "fdb_relative_index_matrix",
     "fdb_quantize_e4m3", "fdb_add_layernorm", "fdb_linear_gelu", "fdb_embed_layernorm",
     "fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums", "fdb_expanded_rows", "fdb_expand_tables", "fdb_encoder_create",
     "fdb_encoder_destroy", "fdb_encoder_workspace_bytes", "fdb_encoder_forward", "fdb_attn_bwd_workspace_bytes", "fdb_attn_bwd",
-    "fdb_lengths_from_mask", "fdb_column_sums_workspace_bytes", "fdb_column_sums",
+    "fdb_lengths_from_mask", "fdb_column_sums_workspace_bytes", "fdb_column_sums", "fdb_quantize_attn",
 )
 
 _lib = None
@@ -96,6 +104,8 @@ def load() -> C.CDLL:
     lib.fdb_quantize_e4m3.restype = C.c_int
     lib.fdb_quantize_e4m3.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
                                       C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.fdb_quantize_attn.restype = C.c_int
+    lib.fdb_quantize_attn.argtypes = [C.c_void_p, C.c_void_p]
     lib.fdb_add_layernorm.restype = C.c_int
     lib.fdb_add_layernorm.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int32,
                                       C.c_float, C.c_void_p]

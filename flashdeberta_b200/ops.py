@@ -338,28 +338,36 @@ def disentangled_attention_fp8(
     reference.  Returns bf16."""
     if wants_grad(q, k, v, pos_key, pos_query):
         raise RuntimeError("the e4m3 attention is forward-only; train with attn_fp8 off")
-    if q.dim() == 4:
-        B, L = q.shape[0], q.shape[1]
-        slabs = torch.arange(0, (B + 1) * L, L, dtype=torch.int32, device=q.device)
-    else:
-        if cu_seqlens is None:
-            raise ValueError("packed inputs need cu_seqlens")
-        slabs = cu_seqlens.to(torch.int32)
-    q8, sq = quantize_e4m3(q, slabs)
-    k8, sk = quantize_e4m3(k, slabs)
-    v8, sv = quantize_e4m3(v, slabs)
-    scales = {"q_scale": sq, "k_scale": sk, "v_scale": sv}
-    tabs = {}
-    for name, t in (("pos_key", pos_key), ("pos_query", pos_query)):
-        if t is None:
-            tabs[name] = None
-            continue
-        H, R, D = t.shape
-        rows = t.contiguous().view(H * R, 1, D)
-        y, sc = quantize_e4m3(rows, torch.arange(0, (H + 1) * R, R, dtype=torch.int32, device=t.device))
-        tabs[name] = y.view(H, R, D)
-        scales[name + "_scale"] = sc.view(H)
-    return disentangled_attention(q8, k8, v8, tabs["pos_key"], tabs["pos_query"], cu_seqlens=cu_seqlens,
+    if q.dim() != 4 and cu_seqlens is None:
+        raise ValueError("packed inputs need cu_seqlens")
+    if not q.is_cuda:
+        raise RuntimeError("flashdeberta_b200 runs on CUDA devices only; there is no CPU path")
+    global _launches
+    if sm_scale is None:
+        sm_scale = 1.0 / math.sqrt(q.shape[-1] * (1 + int(pos_key is not None) + int(pos_query is not None)))
+    if cu_seqlens is not None:
+        cu_seqlens = _int32(cu_seqlens)
+    lib, dev, H = _lib.load(), q.device, q.shape[-2]
+    given = {"q": q, "k": k, "v": v, "pos_key": pos_key, "pos_query": pos_query}
+    p, keep = _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_relative_positions, q, None)
+    quant = _lib.QuantizeAttnParams()
+    quant.struct_bytes, quant.input = C.sizeof(_lib.QuantizeAttnParams), C.pointer(p)
+    sizes = {n: H if n.startswith("pos") else p.batch * H for n, t in given.items() if t is not None}
+    total = sum(sizes.values())
+    scale = torch.empty(2 * total, dtype=torch.float32, device=dev)  # scales, then the maxima they come from
+    low, scales, at = {"pos_key": None, "pos_query": None}, {}, 0
+    for name, n in sizes.items():
+        low[name] = torch.empty(given[name].shape, dtype=torch.float8_e4m3fn, device=dev)
+        scales[name + "_scale"] = scale[at:at + n]
+        setattr(quant, name, low[name].data_ptr())
+        setattr(quant, name + "_scale", scale.data_ptr() + 4 * at)
+        at += n
+    quant.amax, quant.amax_bytes = scale.data_ptr() + 4 * total, 4 * total
+    with on_device(dev):
+        _lib.check(lib.fdb_quantize_attn(C.byref(quant), C.c_void_p(raw_stream(dev))))
+        _launches += 2
+    del keep
+    return disentangled_attention(low["q"], low["k"], low["v"], low["pos_key"], low["pos_query"], cu_seqlens=cu_seqlens,
                                   seq_lens=seq_lens, max_seqlen=max_seqlen, sm_scale=sm_scale,
                                   position_buckets=position_buckets, max_relative_positions=max_relative_positions,
                                   scales=scales)

@@ -302,6 +302,21 @@ FDB_API int fdb_quantize_e4m3(const void* x_bf16, int64_t rows, int64_t row_stri
                       const int32_t* slab_start, int32_t n_slabs, int32_t heads, int32_t head_dim, void* y_e4m3,
                       float* scale, void* stream);
 
+/* The same for everything that one attention call reads, in two launches: q, k, v per (sequence, head) (dense sequences with
+ * their padding) and the position tables per head. */
+typedef struct fdb_quantize_attn_params {
+  uint32_t struct_bytes;       /* sizeof(fdb_quantize_attn_params) */
+  int32_t reserved;
+  const fdb_attn_params* in;   /* the call in bf16: tensors, strides and layout are looked at */
+  void *q, *k, *v;             /* out, e4m3, contiguous (total_rows, heads, 64) */
+  void *pos_key, *pos_query;   /* out, e4m3 (heads, 2*att_span, 64), each with its table */
+  float *q_scale, *k_scale, *v_scale;          /* out (batch, heads) */
+  float *pos_key_scale, *pos_query_scale;      /* out (heads) */
+  void* amax;                  /* device scratch: 4 bytes for every scale, 16-byte aligned */
+  uint64_t amax_bytes;
+} fdb_quantize_attn_params;
+FDB_API int fdb_quantize_attn(const fdb_quantize_attn_params* p, void* stream);
+
 /*
  * out = LayerNorm(x + residual) over the last dimension (eps inside the square root), bf16 in and out, fp32 statistics; the
  * sum is rounded to bf16 first, as the eager expression does.  Replaces the tail of both output blocks of a layer, which
