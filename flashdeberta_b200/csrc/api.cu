@@ -140,8 +140,9 @@ int fdb_attn_fwd(const fdb_attn_params* p, void* stream) {
                 (unsigned long long)(p->workspace ? p->workspace_bytes : 0));
   if ((reinterpret_cast<uintptr_t>(p->workspace) & 255u) != 0) return fail(FDB_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
   const AttnBuffers b = attn_buffers(*p, w);
-  if ((rc = launch_prepare(*p, g, b, stream)) != FDB_OK) return rc;
-  return launch_attn_fwd_sm100(*p, g, b, stream);
+  bool prepared;
+  if ((rc = launch_prepare(*p, g, b, stream, &prepared)) != FDB_OK) return rc;
+  return launch_attn_fwd_sm100(*p, g, b, stream, prepared);
 }
 
 int fdb_attn_fwd_check(const fdb_attn_params* p, void* stream) {

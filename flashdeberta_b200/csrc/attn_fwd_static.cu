@@ -71,6 +71,7 @@ extern "C" FDB_API int fdb_attn_fwd_static(const fdb_attn_params* p, void* strea
   // Nothing in the scratch has to start at zero: seq_info_kernel and expand_tables_kernel write every entry the fused
   // kernel reads, on this stream, before it runs.
   const AttnBuffers b = attn_buffers(q, w);
-  if ((rc = launch_prepare(q, g, b, stream)) != FDB_OK) return rc;
-  return launch_attn_fwd_sm100(q, g, b, stream);
+  bool prepared;
+  if ((rc = launch_prepare(q, g, b, stream, &prepared)) != FDB_OK) return rc;
+  return launch_attn_fwd_sm100(q, g, b, stream, prepared);
 }
