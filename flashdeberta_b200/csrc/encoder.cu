@@ -14,6 +14,7 @@
 #include <new>
 #include <vector>
 
+#include "encoder_small.h"
 #include "internal.h"
 #include "linear.h"
 #include "sm100_ptx.cuh"
@@ -134,7 +135,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(const void* mask, in
 }
 
 struct Layout {  // byte offsets into the workspace
-  uint64_t counts, index, cu, rows, attn, x, h, qkv, ctx, proj, mid, total;
+  uint64_t counts, index, cu, rows, barrier, attn, x, h, qkv, ctx, proj, mid, total;
   WorkspaceLayout attn_layout;
 };
 
@@ -164,6 +165,12 @@ fdb_attn_params attn_params(const fdb_encoder_call& c, const EncoderPlan& plan) 
   return p;
 }
 
+SmallLayer small_layer(const fdb_encoder_layer& d) {
+  auto p = [](const void* x) { return static_cast<const __nv_bfloat16*>(x); };
+  return {p(d.wq), p(d.bq), p(d.wk), p(d.bk), p(d.wv), p(d.bv), p(d.wo), p(d.bo), p(d.ln1_gamma), p(d.ln1_beta), p(d.wi), p(d.bi),
+          p(d.wd), p(d.bd), p(d.ln2_gamma), p(d.ln2_beta), p(d.exp_key), p(d.exp_query), d.ln1_eps, d.ln2_eps};
+}
+
 Layout layout_of(const fdb_encoder_call& c, const EncoderPlan& plan, const fdb_attn_params& p) {
   Layout l;
   const uint64_t rows = (uint64_t)c.total_rows, h = (uint64_t)plan.hidden * 2;
@@ -173,6 +180,7 @@ Layout layout_of(const fdb_encoder_call& c, const EncoderPlan& plan, const fdb_a
   l.index = off;  off = align256(off + (c.mask ? rows * 4 : 0));
   l.cu = off;     off = align256(off + (uint64_t)(c.batch + 1) * 4);
   l.rows = off;   off = align256(off + 4);
+  l.barrier = off; off = align256(off + 8);
   fdb_attn_params q = p;
   q.pos_key = q.pos_query = nullptr;  // no room for gathered tables: they are the plan's
   ExpandGeometry none = {0, 0, 0, 0};
@@ -296,6 +304,12 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
   char* ws = static_cast<char*>(c->workspace);
   const int64_t rows = c->total_rows;
   int launches = 0;
+  // Up to 64 rows the layers are one kernel.  (Timing events around the attention of every layer need launches of their own.)
+  const bool small = c->attn_events == nullptr && small_encoder_covers(rows, plan.hidden, plan.ffn, (int)plan.layers.size());
+  if (small) {
+    const cudaError_t e = cudaMemsetAsync(ws + l.barrier, 0, 8, s);
+    if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "encoder memset: %s", cudaGetErrorString(e));
+  }
 
   // ---- which rows there are -------------------------------------------------------------------------------------------
   const int32_t *index = nullptr, *rows_dev = nullptr;
@@ -319,8 +333,10 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
   }
   p.workspace = ws + l.attn;
   AttnBuffers b = attn_buffers(p, l.attn_layout);
-  if ((rc = launch_seq_info(p, b, stream)) != FDB_OK) return rc;
-  ++launches;
+  if (!small) {
+    if ((rc = launch_seq_info(p, b, stream)) != FDB_OK) return rc;
+    ++launches;
+  }
 
   // ---- embedding stage --------------------------------------------------------------------------------------------------
   LayerNormCall ln = {};
@@ -332,6 +348,25 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
   if (rows_dev != nullptr) ln.zero_tail = ws + l.qkv + 2 * (uint64_t)rows * plan.hidden * 2;
   if ((rc = launch_layernorm(ln, stream)) != FDB_OK) return rc;
   ++launches;
+
+  if (small) {
+    SmallEncoderArgs a;
+    a.n_layers = (int)plan.layers.size();
+    for (int i = 0; i < a.n_layers; ++i) a.layer[i] = small_layer(plan.layers[i].d);
+    a.hidden = plan.hidden; a.ffn = plan.ffn;
+    a.row_bound = (int)rows; a.rows_dev = rows_dev;
+    a.cu_seqlens = p.cu_seqlens; a.batch = c->batch; a.max_seqlen = c->max_seqlen;
+    a.xrows = g.rows; a.d_first = g.d_first;
+    a.sm_scale = c->sm_scale;
+    auto at = [&](uint64_t offset) { return reinterpret_cast<__nv_bfloat16*>(ws + offset); };
+    a.x = at(l.x); a.qkv = at(l.qkv); a.ctx = at(l.ctx); a.y = at(l.proj); a.mid = at(l.mid);
+    a.out = static_cast<__nv_bfloat16*>(c->out); a.out_index = index;
+    a.barrier = reinterpret_cast<uint32_t*>(ws + l.barrier);
+    a.status = c->status;
+    if ((rc = launch_small_encoder(a, stream)) != FDB_OK) return rc;
+    c->launches = launches + 1;
+    return FDB_OK;
+  }
 
   // ---- layers -------------------------------------------------------------------------------------------------------------
   CUtensorMap map_x, map_ctx, map_h, map_mid;

@@ -1,0 +1,440 @@
+// The whole encoder stack in one kernel for a handful of tokens (a query, a short sentence): at most 64 rows.
+//
+// At that size a layer's seven launches are all latency: 4 to 10 us each for a microsecond of work, one behind the other.  Here one
+// CTA per SM stays for the whole forward and the steps of a layer are separated by grid barriers:
+//   1  LayerNorm of the layer before -> shared memory; query, key and value projections
+//   2  attention, a warp per (row, head), on the CUDA cores
+//   3  output projection, + residual
+//   4  LayerNorm -> shared memory; first feed-forward product, GELU
+//   5  second feed-forward product, + residual
+// Every CTA normalises all rows for itself (the next product needs them all) and keeps them, so the residuals of steps 3 and 5 come from
+// shared memory too.  A product's columns are dealt over the CTAs in tiles of 8, its K over the warps; the warps' partial sums
+// meet in shared memory.  What bounds a step is latency (barrier, one trip to L2 for the rows, one for the weights, which are
+// fetched to L2 ahead of the barrier): with 16 to 64 rows there is nothing to fill tcgen05 tiles of 128 rows with, and fragments
+// that go from memory to registers save the trip through shared memory and tensor memory, so the products are warp MMAs.  Both
+// operands are read 32 bytes per thread: K is permuted the same way in both, which a sum over K does not see.
+//
+// 12 layers of 768, 29 tokens: @@
+#include <cuda_bf16.h>
+#include <cuda_runtime.h>
+
+#include <algorithm>
+
+#include "encoder_small.h"
+#include "gelu.cuh"
+#include "internal.h"
+#include "launch.h"
+#include "sm100_ptx.cuh"
+
+namespace fdb {
+namespace {
+
+constexpr int kThreads = 512, kWarps = kThreads / 32;
+constexpr int kMaxTiles = 4;  // 8-column tiles of one product per CTA
+
+struct Ctx {
+  const SmallEncoderArgs* a;
+  uint8_t* s_x;        // rows of hidden bf16 + 16 bytes: with 32 bytes per thread, eight threads read all banks
+  float* s_red;
+  int rows, pitch, tid, warp, lane;
+};
+
+__device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+__device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+__device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+
+// All CTAs' writes before it are visible after it.  Bounded: after about two seconds of SM clock, or once another CTA has given up,
+// every CTA returns.
+__device__ __forceinline__ bool grid_barrier(const SmallEncoderArgs& a, uint32_t* s_ok, uint32_t target) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    uint32_t ok = 1;
+    __threadfence();
+    atomicAdd(a.barrier, 1u);
+    const long long t0 = clock64();
+    uint32_t seen = 0;
+    for (uint32_t i = 0; i < (1u << 30); ++i) {
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.barrier) : "memory");
+      if (seen >= target) break;
+      if ((i & 63u) == 63u && (clock64() - t0 > 4000000000LL || *reinterpret_cast<volatile uint32_t*>(a.barrier + 1) != 0u)) break;
+    }
+    if (seen < target) {
+      ok = 0;
+      atomicExch(a.barrier + 1, 1u);
+      if (a.status != nullptr) atomicOr(reinterpret_cast<unsigned int*>(a.status), FDB_DEV_TIMEOUT);
+    }
+    *s_ok = ok;
+  }
+  __syncthreads();
+  return *s_ok != 0;
+}
+
+// One product out[rows][n] = x . w^T over K = k; this CTA's tiles of 8 columns are [tile0, tile0 + tiles).
+struct Product {
+  const __nv_bfloat16 *w0, *w1, *w2;   // (group columns, k) each; group g holds columns g * group_cols ...
+  const __nv_bfloat16 *b0, *b1, *b2;
+  int group_cols, k, tile0, tiles;
+};
+
+__device__ __forceinline__ Product make_product(const Ctx& c, const __nv_bfloat16* w0, const __nv_bfloat16* w1, const __nv_bfloat16* w2,
+                                                const __nv_bfloat16* b0, const __nv_bfloat16* b1, const __nv_bfloat16* b2, int group_cols,
+                                                int groups, int k) {
+  Product p = {w0, w1, w2, b0, b1, b2, group_cols, k, 0, 0};
+  const int all = group_cols * groups / 8, per = (all + (int)gridDim.x - 1) / (int)gridDim.x;
+  p.tile0 = blockIdx.x * per;
+  p.tiles = max(0, min(per, all - p.tile0));
+  return p;
+}
+__device__ __forceinline__ const __nv_bfloat16* weight_row(const Product& p, int tile, int r) {
+  const int col = tile * 8, g = col / p.group_cols;
+  return (g == 0 ? p.w0 : (g == 1 ? p.w1 : p.w2)) + (int64_t)(col - g * p.group_cols + r) * p.k;
+}
+// the CTA's weights of a coming product to L2
+__device__ __forceinline__ void prefetch(const Ctx& c, const Product& p) {
+  const int lines = p.k / 64;
+  for (int i = c.tid; i < p.tiles * 8 * lines; i += kThreads) {
+    const int row = i / lines;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(weight_row(p, p.tile0 + (row >> 3), row & 7) + (i - row * lines) * 64));
+  }
+}
+
+// Partial sums of the warps over their share of K, then `store(row, column, v0, v1)` for pairs of columns with the bias added.  The
+// rows come from shared memory (src == NULL) or from memory.
+template <int MT, int NT, typename Store>
+__device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, const __nv_bfloat16* src, int split, Store&& store) {
+  const int g = c.lane >> 2, t = c.lane & 3;
+  const int kgs = kWarps / split, kg = c.warp % kgs, tile = (c.warp / kgs) * NT;  // split: the tiles are dealt to this many sets of warps
+  const int cols = p.tiles * 8, blocks = p.k / 64;
+  float acc[MT][NT][4];
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
+  // of each 64 of K, thread t of a fragment's row has the 16 values from 16 t on: four steps of the MMA
+  const __nv_bfloat16* w[NT];
+#pragma unroll
+  for (int n = 0; n < NT; ++n) w[n] = weight_row(p, p.tile0 + min(tile + n, p.tiles - 1), g) + t * 16;
+#pragma unroll(MT <= 2 ? 3 : 1)
+  for (int b = kg; b < blocks; b += kgs) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint4 x[MT][2], y[NT];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) y[n] = __ldg(reinterpret_cast<const uint4*>(w[n] + b * 64) + u);
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int row = m * 16 + h * 8 + g, at = b * 64 + t * 16 + u * 8;
+          if (src == nullptr) x[m][h] = *reinterpret_cast<const uint4*>(c.s_x + row * c.pitch + at * 2);
+          else x[m][h] = row < c.rows ? __ldcg(reinterpret_cast<const uint4*>(src + (int64_t)row * p.k + at)) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+      for (int m = 0; m < MT; ++m)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) {
+          mma16816(acc[m][n], x[m][0].x, x[m][1].x, x[m][0].y, x[m][1].y, y[n].x, y[n].y);
+          mma16816(acc[m][n], x[m][0].z, x[m][1].z, x[m][0].w, x[m][1].w, y[n].z, y[n].w);
+        }
+    }
+  }
+#pragma unroll
+  for (int m = 0; m < MT; ++m)
+#pragma unroll
+    for (int n = 0; n < NT; ++n)
+      if (tile + n < p.tiles) {
+        float* at = c.s_red + ((int64_t)(kg * MT * 16 + m * 16 + g)) * cols + (tile + n) * 8 + 2 * t;
+        *reinterpret_cast<float2*>(at) = make_float2(acc[m][n][0], acc[m][n][1]);
+        *reinterpret_cast<float2*>(at + 8 * cols) = make_float2(acc[m][n][2], acc[m][n][3]);
+      }
+  __syncthreads();
+  for (int i = c.tid; i < c.rows * (cols / 2); i += kThreads) {
+    const int row = i / (cols / 2), cp = (i - row * (cols / 2)) * 2;
+    float2 s = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int k = 0; k < kgs; ++k) {
+      const float2 v = *reinterpret_cast<const float2*>(c.s_red + (int64_t)(k * MT * 16 + row) * cols + cp);
+      s.x += v.x;
+      s.y += v.y;
+    }
+    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols, in = col - grp * p.group_cols;
+    const __nv_bfloat16* bias = grp == 0 ? p.b0 : (grp == 1 ? p.b1 : p.b2);
+    if (bias != nullptr) {
+      const uint32_t b = *reinterpret_cast<const uint32_t*>(bias + in);
+      s.x += lo(b);
+      s.y += hi(b);
+    }
+    store(row, grp, in, round_bf16(s.x), round_bf16(s.y));
+  }
+}
+
+template <int MT, typename Store>
+__device__ __forceinline__ void product(const Ctx& c, const Product& p, const __nv_bfloat16* src, Store&& store) {
+  if (p.tiles == 0) return;  // (uniform over the CTA)
+  if (p.tiles == 1) product_tiles<MT, 1>(c, p, src, 1, store);
+  else if (p.tiles == 2) product_tiles<MT, 2>(c, p, src, 1, store);
+  else if (p.tiles == 3) product_tiles<MT, 3>(c, p, src, 1, store);
+  else product_tiles<MT, 2>(c, p, src, 2, store);  // (four: the partial sums of 16 warps would not fit)
+}
+
+// LayerNorm of the rows of `y`, a warp per row (the arithmetic of add_layernorm.cu); gamma == NULL: the rows as they are
+template <typename Out>
+__device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, float eps,
+                                          int first, int step, Out&& out) {
+  const int vec = c.a->hidden / 256;
+  for (int row = first; row < c.rows; row += step) {
+    uint4 raw[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      raw[i] = i < vec ? __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)row * c.a->hidden) + i * 32 + c.lane) : make_uint4(0, 0, 0, 0);
+    if (gamma != nullptr) {
+      float sum = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { sum += lo(w[k]); sum += hi(w[k]); }
+      }
+      const float inv = 1.f / (float)c.a->hidden, mean = warp_sum(sum) * inv;
+      float sq = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < vec) {
+          const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            const float d0 = lo(w[k]) - mean, d1 = hi(w[k]) - mean;
+            sq = fmaf(d0, d0, sq);
+            sq = fmaf(d1, d1, sq);
+          }
+        }
+      const float rstd = rsqrtf(warp_sum(sq) * inv + eps);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < vec) {
+          const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma) + i * 32 + c.lane), bv = __ldg(reinterpret_cast<const uint4*>(beta) + i * 32 + c.lane);
+          const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
+          uint32_t o[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k)
+            o[k] = ptx::pack_bf16x2(fmaf((lo(w[k]) - mean) * rstd, lo(gw[k]), lo(bw[k])), fmaf((hi(w[k]) - mean) * rstd, hi(gw[k]), hi(bw[k])));
+          raw[i] = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (i < vec) out(row, i * 32 + c.lane, raw[i]);
+  }
+}
+
+// softmax((q.k + c2p + p2c) * scale) v of one row and head by a warp: lanes are keys for the scores, pairs of features for the output
+__device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l, int row, int head, int start, int len) {
+  const SmallEncoderArgs& a = *c.a;
+  const int64_t hd = (int64_t)head * 64;
+  uint32_t* out = reinterpret_cast<uint32_t*>(a.ctx + (int64_t)row * a.hidden + hd) + c.lane;
+  if (len == 0) {  // a row of no sequence
+    *out = 0u;
+    return;
+  }
+  const int64_t plane = (int64_t)a.row_bound * a.hidden;
+  const __nv_bfloat16 *q = a.qkv, *k = a.qkv + plane, *v = a.qkv + 2 * plane;
+  const uint4* qr = reinterpret_cast<const uint4*>(q + (int64_t)row * a.hidden + hd);
+  const int m = row - start;
+  float s[2];
+#pragma unroll
+  for (int ch = 0; ch < 2; ++ch) {
+    s[ch] = -INFINITY;
+    if (ch * 32 >= len) continue;
+    const int n = min(ch * 32 + c.lane, len - 1);
+    const uint4* kr = reinterpret_cast<const uint4*>(k + (int64_t)(start + n) * a.hidden + hd);
+    const int64_t at = ((int64_t)head * a.xrows + (m - n - a.d_first)) * 64;
+    const uint4* xk = reinterpret_cast<const uint4*>(l.exp_key + at);
+    const uint4* xq = reinterpret_cast<const uint4*>(l.exp_query + at);
+    float sum = 0.f;
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      uint4 qv[4], kv[4], kp[4], qp[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        qv[i] = __ldcg(qr + half * 4 + i);
+        kv[i] = __ldcg(kr + half * 4 + i);
+        kp[i] = l.exp_key != nullptr ? __ldg(xk + half * 4 + i) : make_uint4(0, 0, 0, 0);
+        qp[i] = l.exp_query != nullptr ? __ldg(xq + half * 4 + i) : make_uint4(0, 0, 0, 0);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t qw[4] = {qv[i].x, qv[i].y, qv[i].z, qv[i].w}, kw[4] = {kv[i].x, kv[i].y, kv[i].z, kv[i].w};
+        const uint32_t pw[4] = {kp[i].x, kp[i].y, kp[i].z, kp[i].w}, rw[4] = {qp[i].x, qp[i].y, qp[i].z, qp[i].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          sum = fmaf(lo(qw[e]), lo(kw[e]) + lo(pw[e]), fmaf(lo(kw[e]), lo(rw[e]), sum));
+          sum = fmaf(hi(qw[e]), hi(kw[e]) + hi(pw[e]), fmaf(hi(kw[e]), hi(rw[e]), sum));
+        }
+      }
+    }
+    if (ch * 32 + c.lane < len) s[ch] = sum * (a.sm_scale * 1.4426950408889634f);
+  }
+  float top = fmaxf(s[0], s[1]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  const float p0 = ptx::ex2(s[0] - top), p1 = ptx::ex2(s[1] - top);
+  const float inv = 1.f / warp_sum(p0 + p1);
+  float o0 = 0.f, o1 = 0.f;
+  const uint32_t* vr = reinterpret_cast<const uint32_t*>(v + (int64_t)start * a.hidden + hd) + c.lane;
+  for (int n0 = 0; n0 < len; n0 += 8) {
+    uint32_t w[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = n0 + i < len ? __ldcg(vr + (int64_t)(n0 + i) * (a.hidden / 2)) : 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int n = n0 + i;  // keys behind the sequence have probability zero
+      const float pn = __shfl_sync(0xffffffffu, n < 32 ? p0 : p1, n & 31);
+      o0 = fmaf(pn, lo(w[i]), o0);
+      o1 = fmaf(pn, hi(w[i]), o1);
+    }
+  }
+  *out = ptx::pack_bf16x2(o0 * inv, o1 * inv);
+}
+
+template <int MT>
+__global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid_constant__ SmallEncoderArgs args) {
+  extern __shared__ __align__(16) uint8_t smem[];
+  __shared__ int s_start[kSmallRows], s_len[kSmallRows];
+  __shared__ uint32_t s_ok;
+  Ctx c;
+  c.a = &args;
+  c.tid = threadIdx.x; c.warp = threadIdx.x >> 5; c.lane = threadIdx.x & 31;
+  c.rows = args.rows_dev != nullptr ? min(*args.rows_dev, args.row_bound) : args.row_bound;
+  c.pitch = args.hidden * 2 + 16;
+  c.s_x = smem;
+  c.s_red = reinterpret_cast<float*>(smem + MT * 16 * c.pitch);
+
+  // the sequence of every row
+  for (int i = c.tid; i < kSmallRows; i += kThreads) s_start[i] = s_len[i] = 0;
+  for (int i = c.tid; i < (MT * 16 - c.rows) * (c.pitch / 16); i += kThreads)  // rows of the tiles behind the last one
+    reinterpret_cast<uint4*>(c.s_x + c.rows * c.pitch)[i] = make_uint4(0, 0, 0, 0);
+  __syncthreads();
+  for (int b = c.tid; b < args.batch; b += kThreads) {
+    int start = b * args.max_seqlen, end = start + args.max_seqlen;
+    if (args.cu_seqlens != nullptr) {
+      start = args.cu_seqlens[b];
+      end = args.cu_seqlens[b + 1];
+      if (start < 0 || end < start || end - start > args.max_seqlen || end > args.row_bound) {
+        if (blockIdx.x == 0 && args.status != nullptr) atomicOr(reinterpret_cast<unsigned int*>(args.status), FDB_DEV_BAD_SEQLEN);
+        continue;
+      }
+    }
+    for (int r = start; r < min(end, c.rows); ++r) { s_start[r] = start; s_len[r] = end - start; }
+  }
+  __syncthreads();
+
+  const int hidden = args.hidden, heads = hidden / 64;
+  uint32_t barriers = 0;
+  auto sync_grid = [&]() -> bool { return grid_barrier(args, &s_ok, ++barriers * gridDim.x); };
+  auto keep = [&](int row, int i, uint4 v) { *reinterpret_cast<uint4*>(c.s_x + row * c.pitch + i * 16) = v; };
+  auto residual = [&](int row, int col) -> uint32_t { return *reinterpret_cast<const uint32_t*>(c.s_x + row * c.pitch + col * 2); };
+  auto add_to = [&](__nv_bfloat16* y) {
+    return [=](int row, int, int col, float v0, float v1) {
+      const uint32_t r = residual(row, col);
+      *reinterpret_cast<uint32_t*>(y + (int64_t)row * hidden + col) = ptx::pack_bf16x2(v0 + lo(r), v1 + hi(r));
+    };
+  };
+
+  for (int i = 0; i < args.n_layers; ++i) {
+    const SmallLayer& l = args.layer[i];
+    const Product qkv = make_product(c, l.wq, l.wk, l.wv, l.bq, l.bk, l.bv, hidden, 3, hidden);
+    const Product proj = make_product(c, l.wo, nullptr, nullptr, l.bo, nullptr, nullptr, hidden, 1, hidden);
+    const Product up = make_product(c, l.wi, nullptr, nullptr, l.bi, nullptr, nullptr, args.ffn, 1, hidden);
+    const Product down = make_product(c, l.wd, nullptr, nullptr, l.bd, nullptr, nullptr, hidden, 1, args.ffn);
+    // 1
+    if (i == 0) normalise(c, args.x, nullptr, nullptr, 0.f, c.warp, kWarps, keep);
+    else normalise(c, args.y, args.layer[i - 1].ln2_gamma, args.layer[i - 1].ln2_beta, args.layer[i - 1].ln2_eps, c.warp, kWarps, keep);
+    __syncthreads();
+    product<MT>(c, qkv, nullptr, [&](int row, int grp, int col, float v0, float v1) {
+      *reinterpret_cast<uint32_t*>(args.qkv + ((int64_t)grp * args.row_bound + row) * hidden + col) = ptx::pack_bf16x2(v0, v1);
+    });
+    prefetch(c, proj);
+    if (!sync_grid()) return;
+    // 2
+    for (int item = blockIdx.x + gridDim.x * c.warp; item < c.rows * heads; item += gridDim.x * kWarps) {
+      const int row = item / heads;
+      attention_row(c, l, row, item - row * heads, s_start[row], s_len[row]);
+    }
+    prefetch(c, up);
+    if (!sync_grid()) return;
+    // 3
+    product<MT>(c, proj, args.ctx, add_to(args.y));
+    prefetch(c, down);
+    if (!sync_grid()) return;
+    // 4
+    normalise(c, args.y, l.ln1_gamma, l.ln1_beta, l.ln1_eps, c.warp, kWarps, keep);
+    __syncthreads();
+    product<MT>(c, up, nullptr, [&](int row, int, int col, float v0, float v1) {
+      float g0, g1;
+      ptx::unpack_f32x2(gelu_erf2(ptx::pack_f32x2(v0, v1)), g0, g1);
+      *reinterpret_cast<uint32_t*>(args.mid + (int64_t)row * args.ffn + col) = ptx::pack_bf16x2(g0, g1);
+    });
+    if (i + 1 < args.n_layers) {
+      const SmallLayer& n = args.layer[i + 1];
+      prefetch(c, make_product(c, n.wq, n.wk, n.wv, nullptr, nullptr, nullptr, hidden, 3, hidden));
+    }
+    if (!sync_grid()) return;
+    // 5
+    product<MT>(c, down, args.mid, add_to(args.y));
+    if (!sync_grid()) return;
+  }
+  const SmallLayer& l = args.layer[args.n_layers - 1];
+  normalise(c, args.y, l.ln2_gamma, l.ln2_beta, l.ln2_eps, blockIdx.x + gridDim.x * c.warp, gridDim.x * kWarps, [&](int row, int i, uint4 v) {
+    reinterpret_cast<uint4*>(args.out + (int64_t)(args.out_index != nullptr ? args.out_index[row] : row) * hidden)[i] = v;
+  });
+}
+
+size_t smem_bytes(int mt, int hidden, int ffn, int sms) {
+  int tiles = 0;  // per CTA; with four of them half as many partial sums (the last CTA may have three)
+  for (int n : {3 * hidden, hidden, ffn}) tiles = std::max(tiles, (n / 8 + sms - 1) / sms);
+  return size_t(mt) * 16 * (hidden * 2 + 16) + size_t(mt) * 16 * 4 * std::min(tiles, 3) * 8 * kWarps;
+}
+
+}  // namespace
+
+bool small_encoder_covers(int64_t row_bound, int hidden, int ffn, int n_layers) {
+  const int sms = sm_count();
+  if (sms <= 0 || row_bound > kSmallRows || hidden > 1024 || n_layers > kSmallLayers) return false;
+  const int most = std::max(3 * hidden, ffn);
+  return (most / 8 + sms - 1) / sms <= kMaxTiles && smem_bytes(row_bound <= 16 ? 1 : (row_bound <= 32 ? 2 : 4), hidden, ffn, sms) <= 227 * 1024 - 1024;
+}
+
+int launch_small_encoder(const SmallEncoderArgs& a, void* stream) {
+  const int sms = sm_count(), mt = a.row_bound <= 16 ? 1 : (a.row_bound <= 32 ? 2 : 4);
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  auto kernel = mt == 1 ? encoder_small_kernel<1> : (mt == 2 ? encoder_small_kernel<2> : encoder_small_kernel<4>);
+  static std::atomic<uint64_t> smem_done[3];
+  cudaError_t e = allow_smem(smem_done[mt >> 1], reinterpret_cast<const void*>(kernel), 227 * 1024 - 1024);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)sms);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = smem_bytes(mt, a.hidden, a.ffn, sms);
+  cfg.stream = s;
+  cudaLaunchAttribute at;  // the CTAs wait for one another: all of them have to be resident
+  at.id = cudaLaunchAttributeCooperative;
+  at.val.cooperative = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  void* ptr = const_cast<SmallEncoderArgs*>(&a);
+  if (e == cudaSuccess) e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kernel), &ptr);
+  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "small encoder launch: %s", cudaGetErrorString(e));
+  return FDB_OK;
+}
+
+}  // namespace fdb

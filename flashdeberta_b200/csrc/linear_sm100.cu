@@ -17,15 +17,13 @@
 // 128 bytes per clock.  Per 64 of K a 128 x 256 tile moves 96 KB (750 clocks for 512 clocks of MMA); the pair of CTAs halves
 // the W traffic of each SM and brings 256 x 256 to 64 KB (512 for 512).  `kConfigs` holds these costs, and the launcher takes
 // the tile whose waves over the SMs cost least.
-// GELU(v) = v * Phi(v) with Phi from the complementary error function in the rational form of Abramowitz & Stegun 7.1.26
-// (absolute error 1.5e-7, far below half a bf16 ulp of the result): one reciprocal, one exponential and nine FMAs per
-// element, about half of what erff costs — with erff the epilogue would be longer than the main loop.
 // Every wait is bounded; on a timeout the CTA raises FDB_DEV_TIMEOUT in the status word, frees its tensor memory and
 // returns.  No TMA multicast.
 #include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include "gelu.cuh"
 #include "internal.h"
 #include "launch.h"
 #include "linear.h"
@@ -50,27 +48,6 @@ struct LinearArgs {
   int64_t rows, out_stride;
   int k, groups, tiles_n;        // groups = weights over the same x; tiles_n = feature tiles of one weight
 };
-
-// v * Phi(v) with Phi(v) = 1/2 erfc(-v / sqrt 2):  v * Phi(v) = v / 2 + |v| * (1/2 - q),  q = 1/2 erfc(|v| / sqrt 2), for a pair.
-// Two-wide forms where they exist: a third fewer instructions beside a main loop that is bound by power at large sizes
-// (16384 x 768 -> 3072: 75.8 -> 74.7 us, against 63 us without the activation).
-__device__ __forceinline__ uint64_t gelu_erf2(uint64_t v) {
-  const uint64_t av = v & 0x7fffffff7fffffffull;
-  const uint64_t z = mul_f32x2(av, pack_f32x2(0.70710678118654752f, 0.70710678118654752f));
-  float d0, d1, e0, e1, t0, t1;
-  unpack_f32x2(fma_f32x2(pack_f32x2(0.3275911f, 0.3275911f), z, pack_f32x2(1.f, 1.f)), d0, d1);
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t0) : "f"(d0));
-  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(t1) : "f"(d1));
-  unpack_f32x2(mul_f32x2(mul_f32x2(z, z), pack_f32x2(-1.4426950408889634f, -1.4426950408889634f)), e0, e1);
-  const uint64_t e = pack_f32x2(ex2(e0), ex2(e1)), t = pack_f32x2(t0, t1);
-  auto both = [](float c) { return pack_f32x2(c, c); };
-  uint64_t p = fma_f32x2(both(-0.5f * 1.061405429f), t, both(-0.5f * -1.453152027f));  // negated: h = 1/2 - p t e below
-  p = fma_f32x2(p, t, both(-0.5f * 1.421413741f));
-  p = fma_f32x2(p, t, both(-0.5f * -0.284496736f));
-  p = fma_f32x2(p, t, both(-0.5f * 0.254829592f));
-  const uint64_t h = fma_f32x2(mul_f32x2(p, t), e, both(0.5f));
-  return fma_f32x2(av, h, mul_f32x2(v, both(0.5f)));
-}
 
 // 32 bytes per thread in one store (whole sectors)
 __device__ __forceinline__ void st_global_32B(void* p, const uint32_t (&o)[16], int at) {
