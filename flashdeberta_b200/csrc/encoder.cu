@@ -180,7 +180,7 @@ Layout layout_of(const fdb_encoder_call& c, const EncoderPlan& plan, const fdb_a
   l.index = off;  off = align256(off + (c.mask ? rows * 4 : 0));
   l.cu = off;     off = align256(off + (uint64_t)(c.batch + 1) * 4);
   l.rows = off;   off = align256(off + 4);
-  l.barrier = off; off = align256(off + small_encoder_barrier_bytes());
+  l.barrier = off; off = align256(off + 8);
   fdb_attn_params q = p;
   q.pos_key = q.pos_query = nullptr;  // no room for gathered tables: they are the plan's
   ExpandGeometry none = {0, 0, 0, 0};
@@ -307,7 +307,7 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
   // Up to 64 rows the layers are one kernel.  (Timing events around the attention of every layer need launches of their own.)
   const bool small = c->attn_events == nullptr && small_encoder_covers(rows, plan.hidden, plan.ffn, (int)plan.layers.size());
   if (small) {
-    const cudaError_t e = cudaMemsetAsync(ws + l.barrier, 0, small_encoder_barrier_bytes(), s);
+    const cudaError_t e = cudaMemsetAsync(ws + l.barrier, 0, 8, s);
     if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "encoder memset: %s", cudaGetErrorString(e));
   }
 

@@ -42,35 +42,40 @@ struct Ctx {
 __device__ __forceinline__ float lo(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ float round_bf16(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
+__device__ __forceinline__ float warp_sum(float v) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// All CTAs' writes before it are visible after it.  A flag per CTA, polled by a thread each: with one counter the 148 atomics
-// queued up (2900 -> @@ clocks).  Bounded: after about two seconds of SM clock, or once another CTA has given up, every CTA returns.
-__device__ __forceinline__ bool grid_barrier(const SmallEncoderArgs& a, uint32_t epoch) {
+// All CTAs' writes before it are visible after it.  Bounded: after about two seconds of SM clock, or once another CTA has given up,
+// every CTA returns.
+__device__ __forceinline__ bool grid_barrier(const SmallEncoderArgs& a, uint32_t* s_ok, uint32_t target) {
   __syncthreads();
   if (threadIdx.x == 0) {
+    uint32_t ok = 1;
     __threadfence();
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(a.barrier + 1 + blockIdx.x), "r"(epoch) : "memory");
-  }
-  bool ok = true;
-  for (uint32_t n = threadIdx.x; n < gridDim.x; n += kThreads) {
+    atomicAdd(a.barrier, 1u);
     const long long t0 = clock64();
     uint32_t seen = 0;
     for (uint32_t i = 0; i < (1u << 30); ++i) {
-      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.barrier + 1 + n) : "memory");
-      if (seen >= epoch) break;
-      if ((i & 63u) == 63u && (clock64() - t0 > 4000000000LL || *reinterpret_cast<volatile uint32_t*>(a.barrier) != 0u)) break;
+      asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(a.barrier) : "memory");
+      if (seen >= target) break;
+      if ((i & 63u) == 63u && (clock64() - t0 > 4000000000LL || *reinterpret_cast<volatile uint32_t*>(a.barrier + 1) != 0u)) break;
     }
-    ok = ok && seen >= epoch;
+    if (seen < target) {
+      ok = 0;
+      atomicExch(a.barrier + 1, 1u);
+      if (a.status != nullptr) atomicOr(reinterpret_cast<unsigned int*>(a.status), FDB_DEV_TIMEOUT);
+    }
+    *s_ok = ok;
   }
-  if (!ok) {
-    atomicExch(a.barrier, 1u);
-    if (a.status != nullptr) atomicOr(reinterpret_cast<unsigned int*>(a.status), FDB_DEV_TIMEOUT);
-  }
-  return __syncthreads_and(ok) != 0;
+  __syncthreads();
+  return *s_ok != 0;
 }
 
 // One product out[rows][n] = x . w^T over K = k; this CTA's tiles of 8 columns are [tile0, tile0 + tiles).
@@ -103,35 +108,12 @@ __device__ __forceinline__ void prefetch(const Ctx& c, const Product& p) {
 }
 
 // Partial sums of the warps over their share of K, then `store(row, column, v0, v1)` for pairs of columns with the bias added.  The
-// rows come from shared memory (src == NULL) or from memory; `ready` makes them (a grid barrier, a LayerNorm) and is called once the
-// first weights are on their way, which nothing has to wait for.
-template <int MT, int NT, typename Ready, typename Store>
-__device__ __forceinline__ bool product_tiles(const Ctx& c, const Product& p, const __nv_bfloat16* src, int split, Ready&& ready, Store&& store) {
+// rows come from shared memory (src == NULL) or from memory.
+template <int MT, int NT, typename Store>
+__device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, const __nv_bfloat16* src, int split, Store&& store) {
   const int g = c.lane >> 2, t = c.lane & 3;
   const int kgs = kWarps / split, kg = c.warp % kgs, tile = (c.warp / kgs) * NT;  // split: the tiles are dealt to this many sets of warps
   const int cols = p.tiles * 8, blocks = p.k / 64;
-  // of each 64 of K, thread t of a fragment's row has the 16 values from 16 t on: four steps of the MMA
-  constexpr int A = NT == 1 ? (MT == 4 ? 2 : 3) : 1;  // blocks ahead
-  const __nv_bfloat16* w[NT];
-  uint4 y[A][NT][2];
-#pragma unroll
-  for (int n = 0; n < NT; ++n) {
-    w[n] = weight_row(p, p.tile0 + min(tile + n, p.tiles - 1), g) + t * 16;
-#pragma unroll
-    for (int a = 0; a < A; ++a)
-#pragma unroll
-      for (int u = 0; u < 2; ++u)
-        y[a][n][u] = kg + a * kgs < blocks ? __ldg(reinterpret_cast<const uint4*>(w[n] + (kg + a * kgs) * 64) + u) : make_uint4(0, 0, 0, 0);
-  }
-  // the first pair of columns that this thread finishes
-  auto bias_of = [&](int cp) -> uint32_t {
-    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols;
-    const __nv_bfloat16* bias = grp == 0 ? p.b0 : (grp == 1 ? p.b1 : p.b2);
-    return bias != nullptr ? __ldg(reinterpret_cast<const uint32_t*>(bias + col - grp * p.group_cols)) : 0u;
-  };
-  const uint32_t first_bias = bias_of(c.tid % (cols / 2) * 2);
-  if (!ready()) return false;
-
   float acc[MT][NT][4];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -139,50 +121,40 @@ __device__ __forceinline__ bool product_tiles(const Ctx& c, const Product& p, co
     for (int n = 0; n < NT; ++n)
 #pragma unroll
       for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.f;
-  auto block = [&](int b, const uint4 (&yb)[NT][2]) {
-    constexpr int W = MT == 4 ? 1 : 2;  // halves of the block whose rows are loaded together
+  // of each 64 of K, thread t of a fragment's row has the 16 values from 16 t on: four steps of the MMA
+  const __nv_bfloat16* w[NT];
 #pragma unroll
-    for (int u0 = 0; u0 < 2; u0 += W) {
-      uint4 x[MT][2][W];
+  for (int n = 0; n < NT; ++n) w[n] = weight_row(p, p.tile0 + min(tile + n, p.tiles - 1), g) + t * 16;
+#pragma unroll(MT <= 2 ? 3 : 1)
+  for (int b = kg; b < blocks; b += kgs) {
+#pragma unroll
+    for (int u = 0; u < 2; ++u) {
+      uint4 x[MT][2], y[NT];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) y[n] = __ldg(reinterpret_cast<const uint4*>(w[n] + b * 64) + u);
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
+        for (int h = 0; h < 2; ++h) {
+          const int row = m * 16 + h * 8 + g, at = b * 64 + t * 16 + u * 8;
+          if (src == nullptr) x[m][h] = *reinterpret_cast<const uint4*>(c.s_x + row * c.pitch + at * 2);
+          else x[m][h] = row < c.rows ? __ldcg(reinterpret_cast<const uint4*>(src + (int64_t)row * p.k + at)) : make_uint4(0, 0, 0, 0);
+        }
 #pragma unroll
-          for (int u = 0; u < W; ++u) {
-            const int row = m * 16 + h * 8 + g, at = b * 64 + t * 16 + (u0 + u) * 8;
-            if (src == nullptr) x[m][h][u] = *reinterpret_cast<const uint4*>(c.s_x + row * c.pitch + at * 2);
-            else x[m][h][u] = row < c.rows ? __ldcg(reinterpret_cast<const uint4*>(src + (int64_t)row * p.k + at)) : make_uint4(0, 0, 0, 0);
-          }
+      for (int m = 0; m < MT; ++m)
 #pragma unroll
-      for (int u = 0; u < W; ++u)
-#pragma unroll
-        for (int m = 0; m < MT; ++m)
-#pragma unroll
-          for (int n = 0; n < NT; ++n) {
-            const uint4 v = yb[n][u0 + u];
-            mma16816(acc[m][n], x[m][0][u].x, x[m][1][u].x, x[m][0][u].y, x[m][1][u].y, v.x, v.y);
-            mma16816(acc[m][n], x[m][0][u].z, x[m][1][u].z, x[m][0][u].w, x[m][1][u].w, v.z, v.w);
-          }
+        for (int n = 0; n < NT; ++n) {
+          mma16816(acc[m][n], x[m][0].x, x[m][1].x, x[m][0].y, x[m][1].y, y[n].x, y[n].y);
+          mma16816(acc[m][n], x[m][0].z, x[m][1].z, x[m][0].w, x[m][1].w, y[n].z, y[n].w);
+        }
     }
-  };
-#pragma unroll
-  for (int a = 0; a < A; ++a)
-    if (kg + a * kgs < blocks) block(kg + a * kgs, y[a]);
-#pragma unroll 1
-  for (int b = kg + A * kgs; b < blocks; b += kgs) {
-#pragma unroll
-    for (int n = 0; n < NT; ++n)
-#pragma unroll
-      for (int u = 0; u < 2; ++u) y[0][n][u] = __ldg(reinterpret_cast<const uint4*>(w[n] + b * 64) + u);
-    block(b, y[0]);
   }
 #pragma unroll
   for (int m = 0; m < MT; ++m)
 #pragma unroll
     for (int n = 0; n < NT; ++n)
       if (tile + n < p.tiles) {
-        float* at = c.s_red + (kg * MT * 16 + m * 16 + g) * cols + (tile + n) * 8 + 2 * t;
+        float* at = c.s_red + ((int64_t)(kg * MT * 16 + m * 16 + g)) * cols + (tile + n) * 8 + 2 * t;
         *reinterpret_cast<float2*>(at) = make_float2(acc[m][n][0], acc[m][n][1]);
         *reinterpret_cast<float2*>(at + 8 * cols) = make_float2(acc[m][n][2], acc[m][n][3]);
       }
@@ -192,108 +164,81 @@ __device__ __forceinline__ bool product_tiles(const Ctx& c, const Product& p, co
     float2 s = make_float2(0.f, 0.f);
 #pragma unroll 8
     for (int k = 0; k < kgs; ++k) {
-      const float2 v = *reinterpret_cast<const float2*>(c.s_red + (k * MT * 16 + row) * cols + cp);
+      const float2 v = *reinterpret_cast<const float2*>(c.s_red + (int64_t)(k * MT * 16 + row) * cols + cp);
       s.x += v.x;
       s.y += v.y;
     }
-    const uint32_t bias = i < kThreads ? first_bias : bias_of(cp);
-    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols;
-    store(row, grp, col - grp * p.group_cols, round_bf16(s.x + lo(bias)), round_bf16(s.y + hi(bias)));
+    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols, in = col - grp * p.group_cols;
+    const __nv_bfloat16* bias = grp == 0 ? p.b0 : (grp == 1 ? p.b1 : p.b2);
+    if (bias != nullptr) {
+      const uint32_t b = *reinterpret_cast<const uint32_t*>(bias + in);
+      s.x += lo(b);
+      s.y += hi(b);
+    }
+    store(row, grp, in, round_bf16(s.x), round_bf16(s.y));
   }
-  return true;
 }
 
-template <int MT, typename Ready, typename Store>
-__device__ __forceinline__ bool product(const Ctx& c, const Product& p, const __nv_bfloat16* src, Ready&& ready, Store&& store) {
-  if (p.tiles == 0) return ready();  // (uniform over the CTA)
-  if (p.tiles == 1) return product_tiles<MT, 1>(c, p, src, 1, ready, store);
-  if (p.tiles == 2) return product_tiles<MT, 2>(c, p, src, 1, ready, store);
-  if (p.tiles == 3) return product_tiles<MT, 3>(c, p, src, 1, ready, store);
-  return product_tiles<MT, 2>(c, p, src, 2, ready, store);  // (four: the partial sums of 16 warps would not fit)
+template <int MT, typename Store>
+__device__ __forceinline__ void product(const Ctx& c, const Product& p, const __nv_bfloat16* src, Store&& store) {
+  if (p.tiles == 0) return;  // (uniform over the CTA)
+  if (p.tiles == 1) product_tiles<MT, 1>(c, p, src, 1, store);
+  else if (p.tiles == 2) product_tiles<MT, 2>(c, p, src, 1, store);
+  else if (p.tiles == 3) product_tiles<MT, 3>(c, p, src, 1, store);
+  else product_tiles<MT, 2>(c, p, src, 2, store);  // (four: the partial sums of 16 warps would not fit)
 }
 
-// LayerNorm of the rows of `y` (the arithmetic of add_layernorm.cu): R rows of a warp at a time, `step` apart, so that their loads and
-// reductions overlap; gamma == NULL: the rows as they are
-template <int R, typename Out>
+// LayerNorm of the rows of `y`, a warp per row (the arithmetic of add_layernorm.cu); gamma == NULL: the rows as they are
+template <typename Out>
 __device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, float eps,
                                           int first, int step, Out&& out) {
   const int vec = c.a->hidden / 256;
-  for (; first < c.rows; first += R * step) {
-    uint4 raw[R][4];
+  for (int row = first; row < c.rows; row += step) {
+    uint4 raw[4];
 #pragma unroll
-    for (int r = 0; r < R; ++r)
+    for (int i = 0; i < 4; ++i)
+      raw[i] = i < vec ? __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)row * c.a->hidden) + i * 32 + c.lane) : make_uint4(0, 0, 0, 0);
+    if (gamma != nullptr) {
+      float sum = 0.f;
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const int row = min(first + r * step, c.rows - 1);
-        raw[r][i] = i < vec ? __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)row * c.a->hidden) + i * 32 + c.lane) : make_uint4(0, 0, 0, 0);
+        const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) { sum += lo(w[k]); sum += hi(w[k]); }
       }
-    if (gamma != nullptr) {
-      const float inv = 1.f / (float)c.a->hidden;
-      float mean[R], rstd[R];
+      const float inv = 1.f / (float)c.a->hidden, mean = warp_sum(sum) * inv;
+      float sq = 0.f;
 #pragma unroll
-      for (int r = 0; r < R; ++r) {
-        float sum = 0.f;
+      for (int i = 0; i < 4; ++i)
+        if (i < vec) {
+          const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t w[4] = {raw[r][i].x, raw[r][i].y, raw[r][i].z, raw[r][i].w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) { sum += lo(w[k]); sum += hi(w[k]); }
-        }
-        mean[r] = sum;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int r = 0; r < R; ++r) mean[r] += __shfl_xor_sync(0xffffffffu, mean[r], o);
-#pragma unroll
-      for (int r = 0; r < R; ++r) {
-        mean[r] *= inv;
-        float sq = 0.f;
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          if (i < vec) {
-            const uint32_t w[4] = {raw[r][i].x, raw[r][i].y, raw[r][i].z, raw[r][i].w};
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              const float d0 = lo(w[k]) - mean[r], d1 = hi(w[k]) - mean[r];
-              sq = fmaf(d0, d0, sq);
-              sq = fmaf(d1, d1, sq);
-            }
+          for (int k = 0; k < 4; ++k) {
+            const float d0 = lo(w[k]) - mean, d1 = hi(w[k]) - mean;
+            sq = fmaf(d0, d0, sq);
+            sq = fmaf(d1, d1, sq);
           }
-        rstd[r] = sq;
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-        for (int r = 0; r < R; ++r) rstd[r] += __shfl_xor_sync(0xffffffffu, rstd[r], o);
-#pragma unroll
-      for (int r = 0; r < R; ++r) rstd[r] = rsqrtf(rstd[r] * inv + eps);
+        }
+      const float rstd = rsqrtf(warp_sum(sq) * inv + eps);
 #pragma unroll
       for (int i = 0; i < 4; ++i)
         if (i < vec) {
           const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma) + i * 32 + c.lane), bv = __ldg(reinterpret_cast<const uint4*>(beta) + i * 32 + c.lane);
-          const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
+          const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
+          uint32_t o[4];
 #pragma unroll
-          for (int r = 0; r < R; ++r) {
-            const uint32_t w[4] = {raw[r][i].x, raw[r][i].y, raw[r][i].z, raw[r][i].w};
-            uint32_t o[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k)
-              o[k] = ptx::pack_bf16x2(fmaf((lo(w[k]) - mean[r]) * rstd[r], lo(gw[k]), lo(bw[k])), fmaf((hi(w[k]) - mean[r]) * rstd[r], hi(gw[k]), hi(bw[k])));
-            raw[r][i] = make_uint4(o[0], o[1], o[2], o[3]);
-          }
+          for (int k = 0; k < 4; ++k)
+            o[k] = ptx::pack_bf16x2(fmaf((lo(w[k]) - mean) * rstd, lo(gw[k]), lo(bw[k])), fmaf((hi(w[k]) - mean) * rstd, hi(gw[k]), hi(bw[k])));
+          raw[i] = make_uint4(o[0], o[1], o[2], o[3]);
         }
     }
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i < vec && first + r * step < c.rows) out(first + r * step, i * 32 + c.lane, raw[r][i]);
+    for (int i = 0; i < 4; ++i)
+      if (i < vec) out(row, i * 32 + c.lane, raw[i]);
   }
 }
 
-// softmax((q.k + c2p + p2c) * scale) v of one row and head by a warp.  Scores: four lanes per key, 16 features each, so that everything
-// a chunk of 32 keys needs is loaded at once; output: a pair of features per lane.
+// softmax((q.k + c2p + p2c) * scale) v of one row and head by a warp: lanes are keys for the scores, pairs of features for the output
 __device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l, int row, int head, int start, int len) {
   const SmallEncoderArgs& a = *c.a;
   const int64_t hd = (int64_t)head * 64;
@@ -303,73 +248,60 @@ __device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l,
     return;
   }
   const int64_t plane = (int64_t)a.row_bound * a.hidden;
-  const int part = c.lane & 3, m = row - start;
-  const uint4* qr = reinterpret_cast<const uint4*>(a.qkv + (int64_t)row * a.hidden + hd) + part * 2;
-  const uint4 q[2] = {__ldcg(qr), __ldcg(qr + 1)};
-  float s[2][4];  // keys 32 chunk + 8 j + lane / 4
+  const __nv_bfloat16 *q = a.qkv, *k = a.qkv + plane, *v = a.qkv + 2 * plane;
+  const uint4* qr = reinterpret_cast<const uint4*>(q + (int64_t)row * a.hidden + hd);
+  const int m = row - start;
+  float s[2];
 #pragma unroll
   for (int ch = 0; ch < 2; ++ch) {
-#pragma unroll
-    for (int j = 0; j < 4; ++j) s[ch][j] = -INFINITY;
+    s[ch] = -INFINITY;
     if (ch * 32 >= len) continue;
-    uint4 k[4][2], kp[4][2], qp[4][2];
+    const int n = min(ch * 32 + c.lane, len - 1);
+    const uint4* kr = reinterpret_cast<const uint4*>(k + (int64_t)(start + n) * a.hidden + hd);
+    const int64_t at = ((int64_t)head * a.xrows + (m - n - a.d_first)) * 64;
+    const uint4* xk = reinterpret_cast<const uint4*>(l.exp_key + at);
+    const uint4* xq = reinterpret_cast<const uint4*>(l.exp_query + at);
+    float sum = 0.f;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int n = min(ch * 32 + j * 8 + (c.lane >> 2), len - 1);
-      const uint4* kr = reinterpret_cast<const uint4*>(a.qkv + plane + (int64_t)(start + n) * a.hidden + hd) + part * 2;
-      const int64_t at = ((int64_t)head * a.xrows + (m - n - a.d_first)) * 8 + part * 2;
+    for (int half = 0; half < 2; ++half) {
+      uint4 qv[4], kv[4], kp[4], qp[4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        k[j][i] = __ldcg(kr + i);
-        kp[j][i] = l.exp_key != nullptr ? __ldg(reinterpret_cast<const uint4*>(l.exp_key) + at + i) : make_uint4(0, 0, 0, 0);
-        qp[j][i] = l.exp_query != nullptr ? __ldg(reinterpret_cast<const uint4*>(l.exp_query) + at + i) : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < 4; ++i) {
+        qv[i] = __ldcg(qr + half * 4 + i);
+        kv[i] = __ldcg(kr + half * 4 + i);
+        kp[i] = l.exp_key != nullptr ? __ldg(xk + half * 4 + i) : make_uint4(0, 0, 0, 0);
+        qp[i] = l.exp_query != nullptr ? __ldg(xq + half * 4 + i) : make_uint4(0, 0, 0, 0);
       }
-    }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      float sum = 0.f;
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const uint32_t qw[4] = {q[i].x, q[i].y, q[i].z, q[i].w}, kw[4] = {k[j][i].x, k[j][i].y, k[j][i].z, k[j][i].w};
-        const uint32_t pw[4] = {kp[j][i].x, kp[j][i].y, kp[j][i].z, kp[j][i].w}, rw[4] = {qp[j][i].x, qp[j][i].y, qp[j][i].z, qp[j][i].w};
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t qw[4] = {qv[i].x, qv[i].y, qv[i].z, qv[i].w}, kw[4] = {kv[i].x, kv[i].y, kv[i].z, kv[i].w};
+        const uint32_t pw[4] = {kp[i].x, kp[i].y, kp[i].z, kp[i].w}, rw[4] = {qp[i].x, qp[i].y, qp[i].z, qp[i].w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           sum = fmaf(lo(qw[e]), lo(kw[e]) + lo(pw[e]), fmaf(lo(kw[e]), lo(rw[e]), sum));
           sum = fmaf(hi(qw[e]), hi(kw[e]) + hi(pw[e]), fmaf(hi(kw[e]), hi(rw[e]), sum));
         }
       }
-      sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-      sum += __shfl_xor_sync(0xffffffffu, sum, 2);
-      if (ch * 32 + j * 8 + (c.lane >> 2) < len) s[ch][j] = sum * (a.sm_scale * 1.4426950408889634f);
     }
+    if (ch * 32 + c.lane < len) s[ch] = sum * (a.sm_scale * 1.4426950408889634f);
   }
-  float top = s[0][0];
+  float top = fmaxf(s[0], s[1]);
 #pragma unroll
-  for (int i = 1; i < 8; ++i) top = fmaxf(top, s[i >> 2][i & 3]);
-#pragma unroll
-  for (int o = 16; o >= 4; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  float total = 0.f;
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    s[i >> 2][i & 3] = ptx::ex2(s[i >> 2][i & 3] - top);  // keys behind the sequence: zero
-    total += s[i >> 2][i & 3];
-  }
-#pragma unroll
-  for (int o = 16; o >= 4; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
-  const float inv = 1.f / total;
+  for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+  const float p0 = ptx::ex2(s[0] - top), p1 = ptx::ex2(s[1] - top);
+  const float inv = 1.f / warp_sum(p0 + p1);
   float o0 = 0.f, o1 = 0.f;
-  const uint32_t* vr = reinterpret_cast<const uint32_t*>(a.qkv + 2 * plane + (int64_t)start * a.hidden + hd) + c.lane;
+  const uint32_t* vr = reinterpret_cast<const uint32_t*>(v + (int64_t)start * a.hidden + hd) + c.lane;
+  for (int n0 = 0; n0 < len; n0 += 8) {
+    uint32_t w[8];
 #pragma unroll
-  for (int ch = 0; ch < 2; ++ch) {
-    if (ch * 32 >= len) continue;
-    uint32_t w[32];
+    for (int i = 0; i < 8; ++i) w[i] = n0 + i < len ? __ldcg(vr + (int64_t)(n0 + i) * (a.hidden / 2)) : 0u;
 #pragma unroll
-    for (int n = 0; n < 32; ++n) w[n] = ch * 32 + n < len ? __ldcg(vr + (int64_t)(ch * 32 + n) * (a.hidden / 2)) : 0u;
-#pragma unroll
-    for (int n = 0; n < 32; ++n) {
-      const float p = __shfl_sync(0xffffffffu, s[ch][n >> 3], (n & 7) * 4);
-      o0 = fmaf(p, lo(w[n]), o0);
-      o1 = fmaf(p, hi(w[n]), o1);
+    for (int i = 0; i < 8; ++i) {
+      const int n = n0 + i;  // keys behind the sequence have probability zero
+      const float pn = __shfl_sync(0xffffffffu, n < 32 ? p0 : p1, n & 31);
+      o0 = fmaf(pn, lo(w[i]), o0);
+      o1 = fmaf(pn, hi(w[i]), o1);
     }
   }
   *out = ptx::pack_bf16x2(o0 * inv, o1 * inv);
@@ -379,6 +311,7 @@ template <int MT>
 __global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid_constant__ SmallEncoderArgs args) {
   extern __shared__ __align__(16) uint8_t smem[];
   __shared__ int s_start[kSmallRows], s_len[kSmallRows];
+  __shared__ uint32_t s_ok;
   Ctx c;
   c.a = &args;
   c.tid = threadIdx.x; c.warp = threadIdx.x >> 5; c.lane = threadIdx.x & 31;
@@ -408,7 +341,7 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid
 
   const int hidden = args.hidden, heads = hidden / 64;
   uint32_t barriers = 0;
-  auto sync_grid = [&]() -> bool { return grid_barrier(args, ++barriers); };
+  auto sync_grid = [&]() -> bool { return grid_barrier(args, &s_ok, ++barriers * gridDim.x); };
   auto keep = [&](int row, int i, uint4 v) { *reinterpret_cast<uint4*>(c.s_x + row * c.pitch + i * 16) = v; };
   auto residual = [&](int row, int col) -> uint32_t { return *reinterpret_cast<const uint32_t*>(c.s_x + row * c.pitch + col * 2); };
   auto add_to = [&](__nv_bfloat16* y) {
@@ -425,66 +358,44 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid
     const Product up = make_product(c, l.wi, nullptr, nullptr, l.bi, nullptr, nullptr, args.ffn, 1, hidden);
     const Product down = make_product(c, l.wd, nullptr, nullptr, l.bd, nullptr, nullptr, hidden, 1, args.ffn);
     // 1
-    if (!product<MT>(c, qkv, nullptr,
-                     [&]() -> bool {
-                       if (i == 0) {
-                         normalise<MT == 1 ? 1 : 2>(c, args.x, nullptr, nullptr, 0.f, c.warp, kWarps, keep);
-                       } else {
-                         if (!sync_grid()) return false;
-                         const SmallLayer& b = args.layer[i - 1];
-                         normalise<MT == 1 ? 1 : 2>(c, args.y, b.ln2_gamma, b.ln2_beta, b.ln2_eps, c.warp, kWarps, keep);
-                       }
-                       __syncthreads();
-                       return true;
-                     },
-                     [&](int row, int grp, int col, float v0, float v1) {
-                       *reinterpret_cast<uint32_t*>(args.qkv + ((int64_t)grp * args.row_bound + row) * hidden + col) = ptx::pack_bf16x2(v0, v1);
-                     }))
-      return;
+    if (i == 0) normalise(c, args.x, nullptr, nullptr, 0.f, c.warp, kWarps, keep);
+    else normalise(c, args.y, args.layer[i - 1].ln2_gamma, args.layer[i - 1].ln2_beta, args.layer[i - 1].ln2_eps, c.warp, kWarps, keep);
+    __syncthreads();
+    product<MT>(c, qkv, nullptr, [&](int row, int grp, int col, float v0, float v1) {
+      *reinterpret_cast<uint32_t*>(args.qkv + ((int64_t)grp * args.row_bound + row) * hidden + col) = ptx::pack_bf16x2(v0, v1);
+    });
     prefetch(c, proj);
-    // 2
-    const int n_items = c.rows * heads, item0 = blockIdx.x + gridDim.x * c.warp;
-    if (item0 < n_items) {  // the rows of the position tables to L2
-      const int row = item0 / heads;
-      for (int n = c.lane; n < s_len[row]; n += 32) {
-        const int64_t at = ((int64_t)(item0 - row * heads) * args.xrows + (row - s_start[row] - n - args.d_first)) * 64;
-        if (l.exp_key != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(l.exp_key + at));
-        if (l.exp_query != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(l.exp_query + at));
-      }
-    }
     if (!sync_grid()) return;
-    for (int item = item0; item < n_items; item += gridDim.x * kWarps) {
+    // 2
+    for (int item = blockIdx.x + gridDim.x * c.warp; item < c.rows * heads; item += gridDim.x * kWarps) {
       const int row = item / heads;
       attention_row(c, l, row, item - row * heads, s_start[row], s_len[row]);
     }
     prefetch(c, up);
+    if (!sync_grid()) return;
     // 3
-    if (!product<MT>(c, proj, args.ctx, sync_grid, add_to(args.y))) return;
+    product<MT>(c, proj, args.ctx, add_to(args.y));
     prefetch(c, down);
+    if (!sync_grid()) return;
     // 4
-    if (!product<MT>(c, up, nullptr,
-                     [&]() -> bool {
-                       if (!sync_grid()) return false;
-                       normalise<MT == 1 ? 1 : 2>(c, args.y, l.ln1_gamma, l.ln1_beta, l.ln1_eps, c.warp, kWarps, keep);
-                       __syncthreads();
-                       return true;
-                     },
-                     [&](int row, int, int col, float v0, float v1) {
-                       float g0, g1;
-                       ptx::unpack_f32x2(gelu_erf2(ptx::pack_f32x2(v0, v1)), g0, g1);
-                       *reinterpret_cast<uint32_t*>(args.mid + (int64_t)row * args.ffn + col) = ptx::pack_bf16x2(g0, g1);
-                     }))
-      return;
+    normalise(c, args.y, l.ln1_gamma, l.ln1_beta, l.ln1_eps, c.warp, kWarps, keep);
+    __syncthreads();
+    product<MT>(c, up, nullptr, [&](int row, int, int col, float v0, float v1) {
+      float g0, g1;
+      ptx::unpack_f32x2(gelu_erf2(ptx::pack_f32x2(v0, v1)), g0, g1);
+      *reinterpret_cast<uint32_t*>(args.mid + (int64_t)row * args.ffn + col) = ptx::pack_bf16x2(g0, g1);
+    });
     if (i + 1 < args.n_layers) {
       const SmallLayer& n = args.layer[i + 1];
       prefetch(c, make_product(c, n.wq, n.wk, n.wv, nullptr, nullptr, nullptr, hidden, 3, hidden));
     }
+    if (!sync_grid()) return;
     // 5
-    if (!product<MT>(c, down, args.mid, sync_grid, add_to(args.y))) return;
+    product<MT>(c, down, args.mid, add_to(args.y));
+    if (!sync_grid()) return;
   }
-  if (!sync_grid()) return;
   const SmallLayer& l = args.layer[args.n_layers - 1];
-  normalise<1>(c, args.y, l.ln2_gamma, l.ln2_beta, l.ln2_eps, blockIdx.x + gridDim.x * c.warp, gridDim.x * kWarps, [&](int row, int i, uint4 v) {
+  normalise(c, args.y, l.ln2_gamma, l.ln2_beta, l.ln2_eps, blockIdx.x + gridDim.x * c.warp, gridDim.x * kWarps, [&](int row, int i, uint4 v) {
     reinterpret_cast<uint4*>(args.out + (int64_t)(args.out_index != nullptr ? args.out_index[row] : row) * hidden)[i] = v;
   });
 }
@@ -496,8 +407,6 @@ size_t smem_bytes(int mt, int hidden, int ffn, int sms) {
 }
 
 }  // namespace
-
-uint64_t small_encoder_barrier_bytes() { return (1 + uint64_t(sm_count())) * sizeof(uint32_t); }
 
 bool small_encoder_covers(int64_t row_bound, int hidden, int ffn, int n_layers) {
   const int sms = sm_count();

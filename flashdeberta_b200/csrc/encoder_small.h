@@ -28,11 +28,10 @@ struct SmallEncoderArgs {
   __nv_bfloat16 *qkv, *ctx, *y, *mid;  // (3, row_bound, hidden), (row_bound, hidden) twice, (row_bound, ffn)
   __nv_bfloat16* out;
   const int32_t* out_index;    // row -> row of out, or NULL
-  uint32_t* barrier;           // small_encoder_barrier_bytes(), zero
+  uint32_t* barrier;           // two words, zero
   int32_t* status;
 };
 
-uint64_t small_encoder_barrier_bytes();
 bool small_encoder_covers(int64_t row_bound, int hidden, int ffn, int n_layers);
 int launch_small_encoder(const SmallEncoderArgs& a, void* stream);
 
