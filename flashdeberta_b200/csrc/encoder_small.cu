@@ -114,6 +114,13 @@ __device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, co
   const int g = c.lane >> 2, t = c.lane & 3;
   const int kgs = kWarps / split, kg = c.warp % kgs, tile = (c.warp / kgs) * NT;  // split: the tiles are dealt to this many sets of warps
   const int cols = p.tiles * 8, blocks = p.k / 64;
+  // the bias of the pair of columns that this thread finishes first, on its way while the product is made
+  auto bias_of = [&](int cp) -> uint32_t {
+    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols;
+    const __nv_bfloat16* bias = grp == 0 ? p.b0 : (grp == 1 ? p.b1 : p.b2);
+    return bias != nullptr ? __ldg(reinterpret_cast<const uint32_t*>(bias + col - grp * p.group_cols)) : 0u;
+  };
+  const uint32_t first_bias = bias_of(c.tid % (cols / 2) * 2);
   float acc[MT][NT][4];
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -168,14 +175,9 @@ __device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, co
       s.x += v.x;
       s.y += v.y;
     }
+    const uint32_t bias = i < kThreads ? first_bias : bias_of(cp);
     const int col = p.tile0 * 8 + cp, grp = col / p.group_cols, in = col - grp * p.group_cols;
-    const __nv_bfloat16* bias = grp == 0 ? p.b0 : (grp == 1 ? p.b1 : p.b2);
-    if (bias != nullptr) {
-      const uint32_t b = *reinterpret_cast<const uint32_t*>(bias + in);
-      s.x += lo(b);
-      s.y += hi(b);
-    }
-    store(row, grp, in, round_bf16(s.x), round_bf16(s.y));
+    store(row, grp, in, round_bf16(s.x + lo(bias)), round_bf16(s.y + hi(bias)));
   }
 }
 
@@ -188,53 +190,90 @@ __device__ __forceinline__ void product(const Ctx& c, const Product& p, const __
   else product_tiles<MT, 2>(c, p, src, 2, store);  // (four: the partial sums of 16 warps would not fit)
 }
 
-// LayerNorm of the rows of `y`, a warp per row (the arithmetic of add_layernorm.cu); gamma == NULL: the rows as they are
+// a bf16 pair as two floats
+__device__ __forceinline__ uint64_t wide(uint32_t w) { return ptx::pack_f32x2(lo(w), hi(w)); }
+__device__ __forceinline__ uint64_t both(float v) { return ptx::pack_f32x2(v, v); }
+__device__ __forceinline__ float across(uint64_t v) {
+  float a, b;
+  ptx::unpack_f32x2(v, a, b);
+  return a + b;
+}
+
+// LayerNorm of the rows of `y` (the sums of add_layernorm.cu, two at a time), two rows of a warp together; gamma == NULL: the rows as
+// they are.  With all rows on every CTA this is bound by instructions, not by memory.
 template <typename Out>
 __device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, float eps,
                                           int first, int step, Out&& out) {
   const int vec = c.a->hidden / 256;
-  for (int row = first; row < c.rows; row += step) {
-    uint4 raw[4];
+  const float inv = 1.f / (float)c.a->hidden;
+#pragma unroll 1
+  for (int row = first; row < c.rows; row += 2 * step) {
+    uint4 raw[2][4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      raw[i] = i < vec ? __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)row * c.a->hidden) + i * 32 + c.lane) : make_uint4(0, 0, 0, 0);
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        raw[r][i] = i < vec ? __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)min(row + r * step, c.rows - 1) * c.a->hidden) + i * 32 + c.lane)
+                            : make_uint4(0, 0, 0, 0);
     if (gamma != nullptr) {
-      float sum = 0.f;
+      uint64_t d[2][16];
+      float mean[2], rstd[2];
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        uint64_t sum = both(0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t w[4] = {raw[r][i].x, raw[r][i].y, raw[r][i].z, raw[r][i].w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) sum = ptx::add_f32x2(sum, d[r][i * 4 + k] = wide(w[k]));
+        }
+        mean[r] = across(sum);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) mean[r] += __shfl_xor_sync(0xffffffffu, mean[r], o);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        const uint64_t m = both(-mean[r] * inv);
+        uint64_t sq = both(0.f);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          if (i / 4 >= vec) continue;
+          d[r][i] = ptx::add_f32x2(d[r][i], m);
+          sq = ptx::fma_f32x2(d[r][i], d[r][i], sq);
+        }
+        rstd[r] = across(sq);
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int r = 0; r < 2; ++r) rstd[r] += __shfl_xor_sync(0xffffffffu, rstd[r], o);
+#pragma unroll
+      for (int r = 0; r < 2; ++r) rstd[r] = rsqrtf(rstd[r] * inv + eps);
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
+        if (i >= vec) continue;
+        const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma) + i * 32 + c.lane), bv = __ldg(reinterpret_cast<const uint4*>(beta) + i * 32 + c.lane);
+        const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
+        uint32_t o[2][4];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) { sum += lo(w[k]); sum += hi(w[k]); }
-      }
-      const float inv = 1.f / (float)c.a->hidden, mean = warp_sum(sum) * inv;
-      float sq = 0.f;
+        for (int k = 0; k < 4; ++k)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i < vec) {
-          const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w};
-#pragma unroll
-          for (int k = 0; k < 4; ++k) {
-            const float d0 = lo(w[k]) - mean, d1 = hi(w[k]) - mean;
-            sq = fmaf(d0, d0, sq);
-            sq = fmaf(d1, d1, sq);
+          for (int r = 0; r < 2; ++r) {
+            float v0, v1;
+            ptx::unpack_f32x2(ptx::fma_f32x2(ptx::mul_f32x2(d[r][i * 4 + k], both(rstd[r])), wide(gw[k]), wide(bw[k])), v0, v1);
+            o[r][k] = ptx::pack_bf16x2(v0, v1);
           }
-        }
-      const float rstd = rsqrtf(warp_sum(sq) * inv + eps);
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i < vec) {
-          const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma) + i * 32 + c.lane), bv = __ldg(reinterpret_cast<const uint4*>(beta) + i * 32 + c.lane);
-          const uint32_t w[4] = {raw[i].x, raw[i].y, raw[i].z, raw[i].w}, gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
-          uint32_t o[4];
-#pragma unroll
-          for (int k = 0; k < 4; ++k)
-            o[k] = ptx::pack_bf16x2(fmaf((lo(w[k]) - mean) * rstd, lo(gw[k]), lo(bw[k])), fmaf((hi(w[k]) - mean) * rstd, hi(gw[k]), hi(bw[k])));
-          raw[i] = make_uint4(o[0], o[1], o[2], o[3]);
-        }
+        for (int r = 0; r < 2; ++r) raw[r][i] = make_uint4(o[r][0], o[r][1], o[r][2], o[r][3]);
+      }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
-      if (i < vec) out(row, i * 32 + c.lane, raw[i]);
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (i < vec && row + r * step < c.rows) out(row + r * step, i * 32 + c.lane, raw[r][i]);
   }
 }
 
@@ -261,7 +300,7 @@ __device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l,
     const int64_t at = ((int64_t)head * a.xrows + (m - n - a.d_first)) * 64;
     const uint4* xk = reinterpret_cast<const uint4*>(l.exp_key + at);
     const uint4* xq = reinterpret_cast<const uint4*>(l.exp_query + at);
-    float sum = 0.f;
+    uint64_t sum_q = both(0.f), sum_k = both(0.f);  // q . (k + pos_key), k . pos_query
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       uint4 qv[4], kv[4], kp[4], qp[4];
@@ -278,32 +317,34 @@ __device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l,
         const uint32_t pw[4] = {kp[i].x, kp[i].y, kp[i].z, kp[i].w}, rw[4] = {qp[i].x, qp[i].y, qp[i].z, qp[i].w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          sum = fmaf(lo(qw[e]), lo(kw[e]) + lo(pw[e]), fmaf(lo(kw[e]), lo(rw[e]), sum));
-          sum = fmaf(hi(qw[e]), hi(kw[e]) + hi(pw[e]), fmaf(hi(kw[e]), hi(rw[e]), sum));
+          const uint64_t kk = wide(kw[e]);
+          sum_q = ptx::fma_f32x2(wide(qw[e]), ptx::add_f32x2(kk, wide(pw[e])), sum_q);
+          sum_k = ptx::fma_f32x2(kk, wide(rw[e]), sum_k);
         }
       }
     }
-    if (ch * 32 + c.lane < len) s[ch] = sum * (a.sm_scale * 1.4426950408889634f);
+    if (ch * 32 + c.lane < len) s[ch] = across(ptx::add_f32x2(sum_q, sum_k)) * (a.sm_scale * 1.4426950408889634f);
   }
   float top = fmaxf(s[0], s[1]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
   const float p0 = ptx::ex2(s[0] - top), p1 = ptx::ex2(s[1] - top);
   const float inv = 1.f / warp_sum(p0 + p1);
-  float o0 = 0.f, o1 = 0.f;
+  uint64_t o = both(0.f);
   const uint32_t* vr = reinterpret_cast<const uint32_t*>(v + (int64_t)start * a.hidden + hd) + c.lane;
-  for (int n0 = 0; n0 < len; n0 += 8) {
-    uint32_t w[8];
+  for (int n0 = 0; n0 < len; n0 += 16) {
+    uint32_t w[16];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) w[i] = n0 + i < len ? __ldcg(vr + (int64_t)(n0 + i) * (a.hidden / 2)) : 0u;
+    for (int i = 0; i < 16; ++i) w[i] = n0 + i < len ? __ldcg(vr + (int64_t)(n0 + i) * (a.hidden / 2)) : 0u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
+    for (int i = 0; i < 16; ++i) {
       const int n = n0 + i;  // keys behind the sequence have probability zero
       const float pn = __shfl_sync(0xffffffffu, n < 32 ? p0 : p1, n & 31);
-      o0 = fmaf(pn, lo(w[i]), o0);
-      o1 = fmaf(pn, hi(w[i]), o1);
+      o = ptx::fma_f32x2(both(pn), wide(w[i]), o);
     }
   }
+  float o0, o1;
+  ptx::unpack_f32x2(o, o0, o1);
   *out = ptx::pack_bf16x2(o0 * inv, o1 * inv);
 }
 
