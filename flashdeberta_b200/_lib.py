@@ -60,6 +60,7 @@ EXPORTS = (
     "fdb_attn_bwd_probs", "fdb_attn_bwd_bucket_sums", "fdb_expanded_rows", "fdb_expand_tables", "fdb_encoder_create",
     "fdb_encoder_destroy", "fdb_encoder_workspace_bytes", "fdb_encoder_forward", "fdb_attn_bwd_workspace_bytes", "fdb_attn_bwd",
     "fdb_lengths_from_mask", "fdb_column_sums_workspace_bytes", "fdb_column_sums", "fdb_quantize_attn",
+    "fdb_projected_forward",
 )
 
 _lib = None
@@ -104,6 +105,8 @@ def load() -> C.CDLL:
     lib.fdb_quantize_e4m3.restype = C.c_int
     lib.fdb_quantize_e4m3.argtypes = [C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_void_p, C.c_int32, C.c_int32, C.c_int32,
                                       C.c_void_p, C.c_void_p, C.c_void_p]
+    lib.fdb_projected_forward.restype = C.c_int
+    lib.fdb_projected_forward.argtypes = [C.c_void_p, C.c_void_p]
     lib.fdb_quantize_attn.restype = C.c_int
     lib.fdb_quantize_attn.argtypes = [C.c_void_p, C.c_void_p]
     lib.fdb_add_layernorm.restype = C.c_int

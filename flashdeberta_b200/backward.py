@@ -44,7 +44,7 @@ class BwdParams(C.Structure):
         ("struct_bytes", C.c_uint32), ("reserved", C.c_int32), ("fwd", C.POINTER(_lib.AttnParams)),
         ("dout", C.c_void_p), ("dout_row_stride", C.c_int64), ("dout_head_stride", C.c_int64),
         ("dq", C.c_void_p), ("dk", C.c_void_p), ("dv", C.c_void_p), ("grad_row_stride", C.c_int64), ("grad_head_stride", C.c_int64),
-        ("dpos_key", C.c_void_p), ("dpos_query", C.c_void_p),
+        ("dpos_key", C.c_void_p), ("dpos_query", C.c_void_p), ("table_row_stride", C.c_int64), ("table_head_stride", C.c_int64),
         ("workspace", C.c_void_p), ("workspace_bytes", C.c_uint64),
     ]
 
@@ -216,39 +216,37 @@ def index_covered(position_buckets, max_relative_positions) -> bool:
     return _steps[key]
 
 
-def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
-           max_relative_positions, grads=None, table_grads=(None, None)):
-    """``grads`` (rows, 3, H, 64) and ``table_grads`` (each table's shape), when given, take the results."""
+def launch(b: BwdParams, dev: torch.device) -> None:
+    """``fdb_attn_bwd`` on the current stream, with a workspace of this call's own."""
     global _launches
-    dev, shape = q.device, q.shape
     lib = _lib.load()
+    need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
+    ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
+    b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
+    _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(ops.raw_stream(dev))))
+    terms = int(b.dpos_key is not None) + int(b.dpos_query is not None)
+    _launches += 4 + int(terms > 0) + 2 * terms
+
+
+def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
+           max_relative_positions):
+    dev, shape = q.device, q.shape
     with ops.on_device(dev):
         p, keep = ops._fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
                                    max_relative_positions, out.contiguous(), lse.contiguous())
         d3, d_rs, d_hs, T = ops._rows_view(dout)
         H = shape[-2]
-        if grads is None:
-            grads, row_stride = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)], H * 64
-        else:
-            grads, row_stride = grads.unbind(1), 3 * H * 64
-        d_key, d_query = table_grads
-        if d_key is None and pos_key is not None:
-            d_key = torch.empty(pos_key.shape, dtype=torch.bfloat16, device=dev)
-        if d_query is None and pos_query is not None:
-            d_query = torch.empty(pos_query.shape, dtype=torch.bfloat16, device=dev)
+        grads = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)]
+        d_key = torch.empty(pos_key.shape, dtype=torch.bfloat16, device=dev) if pos_key is not None else None
+        d_query = torch.empty(pos_query.shape, dtype=torch.bfloat16, device=dev) if pos_query is not None else None
         b = BwdParams()
         b.struct_bytes, b.fwd = C.sizeof(BwdParams), C.pointer(p)
         b.dout, b.dout_row_stride, b.dout_head_stride = d3.data_ptr(), d_rs, d_hs
         b.dq, b.dk, b.dv = (g.data_ptr() for g in grads)
-        b.grad_row_stride, b.grad_head_stride = row_stride, 64
+        b.grad_row_stride, b.grad_head_stride = H * 64, 64
         b.dpos_key, b.dpos_query = _ptr(d_key), _ptr(d_query)
-        need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
-        ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
-        b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
-        _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(ops.raw_stream(dev))))
-        terms = int(pos_key is not None) + int(pos_query is not None)
-        _launches += 4 + int(terms > 0) + 2 * terms
-        del keep, ws
+        launch(b, dev)
+        del keep
     return (*(g.view(shape) for g in grads), d_key, d_query)
 
 

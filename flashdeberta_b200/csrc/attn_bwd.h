@@ -10,13 +10,14 @@ namespace fdb {
 // out = core + sums . table, dtable = sums^T . operand, for every head.
 struct BwdTablesCall {
   const void* sums;     // bf16 (heads, rows, table_rows)
-  const void* table;    // bf16 (heads, table_rows, 64)
+  const void* table;    // bf16 (heads, table_rows, 64) with the strides below
+  int64_t table_row_stride, table_head_stride;
   const void* operand;  // bf16, rows of operand_row_stride elements
   int64_t operand_row_stride, operand_head_stride;
   float* core;          // (rows, heads, 64); overwritten when table_rows is above 512
   void* out;            // bf16
   int64_t out_row_stride, out_head_stride;
-  void* dtable;         // bf16 (heads, table_rows, 64)
+  void* dtable;         // bf16, laid out like the table
   float* partial;       // bwd_tables_partial_bytes()
   int64_t rows;
   int heads, table_rows;

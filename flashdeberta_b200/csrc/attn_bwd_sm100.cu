@@ -682,20 +682,25 @@ __global__ void __launch_bounds__(256) bwd_delta_kernel(const __nv_bfloat16* __r
 __global__ void __launch_bounds__(256) bwd_expand_kernel(const uint4* __restrict__ pos_key, const uint4* __restrict__ pos_query,
                                                          uint4* __restrict__ key, uint4* __restrict__ query,
                                                          uint4* __restrict__ key_rev, uint4* __restrict__ query_rev,
-                                                         const int16_t* __restrict__ lut, int lut_len, int rows, int table_rows, int heads) {
+                                                         const int16_t* __restrict__ lut, int lut_len, int rows, int heads, int64_t row_stride, int64_t head_stride) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;
   if (i >= (int64_t)heads * rows * 8) return;
   const int c = (int)(i & 7);
   const int u = (int)((i >> 3) % rows), h = (int)((i >> 3) / rows);
   int li = u - 254;  // expanded row 0 is 254 distances below the table
   li = li < 0 ? 0 : (li >= lut_len ? lut_len - 1 : li);
-  const int64_t src = ((int64_t)h * table_rows + lut[li]) * 8 + c;
+  const int64_t src = h * head_stride + lut[li] * row_stride + c;
   const int64_t rev = ((int64_t)h * rows + (rows - 1 - u)) * 8 + c;
   if (pos_key != nullptr) { const uint4 v = pos_key[src]; key[i] = v; key_rev[rev] = v; }
   if (pos_query != nullptr) { const uint4 v = pos_query[src]; query[i] = v; query_rev[rev] = v; }
 }
 
 int table_rows_of(const fdb_attn_params& p) { return 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions); }
+
+TableStrides table_strides(const fdb_attn_bwd_params& b) {
+  if (b.table_row_stride > 0) return {b.table_row_stride, b.table_head_stride};
+  return {kHeadDim, (int64_t)table_rows_of(*b.fwd) * kHeadDim};
+}
 
 uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 
@@ -772,6 +777,8 @@ int launch_bwd(const BwdArgs& a, const fdb_attn_bwd_params& b, char* partial, in
   BwdTablesCall c;
   c.sums = a.sums;
   c.table = DKV ? p.pos_query : p.pos_key;
+  const TableStrides strides = table_strides(b);
+  c.table_row_stride = strides.row; c.table_head_stride = strides.head;
   c.operand = DKV ? p.k : p.q;
   c.operand_row_stride = DKV ? p.k_row_stride : p.q_row_stride;
   c.operand_head_stride = DKV ? p.k_head_stride : p.q_head_stride;
@@ -828,6 +835,7 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   const int64_t strides[4] = {b->dout_row_stride, b->dout_head_stride, b->grad_row_stride, b->grad_head_stride};
   bool aligned = (all & 15u) == 0;
   for (int64_t s : strides) aligned = aligned && s > 0 && s % 8 == 0;
+  aligned = aligned && b->table_row_stride >= 0 && b->table_row_stride % 8 == 0 && (b->table_row_stride == 0 || b->table_head_stride > 0) && b->table_head_stride % 8 == 0;
   if (!aligned) return fail(FDB_ERR_ALIGNMENT, "fdb_attn_bwd: pointers must be 16-byte aligned, strides positive multiples of 8 elements");
   const Layout l = layout_of(p, g);
   if (b->workspace == nullptr || b->workspace_bytes < l.total)
@@ -846,10 +854,11 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   if ((rc = make_args<false>(dq, *b, g, l, ws)) != FDB_OK || (rc = make_args<true>(dkv, *b, g, l, ws)) != FDB_OK) return rc;
   if (p.pos_key != nullptr || p.pos_query != nullptr) {
     const int64_t n = (int64_t)p.heads * g.rows * 8;
+    const TableStrides strides = table_strides(*b);
     auto table = [&](int i) { return reinterpret_cast<uint4*>(ws + l.table[i]); };
     bwd_expand_kernel<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(static_cast<const uint4*>(p.pos_key), static_cast<const uint4*>(p.pos_query),
-                                                                 table(0), table(1), table(2), table(3), p.bucket_lut, p.lut_len, g.rows,
-                                                                 table_rows_of(p), p.heads);
+                                                                 table(0), table(1), table(2), table(3), p.bucket_lut, p.lut_len, g.rows, p.heads,
+                                                                 strides.row / 8, strides.head / 8);
   }
   const int64_t cells = (int64_t)p.total_rows * p.heads;
   bwd_delta_kernel<<<(unsigned)((cells * 8 + 255) / 256), 256, 0, s>>>(

@@ -97,7 +97,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tables_kernel(const __grid_co
     if (elect_one()) {
       mbar_expect_tx(bar(kBarTable), uint32_t(pieces) * 16384u);
       for (int p = 0; p < pieces; ++p)
-        tma_load_3d(smem + kSmemTable + uint32_t(p) * 16384u, &args.tm_table, bar(kBarTable), 0, args.w0 + p * 128, head);
+        tma_load_3d(smem + kSmemTable + uint32_t(p) * 16384u, &args.tm_table, bar(kBarTable), 0, head, args.w0 + p * 128);
     }
     uint32_t n = 0;  // pieces so far
 #pragma unroll 1
@@ -227,8 +227,8 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tables_kernel(const __grid_co
 }
 
 // dtable = sum of the CTAs' parts, in bf16
-__global__ void __launch_bounds__(256) bwd_table_reduce_kernel(const float4* __restrict__ partial, int parts, int w_rows, int w0, int table_rows,
-                                                               int heads, uint2* __restrict__ out) {
+__global__ void __launch_bounds__(256) bwd_table_reduce_kernel(const float4* __restrict__ partial, int parts, int w_rows, int w0, int heads,
+                                                               int64_t row_stride, int64_t head_stride, __nv_bfloat16* __restrict__ out) {
   const int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x;  // (head, w, 4 columns)
   const int64_t per_head = (int64_t)w_rows * 16;
   if (i >= per_head * heads) return;
@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(256) bwd_table_reduce_kernel(const float4* __r
     const float4 v = src[p * per_head];
     s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
   }
-  out[(h * table_rows + w0) * 16 + at] = make_uint2(pack_bf16x2(s.x, s.y), pack_bf16x2(s.z, s.w));
+  *reinterpret_cast<uint2*>(out + h * head_stride + (w0 + at / 16) * row_stride + at % 16 * 4) = make_uint2(pack_bf16x2(s.x, s.y), pack_bf16x2(s.z, s.w));
 }
 
 // (heads, rows, width) bf16, contiguous -> box of 64 x 128 x 1 elements, 128-byte swizzle
@@ -272,7 +272,7 @@ int launch_bwd_tables(const BwdTablesCall& c, cudaStream_t stream) {
   TableArgs a;
   int rc;
   if ((rc = make_map_sums(&a.tm_sums, c.sums, c.table_rows, c.rows, c.heads))) return rc;
-  if ((rc = make_map_table(&a.tm_table, c.table, c.table_rows, c.heads, false, "position table", 128))) return rc;
+  if ((rc = make_map_rows(&a.tm_table, c.table, c.table_rows, c.heads, c.table_row_stride, c.table_head_stride, 128, false, "position table"))) return rc;
   if ((rc = make_map_rows(&a.tm_operand, c.operand, c.rows, c.heads, c.operand_row_stride, c.operand_head_stride, 128, false, "backward operand"))) return rc;
   a.core = c.core;
   a.out = static_cast<__nv_bfloat16*>(c.out);
@@ -291,8 +291,8 @@ int launch_bwd_tables(const BwdTablesCall& c, cudaStream_t stream) {
     e = launch_kernel<TableArgs>(bwd_tables_kernel, a, dim3((unsigned)parts, (unsigned)c.heads), kThreads, kSmemBytes, false, stream);
     if (e != cudaSuccess) break;
     const int64_t n = (int64_t)c.heads * a.w_rows * 16;
-    bwd_table_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(reinterpret_cast<const float4*>(c.partial), parts, a.w_rows, w0,
-                                                                            c.table_rows, c.heads, static_cast<uint2*>(c.dtable));
+    bwd_table_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(reinterpret_cast<const float4*>(c.partial), parts, a.w_rows, w0, c.heads,
+                                                                            c.table_row_stride, c.table_head_stride, static_cast<__nv_bfloat16*>(c.dtable));
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd tables launch: %s", cudaGetErrorString(e));

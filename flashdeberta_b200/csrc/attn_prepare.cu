@@ -194,7 +194,8 @@ struct ExpandArgs {
   const uint4 *pos_key, *pos_query;
   uint4 *exp_key, *exp_query;
   const int16_t* lut;
-  int lut_d_min, lut_len, d_first, rows, table_rows, heads, vec_per_row;
+  int lut_d_min, lut_len, d_first, rows, heads, vec_per_row;
+  int64_t row_stride, head_stride;  // of the tables, in 16-byte units
 };
 
 __global__ void __launch_bounds__(256) expand_tables_kernel(ExpandArgs a) {
@@ -208,7 +209,7 @@ __global__ void __launch_bounds__(256) expand_tables_kernel(ExpandArgs a) {
     int li = a.d_first + u - a.lut_d_min;
     li = li < 0 ? 0 : (li >= a.lut_len ? a.lut_len - 1 : li);
     const int src = a.lut[li];
-    const int64_t s = ((int64_t)h * a.table_rows + src) * a.vec_per_row + c;
+    const int64_t s = h * a.head_stride + src * a.row_stride + c;
     if (a.pos_key != nullptr) a.exp_key[i] = a.pos_key[s];
     if (a.pos_query != nullptr) a.exp_query[i] = a.pos_query[s];
   }
@@ -240,7 +241,7 @@ int launch_seq_info(const fdb_attn_params& p, const AttnBuffers& b, void* stream
   return FDB_OK;
 }
 
-int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained) {
+int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained, TableStrides strides) {
   const int esz = p.dtype == FDB_E4M3 ? 1 : 2;
   ExpandArgs a;
   a.pos_key = static_cast<const uint4*>(p.pos_key);
@@ -249,8 +250,10 @@ int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, cons
   a.exp_query = static_cast<uint4*>(b.exp_query);
   a.lut = p.bucket_lut; a.lut_d_min = p.lut_d_min; a.lut_len = p.lut_len;
   a.d_first = g.d_first; a.rows = g.rows; a.heads = p.heads;
-  a.table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
   a.vec_per_row = kHeadDim * esz / 16;
+  const int table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
+  a.row_stride = strides.row > 0 ? strides.row * esz / 16 : a.vec_per_row;
+  a.head_stride = strides.row > 0 ? strides.head * esz / 16 : (int64_t)table_rows * a.vec_per_row;
   const int64_t total = (int64_t)p.heads * g.rows * a.vec_per_row;
   const cudaError_t e = launch_kernel<ExpandArgs>(expand_tables_kernel, a, dim3((unsigned)((total + 255) / 256)), 256, 0, chained,
                                                   static_cast<cudaStream_t>(stream));
@@ -258,12 +261,12 @@ int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, cons
   return FDB_OK;
 }
 
-int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool* launched) {
+int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool* launched, TableStrides strides) {
   int rc = FDB_OK;
   const bool schedule = (p.prepared & FDB_PREPARED_SCHEDULE) == 0;
   const bool tables = (p.pos_key != nullptr || p.pos_query != nullptr) && (p.prepared & FDB_PREPARED_TABLES) == 0;
   if (schedule) rc = launch_seq_info(p, b, stream);
-  if (rc == FDB_OK && tables) rc = launch_expand_tables(p, g, b, stream, schedule);
+  if (rc == FDB_OK && tables) rc = launch_expand_tables(p, g, b, stream, schedule, strides);
   *launched = schedule || tables;
   return rc;
 }

@@ -97,9 +97,10 @@ int launch_layernorm(const LayerNormCall& c, void* stream);
 // ---- launchers (defined in the .cu files) --------------------------------------------------------------------------
 int launch_attn_check(const fdb_attn_params& p, void* stream);
 int launch_seq_info(const fdb_attn_params& p, const AttnBuffers& b, void* stream);
-int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained = false);
+struct TableStrides { int64_t row, head; };  // of the position tables, in elements; 0: contiguous (heads, rows, 64)
+int launch_expand_tables(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained = false, TableStrides strides = {0, 0});
 // `launched`: a kernel chained to what this launched may start early
-int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool* launched);
+int launch_prepare(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool* launched, TableStrides strides = {0, 0});
 int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, const AttnBuffers& b, void* stream, bool chained = false);
 int launch_attn_fwd_far1(const void* fwd_args, int64_t slots, int heads, void* stream, bool chained);  // fwd_args: fwd::FwdArgs
 int launch_relative_index_matrix(const int16_t* lut, int32_t d_min, int32_t len, int32_t lq, int32_t lk, int32_t* out,

@@ -2,6 +2,8 @@
 //
 //  * lengths_kernel   valid lengths of a right-padded batch from its mask, and the check that the mask is one: a CTA per
 //                     sequence.  As tensor operators this was nine launches of a few hundred bytes each.
+//  * fdb_projected_forward  the module's forward in training: two launches of the linear kernel, then the attention.  Operator by
+//                     operator (two concatenations, two GEMMs, a transposition, the attention call) it was 110 us of host time.
 //  * column_sums      bias gradients: sums over the rows of one or two bf16 matrices side by side, fp32 inside.  Bound by
 //                     reading them; the row ranges of a column are summed in a fixed order by a second launch.
 #include <cuda_bf16.h>
@@ -10,6 +12,7 @@
 #include <algorithm>
 
 #include "internal.h"
+#include "linear.h"
 #include "sm100_ptx.cuh"
 
 namespace fdb {
@@ -136,4 +139,51 @@ extern "C" FDB_API int fdb_column_sums(const void* x, int64_t rows, int32_t cols
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "column_sums launch: %s", cudaGetErrorString(e));
   return FDB_OK;
+}
+
+extern "C" FDB_API int fdb_projected_forward(const fdb_projected_params* c, void* stream) {
+  clear_error();
+  if (c == nullptr || c->struct_bytes != sizeof(fdb_projected_params))
+    return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_projected_params: NULL or struct_bytes %u != %zu", c ? c->struct_bytes : 0u, sizeof(fdb_projected_params));
+  int rc = validate(c->attn, true);
+  if (rc != FDB_OK) return rc;
+  const fdb_attn_params& p = *c->attn;
+  const int inner = p.heads * kHeadDim, table_rows = 2 * (p.position_buckets > 0 ? p.position_buckets : p.max_relative_positions);
+  if (p.dtype != FDB_BF16 || c->in_features <= 0 || c->in_features % 64 != 0)
+    return fail(FDB_ERR_UNSUPPORTED, "fdb_projected_forward takes bf16 and in_features a multiple of 64");
+  if (!p.pos_key || !p.pos_query || !c->x || !c->rel || !c->wq || !c->bq || !c->wk || !c->bk || !c->wv || !c->bv)
+    return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_projected_forward: NULL pointer");
+  const uintptr_t all = (uintptr_t)c->x | (uintptr_t)c->rel | (uintptr_t)c->wq | (uintptr_t)c->bq | (uintptr_t)c->wk | (uintptr_t)c->bk |
+                        (uintptr_t)c->wv | (uintptr_t)c->bv;
+  if ((all & 15u) != 0 || p.q_row_stride != p.k_row_stride || p.q_row_stride != p.v_row_stride || p.q_head_stride != kHeadDim ||
+      p.k_head_stride != kHeadDim || p.v_head_stride != kHeadDim || c->table_head_stride != kHeadDim || c->table_row_stride < inner ||
+      c->table_row_stride % 8 != 0)
+    return fail(FDB_ERR_ALIGNMENT, "fdb_projected_forward: pointers must be 16-byte aligned, q, k and v rows of one stride, heads 64 apart");
+  if (p.batch == 0 || p.total_rows == 0) return FDB_OK;
+  const ExpandGeometry g = expand_geometry(p.lut_d_min, p.lut_len);
+  const WorkspaceLayout w = workspace_layout(p, g);
+  if (p.workspace == nullptr || p.workspace_bytes < w.total || (reinterpret_cast<uintptr_t>(p.workspace) & 255u) != 0)
+    return fail(FDB_ERR_WORKSPACE, "workspace of %llu bytes needed (256-byte aligned), %llu given", (unsigned long long)w.total, (unsigned long long)p.workspace_bytes);
+  CUtensorMap map_x, map_rel;
+  LinearWeight wq, wk, wv;
+  if ((rc = make_linear_input_map(&map_x, c->x, p.total_rows, c->in_features)) != FDB_OK) return rc;
+  if ((rc = make_linear_input_map(&map_rel, c->rel, table_rows, c->in_features)) != FDB_OK) return rc;
+  if ((rc = make_linear_maps(&wq, c->wq, inner, c->in_features)) != FDB_OK || (rc = make_linear_maps(&wk, c->wk, inner, c->in_features)) != FDB_OK ||
+      (rc = make_linear_maps(&wv, c->wv, inner, c->in_features)) != FDB_OK) return rc;
+  LinearCall lin = {};
+  lin.x_map = &map_x; lin.rows = p.total_rows; lin.out_stride = p.q_row_stride;
+  lin.k = c->in_features; lin.n = inner; lin.groups = 3; lin.status = p.status;
+  lin.weight[0] = &wq; lin.weight[1] = &wk; lin.weight[2] = &wv;
+  lin.bias[0] = c->bq; lin.bias[1] = c->bk; lin.bias[2] = c->bv;
+  lin.out[0] = const_cast<void*>(p.q); lin.out[1] = const_cast<void*>(p.k); lin.out[2] = const_cast<void*>(p.v);
+  if ((rc = launch_linear(lin, stream)) != FDB_OK) return rc;
+  lin.x_map = &map_rel; lin.rows = table_rows; lin.out_stride = c->table_row_stride; lin.groups = 2;
+  lin.out[0] = const_cast<void*>(p.pos_query); lin.out[1] = const_cast<void*>(p.pos_key);
+  if ((rc = launch_linear(lin, stream)) != FDB_OK) return rc;
+  fdb_attn_params q = p;
+  q.prepared = 0;
+  const AttnBuffers b = attn_buffers(q, w);
+  bool prepared;
+  if ((rc = launch_prepare(q, g, b, stream, &prepared, {c->table_row_stride, c->table_head_stride})) != FDB_OK) return rc;
+  return launch_attn_fwd_sm100(q, g, b, stream, prepared);
 }

@@ -225,6 +225,7 @@ typedef struct fdb_attn_bwd_params {
   void *dq, *dk, *dv;           /* out bf16, (total_rows, heads, 64) with the strides below */
   int64_t grad_row_stride, grad_head_stride;
   void *dpos_key, *dpos_query;  /* out bf16 (heads, 2*att_span, 64), each with its table */
+  int64_t table_row_stride, table_head_stride; /* of the position tables and their gradients, in elements; 0, 0: contiguous */
   void* workspace;              /* device, >= fdb_attn_bwd_workspace_bytes(), 256-byte aligned */
   uint64_t workspace_bytes;
 } fdb_attn_bwd_params;
@@ -401,6 +402,20 @@ FDB_API void fdb_encoder_destroy(void* plan);
  * token_stride; FDB_DEV_BAD_MASK in `status` (or NULL) when the valid tokens of a sequence are not its first ones. */
 FDB_API int fdb_lengths_from_mask(const void* mask, int32_t mask_type, int32_t batch, int32_t seqlen, int64_t batch_stride,
                                   int64_t token_stride, int32_t* lens, int32_t* status, void* stream);
+
+/* Forward of the attention module as training needs it, in one call: the three projections of x, the two of the position
+ * embeddings through the same weights (share_att_key), and the attention with its LSE.  The projections are written where `attn`
+ * says that q, k, v, pos_query and pos_key are (q, k and v with one row stride); the tables have the strides below. */
+typedef struct fdb_projected_params {
+  uint32_t struct_bytes;       /* sizeof(fdb_projected_params) */
+  int32_t in_features;         /* a multiple of 64 */
+  const fdb_attn_params* attn; /* bf16, both tables given; workspace as for fdb_attn_fwd */
+  int64_t table_row_stride, table_head_stride;
+  const void* x;               /* bf16 (total_rows, in_features) */
+  const void* rel;             /* bf16 (2*att_span, in_features) */
+  const void *wq, *bq, *wk, *bk, *wv, *bv; /* bf16 (heads*64, in_features), (heads*64) */
+} fdb_projected_params;
+FDB_API int fdb_projected_forward(const fdb_projected_params* p, void* stream);
 
 /* out[c] = sum over the rows of x (rows, cols) and of more (more_rows, more_cols <= cols), bf16, contiguous, summed in fp32:
  * the bias gradients of projections of two inputs through the same weights. */
