@@ -224,8 +224,13 @@ class EncoderEngine:
         with ops.on_device(device):
             stream = ops.raw_stream(device)
             ops._launches += plan.refresh_tables(model.encoder, stream)
-            if plan.tables is not None and stream != plan.table_stream:
-                torch.cuda.current_stream(device).wait_event(plan.table_event)
+            # tables gathered on another stream: wait for them once, until they are known to be there.  A capture cannot wait for
+            # work outside it, and need not: it begins with a synchronisation
+            if plan.tables is not None and plan.table_event is not None and not torch.cuda.is_current_stream_capturing():
+                if plan.table_event.query():
+                    plan.table_event = None
+                elif stream != plan.table_stream:
+                    torch.cuda.current_stream(device).wait_event(plan.table_event)
             need = lib.fdb_encoder_workspace_bytes(C.byref(p))
             ws = torch.empty(need + 256, dtype=torch.uint8, device=device)
             p.workspace, p.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
