@@ -14,7 +14,9 @@
 // that go from memory to registers save the trip through shared memory and tensor memory, so the products are warp MMAs.  Both
 // operands are read 32 bytes per thread: K is permuted the same way in both, which a sum over K does not see.
 //
-// 12 layers of 768, 29 tokens: @@
+// 12 layers of 768, 29 tokens: 607 us a call as 84 launches, 385 in one kernel.  Of a layer (55000 clocks): five barriers 14000, the two
+// LayerNorms 11500, the four products 4000 to 8300 each, attention 6800.  Up to 64 rows, because every CTA normalises all rows and
+// keeps them: at 64 a layer takes 45 us, about what seven launches take.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 

@@ -34,41 +34,6 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait that also gives up as soon as another thread of the CTA has raised `*abort_flag`.
-__device__ __forceinline__ bool mbar_wait_abortable_slow(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_flag) {
-  const long long t0 = clock64();
-#pragma unroll 1
-  for (uint32_t i = 0; i < (1u << 30); ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 63u) == 63u) {
-      if (*abort_flag != 0u) return false;
-      if (clock64() - t0 > 4000000000LL) break;
-    }
-  }
-  return false;
-}
-__device__ __forceinline__ bool mbar_wait_abortable(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_flag) {
-#pragma unroll 1
-  for (int i = 0; i < 32; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_abortable_slow(bar, parity, abort_flag);
-}
-// The same for a role that is not on the critical path: it sleeps between polls, so that its polling does not take issue
-// slots from the warps that share its scheduler.
-__device__ __forceinline__ bool mbar_wait_abortable_relaxed(uint32_t bar, uint32_t parity, const volatile uint32_t* abort_flag) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-#pragma unroll 1
-  for (uint32_t i = 0; i < (1u << 28); ++i) {
-    __nanosleep(100);
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 15u) == 15u) {
-      if (*abort_flag != 0u) return false;
-      if (clock64() - t0 > 4000000000LL) break;
-    }
-  }
-  return false;
-}
 // One lane of a converged warp.  The issuing warps keep whole warps in their loops and let the elected lane issue: the compiler
 // then keeps addresses and descriptors in uniform registers.  Behind a `lane == 0` branch every tcgen05.mma and every TMA
 // load instead pays for moving its operands there one by one: 800 clocks per four MMAs, a commit and a wait, measured in
@@ -100,26 +65,9 @@ __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, vo
 __device__ __forceinline__ void bar_sync(uint32_t id, uint32_t count) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(count) : "memory");
 }
-// Bounded wait: gives up after about two seconds of SM clock and reports false.
-__device__ __forceinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity) {
-  const long long t0 = clock64();
-#pragma unroll 1
-  for (uint32_t i = 0; i < (1u << 30); ++i) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if ((i & 255u) == 255u && clock64() - t0 > 4000000000LL) break;
-  }
-  return false;
-}
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
-#pragma unroll 1
-  for (int i = 0; i < 64; ++i)
-    if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity);
-}
 
 // ---- fences -----------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
-__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -311,12 +259,6 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
       ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
         "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(taddr)
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&r)[8]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
-      ::"r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(taddr)
       : "memory");
 }
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
