@@ -304,7 +304,7 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
   char* ws = static_cast<char*>(c->workspace);
   const int64_t rows = c->total_rows;
   int launches = 0;
-  // Up to 64 rows the layers are one kernel.  (Timing events around the attention of every layer need launches of their own.)
+  // A handful of rows: the layers are one kernel.  (Timing events around the attention of every layer need launches of their own.)
   const bool small = c->attn_events == nullptr && small_encoder_covers(rows, plan.hidden, plan.ffn, (int)plan.layers.size());
   if (small) {
     const cudaError_t e = cudaMemsetAsync(ws + l.barrier, 0, 8, s);

@@ -15,8 +15,8 @@
 // operands are read 32 bytes per thread: K is permuted the same way in both, which a sum over K does not see.
 //
 // 12 layers of 768, 29 tokens: 607 us a call as 84 launches, 385 in one kernel.  Of a layer (55000 clocks): five barriers 14000, the two
-// LayerNorms 11500, the four products 4000 to 8300 each, attention 6800.  Up to 64 rows, because every CTA normalises all rows and
-// keeps them: at 64 a layer takes 45 us, about what seven launches take.
+// LayerNorms 11500, the four products 4000 to 8300 each, attention 6800.  It ends where every CTA normalising all rows costs what the
+// launches cost: see small_encoder_covers.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -454,6 +454,9 @@ size_t smem_bytes(int mt, int hidden, int ffn, int sms) {
 bool small_encoder_covers(int64_t row_bound, int hidden, int ffn, int n_layers) {
   const int sms = sm_count();
   if (sms <= 0 || row_bound > kSmallRows || hidden > 1024 || n_layers > kSmallLayers) return false;
+  // Where it is the faster form.  16 / 32 / 48 / 64 rows, us against the separate launches: 12 layers of 768 351 / 391 / 534 / 567
+  // against 607; 24 layers of 1024 755 / 872 / 1320 / 1480 against 1375.
+  if (row_bound * hidden > 48 * 1024) return false;
   const int most = std::max(3 * hidden, ffn);
   return (most / 8 + sms - 1) / sms <= kMaxTiles && smem_bytes(row_bound <= 16 ? 1 : (row_bound <= 32 ? 2 : 4), hidden, ffn, sms) <= 227 * 1024 - 1024;
 }
