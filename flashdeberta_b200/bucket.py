@@ -11,7 +11,7 @@ import torch
 from . import _lib
 
 _host_cache: Dict[Tuple[int, int], Tuple[np.ndarray, int]] = {}
-_dev_cache: Dict[Tuple[int, int, str], torch.Tensor] = {}
+_dev_cache: Dict[Tuple[int, int, torch.device], Tuple[torch.Tensor, int]] = {}
 
 
 def att_span(position_buckets: int, max_relative_positions: int) -> int:
@@ -34,11 +34,12 @@ def host_lut(position_buckets: int, max_relative_positions: int) -> Tuple[np.nda
 
 
 def device_lut(position_buckets: int, max_relative_positions: int, device: torch.device) -> Tuple[torch.Tensor, int]:
-    tab, d_min = host_lut(position_buckets, max_relative_positions)
-    key = (int(position_buckets), int(max_relative_positions), str(device))
-    if key not in _dev_cache:
-        _dev_cache[key] = torch.from_numpy(tab).to(device)
-    return _dev_cache[key], d_min
+    key = (int(position_buckets), int(max_relative_positions), device)
+    found = _dev_cache.get(key)
+    if found is None:
+        tab, d_min = host_lut(position_buckets, max_relative_positions)
+        found = _dev_cache[key] = (torch.from_numpy(tab).to(device), d_min)
+    return found
 
 
 def relative_index(distance: int, position_buckets: int, max_relative_positions: int) -> int:

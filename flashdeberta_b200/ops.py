@@ -218,6 +218,8 @@ _PARAMS_BYTES = C.sizeof(_lib.AttnParams)
 
 
 def _out_like(q: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    if q.is_contiguous():  # (the layout of q is the layout of the output: the call with fewest arguments to look at)
+        return torch.empty_like(q) if q.dtype == dtype else torch.empty_like(q, dtype=dtype)
     return torch.empty(q.shape, dtype=dtype, device=q.device)
 
 
