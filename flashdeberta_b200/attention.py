@@ -118,9 +118,10 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
         # (rows, H*D) -> (H, rows, D)
         return x.view(x.shape[0], self.num_attention_heads, -1).permute(1, 0, 2).contiguous()
 
-    def _position_tables(self, rel_embeddings: torch.Tensor, dtype: torch.dtype):
+    def _position_tables(self, rel_embeddings: torch.Tensor, dtype: torch.dtype, keep: bool = True):
         """pos_key_layer / pos_query_layer of model.py:159-177, head-major (H, 2*span, D).  They do not depend on the
-        input, so in eval mode they are kept until a parameter or the embedding table changes."""
+        input, so in eval mode they are kept until a parameter or the embedding table changes (``keep`` false: made from the
+        parameters, and not kept)."""
         c2p = "c2p" in self.pos_att_type
         p2c = "p2c" in self.pos_att_type
         if self.share_att_key:
@@ -128,7 +129,7 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
         else:
             wk, wq = getattr(self, "pos_key_proj", None), getattr(self, "pos_query_proj", None)
         key = None
-        if not self.training and not torch.is_grad_enabled() and not torch.compiler.is_compiling():
+        if keep and not self.training and not torch.is_grad_enabled() and not torch.compiler.is_compiling():
             # the table is kept alive below, so its identity stays its own
             key = (id(rel_embeddings), ops.tensor_stamp(rel_embeddings, held=True), rel_embeddings.device, dtype,
                    tuple(ops.tensor_stamp(p, held=True) for m in (wk, wq) if m is not None for p in m.parameters()))
@@ -138,7 +139,7 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
         rel = self.pos_dropout(rel_embeddings)[:span2]
         pos_key = self._heads_first(wk(rel)).to(dtype) if c2p else None
         pos_query = self._heads_first(wq(rel)).to(dtype) if p2c else None
-        if key is not None:
+        if key is not None and not ops.capturing(rel_embeddings):  # (what a capture records has not been computed)
             self._pos_cache = (key, pos_key, pos_query, rel_embeddings)  # keep the table alive so id() stays unique
         return pos_key, pos_query
 

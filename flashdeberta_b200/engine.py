@@ -149,24 +149,34 @@ class _Plan:
         """No hooks, no module in training mode, no patched ``forward``: nothing a module walk would do beside the arithmetic."""
         return not any(self.hooks) and not any([d["training"] or "forward" in d for d in self.attrs])
 
-    def refresh_tables(self, encoder, stream) -> int:
-        """Gathers the projected position tables of every layer again when a parameter behind them was written to."""
-        versions = [p._version for p in self.table_params]
-        if self.tables is None or versions == self.table_versions:
-            return 0
+    def versions(self):
+        """What the gathered tables depend on, as it is now."""
+        return [p._version for p in self.table_params]
+
+    def gather(self, encoder, stream, keep: bool = True) -> int:
+        """Gathers the projected position tables of every layer, from what the modules keep of them or (``keep`` false) from the
+        parameters alone.  Returns the kernels launched."""
         lib = _lib.load()
-        rel = encoder.get_rel_embedding()
+        rel = encoder.get_rel_embedding(keep)
         for i, a in enumerate(self.attention):
-            pos_key, pos_query = a._position_tables(rel, torch.bfloat16)
+            pos_key, pos_query = a._position_tables(rel, torch.bfloat16, keep)
             any_table = pos_key if pos_key is not None else pos_query
             _lib.check(lib.fdb_expand_tables(
                 pos_key.data_ptr() if self.c2p else None, pos_query.data_ptr() if self.p2c else None,
                 self.tables[i, 0].data_ptr() if self.c2p else None, self.tables[i, 1].data_ptr() if self.p2c else None,
                 self.heads, any_table.shape[1], self.lut.data_ptr(), self.d_min, self.lut.numel(), C.c_void_p(stream)))
+        return len(self.attention)
+
+    def refresh_tables(self, encoder, stream) -> int:
+        """Gathers the tables again when a parameter behind them was written to."""
+        versions = self.versions()
+        if self.tables is None or versions == self.table_versions:
+            return 0
+        launched = self.gather(encoder, stream)
         self.table_versions, self.table_stream = versions, stream
         self.table_event = torch.cuda.Event()
         self.table_event.record()
-        return len(self.attention)
+        return launched
 
 
 class EncoderEngine:
@@ -185,8 +195,14 @@ class EncoderEngine:
                 max_seqlen: int) -> Optional[torch.Tensor]:
         """Last hidden state of (B, L) ids with an optional (B, L) mask, or of (1, T) packed ids with ``cu_seqlens``.  None
         when the model or the call is not covered."""
-        plan = self.plan
-        if plan is None or not plan.current():
+        plan, capturing = self.plan, ops.capturing(ids)
+        # What a captured call launches has not run when the call returns, so nothing that it sets up may be taken for done by
+        # another call: where the plan or its tables are not up to date, a captured call makes its own, and its graph gathers
+        # the tables whenever it is replayed.
+        own = capturing and (plan is None or not plan.current() or (plan.ok and plan.tables is not None and plan.versions() != plan.table_versions))
+        if own:
+            plan = _Plan(model)
+        elif plan is None or not plan.current():
             plan = self.plan = _Plan(model)
         if not plan.ok or ids.device != plan.device or not plan.plain():
             return None
@@ -223,14 +239,17 @@ class EncoderEngine:
         p.status = ops._status_word(device).data_ptr()
         with ops.on_device(device):
             stream = ops.raw_stream(device)
-            ops._launches += plan.refresh_tables(model.encoder, stream)
-            # tables gathered on another stream: wait for them once, until they are known to be there.  A capture cannot wait for
-            # work outside it, and need not: it begins with a synchronisation
-            if plan.tables is not None and plan.table_event is not None and not torch.cuda.is_current_stream_capturing():
-                if plan.table_event.query():
-                    plan.table_event = None
-                elif stream != plan.table_stream:
-                    torch.cuda.current_stream(device).wait_event(plan.table_event)
+            if own and plan.tables is not None:
+                ops._launches += plan.gather(model.encoder, stream, keep=False)
+            elif not capturing:
+                ops._launches += plan.refresh_tables(model.encoder, stream)
+                # tables gathered on another stream: wait for them once, until they are known to be there.  A capture cannot wait for
+                # work outside it, and need not: it begins with a synchronisation
+                if plan.tables is not None and plan.table_event is not None:
+                    if plan.table_event.query():
+                        plan.table_event = None
+                    elif stream != plan.table_stream:
+                        torch.cuda.current_stream(device).wait_event(plan.table_event)
             need = lib.fdb_encoder_workspace_bytes(C.byref(p))
             ws = torch.empty(need + 256, dtype=torch.uint8, device=device)
             p.workspace, p.workspace_bytes = (ws.data_ptr() + 255) & ~255, need

@@ -153,17 +153,20 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
         self._mask_cache = None
         self.config_pack = config
 
-    def get_rel_embedding(self):
+    def get_rel_embedding(self, keep: bool = True):
         """LayerNorm(rel_embeddings) does not depend on the input: in eval mode it is computed once and reused, which
-        also lets every layer keep its projected position tables."""
-        if self.training or torch.is_grad_enabled() or not self.relative_attention:
+        also lets every layer keep its projected position tables (``keep`` false: computed, and not kept)."""
+        if not keep or self.training or torch.is_grad_enabled() or not self.relative_attention:
             return super().get_rel_embedding()
         w = self.rel_embeddings.weight
         key = [ops.tensor_stamp(w, held=True), w.dtype, w.device]
         if "layer_norm" in self.norm_rel_ebd:
             key += [ops.tensor_stamp(self.LayerNorm.weight, held=True), ops.tensor_stamp(self.LayerNorm.bias, held=True)]
         if self._rel_cache is None or self._rel_cache[0] != key:
-            self._rel_cache = (key, super().get_rel_embedding())
+            rel = super().get_rel_embedding()
+            if ops.capturing(w):  # recorded, not computed
+                return rel
+            self._rel_cache = (key, rel)
         return self._rel_cache[1]
 
     def forward(self, hidden_states, attention_mask, output_hidden_states=True, output_attentions=False,

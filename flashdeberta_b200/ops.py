@@ -95,6 +95,14 @@ def raw_stream(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
+def capturing(t: torch.Tensor) -> bool:
+    """Whether the current stream of the tensor's device is being captured into a CUDA graph."""
+    if not t.is_cuda:
+        return False
+    with on_device(t.device):
+        return torch.cuda.is_current_stream_capturing()
+
+
 def lengths_from_mask(mask: torch.Tensor) -> torch.Tensor:
     """int32 lengths of the rows of a (batch, tokens) mask on the GPU, any strides; flags a mask that is not right-padded in
     the device status word."""

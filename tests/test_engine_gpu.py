@@ -1,0 +1,72 @@
+"""GPU tests of what the encoder's one-call inference keeps between calls (flashdeberta_b200/engine.py): when it is made again, and
+who may rely on it.  The reference for every output is the module walk (taken when the layers' hidden states are asked for)."""
+import pytest
+import torch
+
+from tests.test_configs_gpu import _close, _ragged, _small_config
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda"
+
+
+def _model(**kw):
+    from flashdeberta_b200 import FlashDebertaV2Model
+    torch.manual_seed(0)
+    return FlashDebertaV2Model(_small_config("b200", **kw)).eval().to(DEV).bfloat16()
+
+
+def _walk(model, ids, mask):
+    return model(input_ids=ids, attention_mask=mask, output_hidden_states=True).last_hidden_state
+
+
+def _capture(run):
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        out = run()
+    return graph, out
+
+
+@pytest.mark.parametrize("rows", [40, 600])
+def test_capture_after_a_weight_was_written(rows):
+    """The position tables depend on the key projection.  Written to between the warm-up and the capture, a graph has to gather
+    them itself, and the calls around it (eager, before and after a replay) have to be right too."""
+    from flashdeberta_b200 import ops
+    model = _model()
+    ids, mask = _ragged(1, rows, (rows - 3,))
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    with torch.no_grad():
+        old = run()
+        for layer in model.encoder.layer:
+            layer.attention.self.key_proj.weight.mul_(3.0)
+        graph, out = _capture(run)
+        eager = run()                   # before the graph has ever run
+        assert not torch.equal(eager, old)
+        _close(eager, _walk(model, ids, mask), 0.1, 5e-3, "eager after the capture")
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, eager)
+        for layer in model.encoder.layer:
+            layer.attention.self.key_proj.weight.mul_(0.5)
+        graph.replay()                  # the graph that gathers sees the weights of its replay
+        torch.cuda.synchronize()
+        assert torch.equal(out, run())
+    ops.check_status()
+
+
+def test_first_call_of_a_plan_inside_a_capture():
+    """A parameter replaced between warm-up and capture: the plan of the captured call is the graph's own."""
+    model = _model()
+    ids, mask = _ragged(2, 300, (300, 170))
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    with torch.no_grad():
+        run()
+        proj = model.encoder.layer[0].attention.self.key_proj
+        proj.weight = torch.nn.Parameter(proj.weight * 2)
+        graph, out = _capture(run)
+        eager = run()
+        _close(eager, _walk(model, ids, mask), 0.1, 5e-3, "eager after the capture")
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, eager)
