@@ -10,6 +10,7 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 from typing import Optional
 
 import torch
@@ -37,6 +38,17 @@ class EncoderCall(C.Structure):
         ("emb_beta", C.c_void_p), ("emb_rows", C.c_int64), ("out", C.c_void_p), ("workspace", C.c_void_p),
         ("workspace_bytes", C.c_uint64), ("status", C.c_void_p), ("attn_events", C.c_void_p), ("launches", C.c_int32),
     ]
+
+
+class _Tables:
+    """The projected position tables of every layer, gathered through the bucket index.  The lock covers everything but ``data``: a
+    thread that finds ``versions`` up to date also finds the event that its stream has to wait for."""
+
+    def __init__(self, shape, device):
+        self.data = torch.empty(shape, dtype=torch.bfloat16, device=device)
+        self.lock = threading.Lock()
+        self.versions = None             # of the parameters that `data` was gathered from
+        self.stream = self.event = None  # the stream it was gathered on; the end of it, until that is known to be reached
 
 
 class _Plan:
@@ -102,7 +114,7 @@ class _Plan:
         if self.c2p or self.p2c:
             self.lut, self.d_min = bucket.device_lut(self.buckets, self.max_rel, device)
             rows = _lib.load().fdb_expanded_rows(self.d_min, self.lut.numel())
-            self.tables = torch.empty(len(enc.layer), 2, heads, rows, 64, dtype=torch.bfloat16, device=device)
+            self.tables = _Tables((len(enc.layer), 2, heads, rows, 64), device)
         # the parameters that the gathered tables depend on
         table_params = [enc.rel_embeddings.weight, *(enc.LayerNorm.parameters() if "layer_norm" in enc.norm_rel_ebd else ())]
         for a in self.attention:
@@ -112,7 +124,6 @@ class _Plan:
                 if m is not None:
                     table_params += list(m.parameters())
         self.table_params = [p for p in table_params if not p.is_inference()]  # (those cannot be written to)
-        self.table_versions = None
         self._create(enc)
 
     def _create(self, enc):
@@ -127,8 +138,8 @@ class _Plan:
                 setattr(d, "b" + name, ptr(m.bias))
             d.ln1_gamma, d.ln1_beta, d.ln1_eps = ptr(o.LayerNorm.weight), ptr(o.LayerNorm.bias), o.LayerNorm.eps
             d.ln2_gamma, d.ln2_beta, d.ln2_eps = ptr(layer.output.LayerNorm.weight), ptr(layer.output.LayerNorm.bias), layer.output.LayerNorm.eps
-            d.exp_key = ptr(self.tables[i, 0]) if self.c2p else None
-            d.exp_query = ptr(self.tables[i, 1]) if self.p2c else None
+            d.exp_key = ptr(self.tables.data[i, 0]) if self.c2p else None
+            d.exp_query = ptr(self.tables.data[i, 1]) if self.p2c else None
         ffn = enc.layer[0].intermediate.dense.out_features
         with ops.on_device(self.device):
             rc = _lib.load().fdb_encoder_create(C.byref(descs), n, self.hidden, self.heads, ffn, C.byref(self.handle))
@@ -153,29 +164,39 @@ class _Plan:
         """What the gathered tables depend on, as it is now."""
         return [p._version for p in self.table_params]
 
-    def gather(self, encoder, stream, keep: bool = True) -> int:
-        """Gathers the projected position tables of every layer, from what the modules keep of them or (``keep`` false) from the
-        parameters alone.  Returns the kernels launched."""
+    def gather(self, encoder, stream) -> int:
+        """Gathers the projected position tables of every layer, from the parameters alone: what the modules keep of them may be on
+        its way on another stream.  Returns the kernels launched."""
         lib = _lib.load()
-        rel = encoder.get_rel_embedding(keep)
+        rel = encoder.get_rel_embedding(keep=False)
         for i, a in enumerate(self.attention):
-            pos_key, pos_query = a._position_tables(rel, torch.bfloat16, keep)
+            pos_key, pos_query = a._position_tables(rel, torch.bfloat16, keep=False)
             any_table = pos_key if pos_key is not None else pos_query
             _lib.check(lib.fdb_expand_tables(
                 pos_key.data_ptr() if self.c2p else None, pos_query.data_ptr() if self.p2c else None,
-                self.tables[i, 0].data_ptr() if self.c2p else None, self.tables[i, 1].data_ptr() if self.p2c else None,
+                self.tables.data[i, 0].data_ptr() if self.c2p else None, self.tables.data[i, 1].data_ptr() if self.p2c else None,
                 self.heads, any_table.shape[1], self.lut.data_ptr(), self.d_min, self.lut.numel(), C.c_void_p(stream)))
         return len(self.attention)
 
-    def refresh_tables(self, encoder, stream) -> int:
-        """Gathers the tables again when a parameter behind them was written to."""
-        versions = self.versions()
-        if self.tables is None or versions == self.table_versions:
+    def refresh_tables(self, encoder, stream, device) -> int:
+        """Gathers the tables again when a parameter behind them was written to, and lets this stream wait for a gathering on another
+        one, until that is known to be over.  Returns the kernels launched."""
+        t, launched = self.tables, 0
+        if t is None:
             return 0
-        launched = self.gather(encoder, stream)
-        self.table_versions, self.table_stream = versions, stream
-        self.table_event = torch.cuda.Event()
-        self.table_event.record()
+        versions = self.versions()
+        with t.lock:
+            if t.versions != versions:
+                t.versions = None  # should anything below fail
+                launched = self.gather(encoder, stream)
+                event = torch.cuda.Event()
+                event.record()
+                t.versions, t.stream, t.event = versions, stream, event
+            elif t.event is not None:
+                if t.event.query():
+                    t.event = None
+                elif stream != t.stream:
+                    torch.cuda.current_stream(device).wait_event(t.event)
         return launched
 
 
@@ -199,7 +220,7 @@ class EncoderEngine:
         # What a captured call launches has not run when the call returns, so nothing that it sets up may be taken for done by
         # another call: where the plan or its tables are not up to date, a captured call makes its own, and its graph gathers
         # the tables whenever it is replayed.
-        own = capturing and (plan is None or not plan.current() or (plan.ok and plan.tables is not None and plan.versions() != plan.table_versions))
+        own = capturing and (plan is None or not plan.current() or (plan.ok and plan.tables is not None and plan.versions() != plan.tables.versions))
         if own:
             plan = _Plan(model)
         elif plan is None or not plan.current():
@@ -240,16 +261,9 @@ class EncoderEngine:
         with ops.on_device(device):
             stream = ops.raw_stream(device)
             if own and plan.tables is not None:
-                ops._launches += plan.gather(model.encoder, stream, keep=False)
-            elif not capturing:
-                ops._launches += plan.refresh_tables(model.encoder, stream)
-                # tables gathered on another stream: wait for them once, until they are known to be there.  A capture cannot wait for
-                # work outside it, and need not: it begins with a synchronisation
-                if plan.tables is not None and plan.table_event is not None:
-                    if plan.table_event.query():
-                        plan.table_event = None
-                    elif stream != plan.table_stream:
-                        torch.cuda.current_stream(device).wait_event(plan.table_event)
+                ops._launches += plan.gather(model.encoder, stream)
+            elif not capturing:  # (a capture cannot wait for work outside it, and need not: it begins with a synchronisation)
+                ops._launches += plan.refresh_tables(model.encoder, stream, device)
             need = lib.fdb_encoder_workspace_bytes(C.byref(p))
             ws = torch.empty(need + 256, dtype=torch.uint8, device=device)
             p.workspace, p.workspace_bytes = (ws.data_ptr() + 255) & ~255, need

@@ -70,3 +70,54 @@ def test_first_call_of_a_plan_inside_a_capture():
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, eager)
+
+
+def test_tables_are_published_behind_their_event(monkeypatch):
+    """A second thread that calls the model while the first one is still gathering the tables must not take them for gathered: it waits
+    until the gathering and its event are on the first one's stream, and has its own stream wait for that event."""
+    import threading
+    from flashdeberta_b200 import ops
+    from flashdeberta_b200.attention import FlashDisentangledSelfAttention
+    model = _model()
+    ids, mask = _ragged(1, 600, (500,))
+    with torch.no_grad():
+        model(input_ids=ids, attention_mask=mask)  # plan and buffers
+        model.encoder.layer[2].attention.self.key_proj.weight.mul_(3.0)
+        want = _walk(model, ids, mask)
+    torch.cuda.synchronize()
+    started, go_on, outs, errors = threading.Event(), threading.Event(), {}, []
+    position_tables = FlashDisentangledSelfAttention._position_tables
+
+    def late_tables(self, *a, **kw):
+        torch.cuda._sleep(50_000_000)              # the gathering takes some 80 ms on its stream
+        return position_tables(self, *a, **kw)
+
+    class LateEvent(torch.cuda.Event):             # the moment between the making of an event and its record
+        def record(self, *a, **kw):
+            started.set()
+            go_on.wait(2.0)
+            return super().record(*a, **kw)
+
+    monkeypatch.setattr(FlashDisentangledSelfAttention, "_position_tables", late_tables)
+    monkeypatch.setattr(torch.cuda, "Event", LateEvent)
+
+    def call(name):
+        try:
+            with torch.no_grad(), torch.cuda.stream(torch.cuda.Stream()):
+                outs[name] = model(input_ids=ids, attention_mask=mask).last_hidden_state
+                torch.cuda.current_stream().synchronize()
+        except Exception as e:  # noqa: BLE001 (reported below)
+            errors.append(e)
+
+    first = threading.Thread(target=call, args=("first",))
+    first.start()
+    started.wait(10.0)
+    second = threading.Thread(target=call, args=("second",))
+    second.start()
+    second.join(0.3)
+    go_on.set()
+    first.join(), second.join()
+    assert not errors, errors
+    assert torch.equal(outs["first"], outs["second"])
+    _close(outs["second"], want, 0.1, 5e-3, "second thread")
+    ops.check_status()
