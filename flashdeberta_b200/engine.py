@@ -44,8 +44,12 @@ class _Tables:
     """The projected position tables of every layer, gathered through the bucket index.  The lock covers everything but ``data``: a
     thread that finds ``versions`` up to date also finds the event that its stream has to wait for."""
 
-    def __init__(self, shape, device):
-        self.data = torch.empty(shape, dtype=torch.bfloat16, device=device)
+    def __init__(self, shape, device, params):
+        self.params = params             # held, so that nothing else gets their identities
+        with ops.on_device(device):
+            self.data = torch.empty(shape, dtype=torch.bfloat16, device=device)
+            self.streams = {ops.raw_stream(device)}  # those that the allocator knows to read `data`
+        self.captured = False            # a graph may read `data`
         self.lock = threading.Lock()
         self.versions = None             # of the parameters that `data` was gathered from
         self.stream = self.event = None  # the stream it was gathered on; the end of it, until that is known to be reached
@@ -55,7 +59,8 @@ class _Plan:
     """What one walk over the model found: the library's plan, the objects it was made from (to notice a change) and the
     position tables gathered for every layer."""
 
-    def __init__(self, model):
+    def __init__(self, model, kept=()):
+        """``kept``: (key, tables) to take over where they are of the same parameters."""
         from .attention import FlashDisentangledSelfAttention
         from . import model as M
         enc, emb, cfg = model.encoder, model.embeddings, model.config
@@ -110,11 +115,6 @@ class _Plan:
         self.sm_scale = 1.0 / math.sqrt(64 * (1 + int(self.c2p) + int(self.p2c)))
         self.buckets, self.max_rel = attn0.position_buckets, attn0.max_relative_positions
         self.attention = [layer.attention.self for layer in enc.layer]
-        self.lut, self.d_min, self.tables = None, 0, None
-        if self.c2p or self.p2c:
-            self.lut, self.d_min = bucket.device_lut(self.buckets, self.max_rel, device)
-            rows = _lib.load().fdb_expanded_rows(self.d_min, self.lut.numel())
-            self.tables = _Tables((len(enc.layer), 2, heads, rows, 64), device)
         # the parameters that the gathered tables depend on
         table_params = [enc.rel_embeddings.weight, *(enc.LayerNorm.parameters() if "layer_norm" in enc.norm_rel_ebd else ())]
         for a in self.attention:
@@ -123,7 +123,14 @@ class _Plan:
                 m = getattr(a, name, None)
                 if m is not None:
                     table_params += list(m.parameters())
-        self.table_params = [p for p in table_params if not p.is_inference()]  # (those cannot be written to)
+        self.table_params = [p for p in table_params if not p.is_inference()]  # (those have no version counter)
+        self.lut, self.d_min, self.tables = None, 0, None
+        if self.c2p or self.p2c:
+            self.lut, self.d_min = bucket.device_lut(self.buckets, self.max_rel, device)
+            rows = _lib.load().fdb_expanded_rows(self.d_min, self.lut.numel())
+            shape = (len(enc.layer), 2, heads, rows, 64)
+            self.table_key = (device, shape, self.c2p, self.p2c, self.buckets, self.max_rel, [(id(p), p.data_ptr()) for p in table_params])
+            self.tables = next((t for key, t in kept if key == self.table_key), None) or _Tables(shape, device, table_params)
         self._create(enc)
 
     def _create(self, enc):
@@ -197,6 +204,9 @@ class _Plan:
                     t.event = None
                 elif stream != t.stream:
                     torch.cuda.current_stream(device).wait_event(t.event)
+            if stream not in t.streams:  # once freed, the memory may be another tensor's only behind this stream's calls
+                t.data.record_stream(torch.cuda.current_stream(device))
+                t.streams.add(stream)
         return launched
 
 
@@ -205,6 +215,18 @@ class EncoderEngine:
 
     def __init__(self):
         self.plan: Optional[_Plan] = None
+        self.kept = []  # (key, tables) that graphs captured with earlier plans of the same weights read
+
+    def _replace_plan(self, model) -> _Plan:
+        """A plan of the model as it is now.  Tables that a captured graph reads stay until the weights, which it reads too, are
+        others; a plan of the same parameters and bucket table takes its predecessor's over."""
+        old, kept = self.plan, self.kept
+        if old is not None and old.tables is not None:
+            kept = kept + [(old.table_key, old.tables)]
+        plan = _Plan(model, kept)
+        same = old is not None and plan.addresses == old.addresses
+        self.plan, self.kept = plan, [(key, t) for key, t in kept if same and t.captured and t is not plan.tables]
+        return plan
 
     def __deepcopy__(self, memo):
         return EncoderEngine()
@@ -224,7 +246,7 @@ class EncoderEngine:
         if own:
             plan = _Plan(model)
         elif plan is None or not plan.current():
-            plan = self.plan = _Plan(model)
+            plan = self._replace_plan(model)
         if not plan.ok or ids.device != plan.device or not plan.plain():
             return None
         device = plan.device
@@ -264,6 +286,8 @@ class EncoderEngine:
                 ops._launches += plan.gather(model.encoder, stream)
             elif not capturing:  # (a capture cannot wait for work outside it, and need not: it begins with a synchronisation)
                 ops._launches += plan.refresh_tables(model.encoder, stream, device)
+            elif plan.tables is not None:
+                plan.tables.captured = True
             need = lib.fdb_encoder_workspace_bytes(C.byref(p))
             ws = torch.empty(need + 256, dtype=torch.uint8, device=device)
             p.workspace, p.workspace_bytes = (ws.data_ptr() + 255) & ~255, need

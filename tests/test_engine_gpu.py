@@ -121,3 +121,66 @@ def test_tables_are_published_behind_their_event(monkeypatch):
     assert torch.equal(outs["first"], outs["second"])
     _close(outs["second"], want, 0.1, 5e-3, "second thread")
     ops.check_status()
+
+
+def _scribble(nbytes, n=24):
+    """Memory of this size from the current stream's pool, overwritten."""
+    return [torch.full((nbytes // 2,), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(n)]
+
+
+def test_tables_outlive_the_calls_of_other_streams():
+    """A call on another stream still reads the tables when a weight is replaced and the plan they belong to goes: their memory must
+    not be handed out before that call is over."""
+    model = _model()
+    ids, mask = _ragged(1, 600, (500,))
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    side = torch.cuda.Stream()
+    with torch.no_grad():
+        size = 3 * 2 * 4 * 1527 * 64 * 2  # layers, terms, heads, rows, features, bytes
+        proj = model.encoder.layer[0].attention.self.key_proj
+        for _ in range(2):  # (a kernel's first launch may wait for the device)
+            proj.weight = torch.nn.Parameter(proj.weight.clone())
+            want = run()
+            junk = _scribble(size)
+        del junk
+        torch.cuda.synchronize()
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(200_000_000)
+            got = run()
+        assert not side.query()
+        held, proj.weight = proj.weight, torch.nn.Parameter(proj.weight.clone())
+        run()
+        junk = _scribble(size, 48)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+    del held, junk
+
+
+def test_tables_outlive_the_plan_a_graph_was_captured_with():
+    """Another plan for the same weights (a module was swapped): a graph captured before still reads valid tables."""
+    model = _model()
+    ids, mask = _ragged(1, 600, (500,))
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    with torch.no_grad():
+        want = run()
+        graph, out = _capture(run)
+        model.encoder.layer[0].output.dropout = torch.nn.Dropout(0.0).eval()
+        assert torch.equal(run(), want)
+        junk = _scribble(3 * 2 * 4 * 1527 * 64 * 2)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    del junk
+
+
+def test_tables_of_a_weight_with_other_storage():
+    """The same parameter with other storage (no version counted): the tables are gathered again."""
+    model = _model()
+    ids, mask = _ragged(2, 300, (300, 170))
+    with torch.no_grad():
+        model(input_ids=ids, attention_mask=mask)
+        for layer in model.encoder.layer:
+            weight = layer.attention.self.query_proj.weight
+            weight.data = weight.data * 3
+        got = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        _close(got, _walk(model, ids, mask), 0.1, 5e-3, "other storage")
