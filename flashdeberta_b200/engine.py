@@ -2,9 +2,11 @@
 
 The modules of model.py stay the interface and the owner of every parameter; this walks them once, hands their addresses to
 the library, and from then on a forward of the backbone is one C call instead of a dozen torch operators per layer
-(src/flashdeberta/model.py:275-310 of the reference is the module walk it stands for).  Everything it relies on is looked
-at again on every call — parameters replaced or moved, modules swapped, hooks, training mode — and whatever it does not
-cover goes through the modules as before.
+(src/flashdeberta/model.py:275-310 of the reference is the module walk it stands for).  What it relies on is looked
+at again on every call — parameters replaced or moved, modules swapped, the modules' own settings, hooks, training mode — and
+whatever it does not cover goes through the modules as before.  As in the modules' caches, a parameter counts as unchanged while its
+address and version counter are: a write that bypasses the counter (through ``.data``, a raw kernel) to one behind the position
+tables is not seen.
 """
 from __future__ import annotations
 
@@ -38,6 +40,11 @@ class EncoderCall(C.Structure):
         ("emb_beta", C.c_void_p), ("emb_rows", C.c_int64), ("out", C.c_void_p), ("workspace", C.c_void_p),
         ("workspace_bytes", C.c_uint64), ("status", C.c_void_p), ("attn_events", C.c_void_p), ("launches", C.c_int32),
     ]
+
+
+#: settings of the modules that a plan copies or that decide whether it covers the model
+_SETTINGS = ("attn_fp8", "num_attention_heads", "attention_head_size", "pos_att_type", "relative_attention", "position_buckets",
+             "max_relative_positions", "pos_ebd_size", "share_att_key", "eps", "_erf_gelu", "norm_rel_ebd", "max_norm", "position_biased_input")
 
 
 class _Tables:
@@ -76,6 +83,8 @@ class _Plan:
         self.param_ids = [id(v) for d in self.param_dicts for v in d.values()]
         self.addresses = [p.data_ptr() for p in self.params]
         self.keep = modules
+        self.setting_of = [(d, name) for d in self.attrs for name in _SETTINGS if name in d]
+        self.settings = [list(v) if isinstance(v, list) else v for v in (d[name] for d, name in self.setting_of)]  # (lists may be written to)
         if type(enc) is not M.FlashDebertaV2Encoder or enc.conv is not None or not enc.relative_attention or len(enc.layer) == 0 or type(emb) is not M.FlashDebertaV2Embeddings:
             return
         if emb.position_embeddings is not None or emb.position_biased_input or emb.token_type_embeddings is not None or emb.embed_proj is not None:
@@ -129,7 +138,7 @@ class _Plan:
             self.lut, self.d_min = bucket.device_lut(self.buckets, self.max_rel, device)
             rows = _lib.load().fdb_expanded_rows(self.d_min, self.lut.numel())
             shape = (len(enc.layer), 2, heads, rows, 64)
-            self.table_key = (device, shape, self.c2p, self.p2c, self.buckets, self.max_rel, [(id(p), p.data_ptr()) for p in table_params])
+            self.table_key = (device, shape, self.c2p, self.p2c, self.buckets, self.max_rel, getattr(enc, "LayerNorm", enc).__dict__.get("eps"), [(id(p), p.data_ptr()) for p in table_params])
             self.tables = next((t for key, t in kept if key == self.table_key), None) or _Tables(shape, device, table_params)
         self._create(enc)
 
@@ -158,8 +167,10 @@ class _Plan:
             self.handle = None
 
     def current(self) -> bool:
-        """Whether the model still is the one this plan was made from: same modules and parameters at the same addresses."""
-        return ([id(v) for d in self.module_dicts for v in d.values()] == self.module_ids
+        """Whether the model still is the one this plan was made from: same modules and settings, same parameters at the same
+        addresses."""
+        return ([d.get(name) for d, name in self.setting_of] == self.settings
+                and [id(v) for d in self.module_dicts for v in d.values()] == self.module_ids
                 and [id(v) for d in self.param_dicts for v in d.values()] == self.param_ids
                 and [p.data_ptr() for p in self.params] == self.addresses)
 

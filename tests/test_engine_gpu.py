@@ -184,3 +184,44 @@ def test_tables_of_a_weight_with_other_storage():
             weight.data = weight.data * 3
         got = model(input_ids=ids, attention_mask=mask).last_hidden_state
         _close(got, _walk(model, ids, mask), 0.1, 5e-3, "other storage")
+
+
+def _all_layers(set_one):
+    return lambda model: [set_one(layer) for layer in model.encoder.layer]
+
+
+@pytest.mark.parametrize("change", [
+    _all_layers(lambda l: setattr(l.attention.self, "attn_fp8", True)),
+    _all_layers(lambda l: setattr(l.attention.output.LayerNorm, "eps", 0.5)),
+    _all_layers(lambda l: setattr(l.output.LayerNorm, "eps", 0.5)),
+    lambda model: model.encoder.layer[0].attention.self.pos_att_type.remove("p2c"),  # (one list, which the layers share)
+    _all_layers(lambda l: setattr(l.attention.self, "max_relative_positions", 300)),
+    _all_layers(lambda l: setattr(l.intermediate, "_erf_gelu", False) or setattr(l.intermediate, "intermediate_act_fn", torch.nn.ReLU())),
+    lambda model: setattr(model.encoder.layer[1].attention.self, "attn_fp8", True),
+    lambda model: setattr(model.encoder.LayerNorm, "eps", 0.5),
+], ids=["attn_fp8", "attention eps", "output eps", "pos_att_type", "max_relative_positions", "activation", "attn_fp8 of one layer", "table eps"])
+def test_encoder_call_notices_settings(change):
+    """A setting of a module, changed between two calls, holds from the next one on (and so does changing it back)."""
+    from flashdeberta_b200 import ops
+    model = _model()
+    ids, mask = _ragged(2, 600, (600, 333))
+    with torch.no_grad():
+        first = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        change(model)
+        got = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        assert not torch.equal(got, first)
+        _close(got, _walk(model, ids, mask), 0.1, 5e-3, "changed")
+    ops.check_status()
+
+
+def test_settings_back_and_forth():
+    model = _model()
+    ids, mask = _ragged(1, 40, (40,))
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    ln = model.encoder.layer[0].output.LayerNorm
+    with torch.no_grad():
+        first = run()
+        eps, ln.eps = ln.eps, 0.5
+        assert not torch.equal(run(), first)
+        ln.eps = eps
+        assert torch.equal(run(), first)
