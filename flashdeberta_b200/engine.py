@@ -176,7 +176,7 @@ class _Plan:
 
     def plain(self) -> bool:
         """No hooks, no module in training mode, no patched ``forward``: nothing a module walk would do beside the arithmetic."""
-        return not any(self.hooks) and not any([d["training"] or "forward" in d for d in self.attrs])
+        return not any(self.hooks) and not ops.global_module_hooks() and not any([d["training"] or "forward" in d for d in self.attrs])
 
     def versions(self):
         """What the gathered tables depend on, as it is now."""

@@ -16,6 +16,7 @@ import math
 from typing import Dict, Optional, Tuple
 
 import torch
+from torch.nn.modules import module as _nn_module
 
 from . import _lib, bucket
 
@@ -93,6 +94,14 @@ def on_device(device: torch.device):
 def raw_stream(device: torch.device) -> int:
     """Handle of the current stream of a device."""
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
+
+
+def global_module_hooks() -> bool:
+    """Whether hooks on every module are registered (profilers, module trackers): modules have to be called one by one then."""
+    return any(getattr(_nn_module, h, None) for h in _GLOBAL_HOOKS)
 
 
 def capturing(t: torch.Tensor) -> bool:

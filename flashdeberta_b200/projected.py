@@ -14,12 +14,8 @@ import math
 
 import torch
 from torch import nn
-from torch.nn.modules import module as _nn_module
 
 from . import _lib, backward, bucket, ops
-
-_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
-
 
 def _plain_linear(m, device) -> bool:
     w, b = m.weight, m.bias
@@ -32,7 +28,7 @@ def covers(module, x, query_states, mask, rel) -> bool:
     """Whether a call is one that ``attention`` stands for: autograd recording, bf16 on the GPU, both position terms through the
     key and query projections themselves, self-attention over a dense batch, nothing between the operators (dropout, hooks,
     autocast, tracing)."""
-    if torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or any(getattr(_nn_module, h, None) for h in _GLOBAL_HOOKS):
+    if torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or ops.global_module_hooks():
         return False
     if not (torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and module.share_att_key
             and module.relative_attention and not module.attn_fp8 and module.attention_head_size == 64):

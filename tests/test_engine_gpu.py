@@ -225,3 +225,21 @@ def test_settings_back_and_forth():
         assert not torch.equal(run(), first)
         ln.eps = eps
         assert torch.equal(run(), first)
+
+
+def test_hooks_on_every_module_are_called():
+    from torch.nn.modules.module import register_module_forward_hook, register_module_forward_pre_hook
+    model = _model()
+    ids, mask = _ragged(1, 40, (40,))
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    with torch.no_grad():
+        first = run()
+        for register in (register_module_forward_hook, register_module_forward_pre_hook):
+            seen = []
+            hook = register(lambda m, *a: seen.append(m))
+            try:
+                _close(run(), first, 0.1, 5e-3, "with a hook")
+            finally:
+                hook.remove()
+            assert {*model.encoder.layer, model.embeddings} <= set(seen)
+        assert torch.equal(run(), first)
