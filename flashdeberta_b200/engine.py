@@ -82,6 +82,7 @@ class _Plan:
         self.params = [v for d in self.param_dicts for v in d.values() if v is not None]
         self.param_ids = [id(v) for d in self.param_dicts for v in d.values()]
         self.addresses = [p.data_ptr() for p in self.params]
+        self.owner = (enc, emb)
         self.keep = modules
         self.setting_of = [(d, name) for d in self.attrs for name in _SETTINGS if name in d]
         self.settings = [list(v) if isinstance(v, list) else v for v in (d[name] for d, name in self.setting_of)]  # (lists may be written to)
@@ -89,6 +90,8 @@ class _Plan:
             return
         if emb.position_embeddings is not None or emb.position_biased_input or emb.token_type_embeddings is not None or emb.embed_proj is not None:
             return
+        if not self.params or any(type(p) is not nn.Parameter for p in self.params):
+            return  # (a subclass keeps its values elsewhere than where it points)
         hidden, heads = cfg.hidden_size, cfg.num_attention_heads
         ffn = enc.layer[0].intermediate.dense.out_features
         device = self.params[0].device
@@ -97,13 +100,24 @@ class _Plan:
         if any(p.dtype != torch.bfloat16 or p.device != device or not p.is_contiguous() or p.data_ptr() % 16 for p in self.params):
             return
 
+        def own(m, *names):
+            """Whether these tensors are the module's registered parameters: only those are compared from call to call (sharding
+            wrappers and replicas set others, and set them anew)."""
+            return all(n in m._parameters and n not in m.__dict__ for n in names)
+
         def linear(m, n, k):
-            return type(m) is nn.Linear and m.out_features == n and m.in_features == k
+            return type(m) is nn.Linear and m.out_features == n and m.in_features == k and own(m, "weight", "bias") and m.weight is not None
 
         def norm(m):
-            return type(m) is nn.LayerNorm and m.elementwise_affine and m.bias is not None and m.normalized_shape == (hidden,)
+            return (type(m) is nn.LayerNorm and m.elementwise_affine and own(m, "weight", "bias") and m.bias is not None
+                    and m.normalized_shape == (hidden,))
 
-        if not norm(emb.LayerNorm) or type(emb.word_embeddings) is not nn.Embedding or emb.word_embeddings.max_norm is not None:
+        if (not norm(emb.LayerNorm) or type(emb.word_embeddings) is not nn.Embedding or not own(emb.word_embeddings, "weight")
+                or emb.word_embeddings.max_norm is not None):
+            return
+        if type(enc.rel_embeddings) is not nn.Embedding or not own(enc.rel_embeddings, "weight"):
+            return
+        if "layer_norm" in enc.norm_rel_ebd and not own(enc.LayerNorm, "weight", "bias"):
             return
         attn0 = enc.layer[0].attention.self
         for layer in enc.layer:
@@ -118,6 +132,9 @@ class _Plan:
             if not (all(linear(m, hidden, hidden) for m in (a.query_proj, a.key_proj, a.value_proj, layer.attention.output.dense))
                     and linear(layer.intermediate.dense, ffn, hidden) and linear(layer.output.dense, hidden, ffn)
                     and norm(layer.attention.output.LayerNorm) and norm(layer.output.LayerNorm)):
+                return
+            if not a.share_att_key and not all(type(m) is nn.Linear and own(m, "weight", "bias")
+                                               for m in (getattr(a, n, None) for n in ("pos_key_proj", "pos_query_proj")) if m is not None):
                 return
         self.device, self.hidden, self.heads = device, hidden, heads
         self.c2p, self.p2c = "c2p" in attn0.pos_att_type, "p2c" in attn0.pos_att_type
@@ -166,10 +183,11 @@ class _Plan:
             self.destroy(self.handle)
             self.handle = None
 
-    def current(self) -> bool:
+    def current(self, model) -> bool:
         """Whether the model still is the one this plan was made from: same modules and settings, same parameters at the same
         addresses."""
-        return ([d.get(name) for d, name in self.setting_of] == self.settings
+        return (model.encoder is self.owner[0] and model.embeddings is self.owner[1]
+                and [d.get(name) for d, name in self.setting_of] == self.settings
                 and [id(v) for d in self.module_dicts for v in d.values()] == self.module_ids
                 and [id(v) for d in self.param_dicts for v in d.values()] == self.param_ids
                 and [p.data_ptr() for p in self.params] == self.addresses)
@@ -253,10 +271,10 @@ class EncoderEngine:
         # What a captured call launches has not run when the call returns, so nothing that it sets up may be taken for done by
         # another call: where the plan or its tables are not up to date, a captured call makes its own, and its graph gathers
         # the tables whenever it is replayed.
-        own = capturing and (plan is None or not plan.current() or (plan.ok and plan.tables is not None and plan.versions() != plan.tables.versions))
+        own = capturing and (plan is None or not plan.current(model) or (plan.ok and plan.tables is not None and plan.versions() != plan.tables.versions))
         if own:
             plan = _Plan(model)
-        elif plan is None or not plan.current():
+        elif plan is None or not plan.current(model):
             plan = self._replace_plan(model)
         if not plan.ok or ids.device != plan.device or not plan.plain():
             return None

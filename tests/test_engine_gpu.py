@@ -243,3 +243,45 @@ def test_hooks_on_every_module_are_called():
                 hook.remove()
             assert {*model.encoder.layer, model.embeddings} <= set(seen)
         assert torch.equal(run(), first)
+
+
+def test_weights_that_are_no_parameters_are_read_where_they_are():
+    """A sharding wrapper puts plain tensors in the place of parameters, others for every forward: nothing of the model may be read
+    where it was the time before."""
+    model = _model()
+    ids, mask = _ragged(2, 300, (300, 170))
+    linears = [m for m in model.encoder.modules() if type(m) is torch.nn.Linear]
+    with torch.no_grad():
+        first = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        flat = [(m, m._parameters.pop("weight").detach()) for m in linears]
+
+        def forward(scale):
+            for m, w in flat:
+                m.__dict__["weight"] = w * scale
+            got = model(input_ids=ids, attention_mask=mask).last_hidden_state
+            want = _walk(model, ids, mask)
+            held = [m.__dict__.pop("weight") for m, _ in flat]
+            for t in held:
+                t.fill_(float("nan"))
+            return got, want
+
+        got, want = forward(1.0)
+        _close(got, want, 0.1, 5e-3, "gathered weights")
+        _close(got, first, 0.1, 5e-3, "gathered weights")
+        got, want = forward(1.5)
+        _close(got, want, 0.1, 5e-3, "gathered weights, others")
+        assert not torch.equal(got, first)
+
+
+def test_parameters_of_a_subclass_go_through_the_modules():
+    class Wrapped(torch.nn.Parameter):
+        pass
+
+    model = _model()
+    ids, mask = _ragged(1, 40, (40,))
+    with torch.no_grad():
+        want = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        for layer in model.encoder.layer:
+            layer.output.dense.weight = Wrapped(layer.output.dense.weight.data)
+        _close(model(input_ids=ids, attention_mask=mask).last_hidden_state, want, 0.1, 5e-3, "subclass")
+        assert not model._engine.plan.ok
