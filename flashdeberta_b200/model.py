@@ -276,6 +276,8 @@ class FlashDebertaV2Model(DebertaV2Model):
         if (self.training or torch.is_grad_enabled() or not input_ids.is_cuda or input_ids.numel() == 0 or self.z_steps > 1
                 or torch.compiler.is_compiling() or torch.is_autocast_enabled()):
             return None
+        if "_engine" not in self.__dict__:  # a model pickled as a whole before there was one
+            self._engine = EncoderEngine()
         if cu_seqlens is not None:
             if max_seqlen is None or input_ids.dim() > 2 or (input_ids.dim() == 2 and input_ids.shape[0] != 1):
                 return None  # the module path says what is wrong

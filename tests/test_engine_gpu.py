@@ -285,3 +285,13 @@ def test_parameters_of_a_subclass_go_through_the_modules():
             layer.output.dense.weight = Wrapped(layer.output.dense.weight.data)
         _close(model(input_ids=ids, attention_mask=mask).last_hidden_state, want, 0.1, 5e-3, "subclass")
         assert not model._engine.plan.ok
+
+
+def test_model_from_before_there_was_an_engine():
+    """A model pickled whole by an earlier version has no ``_engine``."""
+    model = _model()
+    ids, mask = _ragged(1, 40, (40,))
+    with torch.no_grad():
+        want = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        del model.__dict__["_engine"]
+        assert torch.equal(model(input_ids=ids, attention_mask=mask).last_hidden_state, want)
