@@ -278,6 +278,8 @@ class FlashDebertaV2Model(DebertaV2Model):
             return None
         if "_engine" not in self.__dict__:  # a model pickled as a whole before there was one
             self._engine = EncoderEngine()
+        if getattr(self, "_is_replica", False):  # of torch.nn.DataParallel: it shares its attributes with the original
+            return None
         if cu_seqlens is not None:
             if max_seqlen is None or input_ids.dim() > 2 or (input_ids.dim() == 2 and input_ids.shape[0] != 1):
                 return None  # the module path says what is wrong

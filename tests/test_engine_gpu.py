@@ -295,3 +295,17 @@ def test_model_from_before_there_was_an_engine():
         want = model(input_ids=ids, attention_mask=mask).last_hidden_state
         del model.__dict__["_engine"]
         assert torch.equal(model(input_ids=ids, attention_mask=mask).last_hidden_state, want)
+
+
+def test_replica_of_data_parallel():
+    """torch.nn.DataParallel runs shallow copies of the model with plain tensors for parameters, in threads: they must neither use nor
+    disturb what the original keeps."""
+    model = _model()
+    ids, mask = _ragged(2, 300, (300, 170))
+    with torch.no_grad():
+        want = model(input_ids=ids, attention_mask=mask).last_hidden_state
+        plan = model._engine.plan
+        replica, = torch.nn.parallel.replicate(model, [torch.device(DEV, torch.cuda.current_device())], detach=True)
+        got = replica(input_ids=ids, attention_mask=mask).last_hidden_state
+        _close(got, want, 0.1, 5e-3, "replica")
+        assert model._engine.plan is plan
