@@ -309,3 +309,25 @@ def test_replica_of_data_parallel():
         got = replica(input_ids=ids, attention_mask=mask).last_hidden_state
         _close(got, want, 0.1, 5e-3, "replica")
         assert model._engine.plan is plan
+
+
+@pytest.mark.parametrize("lens", [(597,), (500, 129), (0, 0), (1, 600)])
+def test_masked_call_does_not_depend_on_what_memory_held(lens):
+    """The same bits whatever the workspace was used for before: rows behind the valid ones are nobody's."""
+    model = _model()
+    ids, mask = _ragged(len(lens), 600, lens)
+    run = lambda: model(input_ids=ids, attention_mask=mask).last_hidden_state
+    with torch.no_grad():
+        for layer in model.encoder.layer:  # (scores that spread widely: the running maxima move)
+            layer.attention.self.query_proj.weight.mul_(8.0)
+            layer.attention.self.key_proj.weight.mul_(8.0)
+        first = run()
+        for value in (0.0, 50.0, -3.0, float("inf"), float("nan")):
+            pool = [torch.full((n // 2,), value, dtype=torch.bfloat16, device=DEV) * torch.randn(n // 2, device=DEV).bfloat16()
+                    for n in (1 << 20, 2 << 20, 4 << 20, 8 << 20, 16 << 20, 32 << 20) for _ in range(4)]
+            del pool
+            assert torch.equal(run(), first), value
+        if any(lens):  # (the walk does not take a batch without a token)
+            _close(first, _walk(model, ids, mask), 0.1, 5e-3, "against the walk")
+        else:
+            assert torch.count_nonzero(first) == 0
