@@ -18,6 +18,7 @@ import warnings
 from typing import Optional
 
 import torch
+from torch._subclasses import FakeTensor
 from transformers.models.deberta_v2.modeling_deberta_v2 import DisentangledSelfAttention
 
 from . import _lib, ops, projected
@@ -86,11 +87,11 @@ def lengths_from_mask(attention_mask: Optional[torch.Tensor], check: bool = True
         m = torch.diagonal(m, dim1=-2, dim2=-1)
     elif m.dim() != 2:
         raise ValueError(f"attention_mask with {attention_mask.dim()} dims is not supported")
-    if check and m.is_cuda and m.dtype in ops.MASK_TYPES and m.dim() == 2 and not torch.compiler.is_compiling():
+    if check and m.is_cuda and m.dtype in ops.MASK_TYPES and m.dim() == 2 and not ops.intercepted(m):
         return ops.lengths_from_mask(m)
     valid = m != 0
     lens = valid.sum(dim=-1, dtype=torch.int32)
-    if check and not torch.compiler.is_compiling():
+    if check and not torch.compiler.is_compiling() and not isinstance(m, FakeTensor):  # (that has nothing to check)
         prefix = torch.arange(m.shape[-1], device=m.device)[None, :] < lens[:, None]
         bad = (valid != prefix).any()
         if m.device.type == "cpu":

@@ -274,7 +274,7 @@ class FlashDebertaV2Model(DebertaV2Model):
         """The last hidden state through ``fdb_encoder_forward`` when the call is one it covers (inference, CUDA, no hidden
         states of the layers asked for), else None."""
         if (self.training or torch.is_grad_enabled() or not input_ids.is_cuda or input_ids.numel() == 0 or self.z_steps > 1
-                or torch.compiler.is_compiling() or torch.is_autocast_enabled()):
+                or torch.is_autocast_enabled() or ops.intercepted(input_ids, attention_mask, cu_seqlens)):
             return None
         if "_engine" not in self.__dict__:  # a model pickled as a whole before there was one
             self._engine = EncoderEngine()

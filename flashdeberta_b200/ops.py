@@ -104,6 +104,17 @@ def global_module_hooks() -> bool:
     return any(getattr(_nn_module, h, None) for h in _GLOBAL_HOOKS)
 
 
+def intercepted(*tensors) -> bool:
+    """Whether somebody wants to see the operators, or these tensors have no memory to point at: tracing, a dispatch mode (fake tensors,
+    flop counters, ``make_fx``), a functorch transform (vmap, grad), a batched gradient, a tensor subclass.  Calls then go through the
+    custom operators, which dispatch; a raw address would bypass all of that."""
+    if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0 or torch._C._get_tracing_state() is not None
+            or torch._C._functorch.peek_interpreter_stack() is not None):
+        return True
+    return any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter or torch._C._functorch.is_legacy_batchedtensor(t)
+               for t in tensors if t is not None)
+
+
 def capturing(t: torch.Tensor) -> bool:
     """Whether the current stream of the tensor's device is being captured into a CUDA graph."""
     if not t.is_cuda:
@@ -705,6 +716,8 @@ class _Train(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad, grad_lse):
+        if intercepted(grad):
+            return _train_backward(ctx, grad, grad_lse)
         from . import backward
         q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, out, lse = ctx.saved_tensors
         max_seqlen, sm_scale, position_buckets, max_rel = ctx.fdb_args
@@ -716,8 +729,9 @@ class _Train(torch.autograd.Function):
 
 
 def attn_train(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_rel):
-    """Output of the attention with autograd recorded: one opaque node under tracing, a plain autograd function otherwise."""
-    call = attn_fwd_train_op if torch.compiler.is_compiling() else _Train.apply
+    """Output of the attention with autograd recorded: one opaque node where operators are looked at, a plain autograd function
+    otherwise."""
+    call = attn_fwd_train_op if intercepted(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens) else _Train.apply
     return call(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_rel)[0]
 
 

@@ -19,7 +19,7 @@ from . import _lib, backward, bucket, ops
 
 def _plain_linear(m, device) -> bool:
     w, b = m.weight, m.bias
-    return (type(m) is nn.Linear and b is not None and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and w.device == device
+    return (b is not None and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and w.device == device
             and w.is_contiguous() and w.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and m.in_features % 64 == 0
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and "forward" not in m.__dict__)
 
@@ -28,7 +28,7 @@ def covers(module, x, query_states, mask, rel) -> bool:
     """Whether a call is one that ``attention`` stands for: autograd recording, bf16 on the GPU, both position terms through the
     key and query projections themselves, self-attention over a dense batch, nothing between the operators (dropout, hooks,
     autocast, tracing)."""
-    if torch.compiler.is_compiling() or torch.is_autocast_enabled("cuda") or ops.global_module_hooks():
+    if torch.is_autocast_enabled("cuda") or ops.global_module_hooks():
         return False
     if not (torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and module.share_att_key
             and module.relative_attention and not module.attn_fp8 and module.attention_head_size == 64):
@@ -37,6 +37,9 @@ def covers(module, x, query_states, mask, rel) -> bool:
         return False
     if rel is None or rel.dim() != 2 or rel.dtype != torch.bfloat16 or rel.device != x.device or x.numel() == 0:
         return False
+    linears = (module.query_proj, module.key_proj, module.value_proj)
+    if any(type(m) is not nn.Linear for m in linears) or ops.intercepted(x, rel, mask, *(t for m in linears for t in (m.weight, m.bias))):
+        return False
     if (x.data_ptr() | rel.data_ptr()) % 16:
         return False
     if "c2p" not in module.pos_att_type or "p2c" not in module.pos_att_type or not (mask is None or isinstance(mask, torch.Tensor)):
@@ -44,7 +47,6 @@ def covers(module, x, query_states, mask, rel) -> bool:
     drop = module.pos_dropout
     if (drop.training and drop.p > 0) or drop._forward_hooks or drop._forward_pre_hooks:
         return False
-    linears = (module.query_proj, module.key_proj, module.value_proj)
     if not all(_plain_linear(m, x.device) for m in linears):
         return False
     if rel.shape[0] < 2 * module.pos_ebd_size or not backward.index_covered(module.position_buckets, module.max_relative_positions):
@@ -104,14 +106,18 @@ class _Projected(torch.autograd.Function):
         x2, rel, wq, wk, wv, qkv, tables, out, lse, lens = ctx.saved_tensors
         B, L, heads, buckets, max_rel = ctx.fdb_args
         inner, span2, dev = heads * 64, tables.shape[0], qkv.device
-        grad = grad.contiguous()
-        d_qkv, d_tables = torch.empty_like(qkv), torch.empty_like(tables)
-        p = _params(qkv, tables, out, lse, lens, B, L, heads, buckets, max_rel)
-        d, t = d_qkv.data_ptr(), d_tables.data_ptr()
-        b = backward.BwdParams(C.sizeof(backward.BwdParams), 0, C.pointer(p), grad.data_ptr(), inner, 64, d, d + 2 * inner, d + 4 * inner,
-                               3 * inner, 64, t + 2 * inner, t, 2 * inner, 64)
-        with ops.on_device(dev):
-            backward.launch(b, dev)
+        operators = ops.intercepted(grad)
+        if operators:
+            d_qkv, d_tables = _backward_by_operators(grad, qkv, tables, out, lse, lens, *ctx.fdb_args)
+        else:
+            grad = grad.contiguous()
+            d_qkv, d_tables = torch.empty_like(qkv), torch.empty_like(tables)
+            p = _params(qkv, tables, out, lse, lens, B, L, heads, buckets, max_rel)
+            d, t = d_qkv.data_ptr(), d_tables.data_ptr()
+            b = backward.BwdParams(C.sizeof(backward.BwdParams), 0, C.pointer(p), grad.data_ptr(), inner, 64, d, d + 2 * inner, d + 4 * inner,
+                                   3 * inner, 64, t + 2 * inner, t, 2 * inner, 64)
+            with ops.on_device(dev):
+                backward.launch(b, dev)
         want = ctx.needs_input_grad
         grads = [None] * 8
         if want[0] or want[1]:
@@ -125,12 +131,31 @@ class _Projected(torch.autograd.Function):
                 grads[1] = d_rel
         if want[2] or want[3] or want[4]:
             dw = torch.mm(d_qkv.t(), x2)
-            dw[:2 * inner].addmm_(d_tables.t(), rel[:span2])
+            if operators:
+                dw = torch.cat((dw[:2 * inner] + torch.mm(d_tables.t(), rel[:span2]), dw[2 * inner:]))
+            else:
+                dw[:2 * inner].addmm_(d_tables.t(), rel[:span2])
             grads[2:5] = [g if n else None for g, n in zip(dw.split(inner), want[2:5])]
         if want[5] or want[6] or want[7]:
-            db = ops.column_sums(d_qkv, d_tables)
+            if operators:
+                db = d_qkv.sum(0, dtype=torch.float32)
+                db = torch.cat((db[:2 * inner] + d_tables.sum(0, dtype=torch.float32), db[2 * inner:])).to(qkv.dtype)
+            else:
+                db = ops.column_sums(d_qkv, d_tables)
             grads[5:8] = [g if n else None for g, n in zip(db.split(inner), want[5:8])]
         return (*grads, None, None, None, None)
+
+
+def _backward_by_operators(grad, qkv, tables, out, lse, lens, B, L, heads, buckets, max_rel):
+    """Gradients of the projections' buffers through the custom operator, for gradients that have no address (``ops.intercepted``)."""
+    inner, span2 = heads * 64, tables.shape[0]
+    q, k, v = qkv.view(B, L, 3, heads, 64).unbind(2)
+    pos_query, pos_key = (t.transpose(0, 1) for t in tables.view(span2, 2, heads, 64).unbind(1))
+    dq, dk, dv, dpk, dpq = ops.attn_bwd_op(
+        grad.reshape(B, L, heads, 64), q, k, v, pos_key, pos_query, out.view(B, L, heads, 64), lse, None, lens, L, 1.0 / math.sqrt(64 * 3),
+        buckets, max_rel)
+    return (torch.stack((dq, dk, dv), 2).reshape(B * L, 3 * inner),
+            torch.stack((dpq, dpk), 0).permute(2, 0, 1, 3).reshape(span2, 2 * inner))
 
 
 def attention(module, x: torch.Tensor, lens, rel: torch.Tensor) -> torch.Tensor:
