@@ -17,10 +17,10 @@ from torch import nn
 
 from . import _lib, backward, bucket, ops
 
-def _plain_linear(m, device) -> bool:
+def _plain_linear(m, device, n: int, k: int) -> bool:
     w, b = m.weight, m.bias
-    return (b is not None and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and w.device == device
-            and w.is_contiguous() and w.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and m.in_features % 64 == 0
+    return (b is not None and w.shape == (n, k) and b.shape == (n,) and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and w.device == device and b.device == device
+            and w.is_contiguous() and w.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and k % 64 == 0
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and "forward" not in m.__dict__)
 
 
@@ -37,6 +37,8 @@ def covers(module, x, query_states, mask, rel) -> bool:
         return False
     if rel is None or rel.dim() != 2 or rel.dtype != torch.bfloat16 or rel.device != x.device or x.numel() == 0:
         return False
+    if x.dim() != 3 or rel.shape[1] != x.shape[2]:  # (from here on only addresses are handed on: every size is looked at)
+        return False
     linears = (module.query_proj, module.key_proj, module.value_proj)
     if any(type(m) is not nn.Linear for m in linears) or ops.intercepted(x, rel, mask, *(t for m in linears for t in (m.weight, m.bias))):
         return False
@@ -44,10 +46,12 @@ def covers(module, x, query_states, mask, rel) -> bool:
         return False
     if "c2p" not in module.pos_att_type or "p2c" not in module.pos_att_type or not (mask is None or isinstance(mask, torch.Tensor)):
         return False
+    if mask is not None and (mask.device != x.device or mask.dim() == 0 or mask.shape[0] != x.shape[0] or (mask.dim() > 1 and mask.shape[-1] != x.shape[1])):
+        return False
     drop = module.pos_dropout
     if (drop.training and drop.p > 0) or drop._forward_hooks or drop._forward_pre_hooks:
         return False
-    if not all(_plain_linear(m, x.device) for m in linears):
+    if not all(_plain_linear(m, x.device, module.num_attention_heads * 64, x.shape[2]) for m in linears):
         return False
     if rel.shape[0] < 2 * module.pos_ebd_size or not backward.index_covered(module.position_buckets, module.max_relative_positions):
         return False

@@ -334,3 +334,30 @@ def test_fp8_attention_refuses_to_train():
     q = torch.randn(1, 128, 2, 64, device=DEV).bfloat16().requires_grad_(True)
     with pytest.raises(RuntimeError, match="forward-only"):
         ops.disentangled_attention_fp8(q, q, q, None, None, max_seqlen=128)
+
+
+@pytest.mark.parametrize("x_width,rel_width,weight", [(320, 256, None), (192, 256, None), (256, 320, None), (256, 128, None),
+                                                      (256, 256, (256, 320)), (256, 256, (192, 256)), (256, 256, (320, 256))])
+def test_module_in_training_refuses_widths_that_do_not_fit(x_width, rel_width, weight):
+    """Sizes that the projections do not have are an error, not a read beyond the weights: the fused node hands on addresses alone."""
+    from flashdeberta_b200 import projected
+    from flashdeberta_b200.attention import FlashDisentangledSelfAttention
+    module = FlashDisentangledSelfAttention(_small_config("b200")).to(DEV).bfloat16().train()
+    if weight is not None:
+        module.key_proj.weight = torch.nn.Parameter(torch.randn(*weight, device=DEV).bfloat16())
+    x = torch.randn(2, 100, x_width, device=DEV).bfloat16().requires_grad_(True)
+    rel = torch.randn(512, rel_width, device=DEV).bfloat16()
+    assert not projected.covers(module, x, None, None, rel)
+    with pytest.raises((RuntimeError, ValueError)):
+        module(x, None, rel_embeddings=rel)
+
+
+def test_module_in_training_takes_only_masks_that_fit():
+    from flashdeberta_b200 import projected
+    from flashdeberta_b200.attention import FlashDisentangledSelfAttention
+    module = FlashDisentangledSelfAttention(_small_config("b200")).to(DEV).bfloat16().train()
+    x = torch.randn(2, 100, 256, device=DEV).bfloat16().requires_grad_(True)
+    rel = torch.randn(512, 256, device=DEV).bfloat16()
+    covered = lambda mask: projected.covers(module, x, None, mask, rel)
+    assert covered(torch.ones(2, 100, device=DEV)) and covered(torch.full((2,), 100, device=DEV))
+    assert not any(covered(m) for m in (torch.ones(2, 100), torch.ones(1, 100, device=DEV), torch.ones(2, 99, device=DEV), torch.ones(1, device=DEV)))
