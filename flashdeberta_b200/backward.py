@@ -275,7 +275,7 @@ def attention_backward(
               block_bytes=block_bytes, status=status)
     if cu_seqlens is None:
         B, L = shape[0], shape[1]
-        lens = None if seq_lens is None else seq_lens.to(torch.int32).contiguous()
+        lens = None if seq_lens is None else ops._int32(seq_lens, q.device)
         dq, dk, dv, dpk, dpq = _backward_block(q3, k3, v3, o3, do3, lse2, pos_key, pos_query, B, L, lens, **kw)
     else:
         cu = [int(x) for x in cu_seqlens.tolist()]

@@ -178,8 +178,9 @@ def _rows_view(x: torch.Tensor) -> Tuple[torch.Tensor, int, int, int]:
     return x, stride[0], stride[1], shape[0]
 
 
-def _int32(t: torch.Tensor) -> torch.Tensor:
-    return t if t.dtype == torch.int32 and t.is_contiguous() else t.to(torch.int32).contiguous()
+def _int32(t: torch.Tensor, device: torch.device) -> torch.Tensor:
+    """Lengths or offsets as the kernels read them."""
+    return t if t.dtype == torch.int32 and t.device == device and t.is_contiguous() else t.to(device=device, dtype=torch.int32).contiguous()
 
 
 def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
@@ -213,7 +214,7 @@ def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, 
         lut_ptr, lut_len = lut.data_ptr(), lut.shape[0]
     cu_ptr = lens_ptr = None
     if cu_seqlens is not None:
-        cu_seqlens = _int32(cu_seqlens)
+        cu_seqlens = _int32(cu_seqlens, q.device)
         keep.append(cu_seqlens)
         cu_ptr, batch = cu_seqlens.data_ptr(), cu_seqlens.numel() - 1
     else:
@@ -223,7 +224,9 @@ def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, 
         if max_seqlen != shape[1]:
             raise ValueError("dense layout: max_seqlen must equal the padded length")
         if seq_lens is not None:
-            seq_lens = _int32(seq_lens)
+            seq_lens = _int32(seq_lens, q.device)
+            if seq_lens.numel() < batch:
+                raise ValueError(f"seq_lens has {seq_lens.numel()} entries for a batch of {batch}")
             keep.append(seq_lens)
             lens_ptr = seq_lens.data_ptr()
     p = _lib.AttnParams(  # in the order of the fields
@@ -376,7 +379,7 @@ def disentangled_attention_fp8(
     if sm_scale is None:
         sm_scale = 1.0 / math.sqrt(q.shape[-1] * (1 + int(pos_key is not None) + int(pos_query is not None)))
     if cu_seqlens is not None:
-        cu_seqlens = _int32(cu_seqlens)
+        cu_seqlens = _int32(cu_seqlens, q.device)
     lib, dev, H = _lib.load(), q.device, q.shape[-2]
     given = {"q": q, "k": k, "v": v, "pos_key": pos_key, "pos_query": pos_query}
     p, keep = _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_relative_positions, q, None)

@@ -361,3 +361,34 @@ def test_module_in_training_takes_only_masks_that_fit():
     covered = lambda mask: projected.covers(module, x, None, mask, rel)
     assert covered(torch.ones(2, 100, device=DEV)) and covered(torch.full((2,), 100, device=DEV))
     assert not any(covered(m) for m in (torch.ones(2, 100), torch.ones(1, 100, device=DEV), torch.ones(2, 99, device=DEV), torch.ones(1, device=DEV)))
+
+
+def test_lengths_on_the_host():
+    """Lengths, offsets and masks on the host are brought to the device; too few lengths are an error."""
+    from flashdeberta_b200 import backward, ops
+    from flashdeberta_b200.attention import FlashDisentangledSelfAttention
+    g = torch.Generator().manual_seed(8)
+    q, k, v, dout = (torch.randn(2, 200, 2, 64, generator=g).bfloat16().to(DEV) for _ in range(4))
+    pk, pq = (torch.randn(2, 64, 64, generator=g).bfloat16().to(DEV) for _ in range(2))
+    kw = dict(max_seqlen=200, position_buckets=32, max_relative_positions=64)
+    lens, cu = torch.tensor([200, 77], dtype=torch.int32), torch.tensor([0, 200, 377])
+
+    def both(call, t):
+        want, got = call(t.to(DEV)), call(t)
+        assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+    flat = lambda t: t.reshape(-1, 2, 64)[:377]
+    both(lambda n: _run_op(q, k, v, pk, pq, dout, seq_lens=n, **kw), lens)
+    both(lambda n: _run_op(flat(q), flat(k), flat(v), pk, pq, flat(dout), cu_seqlens=n, **kw), cu)
+    with torch.no_grad():
+        both(lambda n: [ops.disentangled_attention_fp8(q, k, v, pk, pq, seq_lens=n, **kw)], lens)
+        out, lse = ops.disentangled_attention(q, k, v, pk, pq, seq_lens=lens, return_lse=True, **kw)
+        both(lambda n: backward.attention_backward(dout, q, k, v, pk, pq, out, lse, seq_lens=n, sm_scale=0.07, block_bytes=1 << 28, **kw), lens)
+        with pytest.raises(ValueError):
+            ops.disentangled_attention(q, k, v, pk, pq, seq_lens=lens[:1], **kw)
+    module = FlashDisentangledSelfAttention(_small_config("b200")).to(DEV).bfloat16().train()
+    x, rel = torch.randn(2, 200, 256, device=DEV).bfloat16().requires_grad_(True), torch.randn(512, 256, device=DEV).bfloat16()
+    mask = (torch.arange(200)[None] < lens[:, None]).long()
+    got = torch.autograd.grad(module(x, mask, rel_embeddings=rel)[0].sum(), x)[0]
+    _close(got, torch.autograd.grad(module(x, mask.to(DEV), rel_embeddings=rel)[0].sum(), x)[0].float().cpu(), "host mask")
+    ops.check_status()
