@@ -47,6 +47,7 @@ struct LinearArgs {
   int32_t* status;
   int64_t rows, out_stride;
   int k, groups, tiles_n;        // groups = weights over the same x; tiles_n = feature tiles of one weight
+  bool sectors;                  // every row of every output starts on a 32-byte boundary
 };
 
 // 32 bytes per thread in one store (whole sectors)
@@ -234,8 +235,13 @@ __global__ void __launch_bounds__(kThreads, 1) linear_kernel(const __grid_consta
           }
         }
         if (live && ok) {
-          st_global_32B(orow + ch * 32, o, 0);
-          st_global_32B(orow + ch * 32 + 16, o, 8);
+          if (args.sectors) {
+            st_global_32B(orow + ch * 32, o, 0);
+            st_global_32B(orow + ch * 32 + 16, o, 8);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 16; c += 4) *reinterpret_cast<uint4*>(orow + ch * 32 + 2 * c) = make_uint4(o[c], o[c + 1], o[c + 2], o[c + 3]);
+          }
         }
       }
     }
@@ -299,7 +305,12 @@ int launch_linear(const LinearCall& c, void* stream) {
     if (best == nullptr || cost < best_cost) { best = &f; best_cost = cost; best_tiles = tiles; }
   }
   if (best == nullptr || best_tiles * 2 > 2147483647LL) return fail(FDB_ERR_LIMIT, "linear: %lld rows x %d features", (long long)c.rows, c.n);
+  // The epilogue stores 32 bytes per thread where it may, else 16, which callers' buffers have to allow.
+  uintptr_t outs = (uintptr_t)c.out_stride * 2;
+  for (int g = 0; g < c.groups; ++g) outs |= reinterpret_cast<uintptr_t>(c.out[g]);
+  if ((outs & 15u) != 0) return fail(FDB_ERR_ALIGNMENT, "linear: output rows must be 16-byte aligned");
   LinearArgs a;
+  a.sectors = (outs & 31u) == 0;
   a.tm_x = *c.x_map;
   const int box = best->bn / best->cg;
   for (int g = 0; g < 3; ++g) {

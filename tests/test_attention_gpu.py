@@ -922,3 +922,59 @@ def test_model_b200_backend_vs_eager_backend():
     with torch.no_grad():
         logits = head(input_ids=ids, attention_mask=mask).logits
     assert logits.shape == (B, 2) and torch.isfinite(logits.float()).all()
+
+
+@pytest.mark.parametrize("rows", [1, 129, 700])
+def test_linear_gelu_into_rows_that_start_on_16_bytes(rows):
+    """The C entry point takes any 16-byte aligned output; whole 32-byte sectors are stored only where they are ones."""
+    import ctypes as C
+    from flashdeberta_b200 import _lib, ops
+    g = torch.Generator().manual_seed(rows)
+    x, w = torch.randn(rows, 256, generator=g).bfloat16().to(DEV), (0.05 * torch.randn(512, 256, generator=g)).bfloat16().to(DEV)
+    want = ops.linear_gelu(x, w, None)
+    buf = torch.full((rows * 512 + 16,), 7.0, dtype=torch.bfloat16, device=DEV)
+    out = buf[8:8 + rows * 512]
+    assert out.data_ptr() % 32 == 16
+    _lib.check(_lib.load().fdb_linear_gelu(x.data_ptr(), w.data_ptr(), None, out.data_ptr(), rows, 256, 512, ops._status_word(x.device).data_ptr(),
+                                           C.c_void_p(ops.raw_stream(x.device))))
+    torch.cuda.synchronize()
+    assert torch.equal(out.view(rows, 512), want) and (buf[:8] == 7).all() and (buf[-8:] == 7).all()
+    ops.check_status()
+
+
+@pytest.mark.parametrize("pad", [0, 8, 16])
+def test_projected_forward_with_any_stride_it_accepts(pad):
+    """q, k, v and the tables with rows of 3 * inner + pad and 2 * inner + pad elements: the same numbers as with contiguous rows."""
+    import ctypes as C
+    from flashdeberta_b200 import _lib, ops, projected
+    g = torch.Generator().manual_seed(2)
+    make = lambda *s: (0.1 * torch.randn(*s, generator=g)).bfloat16().to(DEV)
+    B, L, heads, k = 2, 150, 4, 256
+    inner = heads * 64
+    x, rel = make(B * L, k), make(64, k)
+    wq, wk, wv, bq, bk, bv = make(inner, k), make(inner, k), make(inner, k), make(inner), make(inner), make(inner)
+
+    def run(extra):
+        qkv = torch.full((B * L, 3 * inner + extra), 3.0, dtype=torch.bfloat16, device=DEV)
+        tables = torch.full((64, 2 * inner + extra), 3.0, dtype=torch.bfloat16, device=DEV)
+        out = torch.empty(B, L, inner, dtype=torch.bfloat16, device=DEV)
+        lse = torch.empty(B * L, heads, dtype=torch.float32, device=DEV)
+        p = projected._params(qkv, tables, out, lse, None, B, L, heads, 32, 64)
+        for n in ("q", "k", "v"):
+            setattr(p, n + "_row_stride", 3 * inner + extra)
+        need = _lib.load().fdb_attn_workspace_bytes(C.byref(p))
+        ws = torch.empty(need + 256, dtype=torch.uint8, device=DEV)
+        p.workspace, p.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
+        c = projected._ProjectedParams(C.sizeof(projected._ProjectedParams), k, C.pointer(p), 2 * inner + extra, 64, x.data_ptr(), rel.data_ptr(),
+                                       *(t.data_ptr() for t in (wq, bq, wk, bk, wv, bv)))
+        _lib.check(_lib.load().fdb_projected_forward(C.byref(c), C.c_void_p(ops.raw_stream(x.device))))
+        torch.cuda.synchronize()
+        ops.check_status()
+        assert (qkv[:, 3 * inner:] == 3).all() and (tables[:, 2 * inner:] == 3).all()
+        return qkv[:, :3 * inner], tables[:, :2 * inner], out, lse
+
+    for a, b in zip(run(pad), run(0)):
+        assert torch.equal(a, b)
+    want = (x.float() @ torch.cat((wq, wk, wv)).float().t() + torch.cat((bq, bk, bv)).float())
+    # one rounding to bf16 of a product summed in fp32: half an ulp, 2^-9 of the value
+    assert ((run(pad)[0].float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
