@@ -247,7 +247,7 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
         b.dpos_key, b.dpos_query = _ptr(d_key), _ptr(d_query)
         launch(b, dev)
         del keep
-    return (*(g.view(shape) for g in grads), d_key, d_query)
+    return (*(g.view(t.shape) for g, t in zip(grads, (q, k, v))), d_key, d_query)
 
 
 @torch.no_grad()
@@ -299,6 +299,6 @@ def attention_backward(
             dpk = torch.zeros(pos_key.shape, dtype=torch.float32, device=q.device)
         if pos_query is not None and dpq is None:
             dpq = torch.zeros(pos_query.shape, dtype=torch.float32, device=q.device)
-    return (dq.to(q.dtype).view(shape), dk.to(k.dtype).view(shape), dv.to(v.dtype).view(shape),
+    return (dq.to(q.dtype).view(shape), dk.to(k.dtype).view(k.shape), dv.to(v.dtype).view(v.shape),
             None if dpk is None else dpk.to(pos_key.dtype).view(pos_key.shape),
             None if dpq is None else dpq.to(pos_query.dtype).view(pos_query.shape))

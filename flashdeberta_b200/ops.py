@@ -186,11 +186,12 @@ def _int32(t: torch.Tensor, device: torch.device) -> torch.Tensor:
 def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
                  max_relative_positions, out, lse, scales=None):
     q3, q_rs, q_hs, rows = _rows_view(q)
-    k3, k_rs, k_hs, _ = _rows_view(k)
-    v3, v_rs, v_hs, _ = _rows_view(v)
+    k3, k_rs, k_hs, k_rows = _rows_view(k)
+    v3, v_rs, v_hs, v_rows = _rows_view(v)
     shape = q.shape
     H, D = shape[-2], shape[-1]
-    if k.shape != shape or v.shape != shape:
+    # as rows: (1, T, H, D) beside (T, H, D) is the same tensor
+    if k_rows != rows or v_rows != rows or k.shape[-2:] != shape[-2:] or v.shape[-2:] != shape[-2:]:
         raise ValueError("q, k and v must have the same shape")
     keep = [q3, k3, v3]
     tables = [None, None]

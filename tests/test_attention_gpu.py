@@ -978,3 +978,26 @@ def test_projected_forward_with_any_stride_it_accepts(pad):
     want = (x.float() @ torch.cat((wq, wk, wv)).float().t() + torch.cat((bq, bk, bv)).float())
     # one rounding to bf16 of a product summed in fp32: half an ulp, 2^-9 of the value
     assert ((run(pad)[0].float() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-4).all()
+
+
+@pytest.mark.parametrize("q_dims,kv_dims", [(4, 3), (3, 4), (4, 4), (3, 3)])
+def test_one_packed_row_with_or_without_its_batch_dimension(q_dims, kv_dims):
+    """(1, T, H, 64) and (T, H, 64) are the same packed tensor, for each of q, k and v by itself, forward and backward."""
+    from flashdeberta_b200 import ops
+    g = torch.Generator().manual_seed(6)
+    q, k, v, dout = (torch.randn(300, 2, 64, generator=g).bfloat16().to(DEV) for _ in range(4))
+    pk, pq = (torch.randn(2, 64, 64, generator=g).bfloat16().to(DEV) for _ in range(2))
+    kw = dict(cu_seqlens=torch.tensor([0, 129, 300], dtype=torch.int32, device=DEV), max_seqlen=171, position_buckets=32, max_relative_positions=64)
+    dims = lambda t, n: t.clone().unsqueeze(0) if n == 4 else t.clone()
+
+    def run(a, b):
+        leaves = [dims(q, a).requires_grad_(), dims(k, b).requires_grad_(), dims(v, a).requires_grad_(), pk.clone().requires_grad_(), pq.clone().requires_grad_()]
+        out = ops.disentangled_attention(*leaves, **kw)
+        grads = torch.autograd.grad(out, leaves, dims(dout, a))
+        assert out.shape == leaves[0].shape and all(x.shape == y.shape for x, y in zip(grads, leaves))
+        with torch.no_grad():
+            return [t.reshape(-1, 2, 64) for t in (out, *grads, ops.disentangled_attention_fp8(*leaves, **kw))]
+
+    for a, b in zip(run(q_dims, kv_dims), run(3, 3)):
+        assert torch.equal(a, b)
+    ops.check_status()
