@@ -228,12 +228,22 @@ def launch(b: BwdParams, dev: torch.device) -> None:
     _launches += 4 + int(terms > 0) + 2 * terms
 
 
+def _aligned(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
+    """The tensor as the kernels can read it, in pieces of 16 bytes: a copy where it starts or strides elsewhere (a gradient may be a
+    slice, or expanded)."""
+    if t is None or (t.data_ptr() % 16 == 0 and t.stride(-1) == 1 and all(s > 0 and s % 8 == 0 for s in t.stride()[-3:-1])):
+        return t
+    return t.clone(memory_format=torch.contiguous_format)
+
+
 def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
            max_relative_positions):
     dev, shape = q.device, q.shape
     with ops.on_device(dev):
+        dout, q, k, v, pos_key, pos_query, out = (_aligned(t) for t in (dout, q, k, v, pos_key, pos_query, out.contiguous()))
+        lse = lse.contiguous()
         p, keep = ops._fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
-                                   max_relative_positions, out.contiguous(), lse.contiguous())
+                                   max_relative_positions, out, lse)
         d3, d_rs, d_hs, T = ops._rows_view(dout)
         H = shape[-2]
         grads = [torch.empty(T, H, 64, dtype=torch.bfloat16, device=dev) for _ in range(3)]

@@ -114,7 +114,7 @@ class _Projected(torch.autograd.Function):
         if operators:
             d_qkv, d_tables = _backward_by_operators(grad, qkv, tables, out, lse, lens, *ctx.fdb_args)
         else:
-            grad = grad.contiguous()
+            grad = backward._aligned(grad.contiguous())
             d_qkv, d_tables = torch.empty_like(qkv), torch.empty_like(tables)
             p = _params(qkv, tables, out, lse, lens, B, L, heads, buckets, max_rel)
             d, t = d_qkv.data_ptr(), d_tables.data_ptr()

@@ -392,3 +392,41 @@ def test_lengths_on_the_host():
     got = torch.autograd.grad(module(x, mask, rel_embeddings=rel)[0].sum(), x)[0]
     _close(got, torch.autograd.grad(module(x, mask.to(DEV), rel_embeddings=rel)[0].sum(), x)[0].float().cpu(), "host mask")
     ops.check_status()
+
+
+@pytest.mark.parametrize("form", ["offset", "transposed", "expanded rows", "expanded"])
+def test_gradients_that_start_or_stride_anywhere(form):
+    """The gradient of the output as autograd or a caller may hand it over: a slice that starts at an odd element, heads outermost,
+    one row for all, one number for all."""
+    from flashdeberta_b200 import backward, ops
+    from flashdeberta_b200.attention import FlashDisentangledSelfAttention
+    g = torch.Generator().manual_seed(9)
+    make = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+
+    def grad(*shape):
+        n = shape.numel() if isinstance(shape, torch.Size) else torch.Size(shape).numel()
+        if form == "offset":
+            return make(n + 3)[3:].view(shape)
+        if form == "transposed":
+            return make(*shape[::-1]).permute(*range(len(shape) - 1, -1, -1))
+        return make(1, 1, *shape[2:]).expand(shape) if form == "expanded rows" else make(1).expand(shape)
+
+    q, k, v = (make(2, 150, 2, 64) for _ in range(3))
+    pk, pq = make(2, 64, 64), make(2, 64, 64)
+    kw = dict(max_seqlen=150, position_buckets=32, max_relative_positions=64)
+    dout = grad(2, 150, 2, 64)
+    want = _run_op(q, k, v, pk, pq, dout.clone(memory_format=torch.contiguous_format), **kw)
+    for a, b in zip(_run_op(q, k, v, pk, pq, dout, **kw), want):
+        assert torch.equal(a, b)
+    with torch.no_grad():  # and the function itself, with every tensor off its boundary
+        out, lse = ops.disentangled_attention(q, k, v, pk, pq, return_lse=True, **kw)
+        odd = lambda t: torch.cat((t.new_zeros(3), t.flatten()))[3:].view(t.shape)
+        got = backward.attention_backward(dout, *(odd(t) for t in (q, k, v, pk, pq, out)), odd(lse), sm_scale=1 / (64 * 3) ** 0.5, **kw)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    module = FlashDisentangledSelfAttention(_small_config("b200")).to(DEV).bfloat16().train()
+    x, rel, dout = make(2, 150, 256).requires_grad_(True), make(512, 256), grad(2, 150, 256)
+    run = lambda d: torch.autograd.grad(module(x, None, rel_embeddings=rel)[0], [x, *module.parameters()], d)
+    for a, b in zip(run(dout), run(dout.clone(memory_format=torch.contiguous_format))):
+        assert torch.equal(a, b)
+    ops.check_status()
