@@ -25,5 +25,7 @@ struct BwdTablesCall {
 };
 uint64_t bwd_tables_partial_bytes(int64_t rows, int heads, int table_rows);
 int launch_bwd_tables(const BwdTablesCall& c, cudaStream_t stream);
+// Zeros for the gradient of a table of a call without rows.
+int launch_zero_table(void* dtable, int64_t row_stride, int64_t head_stride, int heads, int table_rows, cudaStream_t stream);
 
 }  // namespace fdb

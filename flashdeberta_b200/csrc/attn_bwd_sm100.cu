@@ -771,7 +771,7 @@ int launch_bwd(const BwdArgs& a, const fdb_attn_bwd_params& b, char* partial, in
   static std::atomic<uint64_t> smem_done{0};
   auto kernel = bwd_kernel<DKV>;
   cudaError_t e = allow_smem(smem_done, reinterpret_cast<const void*>(kernel), (int)kSmemBytes);
-  if (e == cudaSuccess) e = launch_kernel<BwdArgs>(kernel, a, dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, false, stream);
+  if (e == cudaSuccess && slots > 0) e = launch_kernel<BwdArgs>(kernel, a, dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, false, stream);
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd launch: %s", cudaGetErrorString(e));
   if (a.xrow == nullptr) return FDB_OK;
   BwdTablesCall c;
@@ -827,7 +827,12 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   int rc = check_bwd(b, &g);
   if (rc != FDB_OK) return rc;
   const fdb_attn_params& p = *b->fwd;
-  if (p.batch == 0 || p.total_rows == 0) return FDB_OK;
+  if (p.total_rows == 0) {  // nothing but the tables' gradients to write
+    const TableStrides strides = table_strides(*b);
+    for (void* d : {b->dpos_key, b->dpos_query})
+      if (d != nullptr && (rc = launch_zero_table(d, strides.row, strides.head, p.heads, table_rows_of(p), static_cast<cudaStream_t>(stream))) != FDB_OK) return rc;
+    return FDB_OK;
+  }
   if (b->dout == nullptr || p.lse == nullptr || b->dq == nullptr || b->dk == nullptr || b->dv == nullptr ||
       (p.pos_key != nullptr) != (b->dpos_key != nullptr) || (p.pos_query != nullptr) != (b->dpos_query != nullptr))
     return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_attn_bwd: dout, lse, dq, dk, dv and the gradient of every position table are required");
@@ -841,7 +846,7 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   if (b->workspace == nullptr || b->workspace_bytes < l.total)
     return fail(FDB_ERR_WORKSPACE, "workspace of %llu bytes needed, %llu given", (unsigned long long)l.total, (unsigned long long)b->workspace_bytes);
   if ((reinterpret_cast<uintptr_t>(b->workspace) & 255u) != 0) return fail(FDB_ERR_ALIGNMENT, "workspace must be 256-byte aligned");
-  const int64_t slots = tile_slots(p);
+  const int64_t slots = tile_slots(p);  // none when no sequence is given: every row is outside then
   if (slots > 2147483647LL || p.heads > 65535) return fail(FDB_ERR_LIMIT, "grid too large");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   char* ws = static_cast<char*>(b->workspace);
@@ -849,7 +854,7 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   buf.seq_info = reinterpret_cast<int32_t*>(ws + l.seq_info);
   buf.tile_first = reinterpret_cast<int32_t*>(ws + l.tile_first);
   buf.slot_info = reinterpret_cast<int32_t*>(ws + l.slot_info);
-  if ((rc = launch_seq_info(p, buf, stream)) != FDB_OK) return rc;
+  if (slots > 0 && (rc = launch_seq_info(p, buf, stream)) != FDB_OK) return rc;
   BwdArgs dq, dkv;
   if ((rc = make_args<false>(dq, *b, g, l, ws)) != FDB_OK || (rc = make_args<true>(dkv, *b, g, l, ws)) != FDB_OK) return rc;
   if (p.pos_key != nullptr || p.pos_query != nullptr) {

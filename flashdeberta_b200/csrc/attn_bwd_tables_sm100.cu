@@ -264,6 +264,15 @@ int parts_of(int64_t rows, int heads) {
 
 }  // namespace
 
+int launch_zero_table(void* dtable, int64_t row_stride, int64_t head_stride, int heads, int table_rows, cudaStream_t stream) {
+  const int64_t n = (int64_t)heads * table_rows * 16;  // a sum of no parts
+  bwd_table_reduce_kernel<<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(nullptr, 0, table_rows, 0, heads, row_stride, head_stride,
+                                                                          static_cast<__nv_bfloat16*>(dtable));
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd tables launch: %s", cudaGetErrorString(e));
+  return FDB_OK;
+}
+
 uint64_t bwd_tables_partial_bytes(int64_t rows, int heads, int table_rows) {
   return uint64_t(heads) * parts_of(rows, heads) * std::min(table_rows, 128 * kPieces) * 64 * sizeof(float);
 }

@@ -430,3 +430,33 @@ def test_gradients_that_start_or_stride_anywhere(form):
     for a, b in zip(run(dout), run(dout.clone(memory_format=torch.contiguous_format))):
         assert torch.equal(a, b)
     ops.check_status()
+
+
+@pytest.mark.parametrize("rows", [0, 1, 300])
+@pytest.mark.parametrize("terms", [True, False])
+def test_no_sequence_gives_zero_gradients(rows, terms):
+    """Offsets that name no sequence: every row is outside, every gradient zero whatever the memory held before.  (The library's entry
+    point is called itself for no rows at all, which the Python side answers alone.)"""
+    import ctypes as C
+    from flashdeberta_b200 import _lib, backward, ops
+    g = torch.Generator().manual_seed(9)
+    q, k, v, out, dout = (torch.randn(max(rows, 1), 2, 64, generator=g).bfloat16().to(DEV)[:rows] for _ in range(5))
+    pk, pq = (torch.randn(2, 64, 64, generator=g).bfloat16().to(DEV) for _ in range(2)) if terms else (None, None)
+    cu = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kw = dict(cu_seqlens=cu, max_seqlen=128, sm_scale=0.1, position_buckets=32, max_relative_positions=64)
+    for _ in range(2):
+        junk = [torch.full((n,), float("nan"), dtype=torch.bfloat16, device=DEV) for n in (rows * 128, 8192, 64 * 128, 1 << 20) for _ in range(4)]
+        del junk
+        got = backward.attention_backward(dout, q, k, v, pk, pq, out, torch.zeros(rows, 2, device=DEV), **kw)
+        for t, like in zip(got, (q, k, v, pk, pq)):
+            assert (t is None) == (like is None) and (t is None or (t.shape == like.shape and torch.count_nonzero(t) == 0))
+    if rows == 0 and terms:
+        d = torch.full((2, 2, 64, 64), float("nan"), dtype=torch.bfloat16, device=DEV)
+        one = torch.zeros(1, 2, 64, dtype=torch.bfloat16, device=DEV)
+        p, keep = ops._fill_params(one, one, one, pk, pq, cu, None, 128, 0.1, 32, 64, one, torch.zeros(1, 2, device=DEV))
+        p.total_rows = 0
+        b = backward.BwdParams()
+        b.struct_bytes, b.fwd, b.dpos_key, b.dpos_query = C.sizeof(b), C.pointer(p), d[0].data_ptr(), d[1].data_ptr()
+        _lib.check(_lib.load().fdb_attn_bwd(C.byref(b), C.c_void_p(ops.raw_stream(q.device))))
+        assert torch.count_nonzero(d) == 0
+    ops.check_status()
