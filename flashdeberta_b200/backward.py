@@ -224,8 +224,13 @@ def launch(b: BwdParams, dev: torch.device) -> None:
     ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
     b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
     _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(ops.raw_stream(dev))))
-    terms = int(b.dpos_key is not None) + int(b.dpos_query is not None)
-    _launches += 4 + int(terms > 0) + 2 * terms
+    p = b.fwd.contents
+    sides, groups = [b.dpos_key, b.dpos_query], 1
+    if any(sides):  # heads in groups of at most 2 GiB of bucket sums (csrc/attn_bwd_sm100.cu)
+        span = p.position_buckets if p.position_buckets > 0 else p.max_relative_positions
+        most = max(1, min(p.heads, (1 << 31) // max(1, p.total_rows * 2 * span * 2)))
+        groups = -(-p.heads // -(-p.heads // -(-p.heads // most)))
+    _launches += 2 + int(any(sides)) + sum(3 * groups if side else 1 for side in sides)
 
 
 def _aligned(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:

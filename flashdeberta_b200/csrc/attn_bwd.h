@@ -14,7 +14,8 @@ struct BwdTablesCall {
   int64_t table_row_stride, table_head_stride;
   const void* operand;  // bf16, rows of operand_row_stride elements
   int64_t operand_row_stride, operand_head_stride;
-  float* core;          // (rows, heads, 64); overwritten when table_rows is above 512
+  float* core;          // (heads, 64) per row, rows core_row_stride elements apart; overwritten when table_rows is above 512
+  int64_t core_row_stride;
   void* out;            // bf16
   int64_t out_row_stride, out_head_stride;
   void* dtable;         // bf16, laid out like the table

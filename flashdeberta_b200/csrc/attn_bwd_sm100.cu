@@ -37,6 +37,8 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "attn_bwd.h"
 #include "attn_fwd_common.cuh"
 #include "internal.h"
@@ -95,11 +97,12 @@ struct alignas(64) BwdArgs {
   __nv_bfloat16* grad;                    // without it: dQ or dK
   __nv_bfloat16* dv;                      // <true>
   int64_t grad_rs, grad_hs;               // strides of dQ, dK, dV
-  __nv_bfloat16* sums;                    // (heads, rows, table_rows)
+  __nv_bfloat16* sums;                    // (heads of this launch, rows, table_rows)
   const int16_t* lut;
   int32_t* status;
   int lut_d_min, lut_len, table_rows;
   int heads, packed, max_seqlen, total_rows;
+  int head0, sum_heads;                   // first head of this launch; heads that `sums` has room for
   int sat_lo, sat_hi, d_first, xrows;     // in distances row - column
   float sm_scale;
 };
@@ -122,9 +125,9 @@ __device__ __forceinline__ void zero_row(const BwdArgs& a, int64_t row, int head
     else if (i < 8) *reinterpret_cast<uint4*>(a.grad + at) = z;
     if (DKV && i < 8) *reinterpret_cast<uint4*>(a.dv + at) = z;
   }
-  if (a.xrow != nullptr)
+  if (a.xrow != nullptr && head - a.head0 < a.sum_heads)
     for (int i = lane; i < a.table_rows / 8; i += n)
-      *reinterpret_cast<uint4*>(a.sums + ((int64_t)head * a.total_rows + row) * a.table_rows + i * 8) = z;
+      *reinterpret_cast<uint4*>(a.sums + ((int64_t)(head - a.head0) * a.total_rows + row) * a.table_rows + i * 8) = z;
 }
 
 template <bool DKV>
@@ -133,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem - smem_u32(smem_raw));
   const int tid = threadIdx.x, warp = (int)uniform(uint32_t(tid) >> 5), lane = tid & 31;
-  const int head = blockIdx.y;
+  const int head = args.head0 + (int)blockIdx.y;
 
   const int4 slot = __ldg(args.slot_info + blockIdx.x);  // (sequence, first row of the tile in it, its first row, its length)
   if (slot.x < 0) return;
@@ -323,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
       for (int i = 0; i < 32; ++i) {  // a row at a time: whole lines (a packed row behind the sequence is another one's)
         const int row = r0 + quad * 32 + i;
         if (row >= len && (args.packed || row >= row_limit)) break;
-        uint4* z = reinterpret_cast<uint4*>(args.sums + ((int64_t)head * args.total_rows + seq_row0 + row) * args.table_rows);
+        uint4* z = reinterpret_cast<uint4*>(args.sums + ((int64_t)blockIdx.y * args.total_rows + seq_row0 + row) * args.table_rows);
         for (int c = lane; c < args.table_rows / 8; c += 32) z[c] = make_uint4(0u, 0u, 0u, 0u);
       }
       __syncwarp();
@@ -334,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
       const uint32_t mine = smem + kSmemEmit + uint32_t(quad * 32 + lane) * kEmitPitch;
       constexpr uint32_t kHome = DKV ? 0u : 32u;  // byte offset of the current group
       sts_v4(mine + kHome, 0u, 0u, 0u, 0u);
-      uint4* sums = reinterpret_cast<uint4*>(args.sums + ((int64_t)head * args.total_rows + seq_row0 + (valid_row ? my_row : len - 1)) * args.table_rows);
+      uint4* sums = reinterpret_cast<uint4*>(args.sums + ((int64_t)blockIdx.y * args.total_rows + seq_row0 + (valid_row ? my_row : len - 1)) * args.table_rows);
       const uint32_t* bits = reinterpret_cast<const uint32_t*>(smem_gen + kSmemBits);
 #pragma unroll 1
       for (int j = 0; j < n_tiles; ++j) {
@@ -704,6 +707,17 @@ TableStrides table_strides(const fdb_attn_bwd_params& b) {
 
 uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 
+// Heads whose bucket sums are in memory at a time.  The sums are 2 bytes per row, head and table row, by far the largest thing in the
+// workspace; heads are independent, so the largest calls go through them in groups of at most this many bytes (131072 rows of 16
+// heads and 512 table rows are one group), and the workspace grows with the rows only by what every row needs once.
+constexpr uint64_t kSumBytes = uint64_t(1) << 31;
+int sum_heads_of(const fdb_attn_params& p) {
+  const uint64_t head = uint64_t(p.total_rows) * table_rows_of(p) * 2;
+  const uint64_t most = head == 0 ? p.heads : std::max<uint64_t>(1, std::min<uint64_t>(p.heads, kSumBytes / head));
+  const int groups = (int)((p.heads + most - 1) / most);
+  return (p.heads + groups - 1) / groups;  // groups of about the same size
+}
+
 struct Layout { uint64_t seq_info, tile_first, slot_info, delta, table[4], core, sums, partial, total; };
 
 Layout layout_of(const fdb_attn_params& p, const ExpandGeometry& g) {
@@ -717,10 +731,12 @@ Layout layout_of(const fdb_attn_params& p, const ExpandGeometry& g) {
   for (int i = 0; i < 4; ++i) { l.table[i] = off; off = align256(off + ((i & 1) ? (p.pos_query ? table : 0) : (p.pos_key ? table : 0))); }
   // the two sides run one after the other and share these
   const bool terms = p.pos_key != nullptr || p.pos_query != nullptr;
-  const int table_rows = table_rows_of(p);
+  const int table_rows = table_rows_of(p), group = sum_heads_of(p), rest = p.heads % group;
   l.core = off;    off = align256(off + (terms ? uint64_t(p.total_rows) * p.heads * kHeadDim * 4 : 0));
-  l.sums = off;    off = align256(off + (terms ? uint64_t(p.total_rows) * p.heads * table_rows * 2 : 0));
-  l.partial = off; off = align256(off + (terms ? bwd_tables_partial_bytes(p.total_rows, p.heads, table_rows) : 0));
+  l.sums = off;    off = align256(off + (terms ? uint64_t(p.total_rows) * group * table_rows * 2 : 0));
+  const uint64_t partial = std::max(bwd_tables_partial_bytes(p.total_rows, group, table_rows),
+                                    rest > 0 ? bwd_tables_partial_bytes(p.total_rows, rest, table_rows) : 0);
+  l.partial = off; off = align256(off + (terms ? partial : 0));
   l.total = off;
   return l;
 }
@@ -756,6 +772,7 @@ int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g,
   a.lut = p.bucket_lut; a.lut_d_min = p.lut_d_min; a.lut_len = p.lut_len;
   a.table_rows = table_rows_of(p);
   a.status = p.status;
+  a.head0 = 0; a.sum_heads = sum_heads_of(p);
   a.heads = p.heads; a.packed = p.cu_seqlens != nullptr; a.max_seqlen = p.max_seqlen; a.total_rows = p.total_rows;
   a.sat_lo = DKV ? -g.sat_hi : g.sat_lo;
   a.sat_hi = DKV ? -g.sat_lo : g.sat_hi;
@@ -766,30 +783,38 @@ int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g,
 }
 
 template <bool DKV>
-int launch_bwd(const BwdArgs& a, const fdb_attn_bwd_params& b, char* partial, int64_t slots, cudaStream_t stream) {
+int launch_bwd(BwdArgs a, const fdb_attn_bwd_params& b, char* partial, int64_t slots, cudaStream_t stream) {
   const fdb_attn_params& p = *b.fwd;
   static std::atomic<uint64_t> smem_done{0};
   auto kernel = bwd_kernel<DKV>;
   cudaError_t e = allow_smem(smem_done, reinterpret_cast<const void*>(kernel), (int)kSmemBytes);
-  if (e == cudaSuccess && slots > 0) e = launch_kernel<BwdArgs>(kernel, a, dim3((unsigned)slots, p.heads), kThreads, kSmemBytes, false, stream);
-  if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd launch: %s", cudaGetErrorString(e));
-  if (a.xrow == nullptr) return FDB_OK;
-  BwdTablesCall c;
-  c.sums = a.sums;
-  c.table = DKV ? p.pos_query : p.pos_key;
-  const TableStrides strides = table_strides(b);
-  c.table_row_stride = strides.row; c.table_head_stride = strides.head;
-  c.operand = DKV ? p.k : p.q;
-  c.operand_row_stride = DKV ? p.k_row_stride : p.q_row_stride;
-  c.operand_head_stride = DKV ? p.k_head_stride : p.q_head_stride;
-  c.core = a.core;
-  c.out = a.grad;
-  c.out_row_stride = a.grad_rs; c.out_head_stride = a.grad_hs;
-  c.dtable = DKV ? b.dpos_query : b.dpos_key;
-  c.partial = reinterpret_cast<float*>(partial);
-  c.rows = p.total_rows; c.heads = p.heads; c.table_rows = a.table_rows;
-  c.status = p.status;
-  return launch_bwd_tables(c, stream);
+  const int group = a.xrow != nullptr ? a.sum_heads : p.heads;  // (without a row term there are no sums)
+  for (a.head0 = 0; a.head0 < p.heads; a.head0 += group) {
+    const int heads = std::min(group, p.heads - a.head0);
+    if (e == cudaSuccess && slots > 0) e = launch_kernel<BwdArgs>(kernel, a, dim3((unsigned)slots, heads), kThreads, kSmemBytes, false, stream);
+    if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd launch: %s", cudaGetErrorString(e));
+    if (a.xrow == nullptr) continue;
+    auto at = [&](const void* base, int64_t head_stride) { return static_cast<const __nv_bfloat16*>(base) + a.head0 * head_stride; };
+    BwdTablesCall c;
+    c.sums = a.sums;
+    const TableStrides strides = table_strides(b);
+    c.table = at(DKV ? p.pos_query : p.pos_key, strides.head);
+    c.table_row_stride = strides.row; c.table_head_stride = strides.head;
+    c.operand_row_stride = DKV ? p.k_row_stride : p.q_row_stride;
+    c.operand_head_stride = DKV ? p.k_head_stride : p.q_head_stride;
+    c.operand = at(DKV ? p.k : p.q, c.operand_head_stride);
+    c.core = a.core + (int64_t)a.head0 * kHeadDim;
+    c.core_row_stride = (int64_t)p.heads * kHeadDim;
+    c.out = const_cast<__nv_bfloat16*>(at(a.grad, a.grad_hs));
+    c.out_row_stride = a.grad_rs; c.out_head_stride = a.grad_hs;
+    c.dtable = const_cast<__nv_bfloat16*>(at(DKV ? b.dpos_query : b.dpos_key, strides.head));
+    c.partial = reinterpret_cast<float*>(partial);
+    c.rows = p.total_rows; c.heads = heads; c.table_rows = a.table_rows;
+    c.status = p.status;
+    const int rc = launch_bwd_tables(c, stream);
+    if (rc != FDB_OK) return rc;
+  }
+  return FDB_OK;
 }
 
 int check_bwd(const fdb_attn_bwd_params* b, ExpandGeometry* g) {

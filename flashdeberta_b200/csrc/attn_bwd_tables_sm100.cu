@@ -52,7 +52,8 @@ enum Bar : uint32_t {
 
 struct alignas(64) TableArgs {
   CUtensorMap tm_sums, tm_table, tm_operand;
-  float* core;               // (rows, heads, 64): read; written unless this is the last group of table rows
+  float* core;               // (heads, 64) per row: read; written unless this is the last group of table rows
+  int64_t core_row_stride;
   __nv_bfloat16* out;        // last group: rows of row_stride elements, heads of head_stride
   int64_t row_stride, head_stride;
   float* partial;            // (heads, parts, group rows, 64)
@@ -165,7 +166,7 @@ __global__ void __launch_bounds__(kThreads, 1) bwd_tables_kernel(const __grid_co
       const uint32_t i = uint32_t(t - t0), o = i & 1u;
       const int row = t * 128 + r;
       const bool valid = row < args.rows;
-      float4* core = reinterpret_cast<float4*>(args.core + ((int64_t)(valid ? row : args.rows - 1) * args.heads + head) * 64);
+      float4* core = reinterpret_cast<float4*>(args.core + (int64_t)(valid ? row : args.rows - 1) * args.core_row_stride + head * 64);
       float4 c[16];
 #pragma unroll
       for (int q = 0; q < 16; ++q) c[q] = core[q];
@@ -283,7 +284,7 @@ int launch_bwd_tables(const BwdTablesCall& c, cudaStream_t stream) {
   if ((rc = make_map_sums(&a.tm_sums, c.sums, c.table_rows, c.rows, c.heads))) return rc;
   if ((rc = make_map_rows(&a.tm_table, c.table, c.table_rows, c.heads, c.table_row_stride, c.table_head_stride, 128, false, "position table"))) return rc;
   if ((rc = make_map_rows(&a.tm_operand, c.operand, c.rows, c.heads, c.operand_row_stride, c.operand_head_stride, 128, false, "backward operand"))) return rc;
-  a.core = c.core;
+  a.core = c.core; a.core_row_stride = c.core_row_stride;
   a.out = static_cast<__nv_bfloat16*>(c.out);
   a.row_stride = c.out_row_stride; a.head_stride = c.out_head_stride;
   a.partial = c.partial;

@@ -287,3 +287,21 @@ def test_model_keeps_transformers_parameter_names():
     ids, mask = torch.randint(1, 100, (2, 9)), torch.ones(2, 9)
     with torch.no_grad():
         assert torch.equal(ours.embeddings(input_ids=ids, mask=mask), theirs.embeddings(input_ids=ids, mask=mask))
+
+
+def test_backward_workspace_is_bounded_beside_what_every_row_needs_once():
+    """The bucket sums (2 bytes per row, head and table row) are kept for as many heads at a time as fit 2 GiB."""
+    from flashdeberta_b200 import backward
+    lib, lut = _lib.load(), 0x1000
+    for rows, heads, buckets in [(1 << 20, 16, 256), (400000, 12, 256), (1 << 17, 16, 256), (1 << 20, 16, 1600), (4096, 12, 256)]:
+        p = _params(batch=1, max_seqlen=rows, total_rows=rows, heads=heads, pos_key=0x1000, pos_query=0x1000, position_buckets=buckets,
+                    max_relative_positions=2 * buckets, bucket_lut=lut, lut_d_min=-2 * buckets, lut_len=3000)
+        for n in ("q", "k", "v"):
+            setattr(p, n + "_row_stride", heads * 64)
+        p.out_row_stride = heads * 64
+        b = backward.BwdParams()
+        b.struct_bytes, b.fwd = C.sizeof(b), C.pointer(p)
+        need = lib.fdb_attn_bwd_workspace_bytes(C.byref(b))
+        once = rows * heads * (64 * 4 + 4)                                  # dQ or dK in fp32, delta
+        sums = min(rows * heads * 2 * buckets * 2, max(1 << 31, rows * 2 * buckets * 2))  # (one head at least)
+        assert once < need <= once + sums + (128 << 20), (rows, heads, buckets, need)
