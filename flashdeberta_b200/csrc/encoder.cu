@@ -26,6 +26,7 @@ struct LayerPlan {
   fdb_encoder_layer d;
   LinearWeight wq, wk, wv, wo, wi, wd;
 };
+constexpr int kMaxLayers = 4096;  // (a layer's plan is some 3 KB)
 struct EncoderPlan {
   int hidden, heads, ffn;
   std::vector<LayerPlan> layers;
@@ -247,10 +248,16 @@ extern "C" FDB_API int fdb_encoder_create(const fdb_encoder_layer* layers, int32
   if (layers == nullptr || plan == nullptr || n_layers <= 0) return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_encoder_create: bad argument");
   if (heads <= 0 || hidden != heads * kHeadDim || hidden % 256 != 0 || hidden > 2048 || ffn <= 0 || ffn % 64 != 0)
     return fail(FDB_ERR_UNSUPPORTED, "fdb_encoder_create: hidden %d, heads %d, ffn %d", hidden, heads, ffn);
+  if (n_layers > kMaxLayers) return fail(FDB_ERR_LIMIT, "fdb_encoder_create: %d layers (at most %d)", n_layers, kMaxLayers);
   EncoderPlan* e = new (std::nothrow) EncoderPlan;
   if (e == nullptr) return fail(FDB_ERR_LIMIT, "fdb_encoder_create: out of host memory");
   e->hidden = hidden; e->heads = heads; e->ffn = ffn;
-  e->layers.resize(n_layers);
+  try {  // (no exception leaves a C entry)
+    e->layers.resize(n_layers);
+  } catch (const std::bad_alloc&) {
+    delete e;
+    return fail(FDB_ERR_LIMIT, "fdb_encoder_create: out of host memory");
+  }
   int rc = FDB_OK;
   for (int i = 0; i < n_layers && rc == FDB_OK; ++i) {
     LayerPlan& l = e->layers[i];

@@ -374,7 +374,7 @@ FDB_API int fdb_expand_tables(const void* pos_key, const void* pos_query, void* 
  *
  * fdb_encoder_create copies the layer descriptions and encodes the weights' tensor maps; the weights themselves stay the
  * caller's and must outlive the plan at these addresses (their contents may change).  hidden = heads * 64, hidden a
- * multiple of 256 up to 2048, ffn a multiple of 64; every pointer 16-byte aligned; biases may be NULL.
+ * multiple of 256 up to 2048, ffn a multiple of 64, at most 4096 layers; every pointer 16-byte aligned; biases may be NULL.
  */
 typedef struct fdb_encoder_layer {
   const void *wq, *bq, *wk, *bk, *wv, *bv; /* (hidden, hidden) and (hidden) */

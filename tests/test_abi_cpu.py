@@ -305,3 +305,12 @@ def test_backward_workspace_is_bounded_beside_what_every_row_needs_once():
         once = rows * heads * (64 * 4 + 4)                                  # dQ or dK in fp32, delta
         sums = min(rows * heads * 2 * buckets * 2, max(1 << 31, rows * 2 * buckets * 2))  # (one head at least)
         assert once < need <= once + sums + (128 << 20), (rows, heads, buckets, need)
+
+
+def test_encoder_plan_of_too_many_layers_is_an_error():
+    """Not an exception that leaves the C entry, and no allocation of that size."""
+    from flashdeberta_b200 import engine
+    lib, layer, plan = _lib.load(), engine.EncoderLayer(), C.c_void_p()
+    for n in (4097, 2 ** 31 - 1):
+        assert lib.fdb_encoder_create(C.byref(layer), n, 256, 4, 512, C.byref(plan)) == -6
+    assert not plan.value and "layers" in lib.fdb_last_error().decode()
