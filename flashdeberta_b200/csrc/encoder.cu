@@ -214,6 +214,10 @@ int check_call(const fdb_encoder_call* c) {
   if (c->cu_seqlens == nullptr && (int64_t)c->batch * c->max_seqlen != c->total_rows)
     return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_encoder_call: dense ids need total_rows == batch * max_seqlen");
   if (c->mask_type < FDB_MASK_F32 || c->mask_type > FDB_MASK_BF16) return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_encoder_call: unknown mask_type %d", c->mask_type);
+  const unsigned mask_bytes[] = {4, 8, 4, 1, 2};  // of FDB_MASK_*
+  if (!aligned_to(16, c->out, c->emb_table, c->emb_gamma, c->emb_beta) || !aligned_to(8, c->ids) || !aligned_to(4, c->cu_seqlens, c->status) ||
+      !aligned_to(2, c->lut) || !aligned_to(mask_bytes[c->mask_type], c->mask))
+    return fail(FDB_ERR_ALIGNMENT, "fdb_encoder_call: out and the embedding stage must be 16-byte aligned, the others to their elements");
   if ((int64_t)c->total_rows > (int64_t(1) << 31) - 256) return fail(FDB_ERR_LIMIT, "fdb_encoder_call: total_rows");
   return FDB_OK;
 }
@@ -231,6 +235,8 @@ extern "C" FDB_API int fdb_expand_tables(const void* pos_key, const void* pos_qu
   if ((pos_key != nullptr) != (exp_key != nullptr) || (pos_query != nullptr) != (exp_query != nullptr) || lut == nullptr || lut_len < 2 ||
       heads <= 0 || table_rows <= 0 || table_rows % 2 != 0)
     return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_expand_tables: bad argument");
+  if (!aligned_to(16, pos_key, pos_query, exp_key, exp_query) || !aligned_to(2, lut))
+    return fail(FDB_ERR_ALIGNMENT, "fdb_expand_tables: tables must be 16-byte aligned");
   if (pos_key == nullptr && pos_query == nullptr) return FDB_OK;
   fdb_attn_params p = {};
   p.dtype = FDB_BF16;
@@ -269,7 +275,8 @@ extern "C" FDB_API int fdb_encoder_create(const fdb_encoder_layer* layers, int32
     }
     const uintptr_t all = (uintptr_t)d.wq | (uintptr_t)d.bq | (uintptr_t)d.wk | (uintptr_t)d.bk | (uintptr_t)d.wv | (uintptr_t)d.bv |
                           (uintptr_t)d.wo | (uintptr_t)d.bo | (uintptr_t)d.wi | (uintptr_t)d.bi | (uintptr_t)d.wd | (uintptr_t)d.bd |
-                          (uintptr_t)d.exp_key | (uintptr_t)d.exp_query;
+                          (uintptr_t)d.exp_key | (uintptr_t)d.exp_query | (uintptr_t)d.ln1_gamma | (uintptr_t)d.ln1_beta |
+                          (uintptr_t)d.ln2_gamma | (uintptr_t)d.ln2_beta;
     if ((all & 15u) != 0) { rc = fail(FDB_ERR_ALIGNMENT, "fdb_encoder_create: layer %d has a pointer that is not 16-byte aligned", i); break; }
     struct { LinearWeight* w; const void* p; int n, k; } maps[6] = {
         {&l.wq, d.wq, hidden, hidden}, {&l.wk, d.wk, hidden, hidden}, {&l.wv, d.wv, hidden, hidden},

@@ -14,6 +14,10 @@ void clear_error();
 // argument checks shared by the entry points; `fused` adds the layout rules of the tensor-core kernel
 int validate(const fdb_attn_params* p, bool fused);
 
+// whether every pointer (NULL included) is a multiple of `bytes`
+template <typename... P>
+inline bool aligned_to(unsigned bytes, const P*... p) { return (((reinterpret_cast<uintptr_t>(p) | ... | uintptr_t(0))) & (bytes - 1)) == 0; }
+
 // ---- bucket table (host) -------------------------------------------------------------------------------------------
 int64_t signed_bucket(int32_t bucket_size, int32_t max_position, int64_t rel);
 int32_t relative_index(int32_t position_buckets, int32_t max_relative_positions, int64_t distance);

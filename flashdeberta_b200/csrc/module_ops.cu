@@ -102,6 +102,9 @@ extern "C" FDB_API int fdb_lengths_from_mask(const void* mask, int32_t mask_type
   if (batch < 0 || seqlen < 0) return fail(FDB_ERR_INVALID_ARGUMENT, "lengths_from_mask: batch %d, seqlen %d", batch, seqlen);
   if (batch == 0) return FDB_OK;
   if ((mask == nullptr && seqlen > 0) || lens == nullptr) return fail(FDB_ERR_INVALID_ARGUMENT, "lengths_from_mask: NULL pointer");
+  const unsigned mask_bytes[] = {4, 8, 4, 1, 2};  // of FDB_MASK_*
+  if (mask_type >= FDB_MASK_F32 && mask_type <= FDB_MASK_BF16 && (!aligned_to(mask_bytes[mask_type], mask) || !aligned_to(4, lens, status)))
+    return fail(FDB_ERR_ALIGNMENT, "lengths_from_mask: mask, lens and status must be aligned to their elements");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   switch (mask_type) {  // a float is zero when no bit but the sign is set
     case kMaskF32: lengths<uint32_t>(mask, batch, seqlen, batch_stride, token_stride, 0x7fffffffu, lens, status, s); break;
@@ -126,8 +129,8 @@ extern "C" FDB_API int fdb_column_sums(const void* x, int64_t rows, int32_t cols
   if (x == nullptr || out == nullptr || rows < 0 || cols <= 0 || rows > 2147483647LL || more_rows < 0 || more_rows > 2147483647LL ||
       more_cols > cols || (more_rows > 0 && (more == nullptr || more_cols <= 0)))
     return fail(FDB_ERR_INVALID_ARGUMENT, "column_sums: bad pointer or size");
-  if (cols % 8 != 0 || more_cols % 8 != 0 || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(more)) & 15u) != 0)
-    return fail(FDB_ERR_ALIGNMENT, "column_sums: columns must be a multiple of 8, pointers 16-byte aligned");
+  if (cols % 8 != 0 || more_cols % 8 != 0 || !aligned_to(16, x, more) || !aligned_to(4, workspace) || !aligned_to(2, out))
+    return fail(FDB_ERR_ALIGNMENT, "column_sums: columns must be a multiple of 8, matrices 16-byte aligned, the others to their elements");
   if (workspace == nullptr || workspace_bytes < fdb_column_sums_workspace_bytes(rows, more_rows, cols))
     return fail(FDB_ERR_WORKSPACE, "column_sums: workspace too small");
   cudaStream_t s = static_cast<cudaStream_t>(stream);

@@ -219,6 +219,9 @@ extern "C" FDB_API int fdb_quantize_attn(const fdb_quantize_attn_params* q, void
   // a table is one slab of table_rows rows per head
   if (p.pos_key) add(p.pos_key, q->pos_key, q->pos_key_scale, 64, 64, p.heads * table_rows, nullptr, table_rows, p.heads, 1);
   if (p.pos_query) add(p.pos_query, q->pos_query, q->pos_query_scale, 64, 64, p.heads * table_rows, nullptr, table_rows, p.heads, 1);
+  if (!aligned_to(8, q->q, q->k, q->v, q->pos_key, q->pos_query) ||
+      !aligned_to(4, q->amax, q->q_scale, q->k_scale, q->v_scale, q->pos_key_scale, q->pos_query_scale))
+    return fail(FDB_ERR_ALIGNMENT, "fdb_quantize_attn: e4m3 outputs must be 8-byte aligned, scales and amax to their elements");
   for (int j = 0; j < jobs.n; ++j)
     if (jobs.job[j].y == nullptr || jobs.job[j].scale == nullptr) return fail(FDB_ERR_INVALID_ARGUMENT, "fdb_quantize_attn: NULL output");
   return run(jobs, q->amax, need, static_cast<cudaStream_t>(stream));

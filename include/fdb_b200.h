@@ -309,11 +309,11 @@ typedef struct fdb_quantize_attn_params {
   uint32_t struct_bytes;       /* sizeof(fdb_quantize_attn_params) */
   int32_t reserved;
   const fdb_attn_params* in;   /* the call in bf16: tensors, strides and layout are looked at */
-  void *q, *k, *v;             /* out, e4m3, contiguous (total_rows, heads, 64) */
+  void *q, *k, *v;             /* out, e4m3, contiguous (total_rows, heads, 64), 8-byte aligned like the tables' */
   void *pos_key, *pos_query;   /* out, e4m3 (heads, 2*att_span, 64), each with its table */
   float *q_scale, *k_scale, *v_scale;          /* out (batch, heads) */
   float *pos_key_scale, *pos_query_scale;      /* out (heads) */
-  void* amax;                  /* device scratch: 4 bytes for every scale, 16-byte aligned */
+  void* amax;                  /* device scratch: 4 bytes for every scale */
   uint64_t amax_bytes;
 } fdb_quantize_attn_params;
 FDB_API int fdb_quantize_attn(const fdb_quantize_attn_params* p, void* stream);
@@ -359,7 +359,7 @@ FDB_API int fdb_linear_gelu(const void* x, const void* weight, const void* bias,
 /*
  * Rows of the position tables gathered through the bucket index, as fdb_attn_fwd does on every call that is not prepared:
  * exp_*[h][u] = pos_*[h][idx(d_first + u)], (heads, fdb_expanded_rows(lut_d_min, lut_len), 64) bf16 each.  Either pair may be
- * NULL.  pos_* as in fdb_attn_params.
+ * NULL.  pos_* as in fdb_attn_params; all four 16-byte aligned.
  */
 FDB_API int32_t fdb_expanded_rows(int32_t lut_d_min, int32_t lut_len);
 FDB_API int fdb_expand_tables(const void* pos_key, const void* pos_query, void* exp_key, void* exp_query, int32_t heads,
@@ -436,7 +436,7 @@ typedef struct fdb_encoder_call {
   const int16_t* lut;    /* bucket table as in fdb_attn_params; NULL without position terms */
   float sm_scale;
   float emb_eps;
-  const void *emb_table, *emb_gamma, *emb_beta; /* (emb_rows, hidden), (hidden), (hidden) bf16 */
+  const void *emb_table, *emb_gamma, *emb_beta; /* (emb_rows, hidden), (hidden), (hidden) bf16; 16-byte aligned, as out */
   int64_t emb_rows;
   void* out;             /* total_rows rows of hidden, bf16; rows of invalid tokens are written as zeros */
   void* workspace;       /* device, >= fdb_encoder_workspace_bytes(), 256-byte aligned */

@@ -314,3 +314,131 @@ def test_encoder_plan_of_too_many_layers_is_an_error():
     for n in (4097, 2 ** 31 - 1):
         assert lib.fdb_encoder_create(C.byref(layer), n, 256, 4, 512, C.byref(plan)) == -6
     assert not plan.value and "layers" in lib.fdb_last_error().decode()
+
+
+def _with_tables(**kw):
+    base = dict(pos_key=0x1000, pos_query=0x1000, position_buckets=256, max_relative_positions=512, bucket_lut=0x1000, lut_d_min=-512, lut_len=1019)
+    base.update(kw)
+    return _params(**base)
+
+
+def _refused(rc, code):
+    assert rc == code and _lib.load().fdb_last_error().decode() != ""
+
+
+@pytest.mark.parametrize("change,code", [
+    (dict(struct_bytes=0), -1), (dict(dout=None), -1), (dict(dq=None), -1), (dict(dpos_key=None), -1), (dict(dpos_query=None), -1),
+    (dict(dout=0x1008), -3), (dict(dv=0x1002), -3), (dict(dout_row_stride=100), -3), (dict(grad_head_stride=0), -3),
+    (dict(table_row_stride=4), -3), (dict(workspace=None), -4), (dict(workspace_bytes=16), -4), (dict(workspace=0x1010), -3),
+])
+def test_backward_argument_errors(change, code):
+    from flashdeberta_b200 import backward
+    p = _with_tables(lse=0x1000)
+    b = backward.BwdParams(C.sizeof(backward.BwdParams), 0, C.pointer(p), 0x1000, 128, 64, 0x1000, 0x1000, 0x1000, 128, 64, 0x1000, 0x1000, 0, 0,
+                           0x1000, 1 << 40)
+    for k, v in change.items():
+        setattr(b, k, v)
+    _refused(_lib.load().fdb_attn_bwd(C.byref(b), None), code)
+
+
+@pytest.mark.parametrize("change,code", [
+    (dict(dtype=1), -2), (dict(head_dim=32), -2), (dict(position_buckets=255), -2), (dict(lut_len=4000), -6), (dict(lse=None), -1),
+])
+def test_backward_refuses_calls_it_is_not_for(change, code):
+    from flashdeberta_b200 import backward
+    p = _with_tables(lse=0x1000, **change) if "lse" not in change else _with_tables()
+    b = backward.BwdParams(C.sizeof(backward.BwdParams), 0, C.pointer(p), 0x1000, 128, 64, 0x1000, 0x1000, 0x1000, 128, 64, 0x1000, 0x1000, 0, 0,
+                           0x1000, 1 << 40)
+    _refused(_lib.load().fdb_attn_bwd(C.byref(b), None), code)
+
+
+@pytest.mark.parametrize("change,code", [
+    (dict(struct_bytes=0), -1), (dict(input=None), -1), (dict(q=None), -1), (dict(pos_key=None), -1), (dict(k_scale=None), -1),
+    (dict(v=0x1004), -3), (dict(pos_query=0x1001), -3), (dict(q_scale=0x1002), -3), (dict(amax=0x1001), -3), (dict(amax=None), -4), (dict(amax_bytes=8), -4),
+])
+def test_quantize_attn_argument_errors(change, code):
+    p = _with_tables()
+    q = _lib.QuantizeAttnParams(C.sizeof(_lib.QuantizeAttnParams), 0, C.pointer(p), *[0x1000] * 11, 1 << 20)
+    for k, v in change.items():
+        setattr(q, k, v)
+    _refused(_lib.load().fdb_quantize_attn(C.byref(q), None), code)
+
+
+def test_quantize_attn_without_rows_is_a_no_op():
+    p = _with_tables(batch=0, total_rows=0)
+    q = _lib.QuantizeAttnParams(C.sizeof(_lib.QuantizeAttnParams), 0, C.pointer(p))
+    assert _lib.load().fdb_quantize_attn(C.byref(q), None) == 0
+
+
+@pytest.mark.parametrize("change,code", [
+    (dict(struct_bytes=0), -1), (dict(attn=None), -1), (dict(in_features=100), -2), (dict(x=None), -1), (dict(bv=None), -1),
+    (dict(wk=0x1008), -3), (dict(rel=0x1008), -3), (dict(table_row_stride=64), -3), (dict(table_row_stride=132), -3), (dict(table_head_stride=128), -3),
+])
+def test_projected_forward_argument_errors(change, code):
+    from flashdeberta_b200 import projected
+    p = _with_tables(lse=0x1000, workspace=0x1000, workspace_bytes=1 << 40)
+    c = projected._ProjectedParams(C.sizeof(projected._ProjectedParams), 128, C.pointer(p), 256, 64, *[0x1000] * 8)
+    for k, v in change.items():
+        setattr(c, k, v)
+    _refused(_lib.load().fdb_projected_forward(C.byref(c), None), code)
+
+
+@pytest.mark.parametrize("args,code", [
+    ((None, 0, 2, 8, 8, 1, 0x1000, None), -1), ((0x1000, 0, 2, 8, 8, 1, None, None), -1), ((0x1000, 9, 2, 8, 8, 1, 0x1000, None), -1),
+    ((0x1000, 0, -1, 8, 8, 1, 0x1000, None), -1), ((0x1002, 0, 2, 8, 8, 1, 0x1000, None), -3), ((0x1004, 1, 2, 8, 8, 1, 0x1000, None), -3),
+    ((0x1001, 4, 2, 8, 8, 1, 0x1000, None), -3), ((0x1000, 3, 2, 8, 8, 1, 0x1002, None), -3), ((None, 0, 0, 8, 8, 1, None, None), 0),
+])
+def test_lengths_from_mask_argument_errors(args, code):
+    assert _lib.load().fdb_lengths_from_mask(*args, None) == code
+
+
+@pytest.mark.parametrize("args,code", [
+    ((None, 8, 64, None, 0, 0, 0x1000, 0x1000, 1 << 20), -1), ((0x1000, 8, 64, None, 4, 64, 0x1000, 0x1000, 1 << 20), -1),
+    ((0x1000, 8, 64, 0x1000, 4, 72, 0x1000, 0x1000, 1 << 20), -1), ((0x1000, 8, 60, None, 0, 0, 0x1000, 0x1000, 1 << 20), -3),
+    ((0x1008, 8, 64, None, 0, 0, 0x1000, 0x1000, 1 << 20), -3), ((0x1000, 8, 64, None, 0, 0, 0x1001, 0x1000, 1 << 20), -3),
+    ((0x1000, 8, 64, None, 0, 0, 0x1000, 0x1002, 1 << 20), -3), ((0x1000, 8, 64, None, 0, 0, 0x1000, None, 0), -4), ((0x1000, 8, 64, None, 0, 0, 0x1000, 0x1000, 8), -4),
+])
+def test_column_sums_argument_errors(args, code):
+    _refused(_lib.load().fdb_column_sums(*args, None), code)
+
+
+@pytest.mark.parametrize("args,code", [
+    ((0x1000, None, None, None, 12, 512, 0x1000, -512, 1019), -1), ((0x1000, None, 0x1000, None, 12, 512, None, -512, 1019), -1),
+    ((0x1000, None, 0x1000, None, 0, 512, 0x1000, -512, 1019), -1), ((0x1008, None, 0x1000, None, 12, 512, 0x1000, -512, 1019), -3),
+    ((0x1000, None, 0x1008, None, 12, 512, 0x1000, -512, 1019), -3), ((None, 0x1000, None, 0x1002, 12, 512, 0x1000, -512, 1019), -3),
+    ((0x1000, None, 0x1000, None, 12, 512, 0x1001, -512, 1019), -3), ((None, None, None, None, 12, 512, 0x1000, -512, 1019), 0),
+])
+def test_expand_tables_argument_errors(args, code):
+    assert _lib.load().fdb_expand_tables(*args, None) == code
+
+
+@pytest.mark.parametrize("change,sizes,code", [
+    ({}, (256, 3, 512), -2), ({}, (192, 3, 512), -2), ({}, (256, 4, 500), -2), ({}, (4096, 64, 512), -2), (dict(wq=None), (256, 4, 512), -1),
+    (dict(ln2_beta=None), (256, 4, 512), -1), (dict(wd=0x1008), (256, 4, 512), -3), (dict(ln1_gamma=0x1008), (256, 4, 512), -3),
+    (dict(ln2_beta=0x1004), (256, 4, 512), -3), (dict(exp_query=0x1008), (256, 4, 512), -3),
+])
+def test_encoder_create_argument_errors(change, sizes, code):
+    from flashdeberta_b200 import engine
+    layer, plan = engine.EncoderLayer(*[0x1000] * 18, 1e-7, 1e-7), C.c_void_p()
+    for k, v in change.items():
+        setattr(layer, k, v)
+    _refused(_lib.load().fdb_encoder_create(C.byref(layer), 1, *sizes, C.byref(plan)), code)
+    assert not plan.value
+
+
+@pytest.mark.parametrize("change,code", [
+    (dict(struct_bytes=0), -1), (dict(plan=None), -1), (dict(ids=None), -1), (dict(out=None), -1), (dict(batch=-1), -1), (dict(emb_rows=0), -1),
+    (dict(total_rows=99), -1), (dict(cu_seqlens=0x1000, mask=0x1000), -1), (dict(mask_type=7), -1), (dict(out=0x1008), -3), (dict(emb_table=0x1008), -3),
+    (dict(emb_beta=0x1004), -3), (dict(ids=0x1004), -3), (dict(mask=0x1004, mask_type=1), -3), (dict(mask=0x1001, mask_type=4), -3), (dict(cu_seqlens=0x1002), -3),
+])
+def test_encoder_call_argument_errors(change, code):
+    from flashdeberta_b200 import engine
+    c = engine.EncoderCall()
+    c.struct_bytes, c.plan, c.ids, c.out = C.sizeof(c), 0x1000, 0x1000, 0x1000
+    c.emb_table = c.emb_gamma = c.emb_beta = 0x1000
+    c.batch, c.max_seqlen, c.total_rows, c.emb_rows = 2, 50, 100, 1000
+    for k, v in change.items():
+        setattr(c, k, v)
+    lib = _lib.load()
+    _refused(lib.fdb_encoder_forward(C.byref(c), None), code)
+    assert lib.fdb_encoder_workspace_bytes(C.byref(c)) == 0
