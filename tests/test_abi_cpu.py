@@ -316,6 +316,29 @@ def test_encoder_plan_of_too_many_layers_is_an_error():
     assert not plan.value and "layers" in lib.fdb_last_error().decode()
 
 
+def _structs():
+    from flashdeberta_b200 import backward, engine, projected
+    return [("fdb_attn_bwd_params", backward.BwdParams), ("fdb_quantize_attn_params", _lib.QuantizeAttnParams),
+            ("fdb_encoder_layer", engine.EncoderLayer), ("fdb_projected_params", projected._ProjectedParams),
+            ("fdb_encoder_call", engine.EncoderCall)]
+
+
+@pytest.mark.parametrize("name,struct", _structs(), ids=[n for n, _ in _structs()])
+def test_other_struct_layouts_match_the_header(name, struct, tmp_path):
+    """Size, order and offsets, of every field that the header declares."""
+    text = open(HEADER).read()
+    body = re.sub(r"/\*.*?\*/", "", re.search(r"typedef struct %s \{(.*?)\} %s;" % (name, name), text, re.S).group(1), flags=re.S)
+    declared = [re.search(r"(\w+)$", part.strip()).group(1) for line in body.split(";") for part in line.split(",") if part.strip()]
+    rename = {"fdb_quantize_attn_params": {"in": "input"}}.get(name, {})
+    assert [rename.get(f, f) for f in declared] == [f[0] for f in struct._fields_]
+    src, exe = tmp_path / "layout.c", tmp_path / "layout"
+    src.write_text('#include <stdio.h>\n#include <stddef.h>\n#include "fdb_b200.h"\nint main(void) {\n  printf("%%zu", sizeof(%s));\n' % name
+                   + "".join('  printf(" %%zu", offsetof(%s, %s));\n' % (name, f) for f in declared) + "  return 0;\n}\n")
+    subprocess.check_call(["gcc", "-std=c11", "-I", os.path.join(ROOT, "include"), str(src), "-o", str(exe)])
+    out = [int(v) for v in subprocess.check_output([str(exe)], text=True).split()]
+    assert out == [C.sizeof(struct)] + [getattr(struct, rename.get(f, f)).offset for f in declared]
+
+
 def _with_tables(**kw):
     base = dict(pos_key=0x1000, pos_query=0x1000, position_buckets=256, max_relative_positions=512, bucket_lut=0x1000, lut_d_min=-512, lut_len=1019)
     base.update(kw)
