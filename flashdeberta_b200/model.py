@@ -204,7 +204,8 @@ class FlashDebertaV2Encoder(DebertaV2Encoder):
             # (B,) int32; the only form of the mask the layers see.  A batch that stays padded is addressed by lengths
             # alone: its mask must be right-padded (checked here; the packed path takes any layout)
             seq_lens = lengths_from_mask(attention_mask, check=packed_all is None)
-            self._mask_cache = (key, attention_mask, (input_mask, seq_lens, packed_all, looked))
+            if not ops.capturing(attention_mask):  # (in a capture the lengths have not been counted)
+                self._mask_cache = (key, attention_mask, (input_mask, seq_lens, packed_all, looked))
         # query_states / a list of hidden states are only used by z_steps: those stay padded
         packed = packed_all if (query_states is None and torch.is_tensor(hidden_states)) else None
         if packed is None and packed_all is not None:

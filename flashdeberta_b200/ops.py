@@ -321,7 +321,8 @@ def disentangled_attention(
             return (out, lse) if return_lse else out
         stream = raw_stream(q.device)
         flags = 0
-        if prepared is not None and need <= prepared.max_bytes and prepared.stream in (None, stream):
+        # (a captured call takes scratch of its graph: what it sets up there has not been set up for any other call)
+        if prepared is not None and need <= prepared.max_bytes and prepared.stream in (None, stream) and not capturing(q):
             prepared.stream = stream  # the buffer stays with the first stream that used it; other streams take scratch
             layout = (q.device, stream, need, p.dtype, p.batch, p.max_seqlen, p.total_rows, p.heads, int(position_buckets),
                       int(max_relative_positions), cu_seqlens is not None)

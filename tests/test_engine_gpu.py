@@ -331,3 +331,47 @@ def test_masked_call_does_not_depend_on_what_memory_held(lens):
             _close(first, _walk(model, ids, mask), 0.1, 5e-3, "against the walk")
         else:
             assert torch.count_nonzero(first) == 0
+
+
+def test_captures_of_the_module_leave_each_other_alone():
+    """The attention module called for the first time inside a capture, and again in a second one before the first has run: neither
+    relies on what the other would set up, nor does an eager call on the same stream."""
+    from flashdeberta_b200 import ops
+    module, warm = (_model().encoder.layer[0].attention.self for _ in range(2))
+    x, rel = torch.randn(2, 300, 256, device=DEV).bfloat16(), torch.randn(512, 256, device=DEV).bfloat16()
+    lens = torch.tensor([300, 131], dtype=torch.int32, device=DEV)
+    stream = torch.cuda.Stream()
+    with torch.no_grad():
+        want = warm(x, lens, rel_embeddings=rel)[0]  # (the bucket table, and the kernels)
+        torch.cuda.synchronize()
+        graphs = []
+        for _ in range(2):
+            graph = torch.cuda.CUDAGraph()
+            with torch.cuda.graph(graph, stream=stream):
+                out = module(x, lens, rel_embeddings=rel)[0]
+            graphs.append((graph, out))
+        with torch.cuda.stream(stream):
+            eager = module(x, lens, rel_embeddings=rel)[0]
+        for graph, out in reversed(graphs):
+            graph.replay()
+            torch.cuda.synchronize()
+            assert torch.equal(out, want)
+        assert torch.equal(eager, want)
+    ops.check_status()
+
+
+def test_mask_analysed_in_a_capture_is_analysed_again():
+    """A batch that stays padded (pack_sequences off): the lengths counted in a capture are the graph's."""
+    from flashdeberta_b200 import ops
+    model = _model(pack_sequences=False)
+    ids, mask = _ragged(2, 300, (300, 131))
+    run = lambda m: model(input_ids=ids, attention_mask=m).last_hidden_state
+    with torch.no_grad():
+        want = run(mask)
+        other = mask.clone()
+        graph, out = _capture(lambda: run(other))
+        assert torch.equal(run(other), want)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    ops.check_status()

@@ -121,3 +121,19 @@ def test_make_fx_records_the_attention(mode):
     other = [(2 * t).detach().requires_grad_(True) for t in leaves]
     for a, b in zip(traced(*other), step(*other)):
         assert (a.float() - b.float()).norm() <= 1e-2 * b.float().norm()
+
+
+def test_saved_tensors_may_be_stored_elsewhere():
+    """Hooks that keep what the backward needs on the host: the addresses are those of what comes back."""
+    leaves, module = _leaves(DEV), _module().to(DEV)
+    x = torch.randn(2, 96, 256, device=DEV).bfloat16().requires_grad_(True)
+    rel = torch.randn(512, 256, device=DEV).bfloat16().requires_grad_(True)
+    for run, wrt in ((lambda: ops.disentangled_attention(*leaves, **KW), leaves),
+                     (lambda: module(x, None, rel_embeddings=rel)[0], [x, rel, *module.parameters()])):
+        want = torch.autograd.grad(run().sum(), wrt)
+        with torch.autograd.graph.save_on_cpu():
+            out = run()
+        junk = [torch.full((1 << 20,), float("nan"), device=DEV) for _ in range(8)]
+        for a, b in zip(torch.autograd.grad(out.sum(), wrt), want):
+            assert torch.equal(a, b)
+        del junk
