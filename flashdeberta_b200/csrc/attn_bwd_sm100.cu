@@ -97,12 +97,12 @@ struct alignas(64) BwdArgs {
   __nv_bfloat16* grad;                    // without it: dQ or dK
   __nv_bfloat16* dv;                      // <true>
   int64_t grad_rs, grad_hs;               // strides of dQ, dK, dV
-  __nv_bfloat16* sums;                    // (heads of this launch, rows, table_rows)
+  __nv_bfloat16* sums;                    // (heads of this launch, rows, table_rows); every pointer starts at the launch's first head
   const int16_t* lut;
   int32_t* status;
   int lut_d_min, lut_len, table_rows;
   int heads, packed, max_seqlen, total_rows;
-  int head0, sum_heads;                   // first head of this launch; heads that `sums` has room for
+  int sum_heads;                          // heads that `sums` has room for
   int sat_lo, sat_hi, d_first, xrows;     // in distances row - column
   float sm_scale;
 };
@@ -125,9 +125,9 @@ __device__ __forceinline__ void zero_row(const BwdArgs& a, int64_t row, int head
     else if (i < 8) *reinterpret_cast<uint4*>(a.grad + at) = z;
     if (DKV && i < 8) *reinterpret_cast<uint4*>(a.dv + at) = z;
   }
-  if (a.xrow != nullptr && head - a.head0 < a.sum_heads)
+  if (a.xrow != nullptr && head < a.sum_heads)
     for (int i = lane; i < a.table_rows / 8; i += n)
-      *reinterpret_cast<uint4*>(a.sums + ((int64_t)(head - a.head0) * a.total_rows + row) * a.table_rows + i * 8) = z;
+      *reinterpret_cast<uint4*>(a.sums + ((int64_t)head * a.total_rows + row) * a.table_rows + i * 8) = z;
 }
 
 template <bool DKV>
@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem - smem_u32(smem_raw));
   const int tid = threadIdx.x, warp = (int)uniform(uint32_t(tid) >> 5), lane = tid & 31;
-  const int head = args.head0 + (int)blockIdx.y;
+  const int head = blockIdx.y;
 
   const int4 slot = __ldg(args.slot_info + blockIdx.x);  // (sequence, first row of the tile in it, its first row, its length)
   if (slot.x < 0) return;
@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
       for (int i = 0; i < 32; ++i) {  // a row at a time: whole lines (a packed row behind the sequence is another one's)
         const int row = r0 + quad * 32 + i;
         if (row >= len && (args.packed || row >= row_limit)) break;
-        uint4* z = reinterpret_cast<uint4*>(args.sums + ((int64_t)blockIdx.y * args.total_rows + seq_row0 + row) * args.table_rows);
+        uint4* z = reinterpret_cast<uint4*>(args.sums + ((int64_t)head * args.total_rows + seq_row0 + row) * args.table_rows);
         for (int c = lane; c < args.table_rows / 8; c += 32) z[c] = make_uint4(0u, 0u, 0u, 0u);
       }
       __syncwarp();
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kThreads, 2) bwd_kernel(const __grid_constant_
       const uint32_t mine = smem + kSmemEmit + uint32_t(quad * 32 + lane) * kEmitPitch;
       constexpr uint32_t kHome = DKV ? 0u : 32u;  // byte offset of the current group
       sts_v4(mine + kHome, 0u, 0u, 0u, 0u);
-      uint4* sums = reinterpret_cast<uint4*>(args.sums + ((int64_t)blockIdx.y * args.total_rows + seq_row0 + (valid_row ? my_row : len - 1)) * args.table_rows);
+      uint4* sums = reinterpret_cast<uint4*>(args.sums + ((int64_t)head * args.total_rows + seq_row0 + (valid_row ? my_row : len - 1)) * args.table_rows);
       const uint32_t* bits = reinterpret_cast<const uint32_t*>(smem_gen + kSmemBits);
 #pragma unroll 1
       for (int j = 0; j < n_tiles; ++j) {
@@ -712,6 +712,7 @@ uint64_t align256(uint64_t x) { return (x + 255) & ~uint64_t(255); }
 // heads and 512 table rows are one group), and the workspace grows with the rows only by what every row needs once.
 constexpr uint64_t kSumBytes = uint64_t(1) << 31;
 int sum_heads_of(const fdb_attn_params& p) {
+  if (p.pos_key == nullptr && p.pos_query == nullptr) return p.heads;  // no sums
   const uint64_t head = uint64_t(p.total_rows) * table_rows_of(p) * 2;
   const uint64_t most = head == 0 ? p.heads : std::max<uint64_t>(1, std::min<uint64_t>(p.heads, kSumBytes / head));
   const int groups = (int)((p.heads + most - 1) / most);
@@ -741,11 +742,13 @@ Layout layout_of(const fdb_attn_params& p, const ExpandGeometry& g) {
   return l;
 }
 
+// Arguments for heads [head0, head0 + heads) of the call.
 template <bool DKV>
-int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layout& l, char* ws) {
+int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layout& l, char* ws, int head0, int heads) {
   const fdb_attn_params& p = *b.fwd;
+  auto at = [&](const void* base, int64_t head_stride) { return static_cast<const __nv_bfloat16*>(base) + head0 * head_stride; };
   auto operand = [&](CUtensorMap* m, const void* base, int64_t rs, int64_t hs, int box) {
-    return make_map_rows(m, base, p.total_rows, p.heads, rs, hs, box, false, "backward operand");
+    return make_map_rows(m, at(base, hs), p.total_rows, heads, rs, hs, box, false, "backward operand");
   };
   int rc;
   const int row = 128, col = kCols;
@@ -755,24 +758,24 @@ int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g,
   if ((rc = operand(&a.tm_col[1], DKV ? b.dout : p.v, DKV ? b.dout_row_stride : p.v_row_stride, DKV ? b.dout_head_stride : p.v_head_stride, col))) return rc;
   // <true>: the row term is p2c, distances are key - query
   const bool has_row = DKV ? p.pos_query != nullptr : p.pos_key != nullptr, has_col = DKV ? p.pos_key != nullptr : p.pos_query != nullptr;
-  a.xrow = has_row ? reinterpret_cast<const __nv_bfloat16*>(ws + l.table[DKV ? 3 : 0]) : nullptr;
-  a.xcol = has_col ? reinterpret_cast<const __nv_bfloat16*>(ws + l.table[DKV ? 2 : 1]) : nullptr;
+  a.xrow = has_row ? at(ws + l.table[DKV ? 3 : 0], (int64_t)g.rows * kHeadDim) : nullptr;
+  a.xcol = has_col ? at(ws + l.table[DKV ? 2 : 1], (int64_t)g.rows * kHeadDim) : nullptr;
   a.tm_xrow = a.tm_xcol = a.tm_xcol_sat = a.tm_row[0];
-  if (has_row && (rc = make_map_table(&a.tm_xrow, a.xrow, g.rows, p.heads, false, "row table", kWin))) return rc;
-  if (has_col && (rc = make_map_table(&a.tm_xcol, a.xcol, g.rows, p.heads, false, "column table", kWin))) return rc;
-  if (has_col && (rc = make_map_table(&a.tm_xcol_sat, a.xcol, g.rows, p.heads, false, "saturated rows", 8))) return rc;
+  if (has_row && (rc = make_map_table(&a.tm_xrow, a.xrow, g.rows, heads, false, "row table", kWin))) return rc;
+  if (has_col && (rc = make_map_table(&a.tm_xcol, a.xcol, g.rows, heads, false, "column table", kWin))) return rc;
+  if (has_col && (rc = make_map_table(&a.tm_xcol_sat, a.xcol, g.rows, heads, false, "saturated rows", 8))) return rc;
   a.slot_info = reinterpret_cast<const int4*>(ws + l.slot_info);
-  a.lse = p.lse;
-  a.delta = reinterpret_cast<const float*>(ws + l.delta);
-  a.core = reinterpret_cast<float*>(ws + l.core);
-  a.grad = static_cast<__nv_bfloat16*>(DKV ? b.dk : b.dq);
-  a.dv = DKV ? static_cast<__nv_bfloat16*>(b.dv) : nullptr;
+  a.lse = p.lse + head0;
+  a.delta = reinterpret_cast<const float*>(ws + l.delta) + head0;
+  a.core = reinterpret_cast<float*>(ws + l.core) + (int64_t)head0 * kHeadDim;
+  a.grad = const_cast<__nv_bfloat16*>(at(DKV ? b.dk : b.dq, b.grad_head_stride));
+  a.dv = DKV ? const_cast<__nv_bfloat16*>(at(b.dv, b.grad_head_stride)) : nullptr;
   a.grad_rs = b.grad_row_stride; a.grad_hs = b.grad_head_stride;
   a.sums = reinterpret_cast<__nv_bfloat16*>(ws + l.sums);
   a.lut = p.bucket_lut; a.lut_d_min = p.lut_d_min; a.lut_len = p.lut_len;
   a.table_rows = table_rows_of(p);
   a.status = p.status;
-  a.head0 = 0; a.sum_heads = sum_heads_of(p);
+  a.sum_heads = sum_heads_of(p);
   a.heads = p.heads; a.packed = p.cu_seqlens != nullptr; a.max_seqlen = p.max_seqlen; a.total_rows = p.total_rows;
   a.sat_lo = DKV ? -g.sat_hi : g.sat_lo;
   a.sat_hi = DKV ? -g.sat_lo : g.sat_hi;
@@ -782,19 +785,21 @@ int make_args(BwdArgs& a, const fdb_attn_bwd_params& b, const ExpandGeometry& g,
   return FDB_OK;
 }
 
+// One side for all heads, from the arguments of the first group of them.
 template <bool DKV>
-int launch_bwd(BwdArgs a, const fdb_attn_bwd_params& b, char* partial, int64_t slots, cudaStream_t stream) {
+int launch_bwd(BwdArgs a, const fdb_attn_bwd_params& b, const ExpandGeometry& g, const Layout& l, char* ws, int64_t slots, cudaStream_t stream) {
   const fdb_attn_params& p = *b.fwd;
   static std::atomic<uint64_t> smem_done{0};
   auto kernel = bwd_kernel<DKV>;
   cudaError_t e = allow_smem(smem_done, reinterpret_cast<const void*>(kernel), (int)kSmemBytes);
-  const int group = a.xrow != nullptr ? a.sum_heads : p.heads;  // (without a row term there are no sums)
-  for (a.head0 = 0; a.head0 < p.heads; a.head0 += group) {
-    const int heads = std::min(group, p.heads - a.head0);
+  int rc = FDB_OK;
+  for (int head0 = 0, heads; head0 < p.heads; head0 += heads) {
+    heads = std::min(a.sum_heads, p.heads - head0);
+    if (head0 > 0 && (rc = make_args<DKV>(a, b, g, l, ws, head0, heads)) != FDB_OK) return rc;
     if (e == cudaSuccess && slots > 0) e = launch_kernel<BwdArgs>(kernel, a, dim3((unsigned)slots, heads), kThreads, kSmemBytes, false, stream);
     if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd launch: %s", cudaGetErrorString(e));
     if (a.xrow == nullptr) continue;
-    auto at = [&](const void* base, int64_t head_stride) { return static_cast<const __nv_bfloat16*>(base) + a.head0 * head_stride; };
+    auto at = [&](const void* base, int64_t head_stride) { return static_cast<const __nv_bfloat16*>(base) + head0 * head_stride; };
     BwdTablesCall c;
     c.sums = a.sums;
     const TableStrides strides = table_strides(b);
@@ -803,16 +808,15 @@ int launch_bwd(BwdArgs a, const fdb_attn_bwd_params& b, char* partial, int64_t s
     c.operand_row_stride = DKV ? p.k_row_stride : p.q_row_stride;
     c.operand_head_stride = DKV ? p.k_head_stride : p.q_head_stride;
     c.operand = at(DKV ? p.k : p.q, c.operand_head_stride);
-    c.core = a.core + (int64_t)a.head0 * kHeadDim;
+    c.core = a.core;
     c.core_row_stride = (int64_t)p.heads * kHeadDim;
-    c.out = const_cast<__nv_bfloat16*>(at(a.grad, a.grad_hs));
+    c.out = a.grad;
     c.out_row_stride = a.grad_rs; c.out_head_stride = a.grad_hs;
     c.dtable = const_cast<__nv_bfloat16*>(at(DKV ? b.dpos_query : b.dpos_key, strides.head));
-    c.partial = reinterpret_cast<float*>(partial);
+    c.partial = reinterpret_cast<float*>(ws + l.partial);
     c.rows = p.total_rows; c.heads = heads; c.table_rows = a.table_rows;
     c.status = p.status;
-    const int rc = launch_bwd_tables(c, stream);
-    if (rc != FDB_OK) return rc;
+    if ((rc = launch_bwd_tables(c, stream)) != FDB_OK) return rc;
   }
   return FDB_OK;
 }
@@ -881,7 +885,8 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
   buf.slot_info = reinterpret_cast<int32_t*>(ws + l.slot_info);
   if (slots > 0 && (rc = launch_seq_info(p, buf, stream)) != FDB_OK) return rc;
   BwdArgs dq, dkv;
-  if ((rc = make_args<false>(dq, *b, g, l, ws)) != FDB_OK || (rc = make_args<true>(dkv, *b, g, l, ws)) != FDB_OK) return rc;
+  const int first = sum_heads_of(p);  // (the heads of a group; all of them but in the largest calls)
+  if ((rc = make_args<false>(dq, *b, g, l, ws, 0, first)) != FDB_OK || (rc = make_args<true>(dkv, *b, g, l, ws, 0, first)) != FDB_OK) return rc;
   if (p.pos_key != nullptr || p.pos_query != nullptr) {
     const int64_t n = (int64_t)p.heads * g.rows * 8;
     const TableStrides strides = table_strides(*b);
@@ -896,6 +901,6 @@ extern "C" FDB_API int fdb_attn_bwd(const fdb_attn_bwd_params* b, void* stream) 
       p.out_row_stride, p.out_head_stride, cells, p.heads, reinterpret_cast<float*>(ws + l.delta), p.cu_seqlens, p.batch, dq, dkv);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(FDB_ERR_CUDA, "attn_bwd set-up: %s", cudaGetErrorString(e));
-  if ((rc = launch_bwd<false>(dq, *b, ws + l.partial, slots, s)) != FDB_OK) return rc;
-  return launch_bwd<true>(dkv, *b, ws + l.partial, slots, s);
+  if ((rc = launch_bwd<false>(dq, *b, g, l, ws, slots, s)) != FDB_OK) return rc;
+  return launch_bwd<true>(dkv, *b, g, l, ws, slots, s);
 }
