@@ -10,7 +10,7 @@ import os
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG_DIR, "libfdb_b200.so")
 
-FDB_OK = 0
+FDB_OK, FDB_ERR_ALIGNMENT = 0, -3
 FDB_BF16, FDB_FP32, FDB_E4M3 = 0, 1, 2
 FDB_DEV_TIMEOUT, FDB_DEV_BAD_SEQLEN, FDB_DEV_BAD_INDEX, FDB_DEV_BAD_MASK = 1, 2, 4, 8
 STATIC_SCRATCH_BYTES = 8 << 20

@@ -224,13 +224,13 @@ def launch(b: BwdParams, dev: torch.device) -> None:
     ws = torch.empty(need + 256, dtype=torch.uint8, device=dev)
     b.workspace, b.workspace_bytes = (ws.data_ptr() + 255) & ~255, need
     _lib.check(lib.fdb_attn_bwd(C.byref(b), C.c_void_p(ops.raw_stream(dev))))
-    p = b.fwd.contents
-    sides, groups = [b.dpos_key, b.dpos_query], 1
-    if any(sides):  # heads in groups of at most 2 GiB of bucket sums (csrc/attn_bwd_sm100.cu)
+    terms = int(b.dpos_key is not None) + int(b.dpos_query is not None)
+    _launches += 4 + int(terms > 0) + 2 * terms
+    if terms and need >= 1 << 31:  # heads in groups of at most 2 GiB of bucket sums (csrc/attn_bwd_sm100.cu)
+        p = b.fwd.contents
         span = p.position_buckets if p.position_buckets > 0 else p.max_relative_positions
         most = max(1, min(p.heads, (1 << 31) // max(1, p.total_rows * 2 * span * 2)))
-        groups = -(-p.heads // -(-p.heads // -(-p.heads // most)))
-    _launches += 2 + int(any(sides)) + sum(3 * groups if side else 1 for side in sides)
+        _launches += 3 * terms * (-(-p.heads // -(-p.heads // -(-p.heads // most))) - 1)
 
 
 def _aligned(t: Optional[torch.Tensor]) -> Optional[torch.Tensor]:
@@ -245,8 +245,7 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
            max_relative_positions):
     dev, shape = q.device, q.shape
     with ops.on_device(dev):
-        dout, q, k, v, pos_key, pos_query, out = (_aligned(t) for t in (dout, q, k, v, pos_key, pos_query, out.contiguous()))
-        lse = lse.contiguous()
+        out, lse = out.contiguous(), lse.contiguous()
         p, keep = ops._fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
                                    max_relative_positions, out, lse)
         d3, d_rs, d_hs, T = ops._rows_view(dout)
@@ -260,7 +259,13 @@ def _fused(dout, q, k, v, pos_key, pos_query, out, lse, cu_seqlens, seq_lens, ma
         b.dq, b.dk, b.dv = (g.data_ptr() for g in grads)
         b.grad_row_stride, b.grad_head_stride = H * 64, 64
         b.dpos_key, b.dpos_query = _ptr(d_key), _ptr(d_query)
-        launch(b, dev)
+        try:
+            launch(b, dev)
+        except _lib.FdbError as e:  # (before anything was launched)
+            copies = [_aligned(t) for t in (dout, q, k, v, pos_key, pos_query, out)]
+            if e.code != _lib.FDB_ERR_ALIGNMENT or all(a is b for a, b in zip(copies, (dout, q, k, v, pos_key, pos_query, out))):
+                raise
+            return _fused(*copies, lse, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets, max_relative_positions)
         del keep
     return (*(g.view(t.shape) for g, t in zip(grads, (q, k, v))), d_key, d_query)
 

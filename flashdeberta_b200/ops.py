@@ -96,12 +96,10 @@ def raw_stream(device: torch.device) -> int:
     return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
 
 
-_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
-
-
 def global_module_hooks() -> bool:
     """Whether hooks on every module are registered (profilers, module trackers): modules have to be called one by one then."""
-    return any(getattr(_nn_module, h, None) for h in _GLOBAL_HOOKS)
+    m = _nn_module
+    return bool(m._global_forward_hooks or m._global_forward_pre_hooks or m._global_backward_hooks or m._global_backward_pre_hooks)
 
 
 def intercepted(*tensors) -> bool:
@@ -111,8 +109,13 @@ def intercepted(*tensors) -> bool:
     if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0 or torch._C._get_tracing_state() is not None
             or torch._C._functorch.peek_interpreter_stack() is not None):
         return True
-    return any(type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter or torch._C._functorch.is_legacy_batchedtensor(t)
-               for t in tensors if t is not None)
+    for t in tensors:
+        if t is not None and (type(t) not in _PLAIN or _is_batched(t)):
+            return True
+    return False
+
+
+_PLAIN, _is_batched = (torch.Tensor, torch.nn.Parameter), torch._C._functorch.is_legacy_batchedtensor
 
 
 def capturing(t: torch.Tensor) -> bool:
@@ -180,7 +183,7 @@ def _rows_view(x: torch.Tensor) -> Tuple[torch.Tensor, int, int, int]:
 
 def _int32(t: torch.Tensor, device: torch.device) -> torch.Tensor:
     """Lengths or offsets as the kernels read them."""
-    return t if t.dtype == torch.int32 and t.device == device and t.is_contiguous() else t.to(device=device, dtype=torch.int32).contiguous()
+    return t if t.dtype == torch.int32 and t.is_cuda and t.is_contiguous() else t.to(device=device, dtype=torch.int32).contiguous()
 
 
 def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, sm_scale, position_buckets,
@@ -190,8 +193,8 @@ def _fill_params(q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, max_seqlen, 
     v3, v_rs, v_hs, v_rows = _rows_view(v)
     shape = q.shape
     H, D = shape[-2], shape[-1]
-    # as rows: (1, T, H, D) beside (T, H, D) is the same tensor
-    if k_rows != rows or v_rows != rows or k.shape[-2:] != shape[-2:] or v.shape[-2:] != shape[-2:]:
+    if (k.shape != shape or v.shape != shape) and (  # as rows: (1, T, H, D) beside (T, H, D) is the same tensor
+            k_rows != rows or v_rows != rows or k.shape[-2:] != shape[-2:] or v.shape[-2:] != shape[-2:]):
         raise ValueError("q, k and v must have the same shape")
     keep = [q3, k3, v3]
     tables = [None, None]

@@ -17,10 +17,9 @@ from torch import nn
 
 from . import _lib, backward, bucket, ops
 
-def _plain_linear(m, device, n: int, k: int) -> bool:
-    w, b = m.weight, m.bias
-    return (b is not None and w.shape == (n, k) and b.shape == (n,) and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and w.device == device and b.device == device
-            and w.is_contiguous() and w.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0 and k % 64 == 0
+def _plain_linear(m, w, b, device, n: int, k: int) -> bool:
+    return (b is not None and w.shape == (n, k) and b.shape == (n,) and w.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
+            and w.device == device and b.device == device and w.is_contiguous() and (w.data_ptr() | b.data_ptr()) % 16 == 0
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and "forward" not in m.__dict__)
 
 
@@ -40,7 +39,10 @@ def covers(module, x, query_states, mask, rel) -> bool:
     if x.dim() != 3 or rel.shape[1] != x.shape[2]:  # (from here on only addresses are handed on: every size is looked at)
         return False
     linears = (module.query_proj, module.key_proj, module.value_proj)
-    if any(type(m) is not nn.Linear for m in linears) or ops.intercepted(x, rel, mask, *(t for m in linears for t in (m.weight, m.bias))):
+    if not (type(linears[0]) is type(linears[1]) is type(linears[2]) is nn.Linear):
+        return False
+    weights = [(m, m.weight, m.bias) for m in linears]
+    if ops.intercepted(x, rel, mask, *[t for _, w, b in weights for t in (w, b)]):
         return False
     if (x.data_ptr() | rel.data_ptr()) % 16:
         return False
@@ -51,11 +53,12 @@ def covers(module, x, query_states, mask, rel) -> bool:
     drop = module.pos_dropout
     if (drop.training and drop.p > 0) or drop._forward_hooks or drop._forward_pre_hooks:
         return False
-    if not all(_plain_linear(m, x.device, module.num_attention_heads * 64, x.shape[2]) for m in linears):
+    n, k, device = module.num_attention_heads * 64, x.shape[2], x.device
+    if k % 64 or not all([_plain_linear(m, w, b, device, n, k) for m, w, b in weights]):
         return False
     if rel.shape[0] < 2 * module.pos_ebd_size or not backward.index_covered(module.position_buckets, module.max_relative_positions):
         return False
-    return ops.wants_grad(x, rel, *(t for m in linears for t in (m.weight, m.bias)))
+    return ops.wants_grad(x, rel, *[t for _, w, b in weights for t in (w, b)])
 
 
 class _ProjectedParams(C.Structure):
@@ -114,7 +117,9 @@ class _Projected(torch.autograd.Function):
         if operators:
             d_qkv, d_tables = _backward_by_operators(grad, qkv, tables, out, lse, lens, *ctx.fdb_args)
         else:
-            grad = backward._aligned(grad.contiguous())
+            grad = grad.contiguous()
+            if grad.data_ptr() % 16:
+                grad = grad.clone()
             d_qkv, d_tables = torch.empty_like(qkv), torch.empty_like(tables)
             p = _params(qkv, tables, out, lse, lens, B, L, heads, buckets, max_rel)
             d, t = d_qkv.data_ptr(), d_tables.data_ptr()
