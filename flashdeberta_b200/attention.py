@@ -183,8 +183,9 @@ class FlashDisentangledSelfAttention(DisentangledSelfAttention):
         B, L, _ = hidden_states.shape
         H, D = self.num_attention_heads, self.attention_head_size
         in_dtype = hidden_states.dtype
-        if projected.covers(self, hidden_states, query_states, attention_mask, rel_embeddings):
-            return (projected.attention(self, hidden_states, lengths_from_mask(attention_mask), rel_embeddings), None)
+        weights = projected.covers(self, hidden_states, query_states, attention_mask, rel_embeddings)
+        if weights:
+            return (projected.attention(self, hidden_states, lengths_from_mask(attention_mask), rel_embeddings, weights), None)
 
         q = self.query_proj(query_states).view(B, L, H, D)
         k = self.key_proj(hidden_states).view(B, L, H, D)

@@ -104,18 +104,21 @@ def global_module_hooks() -> bool:
 
 def intercepted(*tensors) -> bool:
     """Whether somebody wants to see the operators, or these tensors have no memory to point at: tracing, a dispatch mode (fake tensors,
-    flop counters, ``make_fx``), a functorch transform (vmap, grad), a batched gradient, a tensor subclass.  Calls then go through the
-    custom operators, which dispatch; a raw address would bypass all of that."""
+    flop counters, ``make_fx``), a functorch transform (vmap, grad), a tensor subclass.  Calls then go through the
+    custom operators, which dispatch; a raw address would bypass all of that.  (A gradient batched by ``is_grads_batched`` looks like a
+    plain tensor: the backwards ask ``batched`` as well.)"""
     if (torch.compiler.is_compiling() or torch._C._len_torch_dispatch_stack() > 0 or torch._C._get_tracing_state() is not None
             or torch._C._functorch.peek_interpreter_stack() is not None):
         return True
     for t in tensors:
-        if t is not None and (type(t) not in _PLAIN or _is_batched(t)):
+        if type(t) not in _PLAIN:
             return True
     return False
 
 
-_PLAIN, _is_batched = (torch.Tensor, torch.nn.Parameter), torch._C._functorch.is_legacy_batchedtensor
+_PLAIN = frozenset((torch.Tensor, torch.nn.Parameter, type(None)))
+#: whether a tensor is a gradient of ``torch.autograd.grad(..., is_grads_batched=True)``
+batched = torch._C._functorch.is_legacy_batchedtensor
 
 
 def capturing(t: torch.Tensor) -> bool:
@@ -724,7 +727,7 @@ class _Train(torch.autograd.Function):
     @staticmethod
     @torch.autograd.function.once_differentiable
     def backward(ctx, grad, grad_lse):
-        if intercepted(grad):
+        if intercepted(grad) or batched(grad):
             return _train_backward(ctx, grad, grad_lse)
         from . import backward
         q, k, v, pos_key, pos_query, cu_seqlens, seq_lens, out, lse = ctx.saved_tensors

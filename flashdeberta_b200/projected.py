@@ -23,10 +23,10 @@ def _plain_linear(m, w, b, device, n: int, k: int) -> bool:
             and not (m._forward_hooks or m._forward_pre_hooks or m._backward_hooks or m._backward_pre_hooks) and "forward" not in m.__dict__)
 
 
-def covers(module, x, query_states, mask, rel) -> bool:
-    """Whether a call is one that ``attention`` stands for: autograd recording, bf16 on the GPU, both position terms through the
+def covers(module, x, query_states, mask, rel):
+    """The projections' weights and biases, [wq, bq, wk, bk, wv, bv], when a call is one that ``attention`` stands for: autograd recording, bf16 on the GPU, both position terms through the
     key and query projections themselves, self-attention over a dense batch, nothing between the operators (dropout, hooks,
-    autocast, tracing)."""
+    autocast, tracing); else False."""
     if torch.is_autocast_enabled("cuda") or ops.global_module_hooks():
         return False
     if not (torch.is_grad_enabled() and x.is_cuda and x.dtype == torch.bfloat16 and module.share_att_key
@@ -41,8 +41,8 @@ def covers(module, x, query_states, mask, rel) -> bool:
     linears = (module.query_proj, module.key_proj, module.value_proj)
     if not (type(linears[0]) is type(linears[1]) is type(linears[2]) is nn.Linear):
         return False
-    weights = [(m, m.weight, m.bias) for m in linears]
-    if ops.intercepted(x, rel, mask, *[t for _, w, b in weights for t in (w, b)]):
+    weights = [linears[0].weight, linears[0].bias, linears[1].weight, linears[1].bias, linears[2].weight, linears[2].bias]
+    if ops.intercepted(x, rel, mask, *weights):
         return False
     if (x.data_ptr() | rel.data_ptr()) % 16:
         return False
@@ -54,11 +54,11 @@ def covers(module, x, query_states, mask, rel) -> bool:
     if (drop.training and drop.p > 0) or drop._forward_hooks or drop._forward_pre_hooks:
         return False
     n, k, device = module.num_attention_heads * 64, x.shape[2], x.device
-    if k % 64 or not all([_plain_linear(m, w, b, device, n, k) for m, w, b in weights]):
+    if k % 64 or not all([_plain_linear(linears[i], weights[2 * i], weights[2 * i + 1], device, n, k) for i in range(3)]):
         return False
     if rel.shape[0] < 2 * module.pos_ebd_size or not backward.index_covered(module.position_buckets, module.max_relative_positions):
         return False
-    return ops.wants_grad(x, rel, *[t for _, w, b in weights for t in (w, b)])
+    return weights if ops.wants_grad(x, rel, *weights) else False
 
 
 class _ProjectedParams(C.Structure):
@@ -113,7 +113,7 @@ class _Projected(torch.autograd.Function):
         x2, rel, wq, wk, wv, qkv, tables, out, lse, lens = ctx.saved_tensors
         B, L, heads, buckets, max_rel = ctx.fdb_args
         inner, span2, dev = heads * 64, tables.shape[0], qkv.device
-        operators = ops.intercepted(grad)
+        operators = ops.intercepted(grad) or ops.batched(grad)
         if operators:
             d_qkv, d_tables = _backward_by_operators(grad, qkv, tables, out, lse, lens, *ctx.fdb_args)
         else:
@@ -167,9 +167,9 @@ def _backward_by_operators(grad, qkv, tables, out, lse, lens, B, L, heads, bucke
             torch.stack((dpq, dpk), 0).permute(2, 0, 1, 3).reshape(span2, 2 * inner))
 
 
-def attention(module, x: torch.Tensor, lens, rel: torch.Tensor) -> torch.Tensor:
-    """Context (B, L, hidden) of ``FlashDisentangledSelfAttention`` where ``covers`` holds."""
+def attention(module, x: torch.Tensor, lens, rel: torch.Tensor, weights) -> torch.Tensor:
+    """Context (B, L, hidden) of ``FlashDisentangledSelfAttention`` where ``covers`` gave these weights."""
     lens = None if lens is None else lens.contiguous()
-    q, k, v = module.query_proj, module.key_proj, module.value_proj
-    return _Projected.apply(x, rel, q.weight, k.weight, v.weight, q.bias, k.bias, v.bias, lens, module.num_attention_heads,
-                            module.position_buckets, module.max_relative_positions)
+    wq, bq, wk, bk, wv, bv = weights
+    return _Projected.apply(x, rel, wq, wk, wv, bq, bk, bv, lens, module.num_attention_heads, module.position_buckets,
+                            module.max_relative_positions)
