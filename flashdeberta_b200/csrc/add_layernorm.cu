@@ -54,14 +54,10 @@ __global__ void __launch_bounds__(32 * kRowsPerBlock) add_layernorm_kernel(const
   constexpr int kVecPerRow = VEC * 32;
   const int64_t rows = c.rows_dev != nullptr ? (int64_t)*c.rows_dev : c.rows;
   if (row >= rows) {
-    if (row < c.rows && row < rows + kTileN) {
+    if (c.zero_tail != nullptr && row < c.rows && row < rows + kTileN) {
+      uint4* z = static_cast<uint4*>(c.zero_tail) + row * kVecPerRow;
 #pragma unroll
-      for (int t = 0; t < 2; ++t) {
-        if (c.zero_tail[t] == nullptr) continue;
-        uint4* z = static_cast<uint4*>(c.zero_tail[t]) + row * kVecPerRow;
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) z[i * 32 + lane] = make_uint4(0, 0, 0, 0);
-      }
+      for (int i = 0; i < VEC; ++i) z[i * 32 + lane] = make_uint4(0, 0, 0, 0);
     }
     return;
   }

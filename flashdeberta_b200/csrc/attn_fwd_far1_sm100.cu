@@ -229,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
       rc_hi = dot_q_row(q_row, r, xk_h + (int64_t)(args.xrows - 1) * kHeadDim);
     }
 
-    float m_used = 0.f, l_run = 0.f;
+    float m_used = my_row < len ? -INFINITY : INFINITY, l_run = 0.f;  // (rows behind the sequence never ask for a rescale)
 #pragma unroll 1
     for (int i = 0; i < n_far; ++i) {
       const uint32_t u = uint32_t(i);
@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
       const float t_max = (max3(mx[0], mx[1], fmaxf(mx[2], mx[3])) + row_const) * args.scale_log2;
       if (lane == 0 && quad == 0) FDB_STAMP(0, i, 2);
       if (u == 0) {
-        m_used = t_max;
+        m_used = fmaxf(m_used, t_max);
       } else {
         const bool need = t_max > m_used + 8.f;
         if (__any_sync(0xffffffffu, need)) {

@@ -462,7 +462,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     }
 
     uint32_t band_idx = 0;
-    float m_used = 0.f, l_run = 0.f;
+    // Rows behind the sequence (padding, the next sequence, unused memory) never ask for a rescale, which the rows of their warp take
+    // part in: a sequence's rounding is its own.
+    float m_used = my_row < len ? -INFINITY : INFINITY, l_run = 0.f;
     if (resume && ok) {
       // continue from what the far kernel accumulated over the plain and saturated tiles of this row: O goes back into
       // tensor memory (this group's 32 columns), the reference maximum and the row sum into registers
@@ -478,7 +480,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       tmem_st32(tmem_lane + kColO + 32 * g, o);
       tmem_wait_st();
       const float2 ml = __ldg(reinterpret_cast<const float2*>(args.part_ml + rh * 2));
-      m_used = ml.x;
+      if (my_row < len) m_used = ml.x;
       l_run = g == 0 ? ml.y : 0.f;
     }
 
@@ -599,7 +601,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 
       const float t_max = (mx + row_const) * c_eff;
       if (jj == 0 && !resume) {
-        m_used = t_max;
+        m_used = fmaxf(m_used, t_max);
       } else {
         // The previous P.V has finished: O may be rescaled and the P columns overwritten.  Observed on every tile (it is
         // long done by now) so that this thread never falls two phases behind the barrier, which a parity wait could

@@ -358,12 +358,8 @@ extern "C" FDB_API int fdb_encoder_forward(fdb_encoder_call* c, void* stream) {
   ln.rows = rows; ln.rows_dev = rows_dev; ln.hidden = plan.hidden; ln.eps = c->emb_eps;
   ln.ids = c->ids; ln.table_rows = c->emb_rows; ln.token_index = index;
   ln.mask = c->mask; ln.mask_type = c->mask_type; ln.status = c->status; ln.chained = true;
-  // The last tiles of the last sequence read behind the valid rows: values, which have to be finite, and queries, which take part in
-  // their warp's decision when to rescale and so in the rounding of the rows beside them.  Zeros, as behind the end of a tensor.
-  if (rows_dev != nullptr) {
-    ln.zero_tail[0] = ws + l.qkv;
-    ln.zero_tail[1] = ws + l.qkv + 2 * (uint64_t)rows * plan.hidden * 2;
-  }
+  // the last key tile of the last sequence reads values behind the valid rows, which have to be finite
+  if (rows_dev != nullptr) ln.zero_tail = ws + l.qkv + 2 * (uint64_t)rows * plan.hidden * 2;
   if ((rc = launch_layernorm(ln, stream)) != FDB_OK) return rc;
   ++launches;
 

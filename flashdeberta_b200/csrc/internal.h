@@ -92,7 +92,7 @@ struct LayerNormCall {
   const void* mask;
   int mask_type;
   const int32_t* out_index;    // row -> row of `out`; NULL: the row itself
-  void* zero_tail[2];          // rows of these (rows, hidden) buffers behind the actual number are zeroed, one tile of them
+  void* zero_tail;             // rows of this (rows, hidden) buffer behind the actual number are zeroed, one key tile of them
   int32_t* status;
   bool chained;                // launch with programmatic stream serialisation
 };

@@ -1001,3 +1001,33 @@ def test_one_packed_row_with_or_without_its_batch_dimension(q_dims, kv_dims):
     for a, b in zip(run(q_dims, kv_dims), run(3, 3)):
         assert torch.equal(a, b)
     ops.check_status()
+
+
+@pytest.mark.parametrize("L,tune", [(700, 0), (700, 2), (4000, 0)])
+@pytest.mark.parametrize("terms", [True, False])
+def test_bits_of_a_sequence_do_not_depend_on_what_lies_behind_it(L, tune, terms):
+    """A query tile's last rows may be another sequence's, or padding.  With scores that spread widely (the running maxima move, some by
+    less than what makes a row rescale by itself) the rows of the sequence keep their bits, whatever those rows hold."""
+    from flashdeberta_b200 import ops
+    g = torch.Generator().manual_seed(12)
+    make = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+    n, H = L - 60, 4
+    q, k, v = 6 * make(L, H, 64), make(L, H, 64), make(L, H, 64)
+    k[:n] *= torch.linspace(0.2, 1.5, n, device=DEV).bfloat16()[:, None, None]  # later keys score higher
+    pk, pq = (make(H, 512, 64), make(H, 512, 64)) if terms else (None, None)
+    kw = dict(position_buckets=256, max_relative_positions=512, sm_scale=1 / (64 * 3) ** 0.5, tune=tune, return_lse=True)
+    lens = torch.tensor([n], dtype=torch.int32, device=DEV)
+    outs = []
+    for behind in (0.0, 1.0, 30.0, -30.0, float("inf")):
+        x = q.clone()
+        x[n:] = x[n:] * behind if behind else 0.0
+        out, lse = ops.disentangled_attention(x[None], k[None], v[None], pk, pq, seq_lens=lens, max_seqlen=L, **kw)
+        outs.append((out[0, :n], lse[:n]))
+        assert torch.count_nonzero(out[0, n:]) == 0 and torch.count_nonzero(lse[n:]) == 0
+        cu = torch.tensor([0, n, L], dtype=torch.int32, device=DEV)
+        if behind != float("inf"):
+            out, lse = ops.disentangled_attention(x, k, v, pk, pq, cu_seqlens=cu, max_seqlen=L, **kw)
+            outs.append((out[:n], lse[:n]))
+    for out, lse in outs[1:]:
+        assert torch.equal(out, outs[0][0]) and torch.equal(lse, outs[0][1])
+    ops.check_status()
