@@ -8,8 +8,8 @@
 // first loads and its output — runs beside the other one's exponentials.  One softmax thread per query row holds all 128
 // keys of a tile, so there is no exchange between threads.
 //
-//   warps 0-3  softmax, thread r = row r          warp 4  lane 0: score MMAs  S = Q.K^T (+ R.K^T), allocates tensor memory
-//   warp 5     lane 0: TMA (Q once, K/V 2 stages)  warp 6  lane 0: O += P.V
+//   warps 0-3  softmax, thread r = row r     warp 4  score MMAs  S = Q.K^T (+ R.K^T), allocates tensor memory
+//   warp 5     TMA (Q once, K/V 2 stages)    warp 6  O += P.V     (4-6 issue through an elected lane)
 //
 // When the call has position terms the band tiles are left to attn_fwd_kernel (band_only mode), which runs next on the same
 // stream: this kernel then stores, per (row, head), the unnormalised accumulator, reference maximum and row sum instead

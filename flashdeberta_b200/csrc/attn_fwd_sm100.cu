@@ -8,9 +8,10 @@
 // producer and drain groups to the softmax groups with setmaxnreg):
 //   warps 0-3   softmax group 0: thread r owns row r of the tile, keys   0..63  of every 128-key tile
 //   warps 4-7   softmax group 1: thread r owns row r of the tile, keys  64..127
-//   warp  8     lane 0 issues the score-side tcgen05.mma: S = Q.K^T and the position products (the warp allocates TMEM)
-//   warp  9     lane 0 issues every TMA load: Q once, K/V double-buffered, position-table windows
-//   warp  10    lane 0 issues O += P.V
+//   warp  8     score-side tcgen05.mma: S = Q.K^T and the position products (the warp allocates TMEM)
+//   warp  9     every TMA load: Q once, K/V double-buffered, position-table windows
+//   warp  10    O += P.V
+//               (8-10 stay converged and issue through an elected lane: see elect_one)
 //   warps 12-15 drain group: moves the c2p product of a band tile from tensor memory to shared memory (bf16)
 // Tensor memory (512 columns): O 64 | P 64 | S 128 | R 256 (position products of a band tile).
 //

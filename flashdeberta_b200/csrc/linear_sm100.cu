@@ -8,9 +8,9 @@
 //
 // Persistent grid; a tile is 128 rows (CG = 1) or 256 rows (CG = 2, a pair of CTAs on two SMs) x BN output features, K in
 // steps of 64 through a ring of stages:
-//   warp 0  lane 0: TMA, the CTA's 128 x 64 tile of x and its BN / CG rows of W
-//   warp 1  lane 0 (of the pair's even CTA): tcgen05.mma, four per stage; two accumulators in tensor memory, so the epilogue
-//           of one tile runs beside the main loop of the next
+//   warp 0  TMA, the CTA's 128 x 64 tile of x and its BN / CG rows of W
+//   warp 1  (of the pair's even CTA) tcgen05.mma, four per stage; two accumulators in tensor memory, so the epilogue
+//           of one tile runs beside the main loop of the next (both warps stay converged and issue through an elected lane)
 //   warps 2-9: epilogue, two warps per 32-lane quarter of tensor memory: + bias, rounded to bf16 as the separate GEMM would
 //           leave it, GELU in fp32, bf16 out with 32-byte stores
 // What bounds a tile is shared memory, not the tensor pipe: a stage is written once by TMA and read once by the MMAs, at
