@@ -29,10 +29,18 @@
 //     128x64 and two 128x32 MMAs groups), arranged so that the value thread (quadrant w, lane l) needs for key 32b+c sits in
 //     its own quadrant at lane (l+31-c)&31 of product t = (l > c): one select on the source side and one warp shuffle per
 //     score element, fp32, no shared memory;
-//     c2p needs a transpose: X_k[window].Q^T (256x128) is computed into R ahead of the p2c product, the drain group writes it
-//     to shared memory as bf16 [position][query] while the softmax of the previous tile is still running, and thread m
-//     reads c2p[m][m+127-i] at compile-time offsets from a per-thread base.
+//     c2p needs a shift by the row: Q.X_k[window]^T goes through tensor memory to the drain group while the softmax of the previous
+//     tile is still running; the group writes row m of it to shared memory as bf16, rotated by m, and thread m reads its 64 values
+//     as one aligned run.
 // No (rows x 2*span) bias tensor is ever written to global memory.
+//
+// What a band tile costs, 8 x 2048 x 12 heads, clocks of 4500: the two products of p2c pulled and shuffled 1200, c2p added and the
+// maximum 810, its exchange and the decision 350, 64 exponentials per thread 1300, hops between the roles the rest; beside it the
+// products of the next tile (20 narrow p2c MMAs 900, drain 1250).  Neither side hides the other wholly: of this kernel with one part
+// left out, the exponentials were worth 10 % of a call, selects and shuffles 7 %, c2p 3 %, the drain's stores 2 to 3 %, the p2c MMAs
+// and the windows' loads nothing.  Hence shuffle sources in registers, c2p added by the mixed-precision add (no unpacking), stores of
+// the drain at fixed distances from two bases, a stage pitch without bank conflicts, and waits that are over by then in front
+// of the ones that are not: 364 -> 353 us a call at this shape, 168 -> 164 at 32 x 512, packed 48 x <= 4099 x 16 heads 1431 -> 1393.
 //
 // Every mbarrier wait is bounded and gives up early once another role has raised the abort flag; the CTA then sets
 // FDB_DEV_TIMEOUT in the status word, waits a millisecond for copies in flight, releases its TMEM and returns.
@@ -74,15 +82,17 @@ constexpr uint32_t kSmemWinQ = 114688;              // 256 x 128 B window of exp
 // c2p stage: bf16 [128 query rows][256 window positions], rows padded by 16 B.  Row m is rotated by m: position p of the
 // window sits in column (p - m) & 255, so the 64 values a softmax thread needs are one aligned 128-byte run whose place does
 // not depend on m.
-constexpr uint32_t kStageCPitch = 528;
+// A pitch of 140 words: neither the drain group's 4-byte stores (a word less per two rows) nor the 16-byte loads of eight rows
+// meet in a bank.
+constexpr uint32_t kStageCPitch = 560;
 constexpr uint32_t kSmemStageC = 147456;
-constexpr uint32_t kSmemSat = kSmemStageC + 69632;  // 217088: 2 x (8 x 128 B) saturated pos_query rows (hi, lo)
-static_assert(128 * kStageCPitch <= 69632, "c2p stage");
+constexpr uint32_t kSmemSat = kSmemStageC + 71680;  // 2 x (8 x 128 B) saturated pos_query rows (hi, lo)
+static_assert(128 * kStageCPitch <= 71680, "c2p stage");
 constexpr uint32_t kSmemXchg = kSmemSat + 2048;     // float [2 parities][2 groups][128 rows] row maxima
 constexpr uint32_t kSmemLsum = kSmemXchg + 2048;    // float [2 groups][128 rows] row sums at the end
 constexpr uint32_t kSmemBars = kSmemLsum + 1024;
 constexpr uint32_t kSmemBytes = kSmemBars + 256 + 1024;  // + alignment slack
-static_assert(kSmemSat == 217088, "shared memory map");
+static_assert(kSmemSat % 1024 == 0, "shared memory map");
 static_assert(kSmemBytes <= 232448, "exceeds 227 KB");
 
 // mbarriers.  "count" = arrivals per phase.
@@ -203,8 +213,8 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     for (int jj = 0; jj < n_proc; ++jj) {
       const int j = j_first + jj;
       if (tile_kind(j) != kBand) continue;
-      wait(bar(kBarC2p), band_idx & 1u);                               // the product is in R
       if (band_idx > 0) wait(bar(kBarGather), (band_idx - 1u) & 1u);   // nobody reads the previous stage any more
+      wait(bar(kBarC2p), band_idx & 1u);                               // the product is there
       tc_fence_after();
       if (has_c2p && ok) {
         // The product has query rows in the lanes and window positions in the columns, so this thread holds row r.  The
@@ -222,6 +232,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           // an odd start puts value 2k-1 and 2k into one 32-bit word: funnel shift over consecutive pairs by 16 bits;
           // an even start keeps the pairs (shift "32" = take the upper word)
           const uint32_t sh = (start & 1u) ? 16u : 32u;
+          const int w0 = int((start & 255u) >> 1);  // word of the block's first value; the row wraps behind word 127
           uint32_t prev = 0;
           uint32_t t[32];
           tmem_ld32(col, t);
@@ -232,17 +243,17 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 #pragma unroll
             for (int i = 0; i < 16; ++i) pk[i] = pack_bf16x2(__uint_as_float(t[2 * i]), __uint_as_float(t[2 * i + 1]));
             if (c4 < 3) tmem_ld32(col + (c4 + 1) * 32, t);  // the next 32 columns are in flight while these are stored
-#pragma unroll
-            for (int k = 0; k < 16; ++k) {
-              const uint32_t word = ((start + uint32_t(32 * c4 + 2 * k)) >> 1) & 127u;
-              const uint32_t v = __funnelshift_rc(k == 0 ? prev : pk[k - 1], pk[k], sh);
-              if (c4 == 0 && k == 0 && (start & 1u)) {
-                // the low half of this word belongs to the other block's last position: write the upper half only
-                sts_u16(row_addr + 4u * word + 2u, pk[0] & 0xffffu);
-              } else {
-                sts_u32(row_addr + 4u * word, v);
-              }
+            // 16 words at a fixed distance from one of two bases: in front of the wrap and behind it
+            const int front = 128 - (w0 + 16 * c4);
+            const uint32_t to = row_addr + 4u * uint32_t(w0 + 16 * c4), to_wrapped = to - 512u;
+            if (c4 == 0 && (start & 1u)) {
+              // the low half of the first word belongs to the other block's last position: write the upper half only
+              sts_u16(to + 2u, pk[0] & 0xffffu);
+            } else {
+              sts_u32(front > 0 ? to : to_wrapped, __funnelshift_rc(prev, pk[0], sh));
             }
+#pragma unroll
+            for (int k = 1; k < 16; ++k) sts_u32((k < front ? to : to_wrapped) + 4u * uint32_t(k), __funnelshift_rc(pk[k - 1], pk[k], sh));
             prev = pk[15];
             if (c4 < 3) tmem_wait_ld();
           }
@@ -287,8 +298,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           if (!ok) break;
           const int u0 = m0 - j * kTileN - (kTileN - 1) - args.d_first;
           if (elect_one()) {
-            mbar_expect_tx(bar(kBarWin), (has_c2p ? G::kWin : 0u) + (has_p2c ? G::kWin : 0u));
+            // (of pos_key the first tile of the run takes the whole window, the others its 128 new rows)
+            mbar_expect_tx(bar(kBarWin), (has_c2p ? (band_idx == 0 ? G::kWin : G::kTile) : 0u) + (has_p2c ? G::kWin : 0u));
             if (has_c2p) tma_load_3d(smem + kSmemWinK, &args.tm_xk, bar(kBarWin), 0, u0, head);
+            if (has_c2p && band_idx == 0) tma_load_3d(smem + kSmemWinK + G::kTile, &args.tm_xk, bar(kBarWin), 0, u0 + 128, head);
             if (has_p2c) tma_load_3d(smem + kSmemWinQ, &args.tm_xq, bar(kBarWin), 0, u0, head);
           }
           ++band_idx;
@@ -321,11 +334,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         const int kind = tile_kind(j);
         const int s = jj & 1;
         const uint64_t dk = dk0 + uint64_t(s) * (16384u >> 4);  // stages are 16 KB apart in either build
+        wait(bar(kBarK + s), uint32_t(jj >> 1) & 1u);
+        if (kind == kBand) wait(bar(kBarWin), uint32_t(band_idx) & 1u);
         // both softmax groups hold tile j-1 in registers: S and R are free
         if (jj > 0) wait(bar(kBarSFree), uint32_t(jj - 1) & 1u);
-        wait(bar(kBarK + s), uint32_t(jj >> 1) & 1u);
         if (kind == kBand) {
-          wait(bar(kBarWin), uint32_t(band_idx) & 1u);
           tc_fence_after();
           // Order of issue.  First band tile of the run: c2p (two 128-position blocks) -> R, scores -> S, and once the
           // drain group has emptied R, the p2c products -> R.  Later tiles bring one c2p block, and it goes to the S
@@ -462,6 +475,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       }
     }
 
+    // lane that holds the p2c value of key c of a 32-key block; kept in registers (an addition per shuffle otherwise)
+    [[maybe_unused]] int from[32];
+    if constexpr (!F8) {
+#pragma unroll
+      for (int c = 0; c < 32; ++c) {
+        from[c] = lane + 31 - c;  // (taken modulo 32)
+        asm volatile("" : "+r"(from[c]));
+      }
+    }
     uint32_t band_idx = 0;
     // Rows behind the sequence (padding, the next sequence, unused memory) never ask for a rescale, which the rows of their warp take
     // part in: a sequence's rounding is its own.
@@ -498,32 +520,70 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       // ---- this thread's 64 scores (+ p2c through the quadrant shuffle) into registers, then S and R are released ----
       float s[64];
       if (kind == kBand && has_p2c) {
-        // 16 keys at a time, the loads of the next 16 in flight while these are combined (two sets of three 16-register runs)
-        uint32_t a[2][16], t0[2][16], t1[2][16];
-        auto pull = [&](int q) {
-          // key block b = 2g + (q >> 1): columns of its two products (see the score-issuing warp)
-          const int b = 2 * g + (q >> 1);
-          const uint32_t c0 = b == 3 ? 224u : 64u * uint32_t(b);
-          const uint32_t c1 = b == 0 ? 192u : 64u * uint32_t(b) - 32u;
-          const uint32_t hf = 16u * uint32_t(q & 1);
-          tmem_ld16(tmem_lane + kColS + 64 * g + 16 * q, a[q & 1]);
-          tmem_ld16(tmem_lane + kColR + c0 + hf, t0[q & 1]);
-          tmem_ld16(tmem_lane + kColR + c1 + hf, t1[q & 1]);
-        };
-        pull(0);
+        if constexpr (F8) {
+          // 16 keys at a time, the loads of the next 16 in flight while these are combined (two sets of three 16-register runs; in the
+          // other form, which needs its registers for the scale ratios too, 438 against 431 us a call of 2 x 4096 x 16 heads)
+          uint32_t a[2][16], t0[2][16], t1[2][16];
+          auto pull = [&](int q) {
+            // key block b = 2g + (q >> 1): columns of its two products (see the score-issuing warp)
+            const int b = 2 * g + (q >> 1);
+            const uint32_t c0 = b == 3 ? 224u : 64u * uint32_t(b);
+            const uint32_t c1 = b == 0 ? 192u : 64u * uint32_t(b) - 32u;
+            const uint32_t hf = 16u * uint32_t(q & 1);
+            tmem_ld16(tmem_lane + kColS + 64 * g + 16 * q, a[q & 1]);
+            tmem_ld16(tmem_lane + kColR + c0 + hf, t0[q & 1]);
+            tmem_ld16(tmem_lane + kColR + c1 + hf, t1[q & 1]);
+          };
+          pull(0);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          tmem_wait_ld();
+          for (int q = 0; q < 4; ++q) {
+            tmem_wait_ld();
 #pragma unroll
-          for (int c = 0; c < 16; ++c)  // nothing below uses them in front of the wait
-            asm volatile("" : "+r"(a[q & 1][c]), "+r"(t0[q & 1][c]), "+r"(t1[q & 1][c]));
-          if (q < 3) pull(q + 1);
+            for (int c = 0; c < 16; ++c)  // nothing below uses them in front of the wait
+              asm volatile("" : "+r"(a[q & 1][c]), "+r"(t0[q & 1][c]), "+r"(t1[q & 1][c]));
+            if (q < 3) pull(q + 1);
 #pragma unroll
-          for (int c = 0; c < 16; ++c) {
-            const int cc = 16 * (q & 1) + c;
-            const uint32_t x = (lane + cc <= 30) ? t1[q & 1][c] : t0[q & 1][c];
-            const uint32_t y = __shfl_sync(0xffffffffu, x, lane + 31 - cc);  // the source lane is taken modulo 32
-            s[16 * q + c] = fmaf(__uint_as_float(y), ratio_p, __uint_as_float(a[q & 1][c]));
+            for (int c = 0; c < 16; ++c) {
+              const int cc = 16 * (q & 1) + c;
+              const uint32_t x = (lane + cc <= 30) ? t1[q & 1][c] : t0[q & 1][c];
+              const uint32_t y = __shfl_sync(0xffffffffu, x, lane + 31 - cc);  // the source lane is taken modulo 32
+              s[16 * q + c] = fmaf(__uint_as_float(y), ratio_p, __uint_as_float(a[q & 1][c]));
+            }
+          }
+        } else {
+          // the scores, then 16 keys at a time the two products: the loads of the next 16 are in flight while these are shuffled
+          uint32_t a0[32], a1[32], t0[16], t1[16], x[16];
+          auto pull = [&](int q) {
+            // key block b = 2g + (q >> 1): columns of its two products (see the score-issuing warp)
+            const int b = 2 * g + (q >> 1);
+            const uint32_t hf = 16u * uint32_t(q & 1);
+            tmem_ld16(tmem_lane + kColR + (b == 3 ? 224u : 64u * uint32_t(b)) + hf, t0);
+            tmem_ld16(tmem_lane + kColR + (b == 0 ? 192u : 64u * uint32_t(b) - 32u) + hf, t1);
+          };
+          tmem_ld32(tmem_lane + kColS + 64 * g, a0);
+          tmem_ld32(tmem_lane + kColS + 64 * g + 32, a1);
+          pull(0);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            tmem_wait_ld();
+            if (q == 0) {
+#pragma unroll
+              for (int c = 0; c < 32; ++c) asm volatile("" : "+r"(a0[c]), "+r"(a1[c]));  // nothing below uses them in front of the wait
+            }
+#pragma unroll
+            for (int c = 0; c < 16; ++c) asm volatile("" : "+r"(t0[c]), "+r"(t1[c]));
+#pragma unroll
+            for (int c = 0; c < 16; ++c) x[c] = (lane + 16 * (q & 1) + c <= 30) ? t1[c] : t0[c];
+            if (q < 3) {
+#pragma unroll
+              for (int c = 0; c < 16; ++c) asm volatile("" : "+r"(x[c]));
+              pull(q + 1);
+            }
+#pragma unroll
+            for (int c = 0; c < 16; ++c) {
+              const uint32_t y = __shfl_sync(0xffffffffu, x[c], from[16 * (q & 1) + c]);
+              s[16 * q + c] = fmaf(__uint_as_float(y), ratio_p, __uint_as_float(q < 2 ? a0[16 * q + c] : a1[16 * q + c - 32]));
+            }
           }
         }
       } else {
@@ -567,8 +627,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
             const uint32_t w[4] = {w4.x, w4.y, w4.z, w4.w};
 #pragma unroll
             for (int e = 0; e < 8; ++e) {  // column 8q + e of the run -> key 63 - (8q + e)
-              const uint32_t bits = (e & 1) ? (w[e >> 1] & 0xffff0000u) : (w[e >> 1] << 16);
-              s[63 - (8 * q + e)] = fmaf(__uint_as_float(bits), ratio_c, s[63 - (8 * q + e)]);
+              float& to = s[63 - (8 * q + e)];
+              if constexpr (F8) to = fmaf(__uint_as_float((e & 1) ? (w[e >> 1] & 0xffff0000u) : (w[e >> 1] << 16)), ratio_c, to);
+              else to = (e & 1) ? add_bf16_hi(to, w[e >> 1]) : add_bf16_lo(to, w[e >> 1]);
             }
           }
         }
@@ -738,7 +799,7 @@ int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, con
   a.q_scale = p.q_scale; a.k_scale = p.k_scale; a.v_scale = p.v_scale;
   a.xk_scale = p.pos_key_scale; a.xq_scale = p.pos_query_scale;
   // a map is always encoded so the kernel argument is well formed; an unused one points at q
-  if (a.xk) { if ((rc = make_map_table(&a.tm_xk, a.xk, g.rows, p.heads, f8, "expanded pos_key"))) return rc; } else a.tm_xk = a.tm_q;
+  if (a.xk) { if ((rc = make_map_table(&a.tm_xk, a.xk, g.rows, p.heads, f8, "expanded pos_key", 128))) return rc; } else a.tm_xk = a.tm_q;
   if (a.xq) { if ((rc = make_map_table(&a.tm_xq, a.xq, g.rows, p.heads, f8, "expanded pos_query"))) return rc; } else a.tm_xq = a.tm_q;
   if (a.xq) { if ((rc = make_map_table(&a.tm_xq_sat, a.xq, g.rows, p.heads, f8, "saturated pos_query rows", 8))) return rc; } else a.tm_xq_sat = a.tm_q;
   a.out = static_cast<__nv_bfloat16*>(p.out);

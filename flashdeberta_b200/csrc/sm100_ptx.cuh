@@ -304,6 +304,17 @@ __device__ __forceinline__ uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+// fp32 plus the lower / upper bf16 of a pair (exact conversion, one rounding)
+__device__ __forceinline__ float add_bf16_lo(float a, uint32_t pair) {
+  float d;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tadd.f32.bf16 %0, l, %2;\n\t}" : "=f"(d) : "r"(pair), "f"(a));
+  return d;
+}
+__device__ __forceinline__ float add_bf16_hi(float a, uint32_t pair) {
+  float d;
+  asm("{\n\t.reg .b16 l, h;\n\tmov.b32 {l, h}, %1;\n\tadd.f32.bf16 %0, h, %2;\n\t}" : "=f"(d) : "r"(pair), "f"(a));
+  return d;
+}
 // four floats -> four e4m3 bytes (a in the lowest byte), saturating
 __device__ __forceinline__ uint32_t pack_e4m3x4(float a, float b, float c, float d) {
   uint16_t lo, hi;
