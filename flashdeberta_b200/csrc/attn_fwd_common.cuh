@@ -108,45 +108,37 @@ __device__ __forceinline__ float lds_f32(uint32_t addr) {
   return v;
 }
 
-// dot product of one query row (128-byte-swizzled in shared memory) with one 64-element bf16 row in global memory
+// sum of eight (e4m3: sixteen) products of one 16-byte chunk each, added to `acc` one by one
+__device__ __forceinline__ float dot_bf16(uint4 a, uint4 b, float acc) {
+  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    acc = fmaf(bf16_bits_to_f32(aw[i] & 0xffffu), bf16_bits_to_f32(bw[i] & 0xffffu), acc);
+    acc = fmaf(bf16_bits_to_f32(aw[i] >> 16), bf16_bits_to_f32(bw[i] >> 16), acc);
+  }
+  return acc;
+}
+__device__ __forceinline__ float dot_f8(uint4 a, uint4 b, float acc) {
+  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    float fa[4], fb[4];
+    unpack_e4m3x4(aw[i], fa);
+    unpack_e4m3x4(bw[i], fb);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) acc = fmaf(fa[k], fb[k], acc);
+  }
+  return acc;
+}
+// dot product of one query row (128-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ (r & 7); e4m3 rows of 64 bytes: at
+// c ^ ((r >> 1) & 3)) in shared memory with one 64-element bf16 row in global memory
 __device__ __forceinline__ float dot_q_row(uint32_t q_row_addr, int row, const __nv_bfloat16* __restrict__ g) {
   float acc = 0.f;
   const uint4* g4 = reinterpret_cast<const uint4*>(g);
 #pragma unroll
-  for (int c = 0; c < 8; ++c) {
-    const uint4 a = lds_v4(q_row_addr + (uint32_t((c ^ (row & 7))) << 4));
-    const uint4 b = __ldg(g4 + c);
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      acc = fmaf(bf16_bits_to_f32(aw[i] & 0xffffu), bf16_bits_to_f32(bw[i] & 0xffffu), acc);
-      acc = fmaf(bf16_bits_to_f32(aw[i] >> 16), bf16_bits_to_f32(bw[i] >> 16), acc);
-    }
-  }
+  for (int c = 0; c < 8; ++c) acc = dot_bf16(lds_v4(q_row_addr + (uint32_t((c ^ (row & 7))) << 4)), __ldg(g4 + c), acc);
   return acc;
 }
-
-// the same for e4m3 rows (64 bytes, 64-byte swizzle: 16-byte chunk c of row r sits at chunk c ^ ((r >> 1) & 3))
-__device__ __forceinline__ float dot_q_row_f8(uint32_t q_row_addr, int row, const uint8_t* __restrict__ g) {
-  float acc = 0.f;
-  const uint4* g4 = reinterpret_cast<const uint4*>(g);
-#pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const uint4 a = lds_v4(q_row_addr + (uint32_t(c ^ ((row >> 1) & 3)) << 4));
-    const uint4 b = __ldg(g4 + c);
-    const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, bw[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float fa[4], fb[4];
-      unpack_e4m3x4(aw[i], fa);
-      unpack_e4m3x4(bw[i], fb);
-#pragma unroll
-      for (int k = 0; k < 4; ++k) acc = fmaf(fa[k], fb[k], acc);
-    }
-  }
-  return acc;
-}
-
 
 // The band tiles of a query tile are one contiguous run of key tiles [first, first + count): this returns it.
 // d0(j) = m0 - 128 j - 127 decreases with j; band <=> sat_lo - 254 < d0 < sat_hi.

@@ -4,13 +4,15 @@
 // src/flashdeberta/ops/flash_attention_varlen.py:85-225) and the two bias GEMMs in front of them
 // (src/flashdeberta/model.py:189-192, :210-214).
 //
-// One CTA = one 128-row query tile of one (sequence, head); 16 warps in four warpgroups (registers move from the
-// producer and drain groups to the softmax groups with setmaxnreg):
+// Work item = one 128-row query tile of one (sequence, head) = one block of the grid; a CTA (one per SM) does its own and then takes
+// blocks over that have not started (cluster launch control), in the grid's order, heaviest tiles first.  16 warps in four
+// warpgroups (registers move from the producer and drain groups to the softmax groups with setmaxnreg):
 //   warps 0-3   softmax group 0: thread r owns row r of the tile, keys   0..63  of every 128-key tile
 //   warps 4-7   softmax group 1: thread r owns row r of the tile, keys  64..127
 //   warp  8     score-side tcgen05.mma: S = Q.K^T and the position products (the warp allocates TMEM)
-//   warp  9     every TMA load: Q once, K/V double-buffered, position-table windows
+//   warp  9     every TMA load: Q once, K/V double-buffered, position-table windows; asks for further work items
 //   warp  10    O += P.V
+//   warp  11    saturated c2p terms (one dot product per row and side)
 //               (8-10 stay converged and issue through an elected lane: see elect_one)
 //   warps 12-15 drain group: moves the c2p product of a band tile from tensor memory to shared memory (bf16)
 // Tensor memory (512 columns): O 64 | P 64 | S 128 | R 256 (position products of a band tile).
@@ -64,9 +66,9 @@ using namespace fwd;
 constexpr int kSoftmaxThreads = 256;
 constexpr int kDrainThreads = 128;
 constexpr int kThreads = 512;            // four warpgroups: softmax 0, softmax 1, producers (warps 10, 11 idle), drain
-constexpr int kMmaWarp = 8, kTmaWarp = 9, kPvWarp = 10, kDrainWarp0 = 12;
-// 128 registers per thread at launch; after setmaxnreg: 40 * 128 + 72 * 128 + 200 * 256 = 65536
-constexpr int kProducerRegs = 40, kDrainRegs = 72, kSoftmaxRegs = 200;
+constexpr int kMmaWarp = 8, kTmaWarp = 9, kPvWarp = 10, kSatWarp = 11, kDrainWarp0 = 12;
+// 128 registers per thread at launch; after setmaxnreg: 48 * 128 + 64 * 128 + 200 * 256 = 65536
+constexpr int kProducerRegs = 48, kDrainRegs = 64, kSoftmaxRegs = 200;
 constexpr uint32_t kTmemCols = 512;
 constexpr uint32_t kColO = 0;     // 64 columns: output accumulator
 constexpr uint32_t kColP = 64;    // 64 columns: P as bf16 pairs (keys 0..63 in the first 32, keys 64..127 in the last 32)
@@ -90,7 +92,9 @@ constexpr uint32_t kSmemSat = kSmemStageC + 71680;  // 2 x (8 x 128 B) saturated
 static_assert(128 * kStageCPitch <= 71680, "c2p stage");
 constexpr uint32_t kSmemXchg = kSmemSat + 2048;     // float [2 parities][2 groups][128 rows] row maxima
 constexpr uint32_t kSmemLsum = kSmemXchg + 2048;    // float [2 groups][128 rows] row sums at the end
-constexpr uint32_t kSmemBars = kSmemLsum + 1024;
+constexpr uint32_t kSmemRc = kSmemLsum + 1024;      // float [2 items][hi, lo][128 rows] saturated c2p terms
+constexpr uint32_t kSmemItem = kSmemRc + 2048;      // 16 B answer to a request for another block; 2 x 32 B work items
+constexpr uint32_t kSmemBars = kSmemItem + 96;
 constexpr uint32_t kSmemBytes = kSmemBars + 256 + 1024;  // + alignment slack
 static_assert(kSmemSat % 1024 == 0, "shared memory map");
 static_assert(kSmemBytes <= 232448, "exceeds 227 KB");
@@ -111,8 +115,36 @@ enum Bar : uint32_t {
   kBarC2p = 15,      // 1   the c2p product of a band tile is in R
   kBarStage = 16,    // 4   the drain group has written the c2p stage (R may be overwritten, the stage may be read)
   kBarGather = 17,   // 8   both softmax groups are done reading the c2p stage
-  kNumBars = 18
+  kBarQFree = 18,    // 1   the MMAs that read Q (and the saturated rows) of an item finished
+  kBarRc = 19,       // 1   the saturated c2p terms of an item are in buffer s (Q has been read for them), 2 buffers: with items of one
+                     //     tile the next item's are there before the softmax groups look for these
+  kBarAnswer = 21,   // 1   the answer to a request for another block is there
+  kBarItem = 22,     // 1   work item in slot s, 2 slots
+  kBarItemFree = 24, // 15  every other role has read it
+  kNumBars = 26
 };
+constexpr uint32_t kItemReaders = 15;  // softmax 8, drain 4, score, P.V, saturated terms
+
+// One work item: a query tile of one (sequence, head) and the key tiles that this launch gives it.
+struct Item {
+  int seq, m0, row0, len, head;
+  int j_first, n_proc;  // key tiles j_first .. j_first + n_proc - 1; none: an empty slot or a padding tile
+  bool resume;          // the far kernel has left a partial result for this tile
+};
+__device__ __forceinline__ Item make_item(const FwdArgs& args, int4 slot, uint32_t head) {
+  Item it;
+  it.seq = (int)uniform(slot.x); it.m0 = (int)uniform(slot.y); it.row0 = (int)uniform(slot.z); it.len = (int)uniform(slot.w);
+  it.head = (int)uniform(head);
+  it.j_first = it.n_proc = 0;
+  it.resume = false;
+  if (it.seq < 0 || it.m0 >= it.len) return it;  // a slot behind the last sequence, a dense padding tile
+  // key tiles this launch works on: all of them, or (split launch) the contiguous run of band tiles
+  const int num_kt = (it.len + kTileN - 1) / kTileN;
+  it.n_proc = num_kt;
+  if (args.band_only && it.len >= args.split_len) band_run(it.m0, num_kt, args.sat_lo, args.sat_hi, it.j_first, it.n_proc);
+  it.resume = args.band_only && it.n_proc < num_kt;
+  return it;
+}
 
 template <bool F8>
 __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_constant__ FwdArgs args) {
@@ -121,43 +153,15 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
   const uint32_t smem = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_gen = smem_raw + (smem - smem_u32(smem_raw));
   const int tid = threadIdx.x, warp = (int)uniform(uint32_t(tid) >> 5), lane = tid & 31;
-  const int head = blockIdx.y;
-
   grid_launch();
   grid_wait();
-  // ---- which tile ------------------------------------------------------------------------------------------------
-  const int4 slot = __ldg(args.slot_info + blockIdx.x);  // (sequence, first row of the tile in it, its first row, its length)
-  if (slot.x < 0) return;                                  // slot past the last sequence
-  const int seq = (int)uniform(slot.x), m0 = (int)uniform(slot.y), seq_row0 = (int)uniform(slot.z), len = (int)uniform(slot.w);
-  // rows of this tile that may be written: packed -> the sequence's own rows; dense -> the padded row range
-  const int row_limit = args.packed ? len : args.max_seqlen;
-
-  if (m0 >= len) {  // dense padding tile: zeros, nothing else (src/flashdeberta/padding.py:30-44)
-    if (tid < kTileM && m0 + tid < row_limit) {
-      uint4* o4 = reinterpret_cast<uint4*>(args.out + (int64_t)(seq_row0 + m0 + tid) * args.o_rs + (int64_t)head * args.o_hs);
-#pragma unroll
-      for (int c = 0; c < 8; ++c) o4[c] = make_uint4(0, 0, 0, 0);
-      if (args.lse != nullptr) args.lse[(int64_t)(seq_row0 + m0 + tid) * args.heads + head] = 0.f;
-    }
-    return;
-  }
-
   const bool has_c2p = args.xk != nullptr, has_p2c = args.xq != nullptr;
   const bool has_pos = has_c2p || has_p2c;
-  const int num_kt = (len + kTileN - 1) / kTileN;
-  // key tiles this launch works on: all of them, or (split launch) the contiguous run of band tiles; `jj` counts them
-  int j_first = 0, n_proc = num_kt;
-  if (args.band_only && len >= args.split_len) band_run(m0, num_kt, args.sat_lo, args.sat_hi, j_first, n_proc);
-  const bool resume = args.band_only && n_proc < num_kt;  // the far kernel has left a partial result for this tile
-  auto tile_kind = [&](int j) -> int {
+  auto tile_kind = [&](const Item& it, int j) -> int {
     if (!has_pos) return kPlain;
-    const int d0 = m0 - j * kTileN - (kTileN - 1);  // smallest distance of the pair; the largest is d0 + 254
+    const int d0 = it.m0 - j * kTileN - (kTileN - 1);  // smallest distance of the pair; the largest is d0 + 254
     return d0 >= args.sat_hi ? kSatHi : (d0 + 254 <= args.sat_lo ? kSatLo : kBand);
   };
-
-  // When the CTA's very first key tile is a band tile, the output and P columns are still unused: the two c2p blocks of
-  // that tile go to the S columns and to O|P instead of R, so its p2c products need not wait for the drain group.
-  const bool c2p_outside_r = !resume && n_proc > 0 && tile_kind(j_first) == kBand;
 
   auto bar = [&](uint32_t i) -> uint32_t { return smem + kSmemBars + 8u * i; };
   const uint32_t tmem_slot = smem + kSmemBars + 8u * kNumBars;
@@ -169,21 +173,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     for (uint32_t i = 0; i < kNumBars; ++i) {
       uint32_t count = 1u;
       if (i == kBarSFree || i == kBarP || i == kBarGather) count = kSoftmaxThreads / 32;  // one arrival per warp
+      if (i == kBarItemFree || i == kBarItemFree + 1) count = kItemReaders;
       if (i == kBarStage) count = kDrainThreads / 32;
       mbar_init(bar(i), count);
     }
     fence_barrier_init();
-  }
-  // e4m3: value = stored * scale.  The three score terms carry different scale products; they are brought to the one of
-  // Q.K^T (ratio_c, ratio_p) when they are added, and that product goes into the softmax scale.
-  float c_eff = args.scale_log2, ratio_c = 1.f, ratio_p = 1.f, v_scale = 1.f;
-  if constexpr (F8) {
-    const float sq = __ldg(args.q_scale + (int64_t)seq * args.heads + head);
-    const float sk = __ldg(args.k_scale + (int64_t)seq * args.heads + head);
-    v_scale = __ldg(args.v_scale + (int64_t)seq * args.heads + head);
-    c_eff = args.scale_log2 * sq * sk;
-    if (has_c2p) ratio_c = __ldg(args.xk_scale + head) / sk;
-    if (has_p2c) ratio_p = __ldg(args.xq_scale + head) / sq;
   }
   if (warp == kMmaWarp) {
     tmem_alloc(tmem_slot, kTmemCols);
@@ -203,18 +197,53 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     if (elect_one()) mbar_arrive(b);
   };
 
+  auto has_saturated = [&](const Item& it) -> bool {  // (the band tiles are one run)
+    return tile_kind(it, it.j_first) != kBand || tile_kind(it, it.j_first + it.n_proc - 1) != kBand;
+  };
+
+  // ---- work items ------------------------------------------------------------------------------------------------------
+  // The CTA stays on its SM and takes further blocks of the grid over (cluster launch control): the roles run ahead of one another
+  // across the border between two items, so the set-up, the first loads, the first c2p blocks and their drain of an item lie
+  // under the last tile and the output of the item before.  As blocks of their own, one behind the other because an SM's tensor memory
+  // and shared memory hold one, those took 11 700 clocks an item beside 4500 per band tile; what is left between two items is 3000.
+  // 353 -> 336 us a call at 8 x 2048 x 12 heads, 164 -> 132 at 32 x 512, padded 24 x <= 779 124 -> 112, packed 48 x <= 4099 x 16
+  // 1393 -> 1310.  Every count below that a barrier's phase depends on runs on from item to item.
+  // The TMA warp asks and hands the items on, worked out: what the other roles execute between two items is code that the
+  // tiles' loops have pushed out of the instruction cache, so there is little of it.
+  uint32_t taken = 0;
+  auto next_item = [&](Item& it) -> bool {
+    const uint32_t slot = taken & 1u, at = smem + kSmemItem + 32u + 32u * slot;
+    wait(bar(kBarItem + slot), (taken >> 1) & 1u);
+    ++taken;
+    if (!ok) return false;
+    const uint4 what = lds_v4(at);
+    const uint4 rest = lds_v4(at + 16u);
+    arrive(bar(kBarItemFree + slot));
+    it.seq = (int)uniform(what.x); it.m0 = (int)uniform(what.y); it.row0 = (int)uniform(what.z); it.len = (int)uniform(what.w);
+    it.head = (int)uniform(rest.x); it.j_first = (int)uniform(rest.y); it.n_proc = (int)uniform(rest.z);
+    const uint32_t flags = uniform(rest.w);
+    it.resume = (flags & 2u) != 0u;
+    return (flags & 1u) != 0u;
+  };
+  // (sequence, first row of the tile in it, its first row, its length)
+  Item it = make_item(args, __ldg(args.slot_info + blockIdx.x), blockIdx.y);
+
   if (warp >= kDrainWarp0) {
     // =================================================== drain group ====================================================
     reg_dealloc<kDrainRegs>();
     const int quad = warp & 3;
     const int r = quad * 32 + lane;  // TMEM lane = position row inside a 128-position block
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
+    uint32_t bands = 0;  // band tiles of all items so far
+    bool first_item = true;
+    do {
     uint32_t band_idx = 0;
-    for (int jj = 0; jj < n_proc; ++jj) {
-      const int j = j_first + jj;
-      if (tile_kind(j) != kBand) continue;
-      if (band_idx > 0) wait(bar(kBarGather), (band_idx - 1u) & 1u);   // nobody reads the previous stage any more
-      wait(bar(kBarC2p), band_idx & 1u);                               // the product is there
+    for (int jj = 0; jj < it.n_proc; ++jj) {
+      const int j = it.j_first + jj;
+      if (tile_kind(it, j) != kBand) continue;
+      if (bands > 0) wait(bar(kBarGather), (bands - 1u) & 1u);   // nobody reads the previous stage any more
+      wait(bar(kBarC2p), bands & 1u);                            // the product is there
+      const bool c2p_outside_r = first_item && jj == 0 && !it.resume;
       tc_fence_after();
       if (has_c2p && ok) {
         // The product has query rows in the lanes and window positions in the columns, so this thread holds row r.  The
@@ -263,57 +292,130 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       tc_fence_before();
       arrive(bar(kBarStage));
       ++band_idx;
+      ++bands;
     }
+    if (it.n_proc > 0) first_item = false;
+    } while (next_item(it));
   } else if (warp >= kMmaWarp) {
     reg_dealloc<kProducerRegs>();
     if (warp == kTmaWarp) {
       // ================================================= TMA producer ===================================================
-      if (elect_one()) {
-        tma_prefetch_desc(&args.tm_q); tma_prefetch_desc(&args.tm_k); tma_prefetch_desc(&args.tm_v);
+      if (elect_one()) { tma_prefetch_desc(&args.tm_q); tma_prefetch_desc(&args.tm_k); tma_prefetch_desc(&args.tm_v); }
+      uint32_t items = 0, tiles = 0, bands = 0, asked = 0;
+      bool more = false;
+      do {
+      if (it.n_proc > 0) {
+        if (items > 0) {
+          wait(bar(kBarQFree), (items - 1u) & 1u);
+          wait(bar(kBarRc + ((items - 1u) & 1u)), ((items - 1u) >> 1) & 1u);
+        }
+        ++items;
+      }
+      if (ok && it.n_proc > 0 && elect_one()) {
         mbar_expect_tx(bar(kBarQ), G::kTile + (has_p2c ? 16u * G::kRow : 0u));
-        tma_load_3d(smem + kSmemQ, &args.tm_q, bar(kBarQ), 0, head, seq_row0 + m0);
+        tma_load_3d(smem + kSmemQ, &args.tm_q, bar(kBarQ), 0, it.head, it.row0 + it.m0);
         if (has_p2c) {
           // Saturated pos_query rows as MMA operands: the last (first) eight rows of an expanded table are all the row of
           // distances beyond sat_hi (sat_lo), so an 8-row box is the 8 identical rows in the swizzled layout.
-          tma_load_3d(smem + kSmemSat, &args.tm_xq_sat, bar(kBarQ), 0, args.xrows - 8, head);
-          tma_load_3d(smem + kSmemSat + 1024, &args.tm_xq_sat, bar(kBarQ), 0, 0, head);
+          tma_load_3d(smem + kSmemSat, &args.tm_xq_sat, bar(kBarQ), 0, args.xrows - 8, it.head);
+          tma_load_3d(smem + kSmemSat + 1024, &args.tm_xq_sat, bar(kBarQ), 0, 0, it.head);
         }
       }
-      int band_idx = 0;
+      uint32_t band_idx = 0;
 #pragma unroll 1
-      for (int jj = 0; jj < n_proc && ok; ++jj) {
-        const int j = j_first + jj;
-        const int s = jj & 1;
-        const uint32_t use = uint32_t(jj >> 1);  // how often this stage was used before
+      for (int jj = 0; jj < it.n_proc && ok; ++jj) {
+        const int j = it.j_first + jj;
+        const uint32_t s = tiles & 1u, use = tiles >> 1;  // how often this stage was used before
         FDB_STAMP(3, j, 0);
-        if (jj >= 2) wait(bar(kBarKFree + s), (use - 1u) & 1u);
+        if (use > 0) wait(bar(kBarKFree + s), (use - 1u) & 1u);
         if (!ok) break;
         FDB_STAMP(3, j, 1);
         if (elect_one()) {
           mbar_expect_tx(bar(kBarK + s), G::kTile);
-          tma_load_3d(smem + kSmemK + s * 16384, &args.tm_k, bar(kBarK + s), 0, head, seq_row0 + j * kTileN);
+          tma_load_3d(smem + kSmemK + s * 16384, &args.tm_k, bar(kBarK + s), 0, it.head, it.row0 + j * kTileN);
         }
-        if (tile_kind(j) == kBand) {
-          if (band_idx > 0) wait(bar(kBarWinFree), uint32_t(band_idx - 1) & 1u);
+        if (tile_kind(it, j) == kBand) {
+          if (bands > 0) wait(bar(kBarWinFree), (bands - 1u) & 1u);
           if (!ok) break;
-          const int u0 = m0 - j * kTileN - (kTileN - 1) - args.d_first;
+          const int u0 = it.m0 - j * kTileN - (kTileN - 1) - args.d_first;
           if (elect_one()) {
             // (of pos_key the first tile of the run takes the whole window, the others its 128 new rows)
             mbar_expect_tx(bar(kBarWin), (has_c2p ? (band_idx == 0 ? G::kWin : G::kTile) : 0u) + (has_p2c ? G::kWin : 0u));
-            if (has_c2p) tma_load_3d(smem + kSmemWinK, &args.tm_xk, bar(kBarWin), 0, u0, head);
-            if (has_c2p && band_idx == 0) tma_load_3d(smem + kSmemWinK + G::kTile, &args.tm_xk, bar(kBarWin), 0, u0 + 128, head);
-            if (has_p2c) tma_load_3d(smem + kSmemWinQ, &args.tm_xq, bar(kBarWin), 0, u0, head);
+            if (has_c2p) tma_load_3d(smem + kSmemWinK, &args.tm_xk, bar(kBarWin), 0, u0, it.head);
+            if (has_c2p && band_idx == 0) tma_load_3d(smem + kSmemWinK + G::kTile, &args.tm_xk, bar(kBarWin), 0, u0 + 128, it.head);
+            if (has_p2c) tma_load_3d(smem + kSmemWinQ, &args.tm_xq, bar(kBarWin), 0, u0, it.head);
           }
           ++band_idx;
+          ++bands;
         }
-        if (jj >= 2) wait(bar(kBarVFree + s), (use - 1u) & 1u);
+        if (use > 0) wait(bar(kBarVFree + s), (use - 1u) & 1u);
         if (!ok) break;
         FDB_STAMP(3, j, 2);
         if (elect_one()) {
           mbar_expect_tx(bar(kBarV + s), G::kTile);
-          tma_load_3d(smem + kSmemV + s * 16384, &args.tm_v, bar(kBarV + s), 0, head, seq_row0 + j * kTileN);
+          tma_load_3d(smem + kSmemV + s * 16384, &args.tm_v, bar(kBarV + s), 0, it.head, it.row0 + j * kTileN);
         }
+        ++tiles;
       }
+        // another item: asked for when this one is on its way (asked for at its start, the items at the end of a launch would go to
+        // whoever started early, not to whoever is done first)
+        if (ok && elect_one()) {
+          mbar_expect_tx(bar(kBarAnswer), 16u);
+          launch_take_over(smem + kSmemItem, bar(kBarAnswer));
+        }
+        wait(bar(kBarAnswer), asked & 1u);
+        if (!ok) break;
+        uint32_t x, y;
+        more = launch_taken_over(smem + kSmemItem, x, y);
+        fence_proxy_async();  // (the answer is written through the asynchronous proxy again)
+        const uint32_t slot = asked & 1u, at = smem + kSmemItem + 32u + 32u * slot;
+        it = make_item(args, __ldg(args.slot_info + (more ? x : 0u)), y);
+        if (asked >= 2) wait(bar(kBarItemFree + slot), ((asked >> 1) - 1u) & 1u);
+        if (elect_one()) {
+          sts_v4(at, (uint32_t)it.seq, (uint32_t)it.m0, (uint32_t)it.row0, (uint32_t)it.len);
+          sts_v4(at + 16u, (uint32_t)it.head, (uint32_t)it.j_first, (uint32_t)it.n_proc, (more ? 1u : 0u) | (it.resume ? 2u : 0u));
+          mbar_arrive(bar(kBarItem + slot));
+        }
+        ++asked;
+      } while (more);
+    } else if (warp == kSatWarp) {
+      // ============================================= saturated c2p terms ================================================
+      // Q[m].X_k[first row] and Q[m].X_k[last row] of the item's rows, for its saturated tiles.  (The buffer of the item before the last
+      // is free: Q of this one is loaded once the scores of the last one's last tile exist.)
+      uint32_t items = 0;
+      do {
+        if (it.n_proc == 0) continue;
+        wait(bar(kBarQ), items & 1u);
+        if (has_c2p && ok && has_saturated(it)) {
+          const uint32_t rc = smem + kSmemRc + 1024u * (items & 1u);
+          const uint8_t* x = static_cast<const uint8_t*>(args.xk) + (int64_t)it.head * args.xrows * G::kRow;
+          float hi[4] = {0.f, 0.f, 0.f, 0.f}, lo[4] = {0.f, 0.f, 0.f, 0.f};
+          auto chunk = [&](int c, const uint8_t* row) { return __ldg(reinterpret_cast<const uint4*>(row) + c); };
+          const uint8_t* x_last = x + (int64_t)(args.xrows - 1) * G::kRow;
+          uint4 first = chunk(0, x), last = chunk(0, x_last);
+#pragma unroll 1
+          for (int c = 0; c < (int)G::kRow / 16; ++c) {
+            const int next = min(c + 1, (int)G::kRow / 16 - 1);
+            const uint4 first_n = chunk(next, x), last_n = chunk(next, x_last);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              const int r = 32 * i + lane;
+              const uint4 a = lds_v4(smem + kSmemQ + uint32_t(r) * G::kRow + (uint32_t(F8 ? c ^ ((r >> 1) & 3) : c ^ (r & 7)) << 4));
+              lo[i] = F8 ? dot_f8(a, first, lo[i]) : dot_bf16(a, first, lo[i]);
+              hi[i] = F8 ? dot_f8(a, last, hi[i]) : dot_bf16(a, last, hi[i]);
+            }
+            first = first_n;
+            last = last_n;
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            sts_f32(rc + 4u * uint32_t(32 * i + lane), hi[i]);
+            sts_f32(rc + 512u + 4u * uint32_t(32 * i + lane), lo[i]);
+          }
+        }
+        arrive(bar(kBarRc + (items & 1u)));
+        ++items;
+      } while (next_item(it));
     } else if (warp == kMmaWarp) {
       // ================================================= score MMA issuer ===============================================
       // S = Q.K^T (+ saturated p2c) and the position products of band tiles.  Descriptors are built once; per MMA only the
@@ -326,18 +428,26 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       const uint64_t dwk = G::desc(smem + kSmemWinK, G::kGroup);
       const uint64_t dwq = G::desc(smem + kSmemWinQ, G::kGroup);
       const uint64_t dsat = G::desc(smem + kSmemSat, 0);  // group stride 0: every 8-row group is the same rows
+      uint32_t items = 0, tiles = 0, bands = 0;
+      do {
       int band_idx = 0;
-      wait(bar(kBarQ), 0);
+      // When the CTA's very first key tile is a band tile, the output and P columns are still unused: the two c2p blocks of
+      // that tile go to the S columns and to O|P instead of R, so its p2c products need not wait for the drain group.
+      const bool c2p_outside_r = items == 0 && !it.resume && it.n_proc > 0 && tile_kind(it, it.j_first) == kBand;
+      if (it.n_proc > 0) {
+        wait(bar(kBarQ), items & 1u);
+        ++items;
+      }
 #pragma unroll 1
-      for (int jj = 0; jj < n_proc; ++jj) {
-        const int j = j_first + jj;
-        const int kind = tile_kind(j);
-        const int s = jj & 1;
+      for (int jj = 0; jj < it.n_proc; ++jj) {
+        const int j = it.j_first + jj;
+        const int kind = tile_kind(it, j);
+        const uint32_t s = tiles & 1u;
         const uint64_t dk = dk0 + uint64_t(s) * (16384u >> 4);  // stages are 16 KB apart in either build
-        wait(bar(kBarK + s), uint32_t(jj >> 1) & 1u);
-        if (kind == kBand) wait(bar(kBarWin), uint32_t(band_idx) & 1u);
-        // both softmax groups hold tile j-1 in registers: S and R are free
-        if (jj > 0) wait(bar(kBarSFree), uint32_t(jj - 1) & 1u);
+        wait(bar(kBarK + s), (tiles >> 1) & 1u);
+        if (kind == kBand) wait(bar(kBarWin), bands & 1u);
+        // both softmax groups hold the tile before in registers: S and R are free
+        if (tiles > 0) wait(bar(kBarSFree), (tiles - 1u) & 1u);
         if (kind == kBand) {
           tc_fence_after();
           // Order of issue.  First band tile of the run: c2p (two 128-position blocks) -> R, scores -> S, and once the
@@ -365,7 +475,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
               G::mma(tmem_base + kColS, dq + uint64_t((ks * 32) >> 4), dk + uint64_t((ks * 32) >> 4), idesc_s, ks > 0);
           }
           if (!scores_last) {
-            wait(bar(kBarStage), uint32_t(band_idx) & 1u);  // the drain group has moved the c2p product out of R
+            wait(bar(kBarStage), bands & 1u);  // the drain group has moved the c2p product out of R
             tc_fence_after();
           }
           if (ok && has_p2c && elect_one()) {
@@ -394,7 +504,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
                      dk + 3 * blk32 + uint64_t((ks * 32) >> 4), idesc_p2c, ks > 0);
           }
           if (scores_last) {
-            wait(bar(kBarStage), uint32_t(band_idx) & 1u);  // the drain group has moved the c2p product out of S
+            wait(bar(kBarStage), bands & 1u);  // the drain group has moved the c2p product out of S
             tc_fence_after();
             if (ok && elect_one()) {
 #pragma unroll
@@ -403,6 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
             }
           }
           ++band_idx;
+          ++bands;
         } else {
           tc_fence_after();
         }
@@ -424,32 +535,40 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           mma_commit(bar(kBarS));
           mma_commit(bar(kBarKFree + s));
           if (kind == kBand) mma_commit(bar(kBarWinFree));
+          if (jj == it.n_proc - 1) mma_commit(bar(kBarQFree));
         }
+        ++tiles;
         FDB_STAMP(2, j, 0);
       }
+      } while (next_item(it));
     } else if (warp == kPvWarp) {
       // ================================================= P.V MMA issuer =================================================
       const uint32_t idesc_pv = instr_desc(128, 64, G::kFmt, 0, 1);
       const uint64_t dv0 = G::desc(smem + kSmemV, G::kGroup);  // V is the MN-major operand: keys run along K
+      uint32_t tiles = 0;
+      do {
 #pragma unroll 1
-      for (int jj = 0; jj < n_proc; ++jj) {
-        const uint64_t dv = dv0 + uint64_t(jj & 1) * (16384u >> 4);
-        wait(bar(kBarV + (jj & 1)), uint32_t(jj >> 1) & 1u);
-        wait(bar(kBarP), uint32_t(jj) & 1u);  // both groups have written P
+      for (int jj = 0; jj < it.n_proc; ++jj) {
+        const uint32_t s = tiles & 1u;
+        const uint64_t dv = dv0 + uint64_t(s) * (16384u >> 4);
+        wait(bar(kBarV + s), (tiles >> 1) & 1u);
+        wait(bar(kBarP), tiles & 1u);  // both groups have written P (and read the output of the item before)
         tc_fence_after();
-        FDB_STAMP(2, j_first + jj, 3);
+        FDB_STAMP(2, it.j_first + jj, 3);
         if (ok && elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < G::kPvSteps; ++ks)  // one step = 2048 bytes of V in either build (16 x 128 B, 32 x 64 B)
             G::mma_ts(tmem_base + kColO, tmem_base + kColP + G::kPColsPerStep * ks, dv + uint64_t((ks * 2048) >> 4),
-                      idesc_pv, (jj > 0 || ks > 0 || resume) ? 1u : 0u);
+                      idesc_pv, (jj > 0 || ks > 0 || it.resume) ? 1u : 0u);
         }
         if (elect_one()) {
           mma_commit(bar(kBarO));
-          mma_commit(bar(kBarVFree + (jj & 1)));
+          mma_commit(bar(kBarVFree + s));
         }
-        FDB_STAMP(2, j_first + jj, 5);
+        ++tiles;
+        FDB_STAMP(2, it.j_first + jj, 5);
       }
+      } while (next_item(it));
     }
   } else {
     // =================================================== softmax groups =================================================
@@ -458,23 +577,6 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     const int quad = warp & 3;
     const int r = quad * 32 + lane;          // row of the tile
     const uint32_t tmem_lane = tmem_base + (uint32_t(quad * 32) << 16);
-    const int my_row = m0 + r;
-
-    wait(bar(kBarQ), 0);
-    float rc_lo = 0.f, rc_hi = 0.f;  // saturated c2p terms of this row: Q[m].X_k[first row], Q[m].X_k[last row]
-    if (has_c2p && ok) {
-      const uint32_t q_row = smem + kSmemQ + uint32_t(r) * G::kRow;
-      if constexpr (F8) {
-        const uint8_t* xk_h = static_cast<const uint8_t*>(args.xk) + (int64_t)head * args.xrows * kHeadDim;
-        rc_lo = ratio_c * dot_q_row_f8(q_row, r, xk_h);
-        rc_hi = ratio_c * dot_q_row_f8(q_row, r, xk_h + (int64_t)(args.xrows - 1) * kHeadDim);
-      } else {
-        const __nv_bfloat16* xk_h = static_cast<const __nv_bfloat16*>(args.xk) + (int64_t)head * args.xrows * kHeadDim;
-        rc_lo = dot_q_row(q_row, r, xk_h);
-        rc_hi = dot_q_row(q_row, r, xk_h + (int64_t)(args.xrows - 1) * kHeadDim);
-      }
-    }
-
     // lane that holds the p2c value of key c of a 32-key block; kept in registers (an addition per shuffle otherwise)
     [[maybe_unused]] int from[32];
     if constexpr (!F8) {
@@ -484,6 +586,38 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         asm volatile("" : "+r"(from[c]));
       }
     }
+    uint32_t items = 0, tiles = 0, bands = 0;
+    do {
+    const int m0 = it.m0, len = it.len, seq_row0 = it.row0, head = it.head, j_first = it.j_first, n_proc = it.n_proc;
+    const bool resume = it.resume;
+    const int my_row = m0 + r;
+    // rows of this tile that may be written: packed -> the sequence's own rows; dense -> the padded row range
+    const int row_limit = args.packed ? len : args.max_seqlen;
+    if (n_proc == 0) {  // dense padding tile: zeros, nothing else (src/flashdeberta/padding.py:30-44)
+      if (it.seq >= 0 && g == 0 && my_row < row_limit) {
+        uint4* o4 = reinterpret_cast<uint4*>(args.out + (int64_t)(seq_row0 + my_row) * args.o_rs + (int64_t)head * args.o_hs);
+#pragma unroll
+        for (int c = 0; c < 8; ++c) o4[c] = make_uint4(0, 0, 0, 0);
+        if (args.lse != nullptr) args.lse[(int64_t)(seq_row0 + my_row) * args.heads + head] = 0.f;
+      }
+      __syncwarp();
+      continue;
+    }
+    // e4m3: value = stored * scale.  The three score terms carry different scale products; they are brought to the one of
+    // Q.K^T (ratio_c, ratio_p) when they are added, and that product goes into the softmax scale.
+    float c_eff = args.scale_log2, ratio_c = 1.f, ratio_p = 1.f, v_scale = 1.f;
+    if constexpr (F8) {
+      const int64_t at = (int64_t)it.seq * args.heads + head;
+      const float sq = __ldg(args.q_scale + at), sk = __ldg(args.k_scale + at);
+      v_scale = __ldg(args.v_scale + at);
+      c_eff = args.scale_log2 * sq * sk;
+      if (has_c2p) ratio_c = __ldg(args.xk_scale + head) / sk;
+      if (has_p2c) ratio_p = __ldg(args.xq_scale + head) / sq;
+    }
+
+    float rc_lo = 0.f, rc_hi = 0.f;  // saturated c2p terms of this row
+    bool rc_read = !has_c2p;
+
     uint32_t band_idx = 0;
     // Rows behind the sequence (padding, the next sequence, unused memory) never ask for a rescale, which the rows of their warp take
     // part in: a sequence's rounding is its own.
@@ -507,13 +641,22 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       l_run = g == 0 ? ml.y : 0.f;
     }
 
+#pragma unroll 1
     for (int jj = 0; jj < n_proc; ++jj) {
       const int j = j_first + jj;
       const int n0 = j * kTileN;
-      const int kind = tile_kind(j);
+      const int kind = tile_kind(it, j);
 
       if (lane == 0 && quad == 0) FDB_STAMP(g, j, 0);
-      wait(bar(kBarS), uint32_t(jj) & 1u);
+      if (!rc_read && kind != kBand) {
+        // (in front of this tile's scores: until they are read nothing of the item after the next one is loaded, which shares the buffer)
+        wait(bar(kBarRc + (items & 1u)), (items >> 1) & 1u);
+        const uint32_t rc = smem + kSmemRc + 1024u * (items & 1u) + 4u * uint32_t(r);
+        rc_hi = ratio_c * lds_f32(rc);
+        rc_lo = ratio_c * lds_f32(rc + 512u);
+        rc_read = true;
+      }
+      wait(bar(kBarS), tiles & 1u);
       tc_fence_after();
       if (lane == 0 && quad == 0) FDB_STAMP(g, j, 1);
 
@@ -614,7 +757,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
 
       float row_const = 0.f;
       if (kind == kBand) {
-        wait(bar(kBarStage), band_idx & 1u);  // the c2p stage of this tile is complete
+        wait(bar(kBarStage), bands & 1u);  // the c2p stage of this tile is complete
         if (has_c2p) {
           // c2p[m][i] is position p = m + 127 - i of the window, stored in column ((p ^ flip) - m) & 255 of row m (see the
           // drain group): for this thread's keys i = 64g .. 64g+63 that is the aligned run of 64 columns ending at
@@ -635,6 +778,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         }
         arrive(bar(kBarGather));
         ++band_idx;
+        ++bands;
       } else if (kind == kSatHi) {
         row_const = rc_hi;
       } else if (kind == kSatLo) {
@@ -654,7 +798,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       for (int q = 0; q < 4; ++q) mx4[q] = fmaxf(mx4[q], s[60 + q]);
       float mx = max3(mx4[0], mx4[1], fmaxf(mx4[2], mx4[3]));
       // the two threads of a row agree on the row maximum
-      const uint32_t xch = smem + kSmemXchg + uint32_t(jj & 1) * 1024u;
+      const uint32_t xch = smem + kSmemXchg + (tiles & 1u) * 1024u;
       sts_f32(xch + uint32_t(g) * 512u + uint32_t(r) * 4u, mx);
       if (lane == 0 && quad == 0) FDB_STAMP(g, j, 3);
       bar_sync(1, kSoftmaxThreads);
@@ -668,7 +812,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         // The previous P.V has finished: O may be rescaled and the P columns overwritten.  Observed on every tile (it is
         // long done by now) so that this thread never falls two phases behind the barrier, which a parity wait could
         // not tell apart.
-        if (jj > 0) wait(bar(kBarO), uint32_t(jj - 1) & 1u);
+        if (jj > 0) wait(bar(kBarO), (tiles - 1u) & 1u);
         tc_fence_after();
         // bf16: O is rescaled only when the maximum moved by more than 2^8 (P <= 256 is harmless in bf16).
         // e4m3: P is stored as 2^8 * exp2(.), so it has to stay <= 1: rescale whenever the maximum moves.
@@ -737,6 +881,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       }
       tc_fence_before();
       arrive(bar(kBarP));
+      ++tiles;
       if (lane == 0 && quad == 0) FDB_STAMP(g, j, 7);
     }
 
@@ -744,7 +889,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     sts_f32(smem + kSmemLsum + uint32_t(g) * 512u + uint32_t(r) * 4u, l_run);
     bar_sync(1, kSoftmaxThreads);
     const float l_tot = l_run + lds_f32(smem + kSmemLsum + uint32_t(g ^ 1) * 512u + uint32_t(r) * 4u);
-    wait(bar(kBarO), uint32_t(n_proc - 1) & 1u);
+    wait(bar(kBarO), (tiles - 1u) & 1u);
     tc_fence_after();
     if (ok) {
       const bool valid = my_row < len;
@@ -771,6 +916,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
               valid ? (m_used + log2f(l_tot) - (F8 ? 8.f : 0.f)) * 0.6931471805599453f : 0.f;
       }
     }
+    tc_fence_before();
+    __syncwarp();
+    ++items;
+    } while (next_item(it));
   }
 
   // ---- teardown -------------------------------------------------------------------------------------------------------

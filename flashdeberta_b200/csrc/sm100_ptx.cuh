@@ -68,6 +68,7 @@ __device__ __forceinline__ void bar_sync(uint32_t id, uint32_t count) {
 
 // ---- fences -----------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void fence_barrier_init() { asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory"); }
+__device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -138,6 +139,25 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar) {
 // stream may start its prologue.  Both do nothing in a kernel launched without the attribute.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// ---- cluster launch control -----------------------------------------------------------------------------------------
+// Asks for a block of this grid that has not started yet: it will not start, its index comes back (16 bytes in shared memory, counted on
+// the mbarrier) and this CTA does its work.  None left: the answer says so, and no further request may be made.
+__device__ __forceinline__ void launch_take_over(uint32_t answer, uint32_t bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];"
+               ::"r"(answer), "r"(bar) : "memory");
+}
+__device__ __forceinline__ bool launch_taken_over(uint32_t answer, uint32_t& x, uint32_t& y) {
+  uint32_t got;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t.reg .b32 z, w;\n\t"
+      "ld.shared.b128 h, [%3];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid.v4.b32.b128 {%1, %2, z, w}, h;\n\t}"
+      : "=r"(got), "=r"(x), "=r"(y) : "r"(answer) : "memory");
+  return got != 0;
+}
 
 // ---- TMEM allocation (one warp, all lanes) -------------------------------------------------------------------------
 __device__ __forceinline__ void tmem_alloc(uint32_t smem_result, uint32_t cols) {

@@ -1031,3 +1031,40 @@ def test_bits_of_a_sequence_do_not_depend_on_what_lies_behind_it(L, tune, terms)
     for out, lse in outs[1:]:
         assert torch.equal(out, outs[0][0]) and torch.equal(lse, outs[0][1])
     ops.check_status()
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "e4m3"])
+@pytest.mark.parametrize("layout, batch, longest, heads", [("packed", 900, 130, 2), ("dense", 300, 300, 3), ("packed", 60, 1500, 4)])
+def test_many_items_per_sm(layout, batch, longest, heads, dtype):
+    """Far more query tiles than SMs, so that every CTA takes many over: items of one tile, empty sequences, padding tiles, items with
+    and without saturated tiles one behind the other.  Sequences computed alone, in a CTA of their own, have the same bits."""
+    ops = _ops()
+    g = torch.Generator().manual_seed(batch)
+    lens = torch.randint(0, longest + 1, (batch,), generator=g).tolist()
+    lens[:6] = [longest, 1, 0, 128, 129, 127]
+    make = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
+    attend = ops.disentangled_attention_fp8 if dtype == "e4m3" else ops.disentangled_attention
+    tables = [0.5 * make(heads, 512, 64) for _ in range(2)]
+    kw = dict(position_buckets=256, max_relative_positions=512)
+    rows = (sum(lens),) if layout == "packed" else (batch, longest)
+    q, k, v = (make(*rows, heads, 64) for _ in range(3))
+    first = torch.tensor([0] + lens).cumsum(0).tolist()
+    if layout == "packed":
+        out = attend(q, k, v, *tables, cu_seqlens=torch.tensor(first, dtype=torch.int32, device=DEV), max_seqlen=longest, **kw)
+        part = lambda t, b: t[first[b]:first[b + 1]]
+    else:
+        out = attend(q, k, v, *tables, seq_lens=torch.tensor(lens, dtype=torch.int32, device=DEV), max_seqlen=longest, **kw)
+        part = lambda t, b: t[b, :lens[b]]
+        for b in range(batch):
+            assert torch.count_nonzero(out[b, lens[b]:]) == 0
+    ops.check_status()
+    for b in [0, 1, 3, 4, 5, *range(6, batch, batch // 12), batch - 1]:
+        if lens[b] == 0:
+            continue
+        if layout == "packed":
+            cu = torch.tensor([0, lens[b]], dtype=torch.int32, device=DEV)
+            alone = attend(*(part(t, b).contiguous() for t in (q, k, v)), *tables, cu_seqlens=cu, max_seqlen=lens[b], **kw)
+        else:  # (as a padded row: the e4m3 scales are those of the row)
+            n = torch.tensor([lens[b]], dtype=torch.int32, device=DEV)
+            alone = attend(*(t[b:b + 1].contiguous() for t in (q, k, v)), *tables, seq_lens=n, max_seqlen=longest, **kw)[0, :lens[b]]
+        assert torch.equal(part(out, b), alone), (b, lens[b])
