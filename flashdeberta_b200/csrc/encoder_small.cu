@@ -3,7 +3,7 @@
 // At that size a layer's seven launches are all latency: 4 to 10 us each for a microsecond of work, one behind the other.  Here one
 // CTA per SM stays for the whole forward and the steps of a layer are separated by grid barriers:
 //   1  LayerNorm of the layer before -> shared memory; query, key and value projections
-//   2  attention, a warp per (row, head), on the CUDA cores
+//   2  attention, four warps per (row, head), on the CUDA cores
 //   3  output projection, + residual
 //   4  LayerNorm -> shared memory; first feed-forward product, GELU
 //   5  second feed-forward product, + residual
@@ -14,9 +14,11 @@
 // that go from memory to registers save the trip through shared memory and tensor memory, so the products are warp MMAs.  Both
 // operands are read 32 bytes per thread: K is permuted the same way in both, which a sum over K does not see.
 //
-// 12 layers of 768, 29 tokens: 607 us a call as 84 launches, 385 in one kernel.  Of a layer (55000 clocks): five barriers 14000, the two
-// LayerNorms 11500, the four products 4000 to 8300 each, attention 6800.  It ends where every CTA normalising all rows costs what the
-// launches cost: see small_encoder_covers.
+// 12 layers of 768, 29 tokens: 610 us a call as 84 launches, 320 in one kernel.  Of a layer (45 000 clocks): five barriers 13 700, the
+// two LayerNorms 8000, the four products 3800 to 7600 each, attention 4000.  It was 391 us (55 300) with a warp for a (row, head) in the
+// attention (6500 clocks), LayerNorms that asked at run time how long a row is (6000 each), integer divisions in the products' last
+// step and loads of the fifth step that came a half block at a time (8750).  Weights ahead of the barrier by a bulk prefetch or not at
+// all made no difference; scale and shift prefetched to the first-level cache cost 130 us.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -96,8 +98,9 @@ __device__ __forceinline__ Product make_product(const Ctx& c, const __nv_bfloat1
   p.tiles = max(0, min(per, all - p.tile0));
   return p;
 }
+__device__ __forceinline__ int group_of(const Product& p, int col) { return (col >= p.group_cols ? 1 : 0) + (col >= 2 * p.group_cols ? 1 : 0); }
 __device__ __forceinline__ const __nv_bfloat16* weight_row(const Product& p, int tile, int r) {
-  const int col = tile * 8, g = col / p.group_cols;
+  const int col = tile * 8, g = group_of(p, col);
   return (g == 0 ? p.w0 : (g == 1 ? p.w1 : p.w2)) + (int64_t)(col - g * p.group_cols + r) * p.k;
 }
 // the CTA's weights of a coming product to L2
@@ -110,15 +113,16 @@ __device__ __forceinline__ void prefetch(const Ctx& c, const Product& p) {
 }
 
 // Partial sums of the warps over their share of K, then `store(row, column, v0, v1)` for pairs of columns with the bias added.  The
-// rows come from shared memory (src == NULL) or from memory.
-template <int MT, int NT, typename Store>
-__device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, const __nv_bfloat16* src, int split, Store&& store) {
+// rows come from shared memory, or (kInMemory) from `src`.
+template <int MT, int NT, int kSplit, bool kInMemory, typename Store>
+__device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, const __nv_bfloat16* src, Store&& store) {
   const int g = c.lane >> 2, t = c.lane & 3;
-  const int kgs = kWarps / split, kg = c.warp % kgs, tile = (c.warp / kgs) * NT;  // split: the tiles are dealt to this many sets of warps
-  const int cols = p.tiles * 8, blocks = p.k / 64;
+  constexpr int kgs = kWarps / kSplit, cols = NT * kSplit * 8;  // kSplit: the tiles are dealt to this many sets of warps
+  const int kg = c.warp % kgs, tile = (c.warp / kgs) * NT;
+  const int blocks = p.k / 64;
   // the bias of the pair of columns that this thread finishes first, on its way while the product is made
   auto bias_of = [&](int cp) -> uint32_t {
-    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols;
+    const int col = p.tile0 * 8 + cp, grp = group_of(p, col);
     const __nv_bfloat16* bias = grp == 0 ? p.b0 : (grp == 1 ? p.b1 : p.b2);
     return bias != nullptr ? __ldg(reinterpret_cast<const uint32_t*>(bias + col - grp * p.group_cols)) : 0u;
   };
@@ -134,29 +138,37 @@ __device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, co
   const __nv_bfloat16* w[NT];
 #pragma unroll
   for (int n = 0; n < NT; ++n) w[n] = weight_row(p, p.tile0 + min(tile + n, p.tiles - 1), g) + t * 16;
-#pragma unroll(MT <= 2 ? 3 : 1)
-  for (int b = kg; b < blocks; b += kgs) {
+  // A batch of steps (half a block each) at a time: all its loads, then its MMAs.  With the rows in memory the batch is what the
+  // registers hold, for it is a trip to L2 each; in shared memory, a warp's one block of the weights.
+  constexpr int kBatch = kInMemory ? (MT == 1 ? 4 : (MT == 2 ? 3 : 1)) : 2;
+  const int steps = kg < blocks ? 2 * ((blocks - kg - 1) / kgs + 1) : 0;
+#pragma unroll 1
+  for (int s0 = 0; s0 < steps; s0 += kBatch) {
+    uint4 x[kBatch][MT][2], y[kBatch][NT];
 #pragma unroll
-    for (int u = 0; u < 2; ++u) {
-      uint4 x[MT][2], y[NT];
+    for (int j = 0; j < kBatch; ++j) {
+      const int at = (kg + ((s0 + j) >> 1) * kgs) * 64 + ((s0 + j) & 1) * 8;
+      const bool live = kBatch <= 2 || s0 + j < steps;  // (the number of steps is even)
 #pragma unroll
-      for (int n = 0; n < NT; ++n) y[n] = __ldg(reinterpret_cast<const uint4*>(w[n] + b * 64) + u);
+      for (int n = 0; n < NT; ++n) y[j][n] = live ? __ldg(reinterpret_cast<const uint4*>(w[n] + at)) : make_uint4(0, 0, 0, 0);
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-          const int row = m * 16 + h * 8 + g, at = b * 64 + t * 16 + u * 8;
-          if (src == nullptr) x[m][h] = *reinterpret_cast<const uint4*>(c.s_x + row * c.pitch + at * 2);
-          else x[m][h] = row < c.rows ? __ldcg(reinterpret_cast<const uint4*>(src + (int64_t)row * p.k + at)) : make_uint4(0, 0, 0, 0);
+          const int row = m * 16 + h * 8 + g;
+          if constexpr (kInMemory) x[j][m][h] = live && row < c.rows ? __ldcg(reinterpret_cast<const uint4*>(src + (int64_t)row * p.k + at + t * 16)) : make_uint4(0, 0, 0, 0);
+          else x[j][m][h] = *reinterpret_cast<const uint4*>(c.s_x + row * c.pitch + (at + t * 16) * 2);
         }
+    }
+#pragma unroll
+    for (int j = 0; j < kBatch; ++j)
 #pragma unroll
       for (int m = 0; m < MT; ++m)
 #pragma unroll
         for (int n = 0; n < NT; ++n) {
-          mma16816(acc[m][n], x[m][0].x, x[m][1].x, x[m][0].y, x[m][1].y, y[n].x, y[n].y);
-          mma16816(acc[m][n], x[m][0].z, x[m][1].z, x[m][0].w, x[m][1].w, y[n].z, y[n].w);
+          mma16816(acc[m][n], x[j][m][0].x, x[j][m][1].x, x[j][m][0].y, x[j][m][1].y, y[j][n].x, y[j][n].y);
+          mma16816(acc[m][n], x[j][m][0].z, x[j][m][1].z, x[j][m][0].w, x[j][m][1].w, y[j][n].z, y[j][n].w);
         }
-    }
   }
 #pragma unroll
   for (int m = 0; m < MT; ++m)
@@ -178,18 +190,18 @@ __device__ __forceinline__ void product_tiles(const Ctx& c, const Product& p, co
       s.y += v.y;
     }
     const uint32_t bias = i < kThreads ? first_bias : bias_of(cp);
-    const int col = p.tile0 * 8 + cp, grp = col / p.group_cols, in = col - grp * p.group_cols;
+    const int col = p.tile0 * 8 + cp, grp = group_of(p, col), in = col - grp * p.group_cols;
     store(row, grp, in, round_bf16(s.x + lo(bias)), round_bf16(s.y + hi(bias)));
   }
 }
 
-template <int MT, typename Store>
+template <int MT, bool kInMemory, typename Store>
 __device__ __forceinline__ void product(const Ctx& c, const Product& p, const __nv_bfloat16* src, Store&& store) {
   if (p.tiles == 0) return;  // (uniform over the CTA)
-  if (p.tiles == 1) product_tiles<MT, 1>(c, p, src, 1, store);
-  else if (p.tiles == 2) product_tiles<MT, 2>(c, p, src, 1, store);
-  else if (p.tiles == 3) product_tiles<MT, 3>(c, p, src, 1, store);
-  else product_tiles<MT, 2>(c, p, src, 2, store);  // (four: the partial sums of 16 warps would not fit)
+  if (p.tiles == 1) product_tiles<MT, 1, 1, kInMemory>(c, p, src, store);
+  else if (p.tiles == 2) product_tiles<MT, 2, 1, kInMemory>(c, p, src, store);
+  else if (p.tiles == 3) product_tiles<MT, 3, 1, kInMemory>(c, p, src, store);
+  else product_tiles<MT, 2, 2, kInMemory>(c, p, src, store);  // (four: the partial sums of 16 warps would not fit)
 }
 
 // a bf16 pair as two floats
@@ -203,28 +215,26 @@ __device__ __forceinline__ float across(uint64_t v) {
 
 // LayerNorm of the rows of `y` (the sums of add_layernorm.cu, two at a time), two rows of a warp together; gamma == NULL: the rows as
 // they are.  With all rows on every CTA this is bound by instructions, not by memory.
-template <typename Out>
-__device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, float eps,
+template <int kVec, typename Out>
+__device__ __forceinline__ void normalise_rows(const Ctx& c, const __nv_bfloat16* y, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, float eps,
                                           int first, int step, Out&& out) {
-  const int vec = c.a->hidden / 256;
   const float inv = 1.f / (float)c.a->hidden;
 #pragma unroll 1
   for (int row = first; row < c.rows; row += 2 * step) {
-    uint4 raw[2][4];
+    uint4 raw[2][kVec];
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        raw[r][i] = i < vec ? __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)min(row + r * step, c.rows - 1) * c.a->hidden) + i * 32 + c.lane)
-                            : make_uint4(0, 0, 0, 0);
+      for (int i = 0; i < kVec; ++i)
+        raw[r][i] = __ldcg(reinterpret_cast<const uint4*>(y + (int64_t)min(row + r * step, c.rows - 1) * c.a->hidden) + i * 32 + c.lane);
     if (gamma != nullptr) {
-      uint64_t d[2][16];
+      uint64_t d[2][4 * kVec];
       float mean[2], rstd[2];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         uint64_t sum = both(0.f);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
+        for (int i = 0; i < kVec; ++i) {
           const uint32_t w[4] = {raw[r][i].x, raw[r][i].y, raw[r][i].z, raw[r][i].w};
 #pragma unroll
           for (int k = 0; k < 4; ++k) sum = ptx::add_f32x2(sum, d[r][i * 4 + k] = wide(w[k]));
@@ -240,8 +250,7 @@ __device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, 
         const uint64_t m = both(-mean[r] * inv);
         uint64_t sq = both(0.f);
 #pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          if (i / 4 >= vec) continue;
+        for (int i = 0; i < 4 * kVec; ++i) {
           d[r][i] = ptx::add_f32x2(d[r][i], m);
           sq = ptx::fma_f32x2(d[r][i], d[r][i], sq);
         }
@@ -254,8 +263,7 @@ __device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, 
 #pragma unroll
       for (int r = 0; r < 2; ++r) rstd[r] = rsqrtf(rstd[r] * inv + eps);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        if (i >= vec) continue;
+      for (int i = 0; i < kVec; ++i) {
         const uint4 gv = __ldg(reinterpret_cast<const uint4*>(gamma) + i * 32 + c.lane), bv = __ldg(reinterpret_cast<const uint4*>(beta) + i * 32 + c.lane);
         const uint32_t gw[4] = {gv.x, gv.y, gv.z, gv.w}, bw[4] = {bv.x, bv.y, bv.z, bv.w};
         uint32_t o[2][4];
@@ -274,80 +282,100 @@ __device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, 
 #pragma unroll
     for (int r = 0; r < 2; ++r)
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (i < vec && row + r * step < c.rows) out(row + r * step, i * 32 + c.lane, raw[r][i]);
+      for (int i = 0; i < kVec; ++i)
+        if (row + r * step < c.rows) out(row + r * step, i * 32 + c.lane, raw[r][i]);
+  }
+}
+// (with the length of a row known at compile time: a branch per 16 bytes kept the rows' arithmetic apart, 6000 against 4000 clocks for 29 rows)
+template <typename Out>
+__device__ __forceinline__ void normalise(const Ctx& c, const __nv_bfloat16* y, const __nv_bfloat16* gamma, const __nv_bfloat16* beta, float eps,
+                                          int first, int step, Out&& out) {
+  switch (c.a->hidden / 256) {
+    case 1: normalise_rows<1>(c, y, gamma, beta, eps, first, step, out); break;
+    case 2: normalise_rows<2>(c, y, gamma, beta, eps, first, step, out); break;
+    case 3: normalise_rows<3>(c, y, gamma, beta, eps, first, step, out); break;
+    default: normalise_rows<4>(c, y, gamma, beta, eps, first, step, out); break;
   }
 }
 
-// softmax((q.k + c2p + p2c) * scale) v of one row and head by a warp: lanes are keys for the scores, pairs of features for the output
-__device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l, int row, int head, int start, int len) {
+// softmax((q.k + c2p + p2c) * scale) v of one row and head by four warps (a head of 29 rows leaves a CTA two or three of these to do, and
+// one warp alone is a chain of latencies: 6500 clocks against 4000).  Scores: warp w has keys 8w .. 8w+7 (and 32 more), four lanes a
+// key, 16 features each.  Output: warp w has features 16w .. 16w+15, a lane a pair of them over every fourth key.  `scores`: 64
+// floats that the last row but one of these warps used.
+__device__ __forceinline__ void attention_row(const Ctx& c, const SmallLayer& l, int row, int head, int start, int len, float* scores) {
   const SmallEncoderArgs& a = *c.a;
+  const int w = c.warp & 3;
   const int64_t hd = (int64_t)head * 64;
-  uint32_t* out = reinterpret_cast<uint32_t*>(a.ctx + (int64_t)row * a.hidden + hd) + c.lane;
+  uint32_t* out = reinterpret_cast<uint32_t*>(a.ctx + (int64_t)row * a.hidden + hd) + w * 8 + (c.lane & 7);
   if (len == 0) {  // a row of no sequence
-    *out = 0u;
+    if (c.lane < 8) *out = 0u;
     return;
   }
   const int64_t plane = (int64_t)a.row_bound * a.hidden;
   const __nv_bfloat16 *q = a.qkv, *k = a.qkv + plane, *v = a.qkv + 2 * plane;
-  const uint4* qr = reinterpret_cast<const uint4*>(q + (int64_t)row * a.hidden + hd);
-  const int m = row - start;
-  float s[2];
+  const int sub = c.lane >> 3;
+  const uint32_t* vr = reinterpret_cast<const uint32_t*>(v + (int64_t)start * a.hidden + hd) + w * 8 + (c.lane & 7);
+  uint32_t vw[8];  // keys sub, sub + 4, .. of the first 32, on their way beside the scores
 #pragma unroll
-  for (int ch = 0; ch < 2; ++ch) {
-    s[ch] = -INFINITY;
-    if (ch * 32 >= len) continue;
-    const int n = min(ch * 32 + c.lane, len - 1);
-    const uint4* kr = reinterpret_cast<const uint4*>(k + (int64_t)(start + n) * a.hidden + hd);
-    const int64_t at = ((int64_t)head * a.xrows + (m - n - a.d_first)) * 64;
-    const uint4* xk = reinterpret_cast<const uint4*>(l.exp_key + at);
-    const uint4* xq = reinterpret_cast<const uint4*>(l.exp_query + at);
+  for (int i = 0; i < 8; ++i) vw[i] = sub + 4 * i < len ? __ldcg(vr + (int64_t)(sub + 4 * i) * (a.hidden / 2)) : 0u;
+  const int m = row - start, part = (c.lane & 3) * 2;  // 16-byte pieces of the row
+  const uint4* qr = reinterpret_cast<const uint4*>(q + (int64_t)row * a.hidden + hd) + part;
+#pragma unroll 1
+  for (int n = w * 8 + (c.lane >> 2); n - (c.lane >> 2) < 64 && (n & 32 ? len > 32 : true); n += 32) {
+    const int key = min(n, len - 1);
+    const uint4* kr = reinterpret_cast<const uint4*>(k + (int64_t)(start + key) * a.hidden + hd) + part;
+    const int64_t at = ((int64_t)head * a.xrows + (m - key - a.d_first)) * 64;
+    const uint4* xk = reinterpret_cast<const uint4*>(l.exp_key + at) + part;
+    const uint4* xq = reinterpret_cast<const uint4*>(l.exp_query + at) + part;
+    uint4 qv[2], kv[2], kp[2], qp[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      qv[i] = __ldcg(qr + i);
+      kv[i] = __ldcg(kr + i);
+      kp[i] = l.exp_key != nullptr ? __ldg(xk + i) : make_uint4(0, 0, 0, 0);
+      qp[i] = l.exp_query != nullptr ? __ldg(xq + i) : make_uint4(0, 0, 0, 0);
+    }
     uint64_t sum_q = both(0.f), sum_k = both(0.f);  // q . (k + pos_key), k . pos_query
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      uint4 qv[4], kv[4], kp[4], qp[4];
+    for (int i = 0; i < 2; ++i) {
+      const uint32_t qw[4] = {qv[i].x, qv[i].y, qv[i].z, qv[i].w}, kw[4] = {kv[i].x, kv[i].y, kv[i].z, kv[i].w};
+      const uint32_t pw[4] = {kp[i].x, kp[i].y, kp[i].z, kp[i].w}, rw[4] = {qp[i].x, qp[i].y, qp[i].z, qp[i].w};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        qv[i] = __ldcg(qr + half * 4 + i);
-        kv[i] = __ldcg(kr + half * 4 + i);
-        kp[i] = l.exp_key != nullptr ? __ldg(xk + half * 4 + i) : make_uint4(0, 0, 0, 0);
-        qp[i] = l.exp_query != nullptr ? __ldg(xq + half * 4 + i) : make_uint4(0, 0, 0, 0);
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t qw[4] = {qv[i].x, qv[i].y, qv[i].z, qv[i].w}, kw[4] = {kv[i].x, kv[i].y, kv[i].z, kv[i].w};
-        const uint32_t pw[4] = {kp[i].x, kp[i].y, kp[i].z, kp[i].w}, rw[4] = {qp[i].x, qp[i].y, qp[i].z, qp[i].w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          const uint64_t kk = wide(kw[e]);
-          sum_q = ptx::fma_f32x2(wide(qw[e]), ptx::add_f32x2(kk, wide(pw[e])), sum_q);
-          sum_k = ptx::fma_f32x2(kk, wide(rw[e]), sum_k);
-        }
+      for (int e = 0; e < 4; ++e) {
+        const uint64_t kk = wide(kw[e]);
+        sum_q = ptx::fma_f32x2(wide(qw[e]), ptx::add_f32x2(kk, wide(pw[e])), sum_q);
+        sum_k = ptx::fma_f32x2(kk, wide(rw[e]), sum_k);
       }
     }
-    if (ch * 32 + c.lane < len) s[ch] = across(ptx::add_f32x2(sum_q, sum_k)) * (a.sm_scale * 1.4426950408889634f);
+    float s = across(ptx::add_f32x2(sum_q, sum_k));
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    s += __shfl_xor_sync(0xffffffffu, s, 2);
+    if ((c.lane & 3) == 0) scores[n] = n < len ? s * (a.sm_scale * 1.4426950408889634f) : -INFINITY;
   }
-  float top = fmaxf(s[0], s[1]);
+  ptx::bar_sync(1u + uint32_t(c.warp >> 2), 128);
+  const float s0 = scores[c.lane], s1 = len > 32 ? scores[32 + c.lane] : -INFINITY;
+  float top = fmaxf(s0, s1);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
-  const float p0 = ptx::ex2(s[0] - top), p1 = ptx::ex2(s[1] - top);
+  const float p0 = ptx::ex2(s0 - top), p1 = ptx::ex2(s1 - top);
   const float inv = 1.f / warp_sum(p0 + p1);
   uint64_t o = both(0.f);
-  const uint32_t* vr = reinterpret_cast<const uint32_t*>(v + (int64_t)start * a.hidden + hd) + c.lane;
-  for (int n0 = 0; n0 < len; n0 += 16) {
-    uint32_t w[16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) w[i] = n0 + i < len ? __ldcg(vr + (int64_t)(n0 + i) * (a.hidden / 2)) : 0u;
+  for (int i = 0; i < 8; ++i) o = ptx::fma_f32x2(both(__shfl_sync(0xffffffffu, p0, sub + 4 * i)), wide(vw[i]), o);  // (probability zero behind the sequence)
+  if (len > 32) {
 #pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const int n = n0 + i;  // keys behind the sequence have probability zero
-      const float pn = __shfl_sync(0xffffffffu, n < 32 ? p0 : p1, n & 31);
-      o = ptx::fma_f32x2(both(pn), wide(w[i]), o);
-    }
+    for (int i = 0; i < 8; ++i) vw[i] = 32 + sub + 4 * i < len ? __ldcg(vr + (int64_t)(32 + sub + 4 * i) * (a.hidden / 2)) : 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) o = ptx::fma_f32x2(both(__shfl_sync(0xffffffffu, p1, sub + 4 * i)), wide(vw[i]), o);
   }
   float o0, o1;
   ptx::unpack_f32x2(o, o0, o1);
-  *out = ptx::pack_bf16x2(o0 * inv, o1 * inv);
+#pragma unroll
+  for (int d = 8; d < 32; d <<= 1) {
+    o0 += __shfl_xor_sync(0xffffffffu, o0, d);
+    o1 += __shfl_xor_sync(0xffffffffu, o1, d);
+  }
+  if (c.lane < 8) *out = ptx::pack_bf16x2(o0 * inv, o1 * inv);
 }
 
 template <int MT>
@@ -404,26 +432,27 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid
     if (i == 0) normalise(c, args.x, nullptr, nullptr, 0.f, c.warp, kWarps, keep);
     else normalise(c, args.y, args.layer[i - 1].ln2_gamma, args.layer[i - 1].ln2_beta, args.layer[i - 1].ln2_eps, c.warp, kWarps, keep);
     __syncthreads();
-    product<MT>(c, qkv, nullptr, [&](int row, int grp, int col, float v0, float v1) {
+    product<MT, false>(c, qkv, nullptr, [&](int row, int grp, int col, float v0, float v1) {
       *reinterpret_cast<uint32_t*>(args.qkv + ((int64_t)grp * args.row_bound + row) * hidden + col) = ptx::pack_bf16x2(v0, v1);
     });
     prefetch(c, proj);
     if (!sync_grid()) return;
     // 2
-    for (int item = blockIdx.x + gridDim.x * c.warp; item < c.rows * heads; item += gridDim.x * kWarps) {
+    float* scores = c.s_red + (c.warp >> 2) * 128;  // (the products' partial sums have been read)
+    for (int item = blockIdx.x + gridDim.x * (c.warp >> 2), turn = 0; item < c.rows * heads; item += gridDim.x * (kWarps / 4), turn ^= 1) {
       const int row = item / heads;
-      attention_row(c, l, row, item - row * heads, s_start[row], s_len[row]);
+      attention_row(c, l, row, item - row * heads, s_start[row], s_len[row], scores + turn * 64);
     }
     prefetch(c, up);
     if (!sync_grid()) return;
     // 3
-    product<MT>(c, proj, args.ctx, add_to(args.y));
+    product<MT, true>(c, proj, args.ctx, add_to(args.y));
     prefetch(c, down);
     if (!sync_grid()) return;
     // 4
     normalise(c, args.y, l.ln1_gamma, l.ln1_beta, l.ln1_eps, c.warp, kWarps, keep);
     __syncthreads();
-    product<MT>(c, up, nullptr, [&](int row, int, int col, float v0, float v1) {
+    product<MT, false>(c, up, nullptr, [&](int row, int, int col, float v0, float v1) {
       float g0, g1;
       ptx::unpack_f32x2(gelu_erf2(ptx::pack_f32x2(v0, v1)), g0, g1);
       *reinterpret_cast<uint32_t*>(args.mid + (int64_t)row * args.ffn + col) = ptx::pack_bf16x2(g0, g1);
@@ -434,7 +463,7 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid
     }
     if (!sync_grid()) return;
     // 5
-    product<MT>(c, down, args.mid, add_to(args.y));
+    product<MT, true>(c, down, args.mid, add_to(args.y));
     if (!sync_grid()) return;
   }
   const SmallLayer& l = args.layer[args.n_layers - 1];
@@ -454,8 +483,9 @@ size_t smem_bytes(int mt, int hidden, int ffn, int sms) {
 bool small_encoder_covers(int64_t row_bound, int hidden, int ffn, int n_layers) {
   const int sms = sm_count();
   if (sms <= 0 || row_bound > kSmallRows || hidden > 1024 || n_layers > kSmallLayers) return false;
-  // Where it is the faster form.  16 / 32 / 48 / 64 rows, us against the separate launches: 12 layers of 768 351 / 391 / 534 / 567
-  // against 607; 24 layers of 1024 755 / 872 / 1320 / 1480 against 1375.
+  // Where it is the faster form.  16 / 32 / 48 / 64 rows, us against the separate launches: 12 layers of 768 298 / 326 / 443 / 471
+  // against 610; 24 layers of 1024 649 / 751 / 1148 against 1390.  (64 rows of 1024, 1196 against 1380, would be faster here too by
+  // now; 1480 when the line was drawn, and it is where the tests expect it.)
   if (row_bound * hidden > 48 * 1024) return false;
   const int most = std::max(3 * hidden, ffn);
   return (most / 8 + sms - 1) / sms <= kMaxTiles && smem_bytes(row_bound <= 16 ? 1 : (row_bound <= 32 ? 2 : 4), hidden, ffn, sms) <= 227 * 1024 - 1024;

@@ -575,6 +575,12 @@ def test_encoder_of_a_few_tokens_matches_the_module_walk(hidden, ffn, lens):
     ops.check_status()
 
 
+@pytest.mark.parametrize("lens", [[29], [16, 1, 31], [64]])
+def test_encoder_of_a_few_tokens_of_512(lens):
+    """The row length that the cases above leave out: the one-kernel form has a LayerNorm for each."""
+    test_encoder_of_a_few_tokens_matches_the_module_walk(512, 2048, lens)
+
+
 def test_encoder_call_notices_changes_of_the_model():
     """A weight replaced, a module swapped, a hook, training mode: each is seen on the next call."""
     from flashdeberta_b200 import FlashDebertaV2Model
