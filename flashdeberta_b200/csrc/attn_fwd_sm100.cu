@@ -166,10 +166,11 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
   auto bar = [&](uint32_t i) -> uint32_t { return smem + kSmemBars + 8u * i; };
   const uint32_t tmem_slot = smem + kSmemBars + 8u * kNumBars;
   volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(smem_gen + kSmemBars + 8u * kNumBars + 8u);
+  volatile uint32_t* handed_out = abort_flag + 1;  // items handed from role to role, plus one; 0 until the last one was
 
   // ---- set-up ---------------------------------------------------------------------------------------------------------
   if (tid == 0) {
-    *abort_flag = 0u;
+    *abort_flag = *handed_out = 0u;
     for (uint32_t i = 0; i < kNumBars; ++i) {
       uint32_t count = 1u;
       if (i == kBarSFree || i == kBarP || i == kBarGather) count = kSoftmaxThreads / 32;  // one arrival per warp
@@ -211,11 +212,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
   // The TMA warp asks and hands the items on, worked out: what the other roles execute between two items is code that the
   // tiles' loops have pushed out of the instruction cache, so there is little of it.
   uint32_t taken = 0;
-  auto next_item = [&](Item& it) -> bool {
+  auto wait_item = [&]() { wait(bar(kBarItem + (taken & 1u)), (taken >> 1) & 1u); };
+  auto read_item = [&](Item& it) -> bool {
     const uint32_t slot = taken & 1u, at = smem + kSmemItem + 32u + 32u * slot;
-    wait(bar(kBarItem + slot), (taken >> 1) & 1u);
     ++taken;
-    if (!ok) return false;
     const uint4 what = lds_v4(at);
     const uint4 rest = lds_v4(at + 16u);
     arrive(bar(kBarItemFree + slot));
@@ -224,6 +224,25 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     const uint32_t flags = uniform(rest.w);
     it.resume = (flags & 2u) != 0u;
     return (flags & 1u) != 0u;
+  };
+  auto next_item = [&](Item& it) -> bool {
+    wait_item();
+    return ok && read_item(it);
+  };
+  // The softmax warps meet at named barriers, which have no limit of their own and count on every warp.  So they work on the same items,
+  // whichever of them gave up on a wait: such a warp goes on without waiting and without results and takes every item that was handed out.
+  // How many those are is known once the TMA warp has left its loop, which it does at the first wait that it gives up itself.  (A vote
+  // of the eight warps between two items does the same for 2 % of a call with items of one tile.)
+  auto next_item_of_all = [&](Item& it) -> bool {
+    wait_item();
+    if (!ok) {
+      uint32_t n = 0;
+#pragma unroll 1
+      for (uint32_t i = 0; i < (1u << 28) && n == 0u; ++i) n = uniform(*handed_out);
+      __threadfence_block();
+      if (taken + 1u >= n) return false;
+    }
+    return read_item(it);
   };
   // (sequence, first row of the tile in it, its first row, its length)
   Item it = make_item(args, __ldg(args.slot_info + blockIdx.x), blockIdx.y);
@@ -378,6 +397,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         }
         ++asked;
       } while (more);
+      __syncwarp();
+      __threadfence_block();
+      if (elect_one()) *handed_out = asked + 1u;
     } else if (warp == kSatWarp) {
       // ============================================= saturated c2p terms ================================================
       // Q[m].X_k[first row] and Q[m].X_k[last row] of the item's rows, for its saturated tiles.  (The buffer of the item before the last
@@ -919,7 +941,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
     tc_fence_before();
     __syncwarp();
     ++items;
-    } while (next_item(it));
+    } while (next_item_of_all(it));
   }
 
   // ---- teardown -------------------------------------------------------------------------------------------------------
