@@ -390,6 +390,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         const uint32_t slot = asked & 1u, at = smem + kSmemItem + 32u + 32u * slot;
         it = make_item(args, __ldg(args.slot_info + (more ? x : 0u)), y);
         if (asked >= 2) wait(bar(kBarItemFree + slot), ((asked >> 1) - 1u) & 1u);
+        if (!ok) break;  // (somebody may still be reading it)
         if (elect_one()) {
           sts_v4(at, (uint32_t)it.seq, (uint32_t)it.m0, (uint32_t)it.row0, (uint32_t)it.len);
           sts_v4(at + 16u, (uint32_t)it.head, (uint32_t)it.j_first, (uint32_t)it.n_proc, (more ? 1u : 0u) | (it.resume ? 2u : 0u));

@@ -45,6 +45,12 @@ def _softmax_warps_ask():
         "*handed_out = asked + 1u;" in text
 
 
+def _tma_warp_stops():
+    post = re.search(r"wait\(bar\(kBarItemFree \+ slot\), \(\(asked >> 1\) - 1u\) & 1u\);(.*?)sts_v4\(at,", _source("attn_fwd_sm100.cu"), re.S)
+    assert post, "the hand-over of items is not the one modelled here"
+    return "if (!ok) break;" in post.group(1)
+
+
 def _takeover_faults(ask, stop):
     """Faults that some order of steps leads to.  ask: a softmax warp that gave up takes the items that were handed out; stop: the TMA
     warp writes no slot whose readers it gave up on."""
@@ -107,3 +113,9 @@ def test_softmax_warps_that_give_up_leave_none_behind():
     have to work on the same items."""
     assert _takeover_faults(False, True)  # (the model sees the fault)
     assert _takeover_faults(_softmax_warps_ask(), True) == set()
+
+
+def test_items_that_are_still_to_be_read_are_not_written_over():
+    """A TMA warp that gives up on the readers of a slot leaves what is in it: a warp that comes late reads the item that the others read."""
+    assert _takeover_faults(True, False)  # (the model sees the fault)
+    assert _takeover_faults(True, _tma_warp_stops()) == set()
