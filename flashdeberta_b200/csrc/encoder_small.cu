@@ -439,9 +439,11 @@ __global__ void __launch_bounds__(kThreads, 1) encoder_small_kernel(const __grid
     if (!sync_grid()) return;
     // 2
     float* scores = c.s_red + (c.warp >> 2) * 128;  // (the products' partial sums have been read)
-    for (int item = blockIdx.x + gridDim.x * (c.warp >> 2), turn = 0; item < c.rows * heads; item += gridDim.x * (kWarps / 4), turn ^= 1) {
-      const int row = item / heads;
-      attention_row(c, l, row, item - row * heads, s_start[row], s_len[row], scores + turn * 64);
+    int turn = 0;
+    for (int item = blockIdx.x + gridDim.x * (c.warp >> 2); item < c.rows * heads; item += gridDim.x * (kWarps / 4)) {
+      const int row = item / heads, len = s_len[row];
+      attention_row(c, l, row, item - row * heads, s_start[row], len, scores + turn * 64);
+      if (len > 0) turn ^= 1;  // (a row of no sequence passes no barrier: the scores of the row before may still be read)
     }
     prefetch(c, up);
     if (!sync_grid()) return;

@@ -3,6 +3,7 @@
 A wait inside these kernels may give up (two seconds of clock, or another warp gave up), so the models let every wait end either way
 at any time.  What the kernels do at the places that matter is read from their sources.
 """
+import itertools
 import os
 import re
 
@@ -119,3 +120,50 @@ def test_items_that_are_still_to_be_read_are_not_written_over():
     """A TMA warp that gives up on the readers of a slot leaves what is in it: a warp that comes late reads the item that the others read."""
     assert _takeover_faults(True, False)  # (the model sees the fault)
     assert _takeover_faults(True, _tma_warp_stops()) == set()
+
+
+# ---- encoder_small_kernel: the score buffers of attention_row ----------------------------------------------------------------------
+#
+# Four warps share a (row, head); two stand for them.  A row of a sequence: each writes scores, all meet, each reads the scores of all.
+# A row of no sequence does none of it.
+
+
+def _buffers_change_with_the_barrier():
+    text = _source("encoder_small.cu")
+    loop = re.search(r"for \(int item = [^{]*\{.*?attention_row\(.*?\n    \}", text, re.S)
+    assert loop and "scores + turn * 64" in loop.group(0), "the loop over rows and heads is not the one modelled here"
+    return "turn ^= 1) {" not in loop.group(0) and "if (len > 0) turn ^= 1;" in loop.group(0)
+
+
+def _scores_written_over(rows, with_barrier):
+    """Whether some order of steps lets a warp write a score buffer that the other one still has to read."""
+    turns, turn = [], 0
+    for full in rows:
+        turns.append(turn)
+        turn ^= full or not with_barrier
+    program = [(step, i) for i, full in enumerate(rows) if full for step in ("write", "meet", "read")]
+    found = []
+
+    def steps(state):
+        after = []
+        for w in (0, 1):
+            me, other = state[w], state[1 - w]
+            if me == len(program):
+                continue
+            step, row = program[me]
+            if step == "meet" and other < me:
+                continue
+            if step == "write" and any(what == "read" and turns[row] == turns[r] and r < row for what, r in program[other:]):
+                found.append(rows)
+            after.append((me + 1, other) if w == 0 else (other, me + 1))
+        return after
+
+    _walk((0, 0), steps)
+    return bool(found)
+
+
+def test_scores_of_a_row_are_read_before_they_are_written_over():
+    """Whichever rows belong to no sequence (fewer SMs than this kernel usually runs on leave a group of warps more than two of them)."""
+    rows = list(itertools.product((False, True), repeat=5))
+    assert any(_scores_written_over(r, False) for r in rows)  # (the model sees the fault)
+    assert not any(_scores_written_over(r, _buffers_change_with_the_barrier()) for r in rows)
