@@ -51,7 +51,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if not force and not is_stale():
         return LIB_PATH
     nvcc = find_nvcc()
-    extra = os.environ.get("FDB_NVCC_FLAGS", "").split()  # e.g. -DFDB_TRACE for the per-role clock stamps
+    extra = os.environ.get("FDB_NVCC_FLAGS", "").split()  # e.g. -DFDB_TRACE for the clock stamps of a work item
     objdir = os.path.join(PKG_DIR, "build")
     os.makedirs(objdir, exist_ok=True)
     objs = []

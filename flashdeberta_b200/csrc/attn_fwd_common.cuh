@@ -41,22 +41,23 @@ struct alignas(64) FwdArgs {
   int split_len;   // two-launch calls: sequences shorter than this stay whole in attn_fwd_kernel
   int slots;       // query-tile slots of the launch (work items = slots * heads)
 #ifdef FDB_TRACE
-  long long* trace;  // [role 0..3][tile 0..63][event 0..7] clock64 stamps of CTA (0, 0)
+  long long* trace;    // [role 0..3][tile 0..63][event 0..7] clock64 stamps of one work item of CTA (0, 0)
+  uint32_t trace_item; // which of its items: 0 its own block, 1 the first one it takes over, ...
 #endif
 };
 
 #ifdef FDB_TRACE
-// Development builds only (-DFDB_TRACE): clock stamps of one CTA, read back through a buffer whose address comes from the
-// environment.  Compiled out otherwise.
-inline long long* trace_buffer_from_env() {
-  const char* tp = std::getenv("FDB_TRACE_PTR");
-  return tp ? reinterpret_cast<long long*>(std::strtoull(tp, nullptr, 0)) : nullptr;
+// Development builds only (-DFDB_TRACE): clock stamps of one work item of one CTA, read back through a buffer whose address comes from
+// the environment, as does the item's number.  Compiled out otherwise.
+inline unsigned long long trace_from_env(const char* name) {
+  const char* v = std::getenv(name);
+  return v ? std::strtoull(v, nullptr, 0) : 0ull;
 }
-#define FDB_STAMP(role, tile, ev) \
-  do { if (blockIdx.x == 0 && blockIdx.y == 0 && args.trace != nullptr && (tile) < 64) \
+#define FDB_STAMP(item, role, tile, ev) \
+  do { if (blockIdx.x == 0 && blockIdx.y == 0 && args.trace != nullptr && (item) == args.trace_item && (tile) < 64) \
          args.trace[((role) * 64 + (tile)) * 8 + (ev)] = clock64(); } while (0)
 #else
-#define FDB_STAMP(role, tile, ev) do {} while (0)
+#define FDB_STAMP(item, role, tile, ev) do {} while (0)
 #endif
 
 enum TileKind : int { kPlain = 0, kSatHi = 1, kSatLo = 2, kBand = 3 };

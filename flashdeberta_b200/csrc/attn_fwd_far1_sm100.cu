@@ -239,7 +239,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
 
       wait(bar(kBarS), u & 1u);
       tc_fence_after();
-      if (lane == 0 && quad == 0) FDB_STAMP(0, i, 0);
+      if (lane == 0 && quad == 0) FDB_STAMP(0u, 0, i, 0);
       if (n0 + kTileN > len) {
         // ragged last tile of the sequence: overwrite the scores of keys past its end in tensor memory, 32 columns at a
         // time, so the code below is the same for every tile (a select on the 128 register-resident scores under a
@@ -280,7 +280,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
         for (int q = 0; q < 4; ++q) mx[q] = max3(mx[q], __uint_as_float(a1[c + q]), __uint_as_float(a1[c + 4 + q]));
 #pragma unroll
       for (int q = 0; q < 4; ++q) mx[q] = fmaxf(mx[q], __uint_as_float(a1[28 + q]));
-      if (lane == 0 && quad == 0) FDB_STAMP(0, i, 1);
+      if (lane == 0 && quad == 0) FDB_STAMP(0u, 0, i, 1);
 #pragma unroll
       for (int c = 0; c < 32; c += 8)
 #pragma unroll
@@ -292,7 +292,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
 
       const float row_const = kind == kSatHi ? rc_hi : (kind == kSatLo ? rc_lo : 0.f);
       const float t_max = (max3(mx[0], mx[1], fmaxf(mx[2], mx[3])) + row_const) * args.scale_log2;
-      if (lane == 0 && quad == 0) FDB_STAMP(0, i, 2);
+      if (lane == 0 && quad == 0) FDB_STAMP(0u, 0, i, 2);
       if (u == 0) {
         m_used = fmaxf(m_used, t_max);
       } else {
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
           }
         }
       }
-      if (lane == 0 && quad == 0) FDB_STAMP(0, i, 3);
+      if (lane == 0 && quad == 0) FDB_STAMP(0u, 0, i, 3);
       // p = 2^(s * scale + off), two keys per instruction where the hardware has a two-wide form; the first 64 keys go to
       // tensor memory while the other 64 are computed
       const float off = row_const * args.scale_log2 - m_used;
@@ -349,11 +349,11 @@ __global__ void __launch_bounds__(kThreads, 2) attn_fwd_far1_kernel(const __grid
         unpack_f32x2(l2[1], s2, s3);
         l_run += (s0 + s1) + (s2 + s3);
       }
-      if (lane == 0 && quad == 0) FDB_STAMP(0, i, 4);
+      if (lane == 0 && quad == 0) FDB_STAMP(0u, 0, i, 4);
       tmem_wait_st();
       tc_fence_before();
       arrive(bar(kBarP));
-      if (lane == 0 && quad == 0) FDB_STAMP(0, i, 5);
+      if (lane == 0 && quad == 0) FDB_STAMP(0u, 0, i, 5);
     }
 
 

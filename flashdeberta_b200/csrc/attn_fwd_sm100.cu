@@ -345,10 +345,10 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       for (int jj = 0; jj < it.n_proc && ok; ++jj) {
         const int j = it.j_first + jj;
         const uint32_t s = tiles & 1u, use = tiles >> 1;  // how often this stage was used before
-        FDB_STAMP(3, j, 0);
+        FDB_STAMP(asked, 3, j, 0);
         if (use > 0) wait(bar(kBarKFree + s), (use - 1u) & 1u);
         if (!ok) break;
-        FDB_STAMP(3, j, 1);
+        FDB_STAMP(asked, 3, j, 1);
         if (elect_one()) {
           mbar_expect_tx(bar(kBarK + s), G::kTile);
           tma_load_3d(smem + kSmemK + s * 16384, &args.tm_k, bar(kBarK + s), 0, it.head, it.row0 + j * kTileN);
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         }
         if (use > 0) wait(bar(kBarVFree + s), (use - 1u) & 1u);
         if (!ok) break;
-        FDB_STAMP(3, j, 2);
+        FDB_STAMP(asked, 3, j, 2);
         if (elect_one()) {
           mbar_expect_tx(bar(kBarV + s), G::kTile);
           tma_load_3d(smem + kSmemV + s * 16384, &args.tm_v, bar(kBarV + s), 0, it.head, it.row0 + j * kTileN);
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           if (jj == it.n_proc - 1) mma_commit(bar(kBarQFree));
         }
         ++tiles;
-        FDB_STAMP(2, j, 0);
+        FDB_STAMP(taken, 2, j, 0);
       }
       } while (next_item(it));
     } else if (warp == kPvWarp) {
@@ -577,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         wait(bar(kBarV + s), (tiles >> 1) & 1u);
         wait(bar(kBarP), tiles & 1u);  // both groups have written P (and read the output of the item before)
         tc_fence_after();
-        FDB_STAMP(2, it.j_first + jj, 3);
+        FDB_STAMP(taken, 2, it.j_first + jj, 3);
         if (ok && elect_one()) {
 #pragma unroll
           for (int ks = 0; ks < G::kPvSteps; ++ks)  // one step = 2048 bytes of V in either build (16 x 128 B, 32 x 64 B)
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           mma_commit(bar(kBarVFree + s));
         }
         ++tiles;
-        FDB_STAMP(2, it.j_first + jj, 5);
+        FDB_STAMP(taken, 2, it.j_first + jj, 5);
       }
       } while (next_item(it));
     }
@@ -670,7 +670,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       const int n0 = j * kTileN;
       const int kind = tile_kind(it, j);
 
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 0);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 0);
       if (!rc_read && kind != kBand) {
         // (in front of this tile's scores: until they are read nothing of the item after the next one is loaded, which shares the buffer)
         wait(bar(kBarRc + (items & 1u)), (items >> 1) & 1u);
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       }
       wait(bar(kBarS), tiles & 1u);
       tc_fence_after();
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 1);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 1);
 
       // ---- this thread's 64 scores (+ p2c through the quadrant shuffle) into registers, then S and R are released ----
       float s[64];
@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       }
       tc_fence_before();
       arrive(bar(kBarSFree));
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 2);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 2);
 
       float row_const = 0.f;
       if (kind == kBand) {
@@ -823,9 +823,9 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
       // the two threads of a row agree on the row maximum
       const uint32_t xch = smem + kSmemXchg + (tiles & 1u) * 1024u;
       sts_f32(xch + uint32_t(g) * 512u + uint32_t(r) * 4u, mx);
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 3);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 3);
       bar_sync(1, kSoftmaxThreads);
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 4);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 4);
       mx = fmaxf(mx, lds_f32(xch + uint32_t(g ^ 1) * 512u + uint32_t(r) * 4u));
 
       const float t_max = (mx + row_const) * c_eff;
@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           }
         }
       }
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 5);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 5);
       const float off = row_const * c_eff - m_used + (F8 ? 8.f : 0.f);
       if constexpr (F8) {
         float l4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -866,7 +866,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
           l4[i & 3] += s[i];
         }
         l_run += (l4[0] + l4[1]) + (l4[2] + l4[3]);
-        if (lane == 0 && quad == 0) FDB_STAMP(g, j, 6);
+        if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 6);
         {  // 16 columns of e4m3 quadruples
           uint32_t p[16];
 #pragma unroll
@@ -899,13 +899,13 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
         unpack_f32x2(l2[0], s0, s1);
         unpack_f32x2(l2[1], s2, s3);
         l_run += (s0 + s1) + (s2 + s3);
-        if (lane == 0 && quad == 0) FDB_STAMP(g, j, 6);
+        if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 6);
         tmem_wait_st();
       }
       tc_fence_before();
       arrive(bar(kBarP));
       ++tiles;
-      if (lane == 0 && quad == 0) FDB_STAMP(g, j, 7);
+      if (lane == 0 && quad == 0) FDB_STAMP(taken, g, j, 7);
     }
 
     // ---- epilogue: combine the two row sums, O / l, write this group's 32 output columns ----
@@ -988,7 +988,8 @@ int launch_attn_fwd_sm100(const fdb_attn_params& p, const ExpandGeometry& g, con
   a.band_only = b.split ? 1 : 0;
   a.split_len = (p.tune & FDB_TUNE_TWO_LAUNCHES) ? 0 : kSplitSeqlen;  // forced two launches: every sequence is split
 #ifdef FDB_TRACE
-  a.trace = trace_buffer_from_env();
+  a.trace = reinterpret_cast<long long*>(trace_from_env("FDB_TRACE_PTR"));
+  a.trace_item = (uint32_t)trace_from_env("FDB_TRACE_ITEM");
 #endif
 
   const int64_t slots = tile_slots(p);
