@@ -1033,11 +1033,8 @@ def test_bits_of_a_sequence_do_not_depend_on_what_lies_behind_it(L, tune, terms)
     ops.check_status()
 
 
-@pytest.mark.parametrize("dtype", ["bf16", "e4m3"])
-@pytest.mark.parametrize("layout, batch, longest, heads", [("packed", 900, 130, 2), ("dense", 300, 300, 3), ("packed", 60, 1500, 4)])
-def test_many_items_per_sm(layout, batch, longest, heads, dtype):
-    """Far more query tiles than SMs, so that every CTA takes many over: items of one tile, empty sequences, padding tiles, items with
-    and without saturated tiles one behind the other.  Sequences computed alone, in a CTA of their own, have the same bits."""
+def _many_items(layout, batch, longest, heads, dtype, c2p=True, p2c=True, tune=0):
+    """A batch of ragged lengths, some of its sequences alone in CTAs of their own (the same bits) and, in bf16, against the oracle."""
     ops = _ops()
     g = torch.Generator().manual_seed(batch)
     lens = torch.randint(0, longest + 1, (batch,), generator=g).tolist()
@@ -1045,7 +1042,10 @@ def test_many_items_per_sm(layout, batch, longest, heads, dtype):
     make = lambda *s: torch.randn(*s, generator=g).bfloat16().to(DEV)
     attend = ops.disentangled_attention_fp8 if dtype == "e4m3" else ops.disentangled_attention
     tables = [0.5 * make(heads, 512, 64) for _ in range(2)]
+    tables = [tables[0] if c2p else None, tables[1] if p2c else None]
     kw = dict(position_buckets=256, max_relative_positions=512)
+    if tune:
+        kw["tune"] = tune
     rows = (sum(lens),) if layout == "packed" else (batch, longest)
     q, k, v = (make(*rows, heads, 64) for _ in range(3))
     first = torch.tensor([0] + lens).cumsum(0).tolist()
@@ -1068,3 +1068,25 @@ def test_many_items_per_sm(layout, batch, longest, heads, dtype):
             n = torch.tensor([lens[b]], dtype=torch.int32, device=DEV)
             alone = attend(*(t[b:b + 1].contiguous() for t in (q, k, v)), *tables, seq_lens=n, max_seqlen=longest, **kw)[0, :lens[b]]
         assert torch.equal(part(out, b), alone), (b, lens[b])
+    for b in (0, 1, 4) if dtype == "bf16" else ():
+        host = lambda t: None if t is None else t.float().cpu()
+        want = oracle.attention_core(*(host(part(t, b)) for t in (q, k, v)), *(host(t) for t in tables), [0], [lens[b]],
+                                     oracle.sm_scale_for(64, c2p, p2c), 256, 512)
+        _close(part(out, b), want, BF16_MAX, BF16_MEAN, ("oracle", b))
+
+
+@pytest.mark.parametrize("dtype", ["bf16", "e4m3"])
+@pytest.mark.parametrize("layout, batch, longest, heads", [("packed", 900, 130, 2), ("dense", 300, 300, 3), ("packed", 60, 1500, 4)])
+def test_many_items_per_sm(layout, batch, longest, heads, dtype):
+    """Far more query tiles than SMs, so that every CTA takes many over: items of one tile, empty sequences, padding tiles, items with
+    and without saturated tiles one behind the other.  Sequences computed alone, in a CTA of their own, have the same bits."""
+    _many_items(layout, batch, longest, heads, dtype)
+
+
+@pytest.mark.parametrize("c2p, p2c", [(True, False), (False, True), (False, False), (True, True)])
+@pytest.mark.parametrize("layout, batch, longest, heads", [("packed", 900, 130, 2), ("dense", 300, 300, 3), ("packed", 60, 1500, 4)])
+@pytest.mark.parametrize("dtype, tune", [("bf16", 1), ("bf16", 2), ("e4m3", 0)])
+def test_many_items_per_sm_of_every_form(layout, batch, longest, heads, c2p, p2c, dtype, tune):
+    """The same with one position term or none, where other roles have nothing to hand over, and in two launches, where items that go on
+    from what the first launch left stand behind items that start anew."""
+    _many_items(layout, batch, longest, heads, dtype, c2p, p2c, tune)
