@@ -41,7 +41,7 @@
 // products of the next tile (20 narrow p2c MMAs 900, drain 1250).  Neither side hides the other wholly: of this kernel with one part
 // left out, the exponentials were worth 10 % of a call, selects and shuffles 7 %, c2p 3 %, the drain's stores 2 to 3 %, the p2c MMAs
 // and the windows' loads nothing.  Hence shuffle sources in registers, c2p added by the mixed-precision add (no unpacking), stores of
-// the drain at fixed distances from two bases, a stage pitch without bank conflicts, and waits that are over by then in front
+// the drain at fixed distances from two bases, a stage pitch with fewer bank conflicts, and waits that are over by then in front
 // of the ones that are not: 364 -> 353 us a call at this shape, 168 -> 164 at 32 x 512, packed 48 x <= 4099 x 16 heads 1431 -> 1393.
 //
 // Every mbarrier wait is bounded and gives up early once another role has raised the abort flag; the CTA then sets
@@ -65,7 +65,7 @@ using namespace fwd;
 
 constexpr int kSoftmaxThreads = 256;
 constexpr int kDrainThreads = 128;
-constexpr int kThreads = 512;            // four warpgroups: softmax 0, softmax 1, producers (warps 10, 11 idle), drain
+constexpr int kThreads = 512;            // four warpgroups: softmax 0, softmax 1, warps 8-11 (issue and saturated terms), drain
 constexpr int kMmaWarp = 8, kTmaWarp = 9, kPvWarp = 10, kSatWarp = 11, kDrainWarp0 = 12;
 // 128 registers per thread at launch; after setmaxnreg: 48 * 128 + 64 * 128 + 200 * 256 = 65536
 constexpr int kProducerRegs = 48, kDrainRegs = 64, kSoftmaxRegs = 200;
@@ -81,11 +81,11 @@ constexpr uint32_t kSmemK = 16384;                  // 2 stages
 constexpr uint32_t kSmemV = 49152;                  // 2 stages
 constexpr uint32_t kSmemWinK = 81920;               // 256 x 128 B window of expanded pos_key
 constexpr uint32_t kSmemWinQ = 114688;              // 256 x 128 B window of expanded pos_query
-// c2p stage: bf16 [128 query rows][256 window positions], rows padded by 16 B.  Row m is rotated by m: position p of the
+// c2p stage: bf16 [128 query rows][256 window positions], rows padded by 48 B.  Row m is rotated by m: position p of the
 // window sits in column (p - m) & 255, so the 64 values a softmax thread needs are one aligned 128-byte run whose place does
 // not depend on m.
-// A pitch of 140 words: neither the drain group's 4-byte stores (a word less per two rows) nor the 16-byte loads of eight rows
-// meet in a bank.
+// A pitch of 140 words: 16-byte loads of eight rows meet in no bank.  The drain group's 4-byte stores (row r of a warp in bank
+// 12 r - ceil(r / 2)) do in three pairs of the 32 rows, a second wavefront each; at 132 words it was eleven pairs.
 constexpr uint32_t kStageCPitch = 560;
 constexpr uint32_t kSmemStageC = 147456;
 constexpr uint32_t kSmemSat = kSmemStageC + 71680;  // 2 x (8 x 128 B) saturated pos_query rows (hi, lo)
@@ -207,7 +207,7 @@ __global__ void __launch_bounds__(kThreads, 1) attn_fwd_kernel(const __grid_cons
   // across the border between two items, so the set-up, the first loads, the first c2p blocks and their drain of an item lie
   // under the last tile and the output of the item before.  As blocks of their own, one behind the other because an SM's tensor memory
   // and shared memory hold one, those took 11 700 clocks an item beside 4500 per band tile; what is left between two items is 3000.
-  // 353 -> 336 us a call at 8 x 2048 x 12 heads, 164 -> 132 at 32 x 512, padded 24 x <= 779 124 -> 112, packed 48 x <= 4099 x 16
+  // 353 -> 336 us a call at 8 x 2048 x 12 heads, 164 -> 132 at 32 x 512, padded 24 x <= 779 124 -> 110, packed 48 x <= 4099 x 16
   // 1393 -> 1310.  Every count below that a barrier's phase depends on runs on from item to item.
   // The TMA warp asks and hands the items on, worked out: what the other roles execute between two items is code that the
   // tiles' loops have pushed out of the instruction cache, so there is little of it.

@@ -486,8 +486,8 @@ bool small_encoder_covers(int64_t row_bound, int hidden, int ffn, int n_layers) 
   const int sms = sm_count();
   if (sms <= 0 || row_bound > kSmallRows || hidden > 1024 || n_layers > kSmallLayers) return false;
   // Where it is the faster form.  16 / 32 / 48 / 64 rows, us against the separate launches: 12 layers of 768 298 / 326 / 443 / 471
-  // against 610; 24 layers of 1024 649 / 751 / 1148 against 1390.  (64 rows of 1024, 1196 against 1380, would be faster here too by
-  // now; 1480 when the line was drawn, and it is where the tests expect it.)
+  // against 610; 24 layers of 1024 649 / 751 / 1148 against 1390.  The line between 48 and 64 rows of 1024 was drawn when 64 took 1480
+  // here; they take 1196 against 1380 by now, so it lies too low for the row counts in between.
   if (row_bound * hidden > 48 * 1024) return false;
   const int most = std::max(3 * hidden, ffn);
   return (most / 8 + sms - 1) / sms <= kMaxTiles && smem_bytes(row_bound <= 16 ? 1 : (row_bound <= 32 ? 2 : 4), hidden, ffn, sms) <= 227 * 1024 - 1024;
