@@ -167,3 +167,10 @@ def test_scores_of_a_row_are_read_before_they_are_written_over():
     rows = list(itertools.product((False, True), repeat=5))
     assert any(_scores_written_over(r, False) for r in rows)  # (the model sees the fault)
     assert not any(_scores_written_over(r, _buffers_change_with_the_barrier()) for r in rows)
+
+
+def test_clock_stamps_are_of_one_item():
+    """A CTA works on many items and its roles run ahead of one another: every stamp of a development build says which item it is of."""
+    for name, items in (("attn_fwd_sm100.cu", {"taken", "asked"}), ("attn_fwd_far1_sm100.cu", {"0u"})):
+        assert set(re.findall(r"FDB_STAMP\((\w+),", _source(name))) == items
+    assert "(item) == args.trace_item" in _source("attn_fwd_common.cuh")
